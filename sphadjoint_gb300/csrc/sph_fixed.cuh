@@ -86,4 +86,45 @@ SPH_FIXED_HD bool fixed_of(float c, int S, Fixed128 &out)
     return true;
 }
 
+// The same integer as magnitude and shift: |round(c 2^S)| = M << k with
+// 0 <= k (c an FP32 contribution: M <= 2^24; FP64: M <= 2^53). False when it is
+// 0 or c is not finite. Integer instructions only, for both precisions.
+SPH_FIXED_HD bool fixed_parts(float c, int S, uint32_t &M, int &k)
+{
+    const uint32_t bits = fixed_float_bits(c);
+    const uint32_t ex = (bits >> 23) & 0xffu;
+    M = ex ? ((bits & 0x7fffffu) | 0x800000u) : (bits & 0x7fffffu);
+    k = (ex ? (int)ex - 150 : -149) + S;
+    if (ex == 0xffu || k <= -25) M = 0u;
+    if (k < 0 && M) {
+        const int sh = -k;
+        const uint32_t q = M >> sh, r = M & ((1u << sh) - 1u), half = 1u << (sh - 1);
+        M = q + ((r > half || (r == half && (q & 1u))) ? 1u : 0u);
+    }
+    k = k < 0 ? 0 : k;
+    return M != 0u;
+}
+
+SPH_FIXED_HD bool fixed_parts(double c, int S, uint64_t &M, int &k)
+{
+    uint64_t bits;
+#if defined(__CUDA_ARCH__)
+    bits = (uint64_t)__double_as_longlong(c);
+#else
+    std::memcpy(&bits, &c, sizeof bits);
+#endif
+    const uint32_t ex = (uint32_t)(bits >> 52) & 0x7ffu;
+    M = bits & ((1ull << 52) - 1ull);
+    if (ex) M |= 1ull << 52;
+    k = (ex ? (int)ex - 1075 : -1074) + S;
+    if (ex == 0x7ffu || k <= -54) M = 0ull;
+    if (k < 0 && M) {
+        const int sh = -k;
+        const uint64_t q = M >> sh, r = M & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
+        M = q + ((r > half || (r == half && (q & 1ull))) ? 1ull : 0ull);
+    }
+    k = k < 0 ? 0 : k;
+    return M != 0ull;
+}
+
 } // namespace sphgb

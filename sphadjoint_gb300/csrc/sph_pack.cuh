@@ -403,13 +403,14 @@ __global__ void __launch_bounds__(kPackBlock, sizeof(T) == 4 ? 12 : 1)
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
     const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
+    const bool live = i < d.n;
     const NLView<T> &v = d.v;
     const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[i];
-    T gx, gy;
-    pass2_sum<T>(v, I, i, xi, d.grho, gx, gy);
-    pass2_finish<T>(I, 0, i, xi, gx, gy, d.gXs, d.gX, d.galpha, d.emax, d.parity, d.thetaAcc);
+    const T2<T> xi = v.pos[live ? i : d.n - 1];
+    T gx = (T)0, gy = (T)0;
+    if (live) pass2_sum<T>(v, I, i, xi, d.grho, gx, gy);
+    pass2_finish_warp<T>(live, I, 0, i, xi, gx, gy, d.gXs, d.gX, d.galpha, d.emax, d.parity,
+                         d.thetaAcc);
 }
 
 template <typename T>
