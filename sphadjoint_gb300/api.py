@@ -811,13 +811,15 @@ DENSITY_FORMS = {"mask": 0, "tiles": 1, "pairs": 2}
 
 
 def set_density_form(form) -> None:
-    """Density kernel form of FP32 states with one thread per particle (no
-    counterpart in the reference), process-wide: "mask" walks each particle's
-    neighbour masks one candidate at a time, "tiles" uses the cell-tile form
-    (a warp stages its 32 particles' neighbouring cell rows in shared memory
-    and every lane scans all staged candidates; single states), "pairs" (the
-    default) walks the masks two candidates per iteration with packed f32x2
-    arithmetic."""
+    """Kernel form of FP32 states with one thread per particle (no
+    counterpart in the reference), process-wide. "pairs" (the default): the
+    pair passes read neighbour lists and windows staged in shared memory, and the
+    density sum takes two candidates per iteration with packed f32x2 arithmetic.
+    "mask": every pass walks each particle's neighbour masks, the density one
+    candidate at a time (the same bits as "pairs"). "tiles": mask walks with
+    the cell-tile density (a warp stages its 32 particles' neighbouring cell rows
+    in shared memory and every lane scans all staged candidates; single
+    states)."""
     L.check(L.load().sph_set_density_form(DENSITY_FORMS[form] if isinstance(form, str)
                                           else int(form)))
 

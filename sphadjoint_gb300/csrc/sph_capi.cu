@@ -88,6 +88,25 @@ cudaError_t rt_malloc(void **p, size_t bytes, cudaStream_t s)
     return cudaMallocAsync(p, bytes, s);
 }
 
+size_t rt_free_memory()
+{
+    size_t fr = 0, tot = 0;
+    int dev = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    cudaMemPool_t pool;
+    uint64_t held = 0, used = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        held > used)
+        fr += (size_t)(held - used);
+    (void)cudaGetLastError();
+    return fr;
+}
+
 void rt_free(void *p, cudaStream_t s)
 {
     if (cudaFreeAsync(p, s) != cudaSuccess) (void)cudaGetLastError();

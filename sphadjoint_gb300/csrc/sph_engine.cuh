@@ -25,6 +25,7 @@
 #include "sph_coop.cuh"
 #include "sph_iface.hpp"
 #include "sph_kernels.cuh"
+#include "sph_window.cuh"
 
 namespace sphgb {
 
@@ -146,6 +147,17 @@ template <typename T> int &tuned_block(int kid, bool multi)
             const int bs_ = ::sphgb::tuned_block<T>(kid, multi);                              \
             ::sphgb::rt_before_launch(kid);                                                   \
             ::sphgb::launch_k(kern, dim3((unsigned)(((n) + bs_ - 1) / bs_)), dim3(bs_), 0, __VA_ARGS__); \
+            ::sphgb::rt_after_launch(kid);                                                    \
+        }                                                                                     \
+    } while (0)
+
+// One block per tile (sph_window.cuh).
+#define SPH_LAUNCH_TILES(kid, kern, n, ...)                                                   \
+    do {                                                                                      \
+        if ((n) > 0) {                                                                        \
+            ::sphgb::rt_before_launch(kid);                                                   \
+            ::sphgb::launch_k(kern, dim3((unsigned)(((n) + ::sphgb::kTile - 1) / ::sphgb::kTile)), \
+                              dim3(::sphgb::kTile), 0, __VA_ARGS__);                          \
             ::sphgb::rt_after_launch(kid);                                                    \
         }                                                                                     \
     } while (0)
@@ -334,6 +346,11 @@ template <typename T> class Sys final : public StateI {
     DevBuf<int32_t> clStart, clOrder; // build! without a neighbour rebuild
     bool cellsOnlyLatest = false;
     bool keepAccel = false;
+    DevBuf<TileWin> wwin; // windows and neighbour lists of the FP32 tile passes
+    DevBuf<uint2> wcand, wsupp;
+    DevBuf<uint8_t> wcnt; // candidate counts, then in-support counts
+    bool listsTried = false; // the lists were asked for (and may have been refused)
+    bool listsFresh = false; // they belong to the masks the state holds
     StepGraphs graphs;   // simulate's steps, replayed in groups
     bool anyRho = false; // some instance's model reads densities in the adjoint
     bool anyAV = false;  // some instance uses the artificial viscosity
@@ -466,8 +483,9 @@ template <typename T> class Sys final : public StateI {
         scanTmp.alloc((size_t)((ncell + kScanTile - 1) / kScanTile + 1));
         flags.alloc((size_t)B);
         tmask.alloc(6 * n1);
-        rho.alloc(n1);
-        prho.alloc(n1);
+        // staged windows end on multiples of four slots: room for three more
+        rho.alloc(n1 + 4);
+        prho.alloc(n1 + 4);
         stage2.alloc(n1);
         stage1.alloc(n1);
         flags.zero();
@@ -507,6 +525,58 @@ template <typename T> class Sys final : public StateI {
         if (f == 16 || f == 32) return f;
         if (f == 1 || N_ > kCoopMaxN) return 0;
         return N_ <= coop32_max_n<T>() ? 32 : 16;
+    }
+
+    // FP32 states with one thread per particle run their pair passes on tiles
+    // (sph_window.cuh) when their lists are in memory. The lists (about 260
+    // bytes a particle) are scratch that the mask walks do without, so they
+    // are taken only from memory that is plainly free (an eighth of it at most)
+    // and not while a graph is recorded; a state without them gives the same
+    // results. Beyond 2^25 particles they would hold 8.6 GB a state.
+    static constexpr int64_t kListMaxN = int64_t(1) << 25;
+    bool want_tiles() const
+    {
+        return sizeof(T) == 4 && N_ > 0 && N_ <= kListMaxN && group_lanes() == 0 &&
+               rt_density_form() == 2;
+    }
+    bool tiles() const { return want_tiles() && wwin.p; }
+    void reserve_lists()
+    {
+        if (want_tiles()) alloc_lists();
+    }
+    void alloc_lists()
+    {
+        if (listsTried || rt_capturing() || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN) return;
+        listsTried = true;
+        const size_t nt = (size_t)((N_ + kTile - 1) / kTile), e = nt * kQuads * kTile;
+        const size_t bytes = nt * sizeof(TileWin) + 2 * e * sizeof(uint2) + 2 * nt * kTile;
+        if (rt_free_memory() / 8 < bytes) return;
+        try {
+            wcand.alloc(e);
+            wsupp.alloc(e);
+            wcnt.alloc(2 * nt * kTile);
+            wwin.alloc(nt);
+        } catch (const Error &) {
+            wcand.release();
+            wsupp.release();
+            wcnt.release();
+            wwin.release();
+        }
+    }
+    WinLists lists() const
+    {
+        const size_t nt = (size_t)((N_ + kTile - 1) / kTile);
+        return WinLists{wwin.p, wcand.p, wsupp.p, wcnt.p, wcnt.p + nt * kTile};
+    }
+    // the candidate lists of the masks the state holds, if they are not there
+    void fresh_lists(const NLView<T> &v)
+    {
+        if constexpr (sizeof(T) == 4) {
+            if (listsFresh) return;
+            auto kl = B > 1 ? &k_window_lists<true> : &k_window_lists<false>;
+            SPH_LAUNCH_TILES(K_NLBUILD, kl, N_, v, lists());
+            listsFresh = true;
+        }
     }
 
     void upload_inst()
@@ -679,6 +749,7 @@ template <typename T> class Sys final : public StateI {
     // _nl_build! on the freshly sorted particles
     void build_masks()
     {
+        listsFresh = false;
         if (const int G = group_lanes()) {
             auto kn = G == 32 ? &k_nl_build_coop<T, 32> : &k_nl_build_coop<T, 16>;
             SPH_LAUNCH_COOP(K_NLBUILD, G, kn, N_, N_, hinst[0], pos[cur].p, cellStart.p,
@@ -753,6 +824,14 @@ template <typename T> class Sys final : public StateI {
             auto ki = G == 32 ? &k_accel_integrate_coop<T, 32> : &k_accel_integrate_coop<T, 16>;
             SPH_LAUNCH_COOP(K_ACCEL_INTEGRATE, G, ki, N_, v, vel[cur].p, prho.p, rho.p, theta,
                             pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
+        } else if (tiles()) {
+            if constexpr (sizeof(T) == 4) {
+                density_tiles(v, rho.p, prho.p);
+                auto ki = B > 1 ? (anyAV ? &k_accel_win<true, true> : &k_accel_win<true, false>)
+                                : (anyAV ? &k_accel_win<false, true> : &k_accel_win<false, false>);
+                SPH_LAUNCH_TILES(K_ACCEL_INTEGRATE, ki, N_, v, lists(), vel[cur].p, prho.p, rho.p,
+                                 theta, pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
+            }
         } else {
             launch_density(v, rho.p, prho.p);
             v.tmask = tmask.p;
@@ -762,6 +841,16 @@ template <typename T> class Sys final : public StateI {
                              theta, pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
         }
         cur = nxt;
+    }
+
+    // density_kernel! + eos_kernel! on tiles, and this step's in-support lists
+    void density_tiles(const NLView<T> &v, T *rhoOut, T2<T> *prhoOut)
+    {
+        if constexpr (sizeof(T) == 4) {
+            fresh_lists(v);
+            auto kd = B > 1 ? &k_density_win<true> : &k_density_win<false>;
+            SPH_LAUNCH_TILES(K_DENSITY, kd, N_, v, lists(), rhoOut, prhoOut);
+        }
     }
 
     // density_kernel! + eos_kernel! with one thread per particle: the mask
@@ -803,6 +892,7 @@ template <typename T> class Sys final : public StateI {
     {
         use_params(p);
         Field<T> *th = field_of(theta);
+        reserve_lists();
         step_impl(th->th.p, nullptr, nullptr);
         rt_check_launch("step");
     }
@@ -891,6 +981,7 @@ template <typename T> class Sys final : public StateI {
         core.copy_from(s.blob);
         age = s.age;
         cur = s.cur;
+        listsFresh = false;
         cellsOnlyLatest = false;
     }
     void assign(StateI *src) override
@@ -906,6 +997,7 @@ template <typename T> class Sys final : public StateI {
         prho.copy_from(o->prho);
         age = o->age;
         cur = o->cur;
+        listsFresh = false;
         if (std::memcmp(hinst.data(), o->hinst.data(), sizeof(Inst<T>) * B) != 0) {
             prm = o->prm;
             prms = o->prms;
@@ -1125,6 +1217,7 @@ void Sys<T>::simulate(FieldI *theta, const Params *p, int64_t nsteps, TapeI *tap
         for (size_t k = 0; k < tp->descent.size(); ++k)
             if (tp->descent[k] >= tp->n_ && tp->descent[k] < tp->n_ + nsteps)
                 reserve(tp->slot((int)k));
+    reserve_lists();
     graphs.start(step_graph_eligible<T>(N_));
     StepGraphsGuard guard{graphs};
     for (int64_t s = 0; s < nsteps; ++s) {
@@ -1204,8 +1297,8 @@ template <typename T> class Work final : public WorkI {
             gX[k].zero();
             gV[k].zero();
         }
-        abar.alloc(n1); gXs.alloc(n1); stage2.alloc(n1); outX.alloc(n1); outV.alloc(n1);
-        galpha.alloc(n1); grho.alloc(n1);
+        abar.alloc(n1 + 4); gXs.alloc(n1); stage2.alloc(n1); outX.alloc(n1); outV.alloc(n1);
+        galpha.alloc(n1); grho.alloc(n1 + 4); // staged arrays: see Sys
         thetaAcc.alloc(2 * (size_t)nnode);
         emax.alloc(2 * (size_t)B);
         gtheta.alloc((size_t)nnode);
@@ -1274,6 +1367,25 @@ template <typename T> class Work final : public WorkI {
         }
         const bool multi = S.B > 1;
         const bool av = S.anyAV;
+        if (S.tiles()) {
+            if constexpr (sizeof(T) == 4) {
+                S.density_tiles(v, rhoOut, S.prho.p);
+                auto ka = multi ? (av ? &k_drag_win<true, true> : &k_drag_win<true, false>)
+                                : (av ? &k_drag_win<false, true> : &k_drag_win<false, false>);
+                auto k1 = multi ? (av ? &k_pass1_win<true, true> : &k_pass1_win<true, false>)
+                                : (av ? &k_pass1_win<false, true> : &k_pass1_win<false, false>);
+                auto k2 = multi ? &k_pass2_win<true> : &k_pass2_win<false>;
+                const WinLists W = S.lists();
+                SPH_LAUNCH_TILES(K_ACCEL_DRAG, ka, N_, v, W, vel, S.prho.p, S.rho.p, theta,
+                                 gX[gcur].p, gV[gcur].p, abar.p, galpha.p, emax.p, parity);
+                SPH_LAUNCH_TILES(K_PASS1, k1, N_, v, W, vel, S.prho.p, S.rho.p, theta, abar.p,
+                                 galpha.p, gXs.p, grho.p, gV[gcur].p);
+                SPH_LAUNCH_TILES(K_PASS2, k2, N_, v, W, grho.p, gXs.p, gX[gcur].p, galpha.p,
+                                 emax.p, parity, thetaAcc.p);
+            }
+            pendingTheta = parity;
+            return;
+        }
         auto ka = multi ? (av ? &k_accel_drag_adj<T, true, true> : &k_accel_drag_adj<T, true>)
                         : (av ? &k_accel_drag_adj<T, false, true> : &k_accel_drag_adj<T, false>);
         auto k1 = multi ? (av ? &k_pass1_design<T, true, true> : &k_pass1_design<T, true>)
@@ -1579,6 +1691,8 @@ void Work<T>::run_backward(TapeI *tape, FieldI *theta, const Params *pp, const v
     // reverse steps and recomputed forward steps go out in recorded groups
     if (tp->nsnap_ && L > 0)
         for (int k = 0; k < tp->nsnap_; ++k) tp->recomp->reserve(tp->slot(k));
+    S->reserve_lists();
+    if (tp->nsnap_ && L > 0) tp->recomp->reserve_lists();
     graphs.start(step_graph_eligible<T>(N_));
     StepGraphsGuard guard{graphs};
     if (tp->nsnap_ == 0) {

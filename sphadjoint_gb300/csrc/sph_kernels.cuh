@@ -588,6 +588,55 @@ template <typename T> struct Pass1Pair {
 //   d/dd   = K da + A (K/s) w + A ((K/F) G/(h r) - 2K/D) d   (into gx, gy)
 //   d/dv_i = A (K/s) d                                        (into gvx, gvy)
 //   d/drho_i = -A K / (2 rb)                                  (into grho)
+// FP32 with the artificial viscosity: explicit roundings, so that every kernel
+// form (mask walk, lists, lane groups, batched or not) gives the same bits. Left
+// to the compiler, the multiply-adds of the branch on approaching pairs
+// contract differently from kernel to kernel.
+__device__ __forceinline__ Pass1Pair<float>
+pass1_pair_av(float r2, float dx, float dy, float invh, float m, float Fc, float Gc,
+              const Visc<float> &vc, float pti, float rhoi, float rhoj, const float2 &vi,
+              const float2 &ab, const float2 &pj, const float2 &abj, const float2 &vj)
+{
+    const float rinv = r2 > 0.0f ? rsqrtf(r2) : 0.0f;
+    const float q = __fmul_rn(__fmul_rn(r2, rinv), invh);
+    const float u = __fmaf_rn(-0.5f, q, 1.0f);
+    const float F = __fmul_rn(__fmul_rn(__fmul_rn(Fc, u), u), u);
+    const float G = __fmul_rn(__fmul_rn(Gc, u), u);
+    const float Pij = __fmul_rn(m, __fadd_rn(pti, pj.x));
+    const float dax = __fsub_rn(ab.x, abj.x), day = __fsub_rn(ab.y, abj.y);
+    const float dvx = __fsub_rn(vi.x, vj.x), dvy = __fsub_rn(vi.y, vj.y);
+    const float Ad = __fmaf_rn(dax, dx, __fmul_rn(day, dy));
+    const float s = __fmaf_rn(dvx, dx, __fmul_rn(dvy, dy));
+    const float Gr = __fmul_rn(__fmul_rn(G, invh), rinv);
+    const float w = __fmul_rn(__fmul_rn(Pij, -Ad), Gr);
+    const float PF = __fmul_rn(Pij, F);
+    float avx = 0.0f, avy = 0.0f;
+    Pass1Pair<float> o;
+    o.gvx = o.gvy = o.grs = 0.0f;
+    if (s < 0.0f) {
+        const float D = __fadd_rn(r2, vc.eh2);
+        const float rb = __fmul_rn(0.5f, __fadd_rn(rhoi, rhoj));
+        const float Drb = __fmul_rn(D, rb);
+        const float as = __fmul_rn(vc.avc, s);
+        const float K = __fmul_rn(as, F) / Drb;
+        const float Ks = __fmul_rn(vc.avc, F) / Drb;
+        const float KF = as / Drb;
+        const float cd = __fmul_rn(Ad, __fmaf_rn(KF, Gr, -(__fmul_rn(2.0f, K) / D)));
+        const float AK = __fmul_rn(Ad, Ks);
+        avx = __fmaf_rn(cd, dx, __fmaf_rn(AK, dvx, __fmul_rn(K, dax)));
+        avy = __fmaf_rn(cd, dy, __fmaf_rn(AK, dvy, __fmul_rn(K, day)));
+        o.gvx = __fmul_rn(AK, dx);
+        o.gvy = __fmul_rn(AK, dy);
+        o.grs = __fmul_rn(Ad, K) / __fmul_rn(2.0f, rb);
+    }
+    o.gxs = __fmul_rn(PF, dax);
+    o.gys = __fmul_rn(PF, day);
+    o.gxa = __fmaf_rn(w, dx, avx);
+    o.gya = __fmaf_rn(w, dy, avy);
+    o.sS = __fmul_rn(F, -Ad);
+    return o;
+}
+
 template <typename T, bool AV = true>
 __device__ __forceinline__ Pass1Pair<T> pass1_pair(T r2, T dx, T dy, T invh, T m, T Fc, T Gc,
                                                    const Visc<T> &vc, T pti, T iri, T rhoi,
@@ -595,6 +644,11 @@ __device__ __forceinline__ Pass1Pair<T> pass1_pair(T r2, T dx, T dy, T invh, T m
                                                    const T2<T> &pj, const T2<T> &abj,
                                                    const T2<T> &vj)
 {
+    if constexpr (sizeof(T) == 4 && AV) {
+        if (vc.kind == 1)
+            return pass1_pair_av(r2, dx, dy, invh, m, Fc, Gc, vc, pti, rhoi, rhoj, vi, ab, pj, abj,
+                                 vj);
+    }
     const T twomumass = vc.twomumass;
     T r, rinv;
     if constexpr (sizeof(T) == 4) {

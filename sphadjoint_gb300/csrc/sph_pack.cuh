@@ -71,6 +71,7 @@ template <typename T> struct GSys {
     int *emax;
     unsigned long long *thetaAcc;
     double *gtheta;
+    WinLists W; // FP32 windows and lists (W.win NULL: mask walks)
 };
 
 // The per-tick table in constant memory: the descriptors of the requests that
@@ -83,9 +84,9 @@ template <typename T> struct GSys {
 #error "define SPH_PACK_T (this translation unit's precision) before including sph_pack.cuh"
 #endif
 constexpr int kMaxPackSys = 64; // requests one tick can hold
-constexpr int kPackLists = 9;
+constexpr int kPackLists = 10;
 enum PackList : int {
-    PL_GATHER = 0, PL_CELLS, PL_SCANTOP, PL_SCANTILE, PL_PART, PL_ALL, PL_REV, PL_THETA, PL_FWD
+    PL_GATHER = 0, PL_CELLS, PL_SCANTOP, PL_SCANTILE, PL_PART, PL_ALL, PL_REV, PL_THETA, PL_FWD, PL_LISTS
 };
 struct PackLists {
     int32_t cnt[kPackLists];
@@ -299,21 +300,65 @@ __global__ void __launch_bounds__(kPackBlock) g_nl_build(int l)
                     d.flags);
 }
 
+// Windows and candidate lists of the requests whose masks are new (rebuilt this
+// tick, or restored with a snapshot).
+template <typename T>
+__global__ void __launch_bounds__(kTile) g_lists(int l)
+{
+    pdl_enter();
+    if constexpr (sizeof(T) == 4) {
+        const int2 f = glist_find(l);
+        const GSys<T> &d = pack_sys<T>(f.x);
+        window_lists<false>(d.v, d.W, f.y);
+    }
+}
+
 // The pair kernels cap their registers as the tuned single-state kernels do:
 // the request's arrays and constants come from the descriptor table, and
 // holding them all in registers would halve the resident warps.
+static_assert(kPackBlock == kTile, "a block of a grouped launch is one tile");
 template <typename T>
-__global__ void __launch_bounds__(kPackBlock, sizeof(T) == 4 ? 10 : 1)
+__global__ void __launch_bounds__(kPackBlock, sizeof(T) == 4 ? 11 : 1)
     g_density(int l)
 {
     pdl_enter();
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
+    if constexpr (sizeof(T) == 4) {
+        if (d.W.win) {
+            density_window<false>(d.v, d.W, f.y, d.rho, d.prho);
+            return;
+        }
+    }
     const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
     if (i >= d.n) return;
     NLView<T> v = d.v;
     v.tmask = nullptr;
     density_walk<T, false, true>(v, i, d.rho, d.prho, d.tmask);
+}
+
+// The pair sum of a force pass of one request's particle: FP32 requests over
+// their lists and the block's staged window, others by the mask walk. All
+// threads of the block call it (live: this one has a particle).
+template <typename T, bool AV>
+__device__ __forceinline__ void g_accel_sum(const GSys<T> &d, int tile, int64_t i, bool live,
+                                            T2<T> &xi, T2<T> &vi, T &ax, T &ay)
+{
+    const NLView<T> &v = d.v;
+    if constexpr (sizeof(T) == 4) {
+        __shared__ __align__(16) unsigned char s_win[kAccelSmem<AV>];
+        if (d.W.win)
+            stage_window<3, AV>(d.W.win + tile, s_win, v.pos, d.vel, d.prho, nullptr, d.rhoAll);
+        if (!live) return;
+        xi = v.pos[i];
+        vi = d.vel[i];
+        accel_any<false, AV>(v, d.W, tile, s_win, i, v.one, d.vel, d.prho, d.rhoAll, xi, vi, ax, ay);
+    } else {
+        if (!live) return;
+        xi = v.pos[i];
+        vi = d.vel[i];
+        accel_sum<T, AV>(v, v.one, d.vel, d.prho, d.rhoAll, i, xi, vi, ax, ay);
+    }
 }
 
 // accel_kernel! + integrate_kernel! of the requests taking a forward step.
@@ -327,21 +372,18 @@ __global__ void __launch_bounds__(kPackBlock, (sizeof(T) == 4 && !AV) ? 10 : 1)
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
     const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
-    const NLView<T> &v = d.v;
-    const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[i];
-    const T2<T> vi = d.vel[i];
+    T2<T> xi, vi;
     T ax, ay;
-    accel_sum<T, AV>(v, I, d.vel, d.prho, d.rhoAll, i, xi, vi, ax, ay);
-    accel_integrate_finish<T>(I, 0, i, xi, vi, ax, ay, d.theta, d.posOut, d.velOut,
+    g_accel_sum<T, AV>(d, f.y, i, i < d.n, xi, vi, ax, ay);
+    if (i >= d.n) return;
+    accel_integrate_finish<T>(d.v.one, 0, i, xi, vi, ax, ay, d.theta, d.posOut, d.velOut,
                               (T2<T> *)nullptr, (T *)nullptr, d.flags, d.perm, d.tx, d.tv);
 }
 
 // accel recompute + _adj_integrate! + _adj_drag! of the requests taking a
 // reverse step, with the largest exponent of |galpha| (one atomic per warp)
 template <typename T, bool AV>
-__global__ void __launch_bounds__(kPackBlock, (sizeof(T) == 4 && !AV) ? 12 : 1)
+__global__ void __launch_bounds__(kPackBlock, (sizeof(T) == 4 && !AV) ? 10 : 1)
     g_accel_rev(int l)
 {
     pdl_enter();
@@ -350,28 +392,14 @@ __global__ void __launch_bounds__(kPackBlock, (sizeof(T) == 4 && !AV) ? 12 : 1)
     const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
     const bool live = i < d.n;
     int e = INT_MIN;
-    if (live) {
-        const NLView<T> &v = d.v;
-        const Inst<T> &I = v.one;
-        const T2<T> xi = v.pos[i];
-        const T2<T> vi = d.vel[i];
-        T ax, ay;
-        accel_sum<T, AV>(v, I, d.vel, d.prho, d.rhoAll, i, xi, vi, ax, ay);
-        e = drag_adj_finish<T>(I, i, xi, vi, ax, ay, d.theta, d.gX, d.gV, d.abar, d.galpha);
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    if (!live) return;
-    int mx = e;
-    for (unsigned rest = act; rest; rest &= rest - 1) {
-        const int y = __shfl_sync(act, e, __ffs(rest) - 1);
-        mx = y > mx ? y : mx;
-    }
-    if ((int)lane_id() == __ffs(act) - 1 && mx != INT_MIN) atomicMax(d.emax + d.parity, mx);
+    T2<T> xi, vi;
+    T ax, ay;
+    g_accel_sum<T, AV>(d, f.y, i, live, xi, vi, ax, ay);
+    if (live)
+        e = drag_adj_finish<T>(d.v.one, i, xi, vi, ax, ay, d.theta, d.gX, d.gV, d.abar, d.galpha);
+    warp_emax(live, 0, e, d.emax, d.parity, false);
 }
 
-// 8 blocks of 128 (55 registers, no spills): 3.5% faster than 9 blocks (56
-// registers with spills); the reverse force pass keeps its 12 (relaxing it to
-// 10 made it 10% slower)
 template <typename T, bool AV>
 __global__ void __launch_bounds__(kPackBlock, (sizeof(T) == 4 && !AV) ? 8 : 1)
     g_pass1(int l)
@@ -379,20 +407,26 @@ __global__ void __launch_bounds__(kPackBlock, (sizeof(T) == 4 && !AV) ? 8 : 1)
     pdl_enter();
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
-    if (i >= d.n) return;
     const NLView<T> &v = d.v;
-    const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[i];
-    const T2<T> vi = d.vel[i];
-    const T2<T> ab = d.abar[i];
-    const T2<T> pi = d.prho[i];
-    T gx, gy, gvx, gvy, grh, sumS;
-    pass1_sum<T, AV>(v, I, i, d.vel, d.prho, d.rhoAll, d.abar, xi, vi, ab, pi, gx, gy, gvx, gvy,
-                     grh, sumS);
-    const T rhoi = I.p.eos == 1 || (AV && I.p.visc == 1) ? d.rhoAll[i] : (T)0;
-    pass1_finish<T>(I, i, xi, ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, d.theta, d.galpha, d.gXs,
-                    d.grho, d.gV);
+    if constexpr (sizeof(T) == 4) {
+        __shared__ __align__(16) unsigned char s_win[kPass1Smem<AV>];
+        pass1_window<false, AV>(v, d.W, f.y, s_win, d.vel, d.prho, d.rhoAll, d.theta, d.abar,
+                                d.galpha, d.gXs, d.grho, d.gV);
+    } else {
+        const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
+        if (i >= d.n) return;
+        const Inst<T> &I = v.one;
+        const T2<T> xi = v.pos[i];
+        const T2<T> vi = d.vel[i];
+        const T2<T> ab = d.abar[i];
+        const T2<T> pi = d.prho[i];
+        T gx, gy, gvx, gvy, grh, sumS;
+        pass1_sum<T, AV>(v, I, i, d.vel, d.prho, d.rhoAll, d.abar, xi, vi, ab, pi, gx, gy, gvx,
+                         gvy, grh, sumS);
+        const T rhoi = I.p.eos == 1 || (AV && I.p.visc == 1) ? d.rhoAll[i] : (T)0;
+        pass1_finish<T>(I, i, xi, ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, d.theta, d.galpha,
+                        d.gXs, d.grho, d.gV);
+    }
 }
 
 template <typename T>
@@ -402,15 +436,21 @@ __global__ void __launch_bounds__(kPackBlock, sizeof(T) == 4 ? 12 : 1)
     pdl_enter();
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
-    const bool live = i < d.n;
     const NLView<T> &v = d.v;
-    const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[live ? i : d.n - 1];
-    T gx = (T)0, gy = (T)0;
-    if (live) pass2_sum<T>(v, I, i, xi, d.grho, gx, gy);
-    pass2_finish_warp<T>(live, I, 0, i, xi, gx, gy, d.gXs, d.gX, d.galpha, d.emax, d.parity,
-                         d.thetaAcc);
+    if constexpr (sizeof(T) == 4) {
+        __shared__ __align__(16) unsigned char s_win[kWin8 + kWin4];
+        pass2_window<false>(v, d.W, f.y, s_win, d.grho, d.gXs, d.gX, d.galpha, d.emax, d.parity,
+                            d.thetaAcc);
+    } else {
+        const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
+        const bool live = i < d.n;
+        const Inst<T> &I = v.one;
+        const T2<T> xi = v.pos[live ? i : d.n - 1];
+        T gx = (T)0, gy = (T)0;
+        if (live) pass2_sum<T>(v, I, i, xi, d.grho, gx, gy);
+        pass2_finish_warp<T>(live, I, 0, i, xi, gx, gy, d.gXs, d.gX, d.galpha, d.emax, d.parity,
+                             d.thetaAcc);
+    }
 }
 
 template <typename T>
@@ -584,7 +624,9 @@ template <typename T> class Packer final : public PackI {
         if (r.adjoint) {
             q->S.reset(new Sys<T>(ps, ns, nullptr, nullptr, r.opts));
             q->tape.reset(new Tape<T>(r.N, r.nsteps, r.snapshots));
+            q->S->alloc_lists();
         }
+        q->F->alloc_lists();
         q->prog = pack_program(r.nsteps, r.snapshots, r.adjoint);
         SPH_CK(cudaEventCreateWithFlags(&q->done, cudaEventDisableTiming));
         const int id = next_++;
@@ -697,7 +739,7 @@ template <typename T> class Packer final : public PackI {
             }
             int32_t blocks() const { return start.back(); }
         };
-        List lGather, lCells, lScanTop, lScanTile, lPart, lAll, lRev, lTheta, lFwd;
+        List lGather, lCells, lScanTop, lScanTile, lPart, lAll, lRev, lTheta, lFwd, lLists;
         bool anyAV = false;
         auto nb = [](int64_t n, int b) { return (n + b - 1) / b; };
         for (int k = 0; k < P; ++k) {
@@ -738,7 +780,9 @@ template <typename T> class Packer final : public PackI {
             d.theta = q.th->th.p;
             NLView<T> v = Y.view();
             v.pos = Y.pos[post].p;
-            v.tmask = Y.tmask.p;
+            const bool lists = Y.wwin.p && rt_density_form() == 2;
+            if (lists) d.W = Y.lists();
+            v.tmask = lists ? nullptr : Y.tmask.p;
             v.inst = nullptr;
             v.pinst = nullptr;
             d.v = v;
@@ -796,6 +840,11 @@ template <typename T> class Packer final : public PackI {
             }
             lAll.add(k, nb(N, kPackBlock));
             if (!rev) lFwd.add(k, nb(N, kPackBlock));
+            if (rebuild) Y.listsFresh = false;
+            if (lists && !Y.listsFresh) {
+                lLists.add(k, nb(N, kTile));
+                Y.listsFresh = true;
+            }
             // host bookkeeping of maybe_rebuild! and the step
             if (rebuild) Y.age = 0;
             Y.age += 1;
@@ -808,7 +857,7 @@ template <typename T> class Packer final : public PackI {
         ringPos_ = (ringPos_ + 1) % kRing;
         if (R.used) SPH_CK(cudaEventSynchronize(R.ev));
         const List *lists[kPackLists] = {&lGather, &lCells, &lScanTop, &lScanTile, &lPart,
-                                         &lAll, &lRev, &lTheta, &lFwd};
+                                         &lAll, &lRev, &lTheta, &lFwd, &lLists};
         const size_t bytes = sizeof(PackLists) + sizeof(GSys<T>) * (size_t)P;
         if (!R.host) {
             SPH_CK(cudaHostAlloc((void **)&R.host, sizeof(PackTable<T>), cudaHostAllocDefault));
@@ -841,6 +890,7 @@ template <typename T> class Packer final : public PackI {
         launch(K_BUCKET, PL_PART, kPackBlock, g_bucket<T>);
         launch(K_RANK, PL_PART, kPackBlock, g_rank<T>);
         launch(K_NLBUILD, PL_PART, kPackBlock, g_nl_build<T>);
+        launch(K_NLBUILD, PL_LISTS, kTile, g_lists<T>);
         launch(K_DENSITY, PL_ALL, kPackBlock, g_density<T>);
         if (anyAV) launch(K_ACCEL_INTEGRATE, PL_FWD, kPackBlock, g_accel_fwd<T, true>);
         else launch(K_ACCEL_INTEGRATE, PL_FWD, kPackBlock, g_accel_fwd<T, false>);

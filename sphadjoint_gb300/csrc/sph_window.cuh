@@ -1,0 +1,721 @@
+// FP32 pair passes over neighbour lists and staged windows, one thread per
+// particle.
+//
+// A tile is 128 consecutive slots (a thread block). Particles are stored in cell
+// order, so the neighbours of a tile's particles lie in a few contiguous slot
+// ranges: for every run of the tile's particles that share a cell row (and
+// instance), the three neighbouring rows' cells from one before the run's
+// first to one after its last. These ranges, each widened to multiples of four
+// slots, are the tile's window (TileWin, written at a neighbour rebuild): about
+// 470 slots on a lattice at rest. A pass copies the arrays it reads of
+// neighbours into shared memory once per tile (16-byte asynchronous copies,
+// 3.7 slots a particle instead of 21 gathers from L1), and a particle's
+// neighbours are 16-bit byte offsets into that window.
+//
+//   candidates  per particle, the rebuild-time neighbours (the set bits of its
+//               row masks, in slot order), written after a rebuild or when a
+//               restored state has masks but no list
+//   in support  per particle, this step's neighbours with r^2 < 4h^2, written
+//               by the density pass and read by the later passes of the step
+//
+// Lists are stored as quads of four offsets, [tile][quad][thread], so a warp reads
+// four neighbours of all its particles in one coalesced 8-byte load; the last
+// quad is padded with the particle's last entry. Visiting order, pair terms and
+// sums are those of the mask walks (for_each_neighbor), operation by operation,
+// so results are the same bits; what goes away is the walk itself: finding set
+// bits, moving from word to word (some lane of a warp does that in nearly every
+// iteration), and 64-bit addresses for every array. Particles that have no
+// list (a row beyond the 64-slot masks, more than 48 candidates, or a tile
+// whose window exceeds its capacity) are marked and take the mask walk.
+//
+// Bound: shared-memory wavefronts and issue slots together (accel at 1M: 71% of
+// the wavefront rate, 57% of the issue slots, 913 warp instructions a warp where
+// the mask walk ran 1449). Measured per launch at 1,048,576 particles, mask walk
+// -> lists: density 58.1 -> 45.0 us, accel 59.2 -> 46.5, accel + drag 70.8 -> 48.9,
+// pass 1 82.7 -> 60.6, pass 2 64.1 -> 48.2; the lists cost 43 us a rebuild.
+// Solves: 249k particles 2.70 -> 2.17 ms, 8.4M dense (a rebuild a step) 23.5 ->
+// 20.2 ms, 131k with the Tait/artificial-viscosity model 1.83 -> 1.37 ms.
+// Reading the lists two quads ahead (accel 46 -> 49 us), copying a tile's lists
+// to shared memory first (density 45 -> 51) and 16-byte interleaved windows
+// (below) were slower.
+#pragma once
+
+#include "sph_kernels.cuh"
+
+namespace sphgb {
+
+constexpr int kTile = 128;     // slots of a tile = threads of its block
+constexpr int kWinMax = 640;   // window capacity in slots (rest: ~470)
+constexpr int kRunMax = 8;     // cell-row runs of a tile
+constexpr int kRangeMax = 3 * kRunMax;
+constexpr int kQuads = 12;     // list capacity: 48 entries
+constexpr int kNoList = 255;   // count of a particle without a list
+constexpr int kListStride = 8 * kQuads + 4; // bytes per thread while a list is
+                                            // collected: an odd number of words,
+                                            // so a warp's lanes use all banks
+
+struct TileWin {
+    int32_t nr;               // ranges (0: no window, every particle is marked)
+    int32_t pad[3];
+    int32_t start[kRangeMax]; // first slot, a multiple of 4
+    int32_t base[kRangeMax + 1]; // first window slot; base[nr] = window slots
+    int32_t pad2[3];
+};
+
+// The lists of one state (device pointers; win NULL: it has none and every
+// particle takes the mask walk).
+struct WinLists {
+    TileWin *win;
+    uint2 *cand, *supp;        // [tile][kQuads][kTile]
+    uint8_t *candCnt, *suppCnt; // per slot; kNoList: mask walk
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p)
+{
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+// Element at byte offset o of a staged array (s_win is in shared memory).
+__device__ __forceinline__ float2 lds2(const unsigned char *sw, uint32_t o)
+{
+    return *reinterpret_cast<const float2 *>(sw + o);
+}
+__device__ __forceinline__ float lds1(const unsigned char *sw, uint32_t o)
+{
+    return *reinterpret_cast<const float *>(sw + o);
+}
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// Bytes of a staged array.
+constexpr int kWin8 = 8 * kWinMax;
+constexpr int kWin4 = 4 * kWinMax;
+
+// Copy the tile's window of the given arrays into shared memory at sw, sw +
+// kWin8, ... (N8 float2 arrays), then a float array. Range ends are multiples of
+// four slots, so a copy may read up to three elements past the last particle:
+// every staged array has room for them. All threads of the block call it.
+//
+// Neighbours are then read eight bytes at a time: 4.2 wavefronts a warp read
+// (2.1 per 16 lanes; bank padding, swizzles, 4-byte arrays were no better), and
+// 16-byte reads of interleaved arrays measured slower (8.8 wavefronts where two
+// 8-byte reads take 8.4: accel 46 -> 55 us, pass 1 60 -> 74 us at 1M).
+template <int N8, bool F4>
+__device__ __forceinline__ void stage_window(const TileWin *__restrict__ w,
+                                             const unsigned char *sw, const float2 *a0,
+                                             const float2 *a1, const float2 *a2, const float2 *a3,
+                                             const float *f)
+{
+    const uint32_t sm = smem_addr(sw);
+    const int lane = (int)(threadIdx.x & 31u);
+    const int nr = w->nr;
+    const int st = lane < nr ? w->start[lane] : 0;
+    const int bs = lane <= nr ? w->base[lane] : 0;
+    const int total = __shfl_sync(0xffffffffu, bs, nr);
+    const int rounds = (total / 2 + kTile - 1) / kTile;
+    for (int q = 0; q < rounds; ++q) {
+        const int k = 2 * (q * kTile + (int)threadIdx.x);
+        int r = 0;
+        for (int t = 1; t < nr; ++t) r += k >= __shfl_sync(0xffffffffu, bs, t) ? 1 : 0;
+        const int src = __shfl_sync(0xffffffffu, st, r) + k - __shfl_sync(0xffffffffu, bs, r);
+        if (k < total) {
+            const uint32_t d = sm + 8 * k;
+            copy16(d, a0 + src);
+            if (N8 > 1) copy16(d + kWin8, a1 + src);
+            if (N8 > 2) copy16(d + 2 * kWin8, a2 + src);
+            if (N8 > 3) copy16(d + 3 * kWin8, a3 + src);
+            if (F4 && !(k & 2)) copy16(sm + N8 * kWin8 + 4 * k, f + src);
+        }
+    }
+    copy_wait();
+    __syncthreads();
+}
+
+__device__ __forceinline__ uint32_t entry_of(const uint2 &e, int k)
+{
+    const uint32_t w = k < 2 ? e.x : e.y;
+    return (k & 1) ? w >> 16 : w & 0xffffu;
+}
+
+// The collected list of a thread (n entries at its place in shared memory) to
+// its quads, the last one padded with the last entry.
+__device__ __forceinline__ void write_list(unsigned char *place, int n, uint2 *__restrict__ out)
+{
+    uint16_t *p = reinterpret_cast<uint16_t *>(place);
+    if (n & 3) {
+        const uint16_t last = p[n - 1];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (k < (-n & 3)) p[n + k] = last;
+    }
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(place);
+    for (int q = 0; 4 * q < n; ++q) out[q * kTile] = make_uint2(w[2 * q], w[2 * q + 1]);
+}
+
+// Windows and candidate lists from the row masks: after a rebuild, and after a
+// snapshot was restored (a snapshot holds the masks, not the lists).
+template <bool MULTI>
+__device__ __forceinline__ void window_lists(const NLView<float> &v, const WinLists &L, int tile)
+{
+    __shared__ int s_key[kTile];
+    __shared__ int s_cnt[kTile / 32];
+    __shared__ int s_min[kRunMax], s_max[kRunMax], s_inst[kRunMax], s_cy[kRunMax];
+    __shared__ int s_start[32], s_len[32], s_base[33];
+    __shared__ __align__(8) unsigned char s_list[kTile * kListStride];
+    const int t = (int)threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int64_t i = (int64_t)tile * kTile + t;
+    const bool live = i < v.N;
+    const uint32_t cc = live ? v.center[i] : 0u;
+    const int cx = (int)(cc & 0xffffu);
+    const int cy = (int)((cc >> 16) & 0x7fffu);
+    const int b = MULTI && live ? (int)v.pinst[i] : 0;
+    const int key = live ? (b << 15) | cy : -1;
+    s_key[t] = key;
+    if (t < kRunMax) {
+        s_min[t] = INT_MAX;
+        s_max[t] = 0;
+    }
+    if (t < 32) s_len[t] = 0;
+    __syncthreads();
+    const bool first = live && (t == 0 || s_key[t - 1] != key);
+    const unsigned fm = __ballot_sync(0xffffffffu, first);
+    if (lane == 0) s_cnt[warp] = __popc(fm);
+    __syncthreads();
+    int run = __popc(fm & (0xffffffffu >> (31 - lane))) - 1, nrun = 0;
+#pragma unroll
+    for (int w = 0; w < kTile / 32; ++w) {
+        if (w < warp) run += s_cnt[w];
+        nrun += s_cnt[w];
+    }
+    if (live && run < kRunMax) {
+        atomicMin(&s_min[run], cx);
+        atomicMax(&s_max[run], cx);
+        if (first) {
+            s_inst[run] = b;
+            s_cy[run] = cy;
+        }
+    }
+    __syncthreads();
+    bool ok = nrun <= kRunMax;
+    if (ok && t < 3 * nrun) {
+        const int q = t / 3;
+        decltype(auto) I = pick_inst<MULTI>(v.one, v.inst, s_inst[q]);
+        const int jy = s_cy[q] + t % 3 - 1;
+        int a = 0, e = 0;
+        if (jy >= 1 && jy <= I.ny) {
+            const int xa = s_min[q] - 1 > 1 ? s_min[q] - 1 : 1;
+            const int xb = s_max[q] + 1 < I.nx ? s_max[q] + 1 : I.nx;
+            const int row = I.coff + (jy - 1) * I.nx;
+            a = v.cellStart[row + xa - 1];
+            e = v.cellStart[row + xb];
+        }
+        s_start[t] = a & ~3;
+        s_len[t] = e > a ? ((e - (a & ~3) + 3) & ~3) : 0;
+    }
+    __syncthreads();
+    if (t < 32) {
+        const int n = s_len[t];
+        int x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        s_base[t] = x - n;
+        if (t == 31) s_base[32] = x;
+    }
+    __syncthreads();
+    const int total = s_base[32];
+    ok = ok && total <= kWinMax;
+    TileWin *W = L.win + tile;
+    if (t == 0) W->nr = ok ? 3 * nrun : 0;
+    if (t < kRangeMax) W->start[t] = t < 3 * nrun ? s_start[t] : 0;
+    if (t <= kRangeMax) W->base[t] = ok ? s_base[t] : 0;
+    if (!live) return;
+    if (!ok || (cc >> 31)) {
+        L.candCnt[i] = kNoList;
+        return;
+    }
+    // the walk of for_each_neighbor over the masks, as offsets into the window
+    decltype(auto) I = pick_inst<MULTI>(v.one, v.inst, b);
+    const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
+    const int row0 = I.coff + (jx0 - 1) + (cy - 2) * I.nx;
+    unsigned char *const place = s_list + t * kListStride;
+    uint64_t m[3];
+    int off[3];
+    int n = 0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        m[r] = ((uint64_t)v.masks[(2 * r + 1) * v.N + i] << 32) | v.masks[2 * r * v.N + i];
+        n += __popcll(m[r]);
+        off[r] = m[r] ? 8 * (s_base[3 * run + r] + v.cellStart[row0 + r * I.nx] -
+                             s_start[3 * run + r])
+                      : 0;
+    }
+    if (n > 4 * kQuads) {
+        L.candCnt[i] = kNoList;
+        return;
+    }
+    uint16_t *to = reinterpret_cast<uint16_t *>(place);
+    uint32_t w = (uint32_t)m[0];
+    int base = off[0], word = 0;
+    for (;;) {
+        if (w == 0u) {
+            if (++word == 6) break;
+            const uint64_t mr = word < 2 ? m[0] : (word < 4 ? m[1] : m[2]);
+            base = (word < 2 ? off[0] : (word < 4 ? off[1] : off[2])) + ((word & 1) << 8);
+            w = (word & 1) ? (uint32_t)(mr >> 32) : (uint32_t)mr;
+            continue;
+        }
+        const int k = __ffs((int)w) - 1;
+        w &= w - 1u;
+        *to++ = (uint16_t)(base + 8 * k);
+    }
+    write_list(place, n, L.cand + (int64_t)tile * (kQuads * kTile) + t);
+    L.candCnt[i] = (uint8_t)n;
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(kTile)
+    k_window_lists(const __grid_constant__ NLView<float> v, const WinLists L)
+{
+    pdl_enter();
+    window_lists<MULTI>(v, L, (int)blockIdx.x);
+}
+
+// density_kernel! + eos_kernel! and this step's in-support lists: the arithmetic of
+// density_pairs_f32, two candidates at a time.
+template <bool MULTI>
+__device__ __forceinline__ void density_window(const NLView<float> &v, const WinLists &L, int tile,
+                                               float *__restrict__ rho,
+                                               float2 *__restrict__ prho)
+{
+    __shared__ __align__(16) unsigned char s_win[kWin8];
+    __shared__ __align__(8) unsigned char s_list[kTile * kListStride];
+    const int t = (int)threadIdx.x;
+    const int64_t i = (int64_t)tile * kTile + t;
+    const bool live = i < v.N;
+    const unsigned char *sw = s_win;
+    const int n = live ? (int)L.candCnt[i] : 0;
+    stage_window<1, false>(L.win + tile, sw, v.pos, nullptr, nullptr, nullptr, nullptr);
+    if (!live) return;
+    if (n == kNoList) {
+        L.suppCnt[i] = kNoList;
+        density_walk<float, MULTI, true>(v, i, rho, prho, nullptr);
+        return;
+    }
+    decltype(auto) I = load_inst<MULTI>(v, i);
+    const float r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, A = I.p.A;
+    const float2 xi = v.pos[i];
+    const float2 ih2 = make_float2(invh, invh), mh = make_float2(-0.5f, -0.5f);
+    const float2 one2 = make_float2(1.0f, 1.0f), two2 = make_float2(2.0f, 2.0f);
+    const int64_t lbase = (int64_t)tile * (kQuads * kTile) + t;
+    const uint2 *cand = L.cand + lbase;
+    unsigned char *const place = s_list + t * kListStride;
+    int ns = 0;
+    float acc = 0.0f;
+    // one quad of candidates, `left` of them in the list
+    auto quad = [&](const uint2 &cur, int left) {
+        float2 xj[4];
+        bool in[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) xj[k] = lds2(sw, entry_of(cur, k));
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            const float2 da = fsub2(xi, xj[h]);
+            const float2 db = fsub2(xi, xj[h + 1]);
+            const float r2a = da.x * da.x + da.y * da.y;
+            const float r2b = db.x * db.x + db.y * db.y;
+            in[h] = h < left && r2a < r2max;
+            in[h + 1] = h + 1 < left && r2b < r2max;
+            const float2 qq = fmul2(make_float2(pair_sqrt(r2a), pair_sqrt(r2b)), ih2);
+            float2 u = ffma2(qq, mh, one2); // 1 - q/2
+            u.x = in[h] ? u.x : 0.0f;
+            u.y = in[h + 1] ? u.y : 0.0f;
+            const float2 u2 = fmul2(u, u);
+            const float2 u4 = fmul2(u2, u2);
+            const float2 w = ffma2(qq, two2, one2); // 2q + 1
+            acc = fmaf(u4.x, w.x, acc);
+            acc = fmaf(u4.y, w.y, acc);
+        }
+        // every entry is written, and kept by moving on (ns <= 48: the write
+        // after the last kept entry stays inside this thread's place)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            *reinterpret_cast<uint16_t *>(place + ns) = (uint16_t)entry_of(cur, k);
+            if (in[k]) ns += 2;
+        }
+    };
+    uint2 e = n ? cand[0] : make_uint2(0u, 0u);
+    int q = 0;
+    for (; q < (n >> 2); ++q) {
+        const uint2 cur = e;
+        if (4 * q + 4 < n) e = cand[(q + 1) * kTile];
+        quad(cur, 4);
+    }
+    if (n & 3) quad(e, n & 3);
+    ns >>= 1;
+    write_list(place, ns, L.supp + lbase);
+    L.suppCnt[i] = (uint8_t)ns;
+    acc = mul_rn(mul_rn(m, A), acc);
+    density_finish<float>(I, i, acc, rho, prho);
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(kTile, 11)
+    k_density_win(const __grid_constant__ NLView<float> v, const WinLists L,
+                  float *__restrict__ rho, float2 *__restrict__ prho)
+{
+    pdl_enter();
+    density_window<MULTI>(v, L, (int)blockIdx.x, rho, prho);
+}
+
+// Visit a particle's in-support list: f(offset) for each of its n entries, in
+// slot order. Whole quads run four pairs at once, so their loads overlap.
+template <typename F>
+__device__ __forceinline__ void for_each_entry(const uint2 *__restrict__ list, int n, F &&f)
+{
+    const int nq = n >> 2;
+    uint2 e = n ? list[0] : make_uint2(0u, 0u);
+    for (int q = 0; q < nq; ++q) {
+        const uint2 cur = e;
+        if (4 * q + 4 < n) e = list[(q + 1) * kTile];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) f(entry_of(cur, k));
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if (k < (n & 3)) f(entry_of(e, k));
+}
+
+// Pressure + viscosity sum of accel_sum over the staged window: positions,
+// velocities, {p/rho^2, 1/rho} (and densities for the artificial viscosity).
+template <bool AV>
+__device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsigned char *sw,
+                                              const uint2 *__restrict__ list, int n,
+                                              const float2 &xi, const float2 &vi,
+                                              const float2 &pi, float rhoi, float &ax, float &ay)
+{
+    const float invh = I.p.invh, m = I.p.m, Fc = I.p.Fc;
+    // the model is chosen outside the pair loop, so each loop is one straight
+    // body whose multiply-adds contract as in the mask walks' loops
+    Visc<float> vc = visc_of<float>(I);
+    const float pti = pi.x, iri = pi.y;
+    if (!AV || vc.kind != 1) {
+        const float tmm = vc.twomumass;
+        float2 acc = make_float2(0.0f, 0.0f);
+        for_each_entry(list, n, [&](uint32_t o) {
+            const float2 xj = lds2(sw, o);
+            const float2 vj = lds2(sw + kWin8, o);
+            const float2 pj = lds2(sw + 2 * kWin8, o);
+            const float2 d = fsub2(xi, xj);
+            const float r2 = d.x * d.x + d.y * d.y;
+            const float q = pair_sqrt(r2) * invh;
+            const float u = 1.0f - 0.5f * q;
+            const float F = Fc * u * u * u;
+            const float PF = m * (pti + pj.x) * F;
+            const float C = tmm * iri * pj.y * F;
+            acc = ffma2(make_float2(-PF, -PF), d, acc);
+            acc = ffma2(make_float2(C, C), fsub2(vi, vj), acc);
+        });
+        ax = acc.x;
+        ay = acc.y;
+    } else {
+        vc.kind = 1;
+        ax = 0.0f;
+        ay = 0.0f;
+        for_each_entry(list, n, [&](uint32_t o) {
+            const float2 xj = lds2(sw, o);
+            const float2 vj = lds2(sw + kWin8, o);
+            const float2 pj = lds2(sw + 2 * kWin8, o);
+            const float rhoj = lds1(sw + 3 * kWin8, o >> 1);
+            const float dx = xi.x - xj.x;
+            const float dy = xi.y - xj.y;
+            const float r2 = dx * dx + dy * dy;
+            const AccelPair<float> t = accel_pair<float, AV>(r2, dx, dy, invh, m, Fc, vc, pti, iri,
+                                                             rhoi, rhoj, vi, pj, vj);
+            ax -= t.px;
+            ay -= t.py;
+            ax += t.cx;
+            ay += t.cy;
+        });
+    }
+}
+
+// The sum of particle i of a tile: its list, or the mask walk of a marked one.
+template <bool MULTI, bool AV>
+__device__ __forceinline__ void accel_any(const NLView<float> &v, const WinLists &L, int tile,
+                                          const unsigned char *sw, int64_t i, const Inst<float> &I,
+                                          const float2 *__restrict__ vel,
+                                          const float2 *__restrict__ prho,
+                                          const float *__restrict__ rho, const float2 &xi,
+                                          const float2 &vi, float &ax, float &ay)
+{
+    const int n = L.win ? (int)L.suppCnt[i] : kNoList;
+    if (n == kNoList) {
+        accel_sum<float, AV>(v, I, vel, prho, rho, i, xi, vi, ax, ay);
+        return;
+    }
+    const float rhoi = AV && I.p.visc == 1 ? rho[i] : 0.0f;
+    accel_sum_win<AV>(I, sw, L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n, xi, vi,
+                      prho[i], rhoi, ax, ay);
+}
+
+template <bool AV> constexpr int kAccelSmem = 3 * kWin8 + (AV ? kWin4 : 0);
+
+// accel_kernel! + integrate_kernel!
+template <bool MULTI, bool AV>
+__global__ void __launch_bounds__(kTile, AV ? 1 : 12)
+    k_accel_win(const __grid_constant__ NLView<float> v, const WinLists L,
+                const float2 *__restrict__ vel, const float2 *__restrict__ prho,
+                const float *__restrict__ rho, const float *__restrict__ theta,
+                float2 *__restrict__ posOut, float2 *__restrict__ velOut,
+                float2 *__restrict__ aOut, float *__restrict__ alphaOut,
+                uint32_t *__restrict__ flags, const int32_t *__restrict__ perm,
+                float2 *__restrict__ tx, float2 *__restrict__ tv)
+{
+    pdl_enter();
+    __shared__ __align__(16) unsigned char s_win[kAccelSmem<AV>];
+    const unsigned char *sw = s_win;
+    stage_window<3, AV>(L.win + blockIdx.x, sw, v.pos, vel, prho, nullptr, rho);
+    const int64_t i = (int64_t)blockIdx.x * kTile + threadIdx.x;
+    if (i >= v.N) return;
+    const int b = MULTI ? inst_of(v, i) : 0;
+    decltype(auto) I = load_inst<MULTI>(v, i);
+    const float2 xi = v.pos[i];
+    const float2 vi = vel[i];
+    float ax, ay;
+    accel_any<MULTI, AV>(v, L, (int)blockIdx.x, sw, i, I, vel, prho, rho, xi, vi, ax, ay);
+    accel_integrate_finish<float>(I, b, i, xi, vi, ax, ay, theta, posOut, velOut, aOut, alphaOut,
+                                  flags, perm, tx, tv);
+}
+
+// Largest exponent of the lanes of each instance in the warp, one atomic each.
+__device__ __forceinline__ void warp_emax(bool live, int b, int e, int *__restrict__ emax,
+                                          int parity, bool multi)
+{
+    const unsigned act = __ballot_sync(0xffffffffu, live);
+    if (!live) return;
+    const unsigned peers = multi ? __match_any_sync(act, b) : act;
+    const int mx = __reduce_max_sync(peers, e);
+    if ((int)lane_id() == __ffs((int)peers) - 1 && mx != INT_MIN)
+        atomicMax(emax + 2 * b + parity, mx);
+}
+
+// Accel recompute + _adj_integrate! + _adj_drag!
+template <bool MULTI, bool AV>
+__global__ void __launch_bounds__(kTile, AV ? 1 : 12)
+    k_drag_win(const __grid_constant__ NLView<float> v, const WinLists L,
+               const float2 *__restrict__ vel, const float2 *__restrict__ prho,
+               const float *__restrict__ rho, const float *__restrict__ theta,
+               const float2 *__restrict__ gX, float2 *__restrict__ gV, float2 *__restrict__ abar,
+               float *__restrict__ galpha, int *__restrict__ emax, int parity)
+{
+    pdl_enter();
+    __shared__ __align__(16) unsigned char s_win[kAccelSmem<AV>];
+    const unsigned char *sw = s_win;
+    stage_window<3, AV>(L.win + blockIdx.x, sw, v.pos, vel, prho, nullptr, rho);
+    const int64_t i = (int64_t)blockIdx.x * kTile + threadIdx.x;
+    const bool live = i < v.N;
+    int e = INT_MIN, b = 0;
+    if (live) {
+        b = MULTI ? inst_of(v, i) : 0;
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        const float2 xi = v.pos[i];
+        const float2 vi = vel[i];
+        float ax, ay;
+        accel_any<MULTI, AV>(v, L, (int)blockIdx.x, sw, i, I, vel, prho, rho, xi, vi, ax, ay);
+        e = drag_adj_finish<float>(I, i, xi, vi, ax, ay, theta, gX, gV, abar, galpha);
+    }
+    warp_emax(live, b, e, emax, parity, MULTI);
+}
+
+// The pair sums of pass1_sum over the staged window: positions, velocities,
+// {p/rho^2, 1/rho}, abar (and densities).
+template <bool AV>
+__device__ __forceinline__ void pass1_sum_win(const Inst<float> &I, const unsigned char *sw,
+                                              const uint2 *__restrict__ list, int n,
+                                              const float2 &xi, const float2 &vi,
+                                              const float2 &ab, const float2 &pi, float rhoi,
+                                              float &gx, float &gy, float &gvx, float &gvy,
+                                              float &grh, float &sumS)
+{
+    const float invh = I.p.invh, m = I.p.m, Fc = I.p.Fc, Gc = I.p.Gc;
+    Visc<float> vc = visc_of<float>(I);
+    const float pti = pi.x, iri = pi.y;
+    if (!AV || vc.kind != 1) {
+        const float tmm = vc.twomumass;
+        float2 g = make_float2(0.0f, 0.0f), gv = make_float2(0.0f, 0.0f);
+        float gr = 0.0f, sS = 0.0f;
+        for_each_entry(list, n, [&](uint32_t o) {
+            const float2 xj = lds2(sw, o);
+            const float2 vj = lds2(sw + kWin8, o);
+            const float2 pj = lds2(sw + 2 * kWin8, o);
+            const float2 abj = lds2(sw + 3 * kWin8, o);
+            const float2 d = fsub2(xi, xj);
+            const float r2 = d.x * d.x + d.y * d.y;
+            const float rinv = r2 > 0.0f ? rsqrtf(r2) : 0.0f;
+            const float r = r2 * rinv;
+            const float q = r * invh;
+            const float u = 1.0f - 0.5f * q;
+            const float F = Fc * u * u * u;
+            const float G = Gc * u * u;
+            const float PF = m * (pti + pj.x) * F;
+            const float Cbase = tmm * iri * pj.y;
+            const float C = Cbase * F;
+            const float2 da = fsub2(ab, abj);
+            const float2 dv = fsub2(vi, vj);
+            const float ad_d = -(da.x * d.x + da.y * d.y);
+            const float ad_v = da.x * dv.x + da.y * dv.y;
+            const float Fbar = m * (pti + pj.x) * ad_d + Cbase * ad_v;
+            const float w = Fbar * G * invh * rinv;
+            g = ffma2(make_float2(-PF, -PF), da, g);
+            g = ffma2(make_float2(w, w), d, g);
+            gv = ffma2(make_float2(C, C), da, gv);
+            gr -= C * ad_v * iri;
+            sS += F * ad_d;
+        });
+        gx = g.x;
+        gy = g.y;
+        gvx = gv.x;
+        gvy = gv.y;
+        grh = gr;
+        sumS = sS;
+    } else {
+        vc.kind = 1;
+        gx = 0, gy = 0, gvx = 0, gvy = 0, grh = 0, sumS = 0;
+        for_each_entry(list, n, [&](uint32_t o) {
+            const float2 xj = lds2(sw, o);
+            const float2 vj = lds2(sw + kWin8, o);
+            const float2 pj = lds2(sw + 2 * kWin8, o);
+            const float2 abj = lds2(sw + 3 * kWin8, o);
+            const float rhoj = lds1(sw + 4 * kWin8, o >> 1);
+            const float dx = xi.x - xj.x;
+            const float dy = xi.y - xj.y;
+            const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+            const Pass1Pair<float> t = pass1_pair<float, AV>(r2, dx, dy, invh, m, Fc, Gc, vc, pti,
+                                                             iri, rhoi, rhoj, vi, ab, pj, abj, vj);
+            gx -= t.gxs;
+            gy -= t.gys;
+            gx += t.gxa;
+            gy += t.gya;
+            gvx += t.gvx;
+            gvy += t.gvy;
+            grh -= t.grs;
+            sumS += t.sS;
+        });
+    }
+}
+
+template <bool AV> constexpr int kPass1Smem = 4 * kWin8 + (AV ? kWin4 : 0);
+
+template <bool MULTI, bool AV>
+__device__ __forceinline__ void pass1_window(const NLView<float> &v, const WinLists &L, int tile,
+                                             const unsigned char *sw, const float2 *__restrict__ vel,
+                                             const float2 *__restrict__ prho,
+                                             const float *__restrict__ rho,
+                                             const float *__restrict__ theta,
+                                             const float2 *__restrict__ abar,
+                                             const float *__restrict__ galpha,
+                                             float2 *__restrict__ gXs, float *__restrict__ grho,
+                                             float2 *__restrict__ gV)
+{
+    if (L.win) stage_window<4, AV>(L.win + tile, sw, v.pos, vel, prho, abar, rho);
+    const int64_t i = (int64_t)tile * kTile + threadIdx.x;
+    if (i >= v.N) return;
+    decltype(auto) I = load_inst<MULTI>(v, i);
+    const float2 xi = v.pos[i];
+    const float2 vi = vel[i];
+    const float2 ab = abar[i];
+    const float2 pi = prho[i];
+    float gx, gy, gvx, gvy, grh, sumS;
+    const int n = L.win ? (int)L.suppCnt[i] : kNoList;
+    if (n == kNoList)
+        pass1_sum<float, AV>(v, I, i, vel, prho, rho, abar, xi, vi, ab, pi, gx, gy, gvx, gvy, grh,
+                             sumS);
+    else
+        pass1_sum_win<AV>(I, sw, L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n, xi, vi,
+                          ab, pi, AV && I.p.visc == 1 ? rho[i] : 0.0f, gx, gy, gvx, gvy, grh, sumS);
+    const float rhoi = I.p.eos == 1 || (AV && I.p.visc == 1) ? rho[i] : 0.0f;
+    pass1_finish<float>(I, i, xi, ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, theta, galpha, gXs,
+                        grho, gV);
+}
+
+// adj_pass1_kernel! + the gXs half of adj_design_kernel! + _axpy2!(gV, gVs)
+template <bool MULTI, bool AV>
+__global__ void __launch_bounds__(kTile)
+    k_pass1_win(const __grid_constant__ NLView<float> v, const WinLists L,
+                const float2 *__restrict__ vel, const float2 *__restrict__ prho,
+                const float *__restrict__ rho, const float *__restrict__ theta,
+                const float2 *__restrict__ abar, const float *__restrict__ galpha,
+                float2 *__restrict__ gXs, float *__restrict__ grho, float2 *__restrict__ gV)
+{
+    pdl_enter();
+    __shared__ __align__(16) unsigned char s_win[kPass1Smem<AV>];
+    pass1_window<MULTI, AV>(v, L, (int)blockIdx.x, s_win, vel, prho, rho, theta, abar,
+                            galpha, gXs, grho, gV);
+}
+
+// The pair sum of pass2_sum over the staged window: positions and grho.
+template <bool MULTI>
+__device__ __forceinline__ void pass2_window(const NLView<float> &v, const WinLists &L, int tile,
+                                             const unsigned char *sw, const float *__restrict__ grho,
+                                             const float2 *__restrict__ gXs,
+                                             float2 *__restrict__ gX,
+                                             const float *__restrict__ galpha,
+                                             const int *__restrict__ emax, int parity,
+                                             unsigned long long *__restrict__ thetaAcc)
+{
+    if (L.win) stage_window<1, true>(L.win + tile, sw, v.pos, nullptr, nullptr, nullptr, grho);
+    const int64_t i = (int64_t)tile * kTile + threadIdx.x;
+    const bool live = i < v.N;
+    const int64_t s = live ? i : v.N - 1;
+    const int b = MULTI ? inst_of(v, s) : 0;
+    decltype(auto) I = load_inst<MULTI>(v, s);
+    const float2 xi = v.pos[s];
+    float gx = 0.0f, gy = 0.0f;
+    if (live) {
+        const int n = L.win ? (int)L.suppCnt[i] : kNoList;
+        if (n == kNoList) {
+            pass2_sum<float>(v, I, i, xi, grho, gx, gy);
+        } else {
+            const float invh = I.p.invh, m = I.p.m, Fc = I.p.Fc;
+            const float gri = grho[i];
+            float2 acc = make_float2(0.0f, 0.0f);
+            for_each_entry(L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n,
+                           [&](uint32_t o) {
+                               const float2 xj = lds2(sw, o);
+                               const float grj = lds1(sw + kWin8, o >> 1);
+                               const float2 d = fsub2(xi, xj);
+                               const float r2 = d.x * d.x + d.y * d.y;
+                               const float w = pass2_weight<float>(r2, invh, m, Fc, gri, grj);
+                               acc = ffma2(make_float2(w, w), d, acc);
+                           });
+            gx = acc.x;
+            gy = acc.y;
+        }
+    }
+    pass2_finish_warp<float>(live, I, b, i, xi, gx, gy, gXs, gX, galpha, emax, parity, thetaAcc);
+}
+
+// adj_pass2_kernel! + _axpy2!(gX, gXs) + the exact theta write-back
+template <bool MULTI>
+__global__ void __launch_bounds__(kTile, 14)
+    k_pass2_win(const __grid_constant__ NLView<float> v, const WinLists L,
+                const float *__restrict__ grho, const float2 *__restrict__ gXs,
+                float2 *__restrict__ gX, const float *__restrict__ galpha,
+                const int *__restrict__ emax, int parity,
+                unsigned long long *__restrict__ thetaAcc)
+{
+    pdl_enter();
+    __shared__ __align__(16) unsigned char s_win[kWin8 + kWin4];
+    pass2_window<MULTI>(v, L, (int)blockIdx.x, s_win, grho, gXs, gX, galpha, emax,
+                        parity, thetaAcc);
+}
+
+} // namespace sphgb
