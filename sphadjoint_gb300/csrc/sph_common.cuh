@@ -12,6 +12,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sph_exact64.cuh"
+
 namespace sphgb {
 
 template <typename T> struct vec2;
@@ -293,11 +295,11 @@ __device__ __forceinline__ void for_each_neighbor(const NLView<T> &v, const Inst
     }
 }
 
-// Per-pair square root and reciprocal. FP64 keeps IEEE sqrt and division
-// (reference-exact); FP32 uses the PTX approximate square root (one
+// Per-pair square root. FP64 keeps the IEEE result (reference-exact), computed
+// off the FP64 pipe (sph_exact64.cuh, as are the FP64 divisions); FP32 uses the PTX approximate square root (one
 // instruction, sqrt(+0) = +0, within a few ulp; the FP32 path is checked
 // against FP64 by tolerance).
-__device__ __forceinline__ double pair_sqrt(double r2) { return sqrt(r2); }
+__device__ __forceinline__ double pair_sqrt(double r2) { return sqrt_rn(r2); }
 __device__ __forceinline__ float pair_sqrt(float r2)
 {
     float r;
@@ -337,8 +339,8 @@ template <typename T>
 __device__ __forceinline__ void interp_cell(T x, T y, const Phys<T> &p, int &i0, int &j0, T &fx,
                                             T &fy, T &ax, T &ay)
 {
-    const T gx = x / p.hxg;
-    const T gy = y / p.hyg;
+    const T gx = div_rn(x, p.hxg);
+    const T gy = div_rn(y, p.hyg);
     ax = ((gx > (T)0) & (gx < p.ngx1)) ? (T)1 : (T)0;
     ay = ((gy > (T)0) & (gy < p.ngy1)) ? (T)1 : (T)0;
     const T gxc = gx > p.gxmax ? p.gxmax : (gx < (T)0 ? (T)0 : gx);
@@ -369,8 +371,8 @@ __device__ __forceinline__ void interp_alpha(const T *theta, T x, T y, const Phy
     const T t11 = __ldg(theta + l00 + p.ngy + 1);
     a = ((T)1 - fx) * ((T)1 - fy) * t00 + fx * ((T)1 - fy) * t01 + ((T)1 - fx) * fy * t10 +
         fx * fy * t11;
-    dadx = (((T)1 - fy) * (t01 - t00) + fy * (t11 - t10)) / p.hxg * ax;
-    dady = (((T)1 - fx) * (t10 - t00) + fx * (t11 - t01)) / p.hyg * ay;
+    dadx = div_rn(((T)1 - fy) * (t01 - t00) + fy * (t11 - t10), p.hxg) * ax;
+    dady = div_rn(((T)1 - fx) * (t10 - t00) + fx * (t11 - t01), p.hyg) * ay;
 }
 
 template <typename T> __device__ __forceinline__ T interp_alpha_value(const T *theta, T x, T y,

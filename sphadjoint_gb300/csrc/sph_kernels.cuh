@@ -197,8 +197,8 @@ __global__ void k_assign(int64_t N, const T2<T> *__restrict__ pos, const T2<T> *
             if (d2 > I.dmax2) atomicOr(flags + b, FLAG_DISPLACEMENT);
         }
         const T cs = I.cs;
-        const int cx = cell_coord<T>(x.x / cs, I.nx);
-        const int cy = cell_coord<T>(x.y / cs, I.ny);
+        const int cx = cell_coord<T>(div_rn(x.x, cs), I.nx);
+        const int cy = cell_coord<T>(div_rn(x.y, cs), I.ny);
         c = I.coff + (cx - 1) + (cy - 1) * I.nx;
         cellTmp[i] = c;
     }
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(kRebuildSmallThreads)
             const T d2 = r2_exact<T>(sub_rn(x.x, xr.x), sub_rn(x.y, xr.y));
             moved = moved || d2 > I.dmax2;
         }
-        const int cx = cell_coord<T>(x.x / I.cs, I.nx);
-        const int cy = cell_coord<T>(x.y / I.cs, I.ny);
+        const int cx = cell_coord<T>(div_rn(x.x, I.cs), I.nx);
+        const int cy = cell_coord<T>(div_rn(x.y, I.cs), I.ny);
         const int c = I.coff + (cx - 1) + (cy - 1) * I.nx;
         cellOf[i] = c;
         atomicAdd(&cursor[c], 1);
@@ -566,7 +566,7 @@ __device__ __forceinline__ AccelPair<T> accel_pair(T r2, T dx, T dy, T invh, T m
         if (s < (T)0) {
             const T D = r2 + vc.eh2;
             const T rb = half_of(rhoi + rhoj);
-            K = vc.avc * s * F / (D * rb);
+            K = div_rn(vc.avc * s * F, D * rb);
         }
         o.cx = K * dx;
         o.cy = K * dy;
@@ -655,7 +655,7 @@ __device__ __forceinline__ Pass1Pair<T> pass1_pair(T r2, T dx, T dy, T invh, T m
         rinv = r2 > (T)0 ? rsqrtf(r2) : (T)0;
         r = r2 * rinv;
     } else {
-        r = sqrt(r2);
+        r = pair_sqrt(r2);
     }
     const T q = r * invh;
     const T u = (T)1 - half_of(q);
@@ -678,24 +678,24 @@ __device__ __forceinline__ Pass1Pair<T> pass1_pair(T r2, T dx, T dy, T invh, T m
         const T Fbar = Pij * ad_d;
         T w;
         if constexpr (sizeof(T) == 4) w = Fbar * G * invh * rinv;
-        else w = Fbar * G * invh / r;
+        else w = div_rn(Fbar * G * invh, r);
         const T Ad = dax * dx + day * dy;
         T avx = (T)0, avy = (T)0, vx = (T)0, vy = (T)0, rs = (T)0;
         if (s < (T)0) {
             const T D = r2 + vc.eh2;
             const T rb = half_of(rhoi + rhoj);
             const T Drb = D * rb;
-            const T K = vc.avc * s * F / Drb;
-            const T Ks = vc.avc * F / Drb;
-            const T KF = vc.avc * s / Drb;
+            const T K = div_rn(vc.avc * s * F, Drb);
+            const T Ks = div_rn(vc.avc * F, Drb);
+            const T KF = div_rn(vc.avc * s, Drb);
             T cd;
-            if constexpr (sizeof(T) == 4) cd = Ad * (KF * G * invh * rinv - twice_of(K) / D);
-            else cd = Ad * (KF * G * invh / r - twice_of(K) / D);
+            if constexpr (sizeof(T) == 4) cd = Ad * (KF * G * invh * rinv - div_rn(twice_of(K), D));
+            else cd = Ad * (div_rn(KF * G * invh, r) - div_rn(twice_of(K), D));
             avx = K * dax + Ad * Ks * dvx + cd * dx;
             avy = K * day + Ad * Ks * dvy + cd * dy;
             vx = Ad * Ks * dx;
             vy = Ad * Ks * dy;
-            rs = Ad * K / twice_of(rb);
+            rs = div_rn(Ad * K, twice_of(rb));
         }
         o.gxa = w * dx + avx;
         o.gya = w * dy + avy;
@@ -708,7 +708,7 @@ __device__ __forceinline__ Pass1Pair<T> pass1_pair(T r2, T dx, T dy, T invh, T m
     const T Fbar = Pij * ad_d + Cbase * ad_v;
     T w;
     if constexpr (sizeof(T) == 4) w = Fbar * G * invh * rinv;
-    else w = Fbar * G * invh / r;
+    else w = div_rn(Fbar * G * invh, r);
     o.gxa = w * dx;
     o.gya = w * dy;
     o.gvx = C * dax;
@@ -759,9 +759,9 @@ __device__ __forceinline__ void density_finish(const IT &I, int64_t i, T acc, T 
     // (a multiply-add contraction here would depend on the surrounding code)
     const T ri = add_rn(acc, mul_rn(m, A));
     if (rho) rho[i] = ri;
-    const T inv = (T)1 / ri;
+    const T inv = div_rn((T)1, ri);
     T pt;
-    if (I.p.eos == 1) pt = I.p.B * pow1m<T>((ri - I.p.rho0) / I.p.rho0, I.p.gam) * inv * inv;
+    if (I.p.eos == 1) pt = I.p.B * pow1m<T>(div_rn(ri - I.p.rho0, I.p.rho0), I.p.gam) * inv * inv;
     else pt = I.p.c2 * (ri - I.p.rho0) * inv * inv;
     prho[i] = mk2<T>(pt, inv);
 }
@@ -1126,7 +1126,7 @@ __device__ __forceinline__ void accel_integrate_finish(
     if (aOut) aOut[i] = mk2<T>(ax, ay);
     if (alphaOut) alphaOut[i] = al;
     const T dt = p.dt;
-    const T D = (T)1 / ((T)1 + dt * al);
+    const T D = div_rn((T)1, (T)1 + dt * al);
     const T v1 = (vi.x + dt * ax) * D;
     const T v2 = (vi.y + dt * ay) * D;
     const T x1 = xi.x + dt * v1;
@@ -1209,7 +1209,7 @@ __device__ __forceinline__ int drag_adj_finish(const IT &I, int64_t i, const T2<
     T2<T> gv = gV[i];
     gv.x += dt * gx.x;
     gv.y += dt * gx.y;
-    const T D = (T)1 / ((T)1 + dt * al);
+    const T D = div_rn((T)1, (T)1 + dt * al);
     const T vx = (vi.x + dt * ax) * D;
     const T vy = (vi.y + dt * ay) * D;
     abar[i] = mk2<T>(dt * D * gv.x, dt * D * gv.y);
@@ -1393,7 +1393,7 @@ __device__ __forceinline__ void pass1_finish(const IT &I, int64_t i, const T2<T>
     const T pti = pi.x, iri = pi.y;
     const Phys<T> &p = I.p;
     grh += ((T)(-2) * p.m * pti * iri) * sumS;
-    if (p.eos == 1) grh += p.dB * pow_fold<T>(rhoi / p.rho0, p.gam - 1) * p.m * iri * iri * sumS;
+    if (p.eos == 1) grh += p.dB * pow_fold<T>(div_rn(rhoi, p.rho0), p.gam - 1) * p.m * iri * iri * sumS;
     else grh += p.c2 * p.m * iri * iri * sumS;
     gx += ab.x * wall_daccel<T>(xi.x, p.Lx, p.kw);
     gy += ab.y * wall_daccel<T>(xi.y, p.Ly, p.kw);
