@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "sph_coop.cuh"
+#include "sph_flat.cuh"
 #include "sph_iface.hpp"
 #include "sph_kernels.cuh"
 #include "sph_window.cuh"
@@ -147,6 +148,17 @@ template <typename T> int &tuned_block(int kid, bool multi)
             const int bs_ = ::sphgb::tuned_block<T>(kid, multi);                              \
             ::sphgb::rt_before_launch(kid);                                                   \
             ::sphgb::launch_k(kern, dim3((unsigned)(((n) + bs_ - 1) / bs_)), dim3(bs_), 0, __VA_ARGS__); \
+            ::sphgb::rt_after_launch(kid);                                                    \
+        }                                                                                     \
+    } while (0)
+
+// One block per P particles (sph_flat.cuh).
+#define SPH_LAUNCH_FLAT(kid, P, kern, n, ...)                                                 \
+    do {                                                                                      \
+        if ((n) > 0) {                                                                        \
+            ::sphgb::rt_before_launch(kid);                                                   \
+            ::sphgb::launch_k(kern, dim3((unsigned)(((n) + (P) - 1) / (P))),                   \
+                              dim3(::sphgb::kFlatBlock), 0, __VA_ARGS__);                      \
             ::sphgb::rt_after_launch(kid);                                                    \
         }                                                                                     \
     } while (0)
@@ -349,6 +361,9 @@ template <typename T> class Sys final : public StateI {
     DevBuf<TileWin> wwin; // windows and neighbour lists of the FP32 tile passes
     DevBuf<uint2> wcand, wsupp;
     DevBuf<uint8_t> wcnt; // candidate counts, then in-support counts
+    DevBuf<double> fF; // dense pairs of the FP64 flat passes
+    DevBuf<uint32_t> fpair;
+    DevBuf<int32_t> foff;
     bool listsTried = false; // the lists were asked for (and may have been refused)
     bool listsFresh = false; // they belong to the masks the state holds
     StepGraphs graphs;   // simulate's steps, replayed in groups
@@ -540,9 +555,33 @@ template <typename T> class Sys final : public StateI {
                rt_density_form() == 2;
     }
     bool tiles() const { return want_tiles() && wwin.p; }
+    // FP64 states without artificial viscosity run them one lane per pair
+    // (sph_flat.cuh), unless a lane setting is forced; their pair lists (about
+    // 770 bytes a particle) are scratch under the same rule.
+    static constexpr int64_t kFlatMaxN = int64_t(1) << 22;
+    bool want_flat() const
+    {
+        return sizeof(T) == 8 && N_ > 0 && N_ <= kFlatMaxN && rt_group_lanes() == 0;
+    }
+    bool flat() const { return want_flat() && !anyAV && foff.p; }
+    FlatLists flat_lists() const { return FlatLists{fF.p, fpair.p, foff.p, flat_particles(N_)}; }
     void reserve_lists()
     {
         if (want_tiles()) alloc_lists();
+        if (want_flat() && !listsTried && !rt_capturing()) {
+            listsTried = true;
+            const size_t P = (size_t)flat_particles(N_), nb = ((size_t)N_ + P - 1) / P;
+            if (rt_free_memory() / 8 < nb * (P * kFlatRow * 12 + 4 * kFlatOff)) return;
+            try {
+                fF.alloc(nb * P * kFlatRow);
+                fpair.alloc(nb * P * kFlatRow);
+                foff.alloc(nb * kFlatOff);
+            } catch (const Error &) {
+                fF.release();
+                fpair.release();
+                foff.release();
+            }
+        }
     }
     void alloc_lists()
     {
@@ -817,7 +856,16 @@ template <typename T> class Sys final : public StateI {
         const int nxt = 1 - cur;
         T2<T> *aO = keepAccel ? accOut.p : (T2<T> *)nullptr;
         T *alO = keepAccel ? alphaOut.p : (T *)nullptr;
-        if (const int G = group_lanes()) {
+        if (flat()) {
+            if constexpr (sizeof(T) == 8) {
+                const FlatLists W = flat_lists();
+                auto kd = B > 1 ? &k_density_flat<true> : &k_density_flat<false>;
+                auto ki = B > 1 ? &k_accel_flat<true> : &k_accel_flat<false>;
+                SPH_LAUNCH_FLAT(K_DENSITY, W.P, kd, N_, v, W, rho.p, prho.p);
+                SPH_LAUNCH_FLAT(K_ACCEL_INTEGRATE, W.P, ki, N_, v, W, vel[cur].p, prho.p, theta,
+                                pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
+            }
+        } else if (const int G = group_lanes()) {
             auto kd = G == 32 ? &k_density_eos_coop<T, 32> : &k_density_eos_coop<T, 16>;
             SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p);
             v.tmask = tmask.p;
@@ -1348,6 +1396,25 @@ template <typename T> class Work final : public WorkI {
         NLView<T> v = S.view();
         const T2<T> *vel = S.vel[S.cur].p;
         T *rhoOut = S.anyRho ? S.rho.p : (T *)nullptr; // densities only where the model reads them
+        if (S.flat()) {
+            if constexpr (sizeof(T) == 8) {
+                const FlatLists W = S.flat_lists();
+                const bool multi = S.B > 1;
+                auto kd = multi ? &k_density_flat<true> : &k_density_flat<false>;
+                auto ka = multi ? &k_drag_flat<true> : &k_drag_flat<false>;
+                auto k1 = multi ? &k_pass1_flat<true> : &k_pass1_flat<false>;
+                auto k2 = multi ? &k_pass2_flat<true> : &k_pass2_flat<false>;
+                SPH_LAUNCH_FLAT(K_DENSITY, W.P, kd, N_, v, W, rhoOut, S.prho.p);
+                SPH_LAUNCH_FLAT(K_ACCEL_DRAG, W.P, ka, N_, v, W, vel, S.prho.p, theta, gX[gcur].p,
+                                gV[gcur].p, abar.p, galpha.p, emax.p, parity);
+                SPH_LAUNCH_FLAT(K_PASS1, W.P, k1, N_, v, W, vel, S.prho.p, S.rho.p, theta, abar.p,
+                                galpha.p, gXs.p, grho.p, gV[gcur].p);
+                SPH_LAUNCH_FLAT(K_PASS2, W.P, k2, N_, v, W, grho.p, gXs.p, gX[gcur].p, galpha.p,
+                                emax.p, parity, thetaAcc.p);
+            }
+            pendingTheta = parity;
+            return;
+        }
         if (const int G = S.group_lanes()) {
             const bool g32 = G == 32;
             auto kd = g32 ? &k_density_eos_coop<T, 32> : &k_density_eos_coop<T, 16>;
