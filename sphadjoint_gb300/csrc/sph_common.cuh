@@ -319,6 +319,35 @@ template <typename T> __host__ __device__ __forceinline__ int cell_coord(T v, in
     return c > n ? n : c;
 }
 
+// cell_coord of the rounded quotient x / cs (cs > 0). FP64 takes a float
+// estimate of the quotient first: the positions' significands cut to 24 bits and
+// an approximate float division are within 2^-20 of it, so unless that leaves
+// an integer within reach the floor is already known and the division (some
+// hundred integer instructions, div_rn) is not needed. The estimate is off the
+// FP64 pipe. Non-finite, subnormal and out-of-range values take the division.
+__device__ __forceinline__ int cell_div(float x, float cs, int n)
+{
+    return cell_coord<float>(x / cs, n);
+}
+__device__ __forceinline__ int cell_div(double x, double cs, int n)
+{
+    const uint64_t a = ex_bits(x), b = ex_bits(cs);
+    const uint32_t ea = (uint32_t)(a >> 52) & 0x7ffu, eb = (uint32_t)(b >> 52) & 0x7ffu;
+    if (ea - 923u < 200u && eb - 923u < 200u) { // both within 2^-100 .. 2^100
+        const float xf = ex_float((uint32_t)(a >> 32) & 0x80000000u | (ea - 896u) << 23 |
+                                  (uint32_t)(a >> 29) & 0x007fffffu);
+        const float cf = ex_float((eb - 896u) << 23 | (uint32_t)(b >> 29) & 0x007fffffu);
+        const float q = __fdividef(xf, cf);
+        const float tol = 1e-6f * fabsf(q) + 1e-30f, f = floorf(q);
+        if (fabsf(q) < 1e6f && q - f > tol && f + 1.0f - q > tol) {
+            int c = (int)f + 2;
+            c = c < 1 ? 1 : c;
+            return c > n ? n : c;
+        }
+    }
+    return cell_coord<double>(div_rn(x, cs), n);
+}
+
 // wall_accel / wall_daccel (src/params.jl:36-46); max(zero(T), -x) keeps +0.
 template <typename T> __device__ __forceinline__ T wall_accel(T x, T L, T kw)
 {

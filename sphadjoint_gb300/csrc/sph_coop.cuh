@@ -229,9 +229,11 @@ __global__ void __launch_bounds__(kCoopBlock)
 template <typename T, int G>
 __global__ void __launch_bounds__(kCoopBlock)
     k_density_eos_coop(const __grid_constant__ NLView<T> v, T *__restrict__ rho,
-                       T2<T> *__restrict__ prho, uint32_t *__restrict__ tmaskOut)
+                       T2<T> *__restrict__ prho, uint32_t *__restrict__ tmaskOut,
+                       const ThetaFlush<T> flush)
 {
     pdl_enter();
+    if (theta_flush<T>(flush)) return;
     constexpr int NG = kCoopBlock / G;
     __shared__ T buf[NG][G];
     __shared__ uint32_t tws[NG][6];
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(kCoopBlock)
     k_pass2_axpy_coop(const __grid_constant__ NLView<T> v, const T *__restrict__ grho,
                       const T2<T> *__restrict__ gXs, T2<T> *__restrict__ gX,
                       const T *__restrict__ galpha, const int *__restrict__ emax, int parity,
-                      unsigned long long *__restrict__ thetaAcc)
+                      unsigned long long *__restrict__ thetaAcc, NextState<T> next)
 {
     pdl_enter();
     constexpr int NG = kCoopBlock / G;
@@ -537,6 +539,8 @@ __global__ void __launch_bounds__(kCoopBlock)
     const Group<G> g;
     const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
     if (i >= v.N) return;
+    const bool loader = g.gl == G - 1; // a lane with nothing to fold
+    if (loader) next.read(i);
     const Inst<T> &I = v.one;
     const T r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, Fc = I.p.Fc;
     const T2<T> xi = v.pos[i];
@@ -544,6 +548,7 @@ __global__ void __launch_bounds__(kCoopBlock)
     const uint32_t cc = v.center[i];
     T gx = (T)0, gy = (T)0;
     if ((cc >> 31) && I.maxnb > kSpillList) {
+        if (loader) next.write(i);
         if (g.gl != 0) return;
         for_each_neighbor<T>(v, I, i, [&](int j) {
             const T2<T> xj = v.pos[j];
@@ -592,6 +597,7 @@ __global__ void __launch_bounds__(kCoopBlock)
         }
         gx = acc;
         gy = g.from(acc, 1);
+        if (loader) next.write(i);
         if (g.gl != 0) return;
     }
     pass2_finish<T>(I, 0, i, xi, gx, gy, gXs, gX, galpha, emax, parity, thetaAcc);

@@ -153,11 +153,12 @@ template <typename T> int &tuned_block(int kid, bool multi)
     } while (0)
 
 // One block per P particles (sph_flat.cuh).
-#define SPH_LAUNCH_FLAT(kid, P, kern, n, ...)                                                 \
+#define SPH_LAUNCH_FLAT(kid, P, kern, n, ...) SPH_LAUNCH_FLAT_X(kid, P, 0, kern, n, __VA_ARGS__)
+#define SPH_LAUNCH_FLAT_X(kid, P, extra, kern, n, ...)                                        \
     do {                                                                                      \
         if ((n) > 0) {                                                                        \
             ::sphgb::rt_before_launch(kid);                                                   \
-            ::sphgb::launch_k(kern, dim3((unsigned)(((n) + (P) - 1) / (P))),                   \
+            ::sphgb::launch_k(kern, dim3((unsigned)(((n) + (P) - 1) / (P)) + (extra)),         \
                               dim3(::sphgb::kFlatBlock), 0, __VA_ARGS__);                      \
             ::sphgb::rt_after_launch(kid);                                                    \
         }                                                                                     \
@@ -184,13 +185,14 @@ template <typename T> int &tuned_block(int kid, bool multi)
     } while (0)
 
 // Group-per-particle launch: kCoopBlock threads, kCoopBlock / G particles per
-// block.
-#define SPH_LAUNCH_COOP(kid, G, kern, n, ...)                                                \
+// block. The _X forms launch extra blocks behind the particles' ones.
+#define SPH_LAUNCH_COOP(kid, G, kern, n, ...) SPH_LAUNCH_COOP_X(kid, G, 0, kern, n, __VA_ARGS__)
+#define SPH_LAUNCH_COOP_X(kid, G, extra, kern, n, ...)                                        \
     do {                                                                                      \
         if ((n) > 0) {                                                                        \
             const int per_ = ::sphgb::kCoopBlock / (G);                                       \
             ::sphgb::rt_before_launch(kid);                                                   \
-            ::sphgb::launch_k(kern, dim3((unsigned)(((n) + per_ - 1) / per_)),                 \
+            ::sphgb::launch_k(kern, dim3((unsigned)(((n) + per_ - 1) / per_) + (extra)),       \
                               dim3(::sphgb::kCoopBlock), 0, __VA_ARGS__);                       \
             ::sphgb::rt_after_launch(kid);                                                    \
         }                                                                                     \
@@ -508,9 +510,9 @@ template <typename T> class Sys final : public StateI {
         masks.zero();
         center.zero();
         cellStart.zero();
-        if (sizeof(T) == 4) {
-            // the one-launch cell list of small FP32 states (set here, outside
-            // any graph recording)
+        {
+            // the one-launch cell list of small states (set here, outside any
+            // graph recording)
             static bool attr = false;
             if (!attr) {
                 SPH_CK(cudaFuncSetAttribute(k_rebuild_small<T>,
@@ -751,12 +753,11 @@ template <typename T> class Sys final : public StateI {
                  T2<T> *ex1N = nullptr)
     {
         const int check = age != INT64_MAX ? 1 : 0;
-        if (sizeof(T) == 4 && N_ > 0 && B == 1 && N_ <= kRebuildSmallMaxN &&
-            ncell <= kRebuildSmallMaxCells) {
-            // small single FP32 state: the cell list in one launch (the
-            // reference's GPU optimisation set-up, 1500 particles, runs 12%
-            // faster; in FP64 the one block's double-precision cell
-            // coordinates cost more than the launches saved)
+        if (N_ > 0 && B == 1 && N_ <= kRebuildSmallMaxN && ncell <= kRebuildSmallMaxCells) {
+            // small single state: the cell list in one launch (the
+            // reference's GPU optimisation set-up, 1500 FP32 particles, runs 12%
+            // faster; in FP64 the cell coordinates' divisions run on the integer
+            // pipes, div_rn)
             const int nxt = 1 - cur;
             const size_t smem = sizeof(int32_t) * (size_t)(2 * ncell + 1 + 3 * N_);
             rt_before_launch(K_RANK);
@@ -845,6 +846,13 @@ template <typename T> class Sys final : public StateI {
         if (did) *did = r;
     }
 
+    static ThetaFlush<T> no_flush()
+    {
+        ThetaFlush<T> f{};
+        f.first = UINT_MAX;
+        return f;
+    }
+
     // step! (src/forward.jl:161-173); tx/tv: optional tape slot (id order)
     void step_impl(const T *theta, T2<T> *tx, T2<T> *tv)
     {
@@ -861,13 +869,13 @@ template <typename T> class Sys final : public StateI {
                 const FlatLists W = flat_lists();
                 auto kd = B > 1 ? &k_density_flat<true> : &k_density_flat<false>;
                 auto ki = B > 1 ? &k_accel_flat<true> : &k_accel_flat<false>;
-                SPH_LAUNCH_FLAT(K_DENSITY, W.P, kd, N_, v, W, rho.p, prho.p);
+                SPH_LAUNCH_FLAT(K_DENSITY, W.P, kd, N_, v, W, rho.p, prho.p, no_flush());
                 SPH_LAUNCH_FLAT(K_ACCEL_INTEGRATE, W.P, ki, N_, v, W, vel[cur].p, prho.p, theta,
                                 pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
             }
         } else if (const int G = group_lanes()) {
             auto kd = G == 32 ? &k_density_eos_coop<T, 32> : &k_density_eos_coop<T, 16>;
-            SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p);
+            SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush());
             v.tmask = tmask.p;
             auto ki = G == 32 ? &k_accel_integrate_coop<T, 32> : &k_accel_integrate_coop<T, 16>;
             SPH_LAUNCH_COOP(K_ACCEL_INTEGRATE, G, ki, N_, v, vel[cur].p, prho.p, rho.p, theta,
@@ -1371,10 +1379,41 @@ template <typename T> class Work final : public WorkI {
         pendingTheta = -1;
     }
 
-    void reverse_step(Sys<T> &S, const T *theta, const T2<T> *sx, const T2<T> *sv,
-                      const int32_t *srcInv, int parity)
+    // nsx, nsv: the full tape's state of the next reverse step (NULL when there is
+    // none or it is not recorded), which this step's pass 2 loads where launches
+    // count (NextState); the deferred design-node write-back then rides on the
+    // next step's density launch.
+    bool nextLoaded = false;
+
+    // the pending design-node write-back as blocks from `first` on (128 threads)
+    ThetaFlush<T> take_flush(Sys<T> &S, int64_t first, unsigned &extra)
     {
-        if (pendingTheta >= 0 && N_ > 0) {
+        ThetaFlush<T> f = Sys<T>::no_flush();
+        extra = 0;
+        if (pendingTheta < 0) return f;
+        f.first = (unsigned)first;
+        f.parity = pendingTheta;
+        f.B = S.B;
+        f.nnode = nnode;
+        f.inst = S.dinst.p;
+        f.acc = thetaAcc.p;
+        f.emax = emax.p;
+        f.gtheta = gtheta.p;
+        extra = (unsigned)((nnode + 127) / 128);
+        pendingTheta = -1;
+        return f;
+    }
+
+    void reverse_step(Sys<T> &S, const T *theta, const T2<T> *sx, const T2<T> *sv,
+                      const int32_t *srcInv, int parity, const T2<T> *nsx = nullptr,
+                      const T2<T> *nsv = nullptr)
+    {
+        // the forms below that launch per particle of a small or an FP64 state
+        const bool carries = N_ > 0 && (S.flat() || S.group_lanes());
+        if (nextLoaded) {
+            S.cur = 1 - S.cur;
+            if (!carries) flush_theta(S);
+        } else if (pendingTheta >= 0 && N_ > 0) {
             const unsigned gN = grid_for(N_);
             const unsigned gT = grid_for(nnode);
             rt_before_launch(K_GATHER);
@@ -1396,6 +1435,17 @@ template <typename T> class Work final : public WorkI {
         NLView<T> v = S.view();
         const T2<T> *vel = S.vel[S.cur].p;
         T *rhoOut = S.anyRho ? S.rho.p : (T *)nullptr; // densities only where the model reads them
+        const int nb = 1 - S.cur;
+        NextState<T> next{};
+        nextLoaded = nsx && carries;
+        if (nextLoaded) {
+            next.perm = S.perm.p;
+            next.sx = nsx;
+            next.sv = nsv;
+            next.pos = S.pos[nb].p;
+            next.vel = S.vel[nb].p;
+        }
+        unsigned extra = 0;
         if (S.flat()) {
             if constexpr (sizeof(T) == 8) {
                 const FlatLists W = S.flat_lists();
@@ -1404,13 +1454,14 @@ template <typename T> class Work final : public WorkI {
                 auto ka = multi ? &k_drag_flat<true> : &k_drag_flat<false>;
                 auto k1 = multi ? &k_pass1_flat<true> : &k_pass1_flat<false>;
                 auto k2 = multi ? &k_pass2_flat<true> : &k_pass2_flat<false>;
-                SPH_LAUNCH_FLAT(K_DENSITY, W.P, kd, N_, v, W, rhoOut, S.prho.p);
+                const ThetaFlush<T> fl = take_flush(S, (N_ + W.P - 1) / W.P, extra);
+                SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, extra, kd, N_, v, W, rhoOut, S.prho.p, fl);
                 SPH_LAUNCH_FLAT(K_ACCEL_DRAG, W.P, ka, N_, v, W, vel, S.prho.p, theta, gX[gcur].p,
                                 gV[gcur].p, abar.p, galpha.p, emax.p, parity);
                 SPH_LAUNCH_FLAT(K_PASS1, W.P, k1, N_, v, W, vel, S.prho.p, S.rho.p, theta, abar.p,
                                 galpha.p, gXs.p, grho.p, gV[gcur].p);
                 SPH_LAUNCH_FLAT(K_PASS2, W.P, k2, N_, v, W, grho.p, gXs.p, gX[gcur].p, galpha.p,
-                                emax.p, parity, thetaAcc.p);
+                                emax.p, parity, thetaAcc.p, next);
             }
             pendingTheta = parity;
             return;
@@ -1421,14 +1472,16 @@ template <typename T> class Work final : public WorkI {
             auto ka = g32 ? &k_accel_drag_adj_coop<T, 32> : &k_accel_drag_adj_coop<T, 16>;
             auto k1 = g32 ? &k_pass1_design_coop<T, 32> : &k_pass1_design_coop<T, 16>;
             auto k2 = g32 ? &k_pass2_axpy_coop<T, 32> : &k_pass2_axpy_coop<T, 16>;
-            SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rhoOut, S.prho.p, S.tmask.p);
+            const int per = kCoopBlock / G;
+            const ThetaFlush<T> fl = take_flush(S, (N_ + per - 1) / per, extra);
+            SPH_LAUNCH_COOP_X(K_DENSITY, G, extra, kd, N_, v, rhoOut, S.prho.p, S.tmask.p, fl);
             v.tmask = S.tmask.p;
             SPH_LAUNCH_COOP(K_ACCEL_DRAG, G, ka, N_, v, vel, S.prho.p, S.rho.p, theta, gX[gcur].p,
                             gV[gcur].p, abar.p, galpha.p, emax.p, parity);
             SPH_LAUNCH_COOP(K_PASS1, G, k1, N_, v, vel, S.prho.p, S.rho.p, theta, abar.p,
                             galpha.p, gXs.p, grho.p, gV[gcur].p);
             SPH_LAUNCH_COOP(K_PASS2, G, k2, N_, v, grho.p, gXs.p, gX[gcur].p, galpha.p, emax.p,
-                            parity, thetaAcc.p);
+                            parity, thetaAcc.p, next);
             pendingTheta = parity;
             return;
         }
@@ -1753,6 +1806,7 @@ void Work<T>::run_backward(TapeI *tape, FieldI *theta, const Params *pp, const v
 
     const int64_t L = tp->n_;
     pendingTheta = -1;
+    nextLoaded = false;
     int64_t rstep = 0; // reverse steps done (parity of the exponent slot)
     tp->fwdSteps = 0;
     // reverse steps and recomputed forward steps go out in recorded groups
@@ -1765,8 +1819,9 @@ void Work<T>::run_backward(TapeI *tape, FieldI *theta, const Params *pp, const v
     if (tp->nsnap_ == 0) {
         for (int64_t n = L - 1; n >= 0; --n) {
             graphs.before_step();
-            reverse_step(*S, th->th.p, tp->hx.p + (size_t)n * N_, tp->hv.p + (size_t)n * N_,
-                         nullptr, (int)(rstep & 1));
+            const size_t at = (size_t)n * N_, before = (size_t)(n - 1) * N_;
+            reverse_step(*S, th->th.p, tp->hx.p + at, tp->hv.p + at, nullptr, (int)(rstep & 1),
+                         n > 0 ? tp->hx.p + before : nullptr, n > 0 ? tp->hv.p + before : nullptr);
             ++rstep;
             graphs.after_step();
         }

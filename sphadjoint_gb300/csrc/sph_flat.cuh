@@ -86,9 +86,11 @@ __device__ __forceinline__ int flat_scan(int x, int *s_warp, int &tot)
 template <bool MULTI>
 __global__ void __launch_bounds__(kFlatBlock)
     k_density_flat(const __grid_constant__ NLView<double> v, const FlatLists B,
-                   double *__restrict__ rho, double2 *__restrict__ prho)
+                   double *__restrict__ rho, double2 *__restrict__ prho,
+                   const ThetaFlush<double> flush)
 {
     pdl_enter();
+    if (theta_flush<double>(flush)) return;
     __shared__ double s_r2[kFlatMax * kFlatRow];
     __shared__ int32_t s_lst[kFlatMax][kFlatRow]; // rows of spilled particles
     __shared__ uint32_t s_wd[kFlatMax][6];
@@ -481,7 +483,7 @@ __global__ void __launch_bounds__(kFlatBlock)
                  const double *__restrict__ grho, const double2 *__restrict__ gXs,
                  double2 *__restrict__ gX, const double *__restrict__ galpha,
                  const int *__restrict__ emax, int parity,
-                 unsigned long long *__restrict__ thetaAcc)
+                 unsigned long long *__restrict__ thetaAcc, NextState<double> next)
 {
     pdl_enter();
     __shared__ double s_t[2][kFlatChunk], s_acc[2 * kFlatMax];
@@ -491,6 +493,8 @@ __global__ void __launch_bounds__(kFlatBlock)
     const int64_t i0 = (int64_t)blockIdx.x * B.P, bb = i0 * kFlatRow;
     const int np = v.N - i0 < B.P ? (int)(v.N - i0) : B.P;
     flat_offsets(B, np, s_off, &s_serial);
+    const int nt = kFlatBlock - 1 - t; // the last threads load the next state
+    if (nt < np) next.read(i0 + nt);
     __syncthreads();
     const int n = s_off[np], a2 = t >> 1, c2 = t & 1;
     const int b0 = a2 < np ? s_off[a2] : 0, b1 = a2 < np ? s_off[a2 + 1] : 0;
@@ -517,6 +521,7 @@ __global__ void __launch_bounds__(kFlatBlock)
         __syncthreads();
     }
     if (a2 < np) s_acc[t] = acc;
+    if (nt < np) next.write(i0 + nt);
     __syncthreads();
     if (t >= 32) return;
     const bool live = t < np;

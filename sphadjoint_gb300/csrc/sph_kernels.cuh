@@ -197,8 +197,8 @@ __global__ void k_assign(int64_t N, const T2<T> *__restrict__ pos, const T2<T> *
             if (d2 > I.dmax2) atomicOr(flags + b, FLAG_DISPLACEMENT);
         }
         const T cs = I.cs;
-        const int cx = cell_coord<T>(div_rn(x.x, cs), I.nx);
-        const int cy = cell_coord<T>(div_rn(x.y, cs), I.ny);
+        const int cx = cell_div(x.x, cs, I.nx);
+        const int cy = cell_div(x.y, cs, I.ny);
         c = I.coff + (cx - 1) + (cy - 1) * I.nx;
         cellTmp[i] = c;
     }
@@ -266,7 +266,7 @@ __global__ void k_rank_permute(int64_t N, const int32_t *__restrict__ cellTmp,
     if (ex1) ex1N[dst] = ex1[src];
 }
 
-// The whole cell-list rebuild of a small single FP32 state in one block: cells
+// The whole cell-list rebuild of a small single state in one block: cells
 // and the displacement check (k_assign), the exclusive scan (k_scan_*), the
 // bucket and the in-cell rank by particle id (k_bucket, k_rank_permute), with
 // the histogram, scan and buckets in shared memory. Same arithmetic and the
@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(kRebuildSmallThreads)
             const T d2 = r2_exact<T>(sub_rn(x.x, xr.x), sub_rn(x.y, xr.y));
             moved = moved || d2 > I.dmax2;
         }
-        const int cx = cell_coord<T>(div_rn(x.x, I.cs), I.nx);
-        const int cy = cell_coord<T>(div_rn(x.y, I.cs), I.ny);
+        const int cx = cell_div(x.x, I.cs, I.nx);
+        const int cy = cell_div(x.y, I.cs, I.ny);
         const int c = I.coff + (cx - 1) + (cy - 1) * I.nx;
         cellOf[i] = c;
         atomicAdd(&cursor[c], 1);
@@ -1553,6 +1553,34 @@ __device__ __forceinline__ void pass2_sum(const NLView<T> &v, const IT &I, int64
                                           const T2<T> &xi, const T *__restrict__ grho, T &gx,
                                           T &gy);
 
+// _tape_load! of the next reverse step, done by pass 2 of this one: slot i of the
+// state's other buffers takes particle perm[i] of the tape (pos NULL: no next
+// step on a full tape). For states whose passes take little more than their
+// launch (lane groups, FP64 pairs): 128 steps of 2072 FP64 particles 9.2 -> 8.6
+// ms. FP32 tiles keep the gather launch: inside pass 2 it cost 3.0 us at 249k
+// particles, as much as the launch.
+template <typename T> struct NextState {
+    const int32_t *perm;
+    const T2<T> *sx, *sv;
+    T2<T> *pos, *vel;
+    // read early, write late: a store right behind the two dependent loads would
+    // hold the thread up for their latency
+    T2<T> x, v;
+    __device__ __forceinline__ void read(int64_t i)
+    {
+        if (!pos) return;
+        const int32_t id = perm[i];
+        x = sx[id];
+        v = sv[id];
+    }
+    __device__ __forceinline__ void write(int64_t i) const
+    {
+        if (!pos) return;
+        pos[i] = x;
+        vel[i] = v;
+    }
+};
+
 // adj_pass2_kernel! (src/adjoint.jl:126-156) + _axpy2!(gX, gXs) + the theta
 // write-back of adj_design_kernel! (src/adjoint.jl:177-184), done as an exact
 // deterministic reduction keyed by design node instead of float atomics.
@@ -1714,6 +1742,26 @@ __device__ __forceinline__ void theta_node(int64_t n, int64_t nnode, int B,
         gtheta[n] += ldexp(vv, -theta_scale(em, inst[b].lgN));
     }
     if (n < B) emax[2 * n + (1 - parity)] = INT_MIN;
+}
+
+// The design-node write-back of the previous reverse step as extra blocks of a
+// density launch (blocks from `first` on): the pass that follows a reverse
+// step's last one and precedes the next use of the exponent slots.
+template <typename T> struct ThetaFlush {
+    unsigned first; // UINT_MAX: none
+    int parity, B;
+    int64_t nnode;
+    const Inst<T> *inst;
+    unsigned long long *acc;
+    int *emax;
+    double *gtheta;
+};
+template <typename T> __device__ __forceinline__ bool theta_flush(const ThetaFlush<T> &f)
+{
+    if (blockIdx.x < f.first) return false;
+    theta_node<T>((int64_t)(blockIdx.x - f.first) * blockDim.x + threadIdx.x, f.nnode, f.B, f.inst,
+                  f.acc, f.emax, f.parity, f.gtheta);
+    return true;
 }
 
 template <typename T>

@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(kPackBlock) g_assign(int l)
             if (d2 > I.dmax2) atomicOr(d.flags, FLAG_DISPLACEMENT);
         }
         const T cs = I.cs;
-        const int cx = cell_coord<T>(div_rn(x.x, cs), I.nx);
-        const int cy = cell_coord<T>(div_rn(x.y, cs), I.ny);
+        const int cx = cell_div(x.x, cs, I.nx);
+        const int cy = cell_div(x.y, cs, I.ny);
         c = (cx - 1) + (cy - 1) * I.nx;
         d.cellTmp[i] = c;
     }
