@@ -833,8 +833,9 @@ def set_launch_overlap(on: bool) -> None:
 
 def set_step_graphs(steps: int) -> None:
     """Steps per recorded group (no counterpart in the reference),
-    process-wide: simulate and backward record the launches of this many
-    consecutive steps and replay each group as one CUDA graph (default 32;
+    process-wide: simulate and backward record the launches of up to this many
+    consecutive steps and replay each group as one CUDA graph (default 32; a
+    call's first groups are shorter, so that the device starts early;
     0 launches every kernel on its own). Results do not depend on it."""
     L.check(L.load().sph_set_step_graphs(int(steps)))
 

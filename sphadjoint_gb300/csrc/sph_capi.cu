@@ -168,6 +168,7 @@ StepGraphs::~StepGraphs()
 void StepGraphs::start(bool eligible)
 {
     per_ = rt_step_graph();
+    now_ = std::min(per_, kFirst);
     on_ = eligible && per_ > 0 && !rt_capturing() && !rt_timers_on();
     if (on_) {
         // a stream the caller records with the CUDA API itself: its launches
@@ -199,7 +200,9 @@ void StepGraphs::before_step()
 void StepGraphs::after_step()
 {
     if (!open_) return;
-    if (++count_ >= per_) replay();
+    if (++count_ < now_) return;
+    replay();
+    now_ = std::min(per_, 2 * now_);
 }
 
 void StepGraphs::finish()
