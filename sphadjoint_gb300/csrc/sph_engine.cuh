@@ -790,7 +790,14 @@ template <typename T> class Sys final : public StateI {
     void build_masks()
     {
         listsFresh = false;
-        if (const int G = group_lanes()) {
+        if (tiles()) {
+            if constexpr (sizeof(T) == 4) {
+                auto kn = B > 1 ? &k_nl_window<true> : &k_nl_window<false>;
+                SPH_LAUNCH_TILES(K_NLBUILD, kn, N_, N_, hinst[0], dinst.p, pinst.p, pos[cur].p,
+                                 cellStart.p, center.p, masks.p, nbcount.p, flags.p, lists());
+                listsFresh = true;
+            }
+        } else if (const int G = group_lanes()) {
             auto kn = G == 32 ? &k_nl_build_coop<T, 32> : &k_nl_build_coop<T, 16>;
             SPH_LAUNCH_COOP(K_NLBUILD, G, kn, N_, N_, hinst[0], pos[cur].p, cellStart.p,
                             center.p, masks.p, nbcount.p, flags.p);

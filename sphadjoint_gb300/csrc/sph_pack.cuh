@@ -288,20 +288,28 @@ __global__ void __launch_bounds__(kPackBlock) g_rank(int l)
     if (d.ex1) d.ex1N[dst] = d.ex1[src];
 }
 
+static_assert(kPackBlock == kTile, "a block of a grouped launch is one tile");
 template <typename T>
 __global__ void __launch_bounds__(kPackBlock) g_nl_build(int l)
 {
     pdl_enter();
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
+    if constexpr (sizeof(T) == 4) {
+        if (d.W.win) {
+            nl_window<false>(d.n, d.v.one, nullptr, nullptr, d.v.pos, d.cellStart, d.center,
+                             d.masks, d.nbcount, d.flags, d.W, f.y);
+            return;
+        }
+    }
     const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
     if (i >= d.n) return;
     nl_build_one<T>(d.n, d.v.one, 0, i, d.v.pos, d.cellStart, d.center, d.masks, d.nbcount,
                     d.flags);
 }
 
-// Windows and candidate lists of the requests whose masks are new (rebuilt this
-// tick, or restored with a snapshot).
+// Windows and candidate lists of the requests whose masks came with a restored
+// snapshot.
 template <typename T>
 __global__ void __launch_bounds__(kTile) g_lists(int l)
 {
@@ -316,7 +324,6 @@ __global__ void __launch_bounds__(kTile) g_lists(int l)
 // The pair kernels cap their registers as the tuned single-state kernels do:
 // the request's arrays and constants come from the descriptor table, and
 // holding them all in registers would halve the resident warps.
-static_assert(kPackBlock == kTile, "a block of a grouped launch is one tile");
 template <typename T>
 __global__ void __launch_bounds__(kPackBlock, sizeof(T) == 4 ? 11 : 1)
     g_density(int l)
@@ -840,7 +847,7 @@ template <typename T> class Packer final : public PackI {
             }
             lAll.add(k, nb(N, kPackBlock));
             if (!rev) lFwd.add(k, nb(N, kPackBlock));
-            if (rebuild) Y.listsFresh = false;
+            if (rebuild) Y.listsFresh = lists; // the rebuild makes them
             if (lists && !Y.listsFresh) {
                 lLists.add(k, nb(N, kTile));
                 Y.listsFresh = true;
