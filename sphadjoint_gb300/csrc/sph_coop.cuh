@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(kCoopBlock)
     const int64_t i = (int64_t)blockIdx.x * (kCoopBlock / G) + g.gi;
     if (i >= N) return; // the whole group
     const int nx = I.nx, ny = I.ny, maxnb = I.maxnb;
-    const T rc2 = I.rc2, r2min = I.r2min;
     const T2<T> xi = pos[i];
+    const NlTest<T> test(I, xi);
     const int cx = cell_coord<T>(xi.x * I.invcs, nx);
     const int cy = cell_coord<T>(xi.y * I.invcs, ny);
     const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
@@ -193,11 +193,7 @@ __global__ void __launch_bounds__(kCoopBlock)
             for (int base = b; base < e; base += G) {
                 const int j = base + g.gl;
                 bool pass = false;
-                if (j < e) {
-                    const T2<T> xj = pos[j];
-                    const T r2 = r2_exact<T>(sub_rn(xi.x, xj.x), sub_rn(xi.y, xj.y));
-                    pass = lt_nonneg(r2min, r2) && lt_nonneg(r2, rc2);
-                }
+                if (j < e && j != (int)i) pass = test(pos[j]);
                 uint32_t kept = g.ballot(pass);
                 const int np = __popc(kept), room = maxnb - m;
                 if (np > room) {

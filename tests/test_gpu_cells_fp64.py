@@ -36,3 +36,37 @@ def test_cells_on_borders(n, rebuild):
     g, c = st.celllist(), ost.cells()
     for key in ("counts", "starts", "order"):
         assert np.array_equal(g[key], c[key]), key
+
+
+@pytest.mark.parametrize("lanes", [1, 16, 32])
+def test_neighbour_rows_at_the_cutoff(lanes):
+    """Pairs whose distance is the list's cutoff up to a few ulps, coincident
+    particles, particles far outside the tank (clamped into border cells) and tiny
+    offsets: the float estimate of r^2 must leave those to the FP64 test. Rows and
+    counts as the oracle lists them."""
+    rng = np.random.default_rng(5)
+    p = K.dambreak_params()
+    rc = 2.0 * p["h"] * 1.2
+    n = 600
+    X = np.empty((2, n))
+    X[:, 0::3] = np.vstack([0.1 + 1.4 * rng.random(n // 3), 0.1 + 0.8 * rng.random(n // 3)])
+    a = rng.choice([0.0, 0.5 * np.pi, np.pi, 1.0, 2.5], n // 3)
+    d = rc * (1.0 + rng.integers(-3, 4, n // 3) * 2.0 ** -52)
+    X[:, 1::3] = X[:, 0::3] + d * np.vstack([np.cos(a), np.sin(a)])
+    X[:, 2::3] = X[:, 0::3]                       # coincident with the first
+    X[0, 2::6] += p["h"] * 2.0 ** -26             # or at r^2 about eps h^2
+    X[:, 5::60] = 1e3 * (1.0 + rng.random(X[:, 5::60].shape))
+    X[:, 8::60] = -0.2 * rng.random(X[:, 8::60].shape)
+    try:
+        S.set_group_lanes(lanes)
+        st = S.State(X, np.zeros_like(X), S.SPHParams(**p))
+        S.build_neighbors(st)
+        gi, gn = st.neighbors()
+    finally:
+        S.set_group_lanes(0)
+    ost = O.Oracle("f64").state(O.params(**p), X, np.zeros_like(X))
+    ost.build_neighbors(p["h"])
+    oi, on = ost.neighbors()
+    assert np.array_equal(gn, on)
+    for i in range(n):
+        assert np.array_equal(gi[i, : gn[i]], oi[i, : on[i]]), i
