@@ -153,13 +153,14 @@ template <typename T> int &tuned_block(int kid, bool multi)
     } while (0)
 
 // One block per P particles (sph_flat.cuh).
-#define SPH_LAUNCH_FLAT(kid, P, kern, n, ...) SPH_LAUNCH_FLAT_X(kid, P, 0, kern, n, __VA_ARGS__)
-#define SPH_LAUNCH_FLAT_X(kid, P, extra, kern, n, ...)                                        \
+#define SPH_LAUNCH_FLAT(kid, P, kern, n, ...)                                                 \
+    SPH_LAUNCH_FLAT_X(kid, P, 0, ::sphgb::kFlatThreads, kern, n, __VA_ARGS__)
+#define SPH_LAUNCH_FLAT_X(kid, P, extra, threads, kern, n, ...)                                        \
     do {                                                                                      \
         if ((n) > 0) {                                                                        \
             ::sphgb::rt_before_launch(kid);                                                   \
             ::sphgb::launch_k(kern, dim3((unsigned)(((n) + (P) - 1) / (P)) + (extra)),         \
-                              dim3(::sphgb::kFlatBlock), 0, __VA_ARGS__);                      \
+                              dim3(threads), 0, __VA_ARGS__);                                  \
             ::sphgb::rt_after_launch(kid);                                                    \
         }                                                                                     \
     } while (0)
@@ -363,7 +364,7 @@ template <typename T> class Sys final : public StateI {
     DevBuf<TileWin> wwin; // windows and neighbour lists of the FP32 tile passes
     DevBuf<uint2> wcand, wsupp;
     DevBuf<uint8_t> wcnt; // candidate counts, then in-support counts
-    DevBuf<double> fF; // dense pairs of the FP64 flat passes
+    DevBuf<double> fF, fr, ftm; // dense pairs of the FP64 flat passes
     DevBuf<uint32_t> fpair;
     DevBuf<int32_t> foff;
     bool listsTried = false; // the lists were asked for (and may have been refused)
@@ -559,27 +560,31 @@ template <typename T> class Sys final : public StateI {
     bool tiles() const { return want_tiles() && wwin.p; }
     // FP64 states without artificial viscosity run them one lane per pair
     // (sph_flat.cuh), unless a lane setting is forced; their pair lists (about
-    // 770 bytes a particle) are scratch under the same rule.
+    // 1290 bytes a particle) are scratch under the same rule.
     static constexpr int64_t kFlatMaxN = int64_t(1) << 22;
     bool want_flat() const
     {
         return sizeof(T) == 8 && N_ > 0 && N_ <= kFlatMaxN && rt_group_lanes() == 0;
     }
     bool flat() const { return want_flat() && !anyAV && foff.p; }
-    FlatLists flat_lists() const { return FlatLists{fF.p, fpair.p, foff.p, flat_particles(N_)}; }
+    FlatLists flat_lists() const { return FlatLists{fF.p, fr.p, ftm.p, fpair.p, foff.p, flat_particles(N_)}; }
     void reserve_lists()
     {
         if (want_tiles()) alloc_lists();
         if (want_flat() && !listsTried && !rt_capturing()) {
             listsTried = true;
             const size_t P = (size_t)flat_particles(N_), nb = ((size_t)N_ + P - 1) / P;
-            if (rt_free_memory() / 8 < nb * (P * kFlatRow * 12 + 4 * kFlatOff)) return;
+            if (rt_free_memory() / 8 < nb * P * (kFlatRow * 20 + 8) + nb * 4 * kFlatOff) return;
             try {
                 fF.alloc(nb * P * kFlatRow);
+                fr.alloc(nb * P * kFlatRow);
+                ftm.alloc(nb * P);
                 fpair.alloc(nb * P * kFlatRow);
                 foff.alloc(nb * kFlatOff);
             } catch (const Error &) {
                 fF.release();
+                fr.release();
+                ftm.release();
                 fpair.release();
                 foff.release();
             }
@@ -876,7 +881,8 @@ template <typename T> class Sys final : public StateI {
                 const FlatLists W = flat_lists();
                 auto kd = B > 1 ? &k_density_flat<true> : &k_density_flat<false>;
                 auto ki = B > 1 ? &k_accel_flat<true> : &k_accel_flat<false>;
-                SPH_LAUNCH_FLAT(K_DENSITY, W.P, kd, N_, v, W, rho.p, prho.p, no_flush());
+                SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, 0, kFlatBlock, kd, N_, v, W, rho.p, prho.p,
+                                  no_flush());
                 SPH_LAUNCH_FLAT(K_ACCEL_INTEGRATE, W.P, ki, N_, v, W, vel[cur].p, prho.p, theta,
                                 pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
             }
@@ -1462,7 +1468,8 @@ template <typename T> class Work final : public WorkI {
                 auto k1 = multi ? &k_pass1_flat<true> : &k_pass1_flat<false>;
                 auto k2 = multi ? &k_pass2_flat<true> : &k_pass2_flat<false>;
                 const ThetaFlush<T> fl = take_flush(S, (N_ + W.P - 1) / W.P, extra);
-                SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, extra, kd, N_, v, W, rhoOut, S.prho.p, fl);
+                SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, extra, kFlatBlock, kd, N_, v, W, rhoOut, S.prho.p,
+                                  fl);
                 SPH_LAUNCH_FLAT(K_ACCEL_DRAG, W.P, ka, N_, v, W, vel, S.prho.p, theta, gX[gcur].p,
                                 gV[gcur].p, abar.p, galpha.p, emax.p, parity);
                 SPH_LAUNCH_FLAT(K_PASS1, W.P, k1, N_, v, W, vel, S.prho.p, S.rho.p, theta, abar.p,

@@ -14,8 +14,8 @@
 //             The pass leaves, per block, the dense pairs (particle, slot), each
 //             pair's F = Fc u^3, and the particles' offsets.
 //   force and adjoint passes read that sequence: no masks, no support test, and
-//             8 to 10 FP64 operations a pair fewer (r^2, q, u and F are not formed
-//             again; pass 1 needs r itself).
+//             8 to 10 FP64 operations a pair fewer (r, F and each particle's 2 m mu /
+//             rho come with it).
 //
 // Each pair's terms go to shared memory, and one lane per running sum adds them
 // in sequence order, so every sum sees the operations of the serial walk in its
@@ -46,7 +46,8 @@ constexpr int kFlatOff = kFlatMax + 2; // offsets of a block, then its serial ma
 constexpr int kFlatSlotBits = 27;
 
 struct FlatLists {
-    double *F;      // [block][P * kFlatRow]
+    double *F, *r;  // [block][P * kFlatRow]
+    double *tm;     // per slot: 2 m mu / rho
     uint32_t *pair; // local particle << kFlatSlotBits | neighbour slot
     int32_t *off;   // [block][kFlatOff]
     int P;          // particles of a block
@@ -213,10 +214,12 @@ __global__ void __launch_bounds__(kFlatBlock)
     __syncthreads();
     for (int d = t; d < D; d += kFlatBlock) {
         decltype(auto) I = load_inst<MULTI>(v, i0 + s_own[d]);
-        const double q = pair_sqrt(s_r2[d]) * I.p.invh;
+        const double r = pair_sqrt(s_r2[d]);
+        const double q = r * I.p.invh;
         const double u = 1.0 - half_of(q);
         const double u2 = u * u;
         B.F[bb + d] = I.p.Fc * u * u * u;
+        B.r[bb + d] = r;
         s_r2[d] = I.p.m * (I.p.A * u2 * u2 * (twice_of(q) + 1.0));
     }
     int all;
@@ -227,6 +230,8 @@ __global__ void __launch_bounds__(kFlatBlock)
     const int64_t i = i0 + t;
     if ((serial >> t) & 1u) {
         density_walk<double, MULTI, false>(v, i, rho, prho, nullptr);
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        B.tm[i] = I.p.twomumass * prho[i].y;
         return;
     }
     double acc = 0.0;
@@ -234,18 +239,84 @@ __global__ void __launch_bounds__(kFlatBlock)
 #pragma unroll 4
     for (int k = o; k < e; ++k) acc += s_r2[k];
     decltype(auto) I = load_inst<MULTI>(v, i);
-    density_finish<double>(I, i, acc, rho, prho);
+    B.tm[i] = I.p.twomumass * density_finish<double>(I, i, acc, rho, prho).y;
 }
 
-// The offsets of a block's particles in its dense pairs; s_off[np] pairs.
-__device__ __forceinline__ void flat_offsets(const FlatLists &B, int np, int *s_off,
-                                             uint32_t *s_serial)
-{
-    const int t = (int)threadIdx.x;
-    const int32_t *o = B.off + (int64_t)blockIdx.x * kFlatOff;
-    if (t <= np) s_off[t] = o[t];
-    if (t == 0) *s_serial = (uint32_t)o[kFlatOff - 1];
-}
+// ---- the passes that read the dense pairs --------------------------------------
+// Five warps: four take the pairs, the fifth meanwhile does what its particles'
+// results need besides the pair sums (design field, walls, the theta write-back,
+// the next tape state), so that a short pass is one chain of loads, pair terms,
+// fold and a few last operations.
+constexpr int kFlatThreads = kFlatBlock + 32;
+constexpr int kFlatAhead = kFlatChunk / kFlatBlock;
+
+struct FlatShared {
+    int off[kFlatMax + 1];
+    uint32_t serial;
+};
+
+// Where a pass stands: its particles [i0, i0 + np), the thread's role, and the
+// first chunk's pairs, read before the offsets that tell how many there are.
+template <bool MULTI> struct FlatPass {
+    const NLView<double> &v;
+    const FlatLists &B;
+    int64_t i0, bb;
+    int np, t;
+    uint32_t e[kFlatAhead];
+    double F[kFlatAhead];
+    __device__ __forceinline__ FlatPass(const NLView<double> &view, const FlatLists &L,
+                                        FlatShared &S)
+        : v(view), B(L), i0((int64_t)blockIdx.x * L.P), bb(i0 * kFlatRow), t((int)threadIdx.x)
+    {
+        np = v.N - i0 < B.P ? (int)(v.N - i0) : B.P;
+        const int32_t *o = B.off + (int64_t)blockIdx.x * kFlatOff;
+#pragma unroll
+        for (int u = 0; u < kFlatAhead; ++u) {
+            const int p = t + u * kFlatBlock;
+            e[u] = 0u;
+            F[u] = 0.0;
+            if (t < kFlatBlock && p < B.P * kFlatRow) {
+                e[u] = B.pair[bb + p];
+                F[u] = B.F[bb + p];
+            }
+        }
+        if (t <= np) S.off[t] = o[t];
+        if (t == kFlatBlock) S.serial = (uint32_t)o[kFlatOff - 1];
+        __syncthreads();
+    }
+    // f(place in the chunk, particle, neighbour, F) of the chunk's m pairs, done by
+    // the first four warps
+    template <typename Fn> __device__ __forceinline__ void pairs(int base, int m, Fn &&f) const
+    {
+        if (t >= kFlatBlock) return;
+#pragma unroll
+        for (int u = 0; u < kFlatAhead; ++u) {
+            const int p = t + u * kFlatBlock;
+            if (p < m) {
+                const uint32_t q = base ? B.pair[bb + base + p] : e[u];
+                f(p, i0 + (q >> kFlatSlotBits), (int)(q & ((1u << kFlatSlotBits) - 1u)),
+                  base ? B.F[bb + base + p] : F[u]);
+            }
+        }
+    }
+    // The pairs of the chunk from pair `base` of particle a on: those of the next 16
+    // particles where they fit, so that the warp whose lanes fold 16 particles runs
+    // once; a moves to the particle after them.
+    __device__ __forceinline__ int chunk(const FlatShared &S, int base, int &a) const
+    {
+        const int n = S.off[np], a1 = (a & ~15) + 16 < np ? (a & ~15) + 16 : np;
+        if (S.off[a1] - base <= kFlatChunk) {
+            a = a1;
+            return S.off[a1] - base;
+        }
+        return n - base < kFlatChunk ? n - base : kFlatChunk;
+    }
+    // the particle of the fifth warp's lane (-1: none)
+    __device__ __forceinline__ int64_t aside() const
+    {
+        return t >= kFlatBlock && t - kFlatBlock < np ? i0 + t - kFlatBlock : -1;
+    }
+};
 
 // One lane per running sum: chain c adds the terms of its particle's pairs that
 // this chunk holds. sub (may be NULL): a term subtracted before each added one.
@@ -266,44 +337,42 @@ __device__ __forceinline__ double flat_fold(double acc, const double *sub, const
 }
 
 // Pressure + Morris viscosity of the block's particles (accel_pair): s_acc[2 a],
-// s_acc[2 a + 1]. All threads call it; ends with a barrier.
-template <bool MULTI>
-__device__ __forceinline__ void flat_accel(const NLView<double> &v, const FlatLists &B, int np,
-                                           const int *s_off, double (*s_t)[kFlatChunk],
-                                           double *s_acc, const double2 *__restrict__ vel,
-                                           const double2 *__restrict__ prho)
+// s_acc[2 a + 1]. side() is what the fifth warp does during the first chunk. All
+// threads call it; ends with a barrier.
+template <bool MULTI, typename Side>
+__device__ __forceinline__ void flat_accel(const FlatPass<MULTI> &Q, const FlatShared &S,
+                                           double (*s_t)[kFlatChunk], double *s_acc,
+                                           const double2 *__restrict__ vel,
+                                           const double2 *__restrict__ prho, Side &&side)
 {
-    const int t = (int)threadIdx.x;
-    const int64_t i0 = (int64_t)blockIdx.x * B.P, bb = i0 * kFlatRow;
-    const int n = s_off[np], a2 = t >> 1, c2 = t & 1;
-    const int b0 = a2 < np ? s_off[a2] : 0, b1 = a2 < np ? s_off[a2 + 1] : 0;
+    const NLView<double> &v = Q.v;
+    const FlatLists &B = Q.B;
+    const int n = S.off[Q.np], a2 = Q.t >> 1, c2 = Q.t & 1;
+    const int b0 = a2 < Q.np ? S.off[a2] : 0, b1 = a2 < Q.np ? S.off[a2 + 1] : 0;
     double acc = 0.0;
-    for (int base = 0; base < n; base += kFlatChunk) {
-        const int m = n - base < kFlatChunk ? n - base : kFlatChunk;
-        for (int p = t; p < m; p += kFlatBlock) {
-            const uint32_t e = B.pair[bb + base + p];
-            const double F = B.F[bb + base + p];
-            const int64_t i = i0 + (e >> kFlatSlotBits);
-            const int j = (int)(e & ((1u << kFlatSlotBits) - 1u));
+    side();
+    for (int base = 0, at = 0, m; base < n; base += m) {
+        m = Q.chunk(S, base, at);
+        Q.pairs(base, m, [&](int p, int64_t i, int j, double F) {
             decltype(auto) I = load_inst<MULTI>(v, i);
             const double2 xi = v.pos[i], vi = vel[i], pi = prho[i];
             const double2 xj = v.pos[j], vj = vel[j], pj = prho[j];
             const double Pij = I.p.m * (pi.x + pj.x);
             s_t[0][p] = Pij * F * (xi.x - xj.x);
             s_t[1][p] = Pij * F * (xi.y - xj.y);
-            const double C = I.p.twomumass * pi.y * pj.y * F;
+            const double C = B.tm[i] * pj.y * F;
             s_t[2][p] = C * (vi.x - vj.x);
             s_t[3][p] = C * (vi.y - vj.y);
-        }
+        });
         __syncthreads();
-        if (a2 < np) {
+        if (a2 < Q.np) {
             const int k0 = (b0 > base ? b0 : base) - base;
             const int k1 = (b1 < base + m ? b1 : base + m) - base;
             acc = flat_fold(acc, s_t[c2], s_t[2 + c2], k0, k1);
         }
         __syncthreads();
     }
-    if (a2 < np) s_acc[t] = acc;
+    if (a2 < Q.np) s_acc[Q.t] = acc;
     __syncthreads();
 }
 
@@ -324,9 +393,26 @@ __device__ __forceinline__ void flat_force(const NLView<double> &v, uint32_t ser
     }
 }
 
-// accel_kernel! + integrate_kernel!
+// What accel_integrate_finish and drag_adj_finish form without the pair sum:
+// gravity plus wall, the Brinkman alpha and D = 1 / (1 + dt alpha).
+struct FlatForce {
+    double gx, gy, al, D;
+};
+template <typename IT>
+__device__ __forceinline__ FlatForce flat_force_of(const IT &I, const double2 &x,
+                                                   const double *__restrict__ theta)
+{
+    FlatForce f;
+    f.al = interp_alpha_value<double>(theta + I.toff, x.x, x.y, I.p);
+    f.gx = I.p.gx + wall_accel<double>(x.x, I.p.Lx, I.p.kw);
+    f.gy = I.p.gy + wall_accel<double>(x.y, I.p.Ly, I.p.kw);
+    f.D = div_rn(1.0, 1.0 + I.p.dt * f.al);
+    return f;
+}
+
+// accel_kernel! + integrate_kernel! (accel_integrate_finish)
 template <bool MULTI>
-__global__ void __launch_bounds__(kFlatBlock)
+__global__ void __launch_bounds__(kFlatThreads)
     k_accel_flat(const __grid_constant__ NLView<double> v, const FlatLists B,
                  const double2 *__restrict__ vel, const double2 *__restrict__ prho,
                  const double *__restrict__ theta, double2 *__restrict__ posOut,
@@ -337,28 +423,48 @@ __global__ void __launch_bounds__(kFlatBlock)
 {
     pdl_enter();
     __shared__ double s_t[4][kFlatChunk], s_acc[2 * kFlatMax];
-    __shared__ int s_off[kFlatMax + 1];
-    __shared__ uint32_t s_serial;
-    const int64_t i0 = (int64_t)blockIdx.x * B.P;
-    const int np = v.N - i0 < B.P ? (int)(v.N - i0) : B.P;
-    flat_offsets(B, np, s_off, &s_serial);
-    __syncthreads();
-    flat_accel<MULTI>(v, B, np, s_off, s_t, s_acc, vel, prho);
-    const int t = (int)threadIdx.x;
-    if (t >= np) return;
-    const int64_t i = i0 + t;
+    __shared__ FlatForce s_f[kFlatMax];
+    __shared__ FlatShared S;
+    const FlatPass<MULTI> Q(v, B, S);
+    flat_accel<MULTI>(Q, S, s_t, s_acc, vel, prho, [&] {
+        const int64_t i = Q.aside();
+        if (i < 0) return;
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        const double2 xi = v.pos[i];
+        if (tx) {
+            const int32_t id = perm[i];
+            tx[id] = xi;
+            tv[id] = vel[i];
+        }
+        const FlatForce f = flat_force_of(I, xi, theta);
+        if (alphaOut) alphaOut[i] = f.al;
+        s_f[Q.t - kFlatBlock] = f;
+    });
+    if (Q.t >= Q.np) return;
+    const int64_t i = Q.i0 + Q.t;
     const int b = MULTI ? inst_of(v, i) : 0;
     decltype(auto) I = load_inst<MULTI>(v, i);
     const double2 xi = v.pos[i], vi = vel[i];
+    const FlatForce f = s_f[Q.t];
     double ax, ay;
-    flat_force<MULTI>(v, s_serial, i, s_acc, vel, prho, xi, vi, ax, ay);
-    accel_integrate_finish<double>(I, b, i, xi, vi, ax, ay, theta, posOut, velOut, aOut, alphaOut,
-                                   flags, perm, tx, tv);
+    flat_force<MULTI>(v, S.serial, i, s_acc, vel, prho, xi, vi, ax, ay);
+    ax += f.gx;
+    ay += f.gy;
+    if (aOut) aOut[i] = make_double2(ax, ay);
+    const double dt = I.p.dt;
+    const double v1 = (vi.x + dt * ax) * f.D;
+    const double v2 = (vi.y + dt * ay) * f.D;
+    const double x1 = xi.x + dt * v1;
+    const double x2 = xi.y + dt * v2;
+    velOut[i] = make_double2(v1, v2);
+    posOut[i] = make_double2(x1, x2);
+    if (!(isfinite(x1) && isfinite(x2) && isfinite(v1) && isfinite(v2)))
+        atomicOr(flags + b, FLAG_NONFINITE);
 }
 
-// Accel recompute + _adj_integrate! + _adj_drag!
+// Accel recompute + _adj_integrate! + _adj_drag! (drag_adj_finish)
 template <bool MULTI>
-__global__ void __launch_bounds__(kFlatBlock)
+__global__ void __launch_bounds__(kFlatThreads)
     k_drag_flat(const __grid_constant__ NLView<double> v, const FlatLists B,
                 const double2 *__restrict__ vel, const double2 *__restrict__ prho,
                 const double *__restrict__ theta, const double2 *__restrict__ gX,
@@ -367,31 +473,51 @@ __global__ void __launch_bounds__(kFlatBlock)
 {
     pdl_enter();
     __shared__ double s_t[4][kFlatChunk], s_acc[2 * kFlatMax];
-    __shared__ int s_off[kFlatMax + 1];
-    __shared__ uint32_t s_serial;
-    const int64_t i0 = (int64_t)blockIdx.x * B.P;
-    const int np = v.N - i0 < B.P ? (int)(v.N - i0) : B.P;
-    flat_offsets(B, np, s_off, &s_serial);
-    __syncthreads();
-    flat_accel<MULTI>(v, B, np, s_off, s_t, s_acc, vel, prho);
-    const int t = (int)threadIdx.x;
-    if (t >= 32) return;
-    const int64_t i = i0 + t;
+    __shared__ FlatForce s_f[kFlatMax];
+    __shared__ double2 s_gv[kFlatMax];
+    __shared__ FlatShared S;
+    const FlatPass<MULTI> Q(v, B, S);
+    flat_accel<MULTI>(Q, S, s_t, s_acc, vel, prho, [&] {
+        const int64_t i = Q.aside();
+        if (i < 0) return;
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        const FlatForce f = flat_force_of(I, v.pos[i], theta);
+        const double dt = I.p.dt;
+        const double2 gx = gX[i];
+        double2 gv = gV[i];
+        gv.x += dt * gx.x;
+        gv.y += dt * gx.y;
+        abar[i] = make_double2(dt * f.D * gv.x, dt * f.D * gv.y);
+        gV[i] = make_double2(f.D * gv.x, f.D * gv.y);
+        s_f[Q.t - kFlatBlock] = f;
+        s_gv[Q.t - kFlatBlock] = gv;
+    });
+    if (Q.t >= 32) return;
+    const int64_t i = Q.i0 + Q.t;
     int e = INT_MIN, b = 0;
-    if (t < np) {
+    if (Q.t < Q.np) {
         b = MULTI ? inst_of(v, i) : 0;
         decltype(auto) I = load_inst<MULTI>(v, i);
         const double2 xi = v.pos[i], vi = vel[i];
+        const FlatForce f = s_f[Q.t];
+        const double2 gv = s_gv[Q.t];
         double ax, ay;
-        flat_force<MULTI>(v, s_serial, i, s_acc, vel, prho, xi, vi, ax, ay);
-        e = drag_adj_finish<double>(I, i, xi, vi, ax, ay, theta, gX, gV, abar, galpha);
+        flat_force<MULTI>(v, S.serial, i, s_acc, vel, prho, xi, vi, ax, ay);
+        ax += f.gx;
+        ay += f.gy;
+        const double dt = I.p.dt;
+        const double vx = (vi.x + dt * ax) * f.D;
+        const double vy = (vi.y + dt * ay) * f.D;
+        const double ga = -dt * f.D * (vx * gv.x + vy * gv.y);
+        galpha[i] = ga;
+        e = (ga != 0.0 && isfinite(ga)) ? ilogb(ga) + 1 : INT_MIN;
     }
-    warp_emax(t < np, b, e, emax, parity, MULTI);
+    warp_emax(Q.t < Q.np, b, e, emax, parity, MULTI);
 }
 
 // adj_pass1_kernel! + the gXs half of adj_design_kernel! + _axpy2!(gV, gVs)
 template <bool MULTI>
-__global__ void __launch_bounds__(kFlatBlock)
+__global__ void __launch_bounds__(kFlatThreads)
     k_pass1_flat(const __grid_constant__ NLView<double> v, const FlatLists B,
                  const double2 *__restrict__ vel, const double2 *__restrict__ prho,
                  const double *__restrict__ rho, const double *__restrict__ theta,
@@ -401,34 +527,39 @@ __global__ void __launch_bounds__(kFlatBlock)
     pdl_enter();
     __shared__ double s_t[8][kFlatChunk];
     __shared__ double s_acc[6 * kFlatMax]; // gx gy per particle, then gvx gvy grho S
-    __shared__ int s_off[kFlatMax + 1];
-    __shared__ uint32_t s_serial;
-    const int t = (int)threadIdx.x;
-    const int64_t i0 = (int64_t)blockIdx.x * B.P, bb = i0 * kFlatRow;
-    const int np = v.N - i0 < B.P ? (int)(v.N - i0) : B.P;
-    flat_offsets(B, np, s_off, &s_serial);
-    for (int k = t; k < 6 * kFlatMax; k += kFlatBlock) s_acc[k] = 0.0;
-    __syncthreads();
-    const int n = s_off[np];
-    for (int base = 0; base < n; base += kFlatChunk) {
-        const int m = n - base < kFlatChunk ? n - base : kFlatChunk;
-        for (int p = t; p < m; p += kFlatBlock) {
-            const uint32_t e = B.pair[bb + base + p];
-            const double F = B.F[bb + base + p];
-            const int64_t i = i0 + (e >> kFlatSlotBits);
-            const int j = (int)(e & ((1u << kFlatSlotBits) - 1u));
+    __shared__ double s_side[4][kFlatMax]; // wall and design-field terms of gXs
+    __shared__ FlatShared S;
+    const FlatPass<MULTI> Q(v, B, S);
+    const int t = Q.t, np = Q.np;
+    for (int k = t; k < 6 * kFlatMax; k += kFlatThreads) s_acc[k] = 0.0;
+    if (const int64_t i = Q.aside(); i >= 0) {
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        const double2 x = v.pos[i], ab = abar[i];
+        double al, dadx, dady;
+        interp_alpha<double>(theta + I.toff, x.x, x.y, I.p, al, dadx, dady);
+        const double ga = galpha[i];
+        s_side[0][t - kFlatBlock] = ab.x * wall_daccel<double>(x.x, I.p.Lx, I.p.kw);
+        s_side[1][t - kFlatBlock] = ab.y * wall_daccel<double>(x.y, I.p.Ly, I.p.kw);
+        s_side[2][t - kFlatBlock] = ga * dadx;
+        s_side[3][t - kFlatBlock] = ga * dady;
+    }
+    const int n = S.off[np];
+    if (n == 0) __syncthreads();
+    for (int base = 0, at = 0, m; base < n; base += m) {
+        m = Q.chunk(S, base, at);
+        Q.pairs(base, m, [&](int p, int64_t i, int j, double F) {
             decltype(auto) I = load_inst<MULTI>(v, i);
             const double2 xi = v.pos[i], vi = vel[i], pi = prho[i], ab = abar[i];
             const double2 xj = v.pos[j], vj = vel[j], pj = prho[j], abj = abar[j];
             // pass1_pair, with F from the density pass
             const double dx = xi.x - xj.x;
             const double dy = xi.y - xj.y;
-            const double r = pair_sqrt(dx * dx + dy * dy);
+            const double r = B.r[Q.bb + base + p];
             const double q = r * I.p.invh;
             const double u = 1.0 - half_of(q);
             const double G = I.p.Gc * u * u;
             const double Pij = I.p.m * (pi.x + pj.x);
-            const double Cbase = I.p.twomumass * pi.y * pj.y;
+            const double Cbase = B.tm[i] * pj.y;
             const double C = Cbase * F;
             const double dax = ab.x - abj.x;
             const double day = ab.y - abj.y;
@@ -444,41 +575,53 @@ __global__ void __launch_bounds__(kFlatBlock)
             s_t[5][p] = C * day;
             s_t[6][p] = -(C * ad_v * pi.y); // subtracted
             s_t[7][p] = F * ad_d;
-        }
+        });
         __syncthreads();
-        // gx and gy (two terms a pair) on the first warps, then the four sums
-        // with one
-        for (int c = t; c < 2 * np; c += kFlatBlock) {
-            const int a = c >> 1, k0 = s_off[a] > base ? s_off[a] - base : 0;
-            const int k1 = s_off[a + 1] < base + m ? s_off[a + 1] - base : m;
+        // gx and gy (two terms a pair) on the first warps, the four sums with one
+        // term from the last warp down
+        for (int c = t; c < 2 * np; c += kFlatThreads) {
+            const int a = c >> 1, k0 = S.off[a] > base ? S.off[a] - base : 0;
+            const int k1 = S.off[a + 1] < base + m ? S.off[a + 1] - base : m;
             s_acc[c] = flat_fold(s_acc[c], s_t[c & 1], s_t[2 + (c & 1)], k0, k1);
         }
-        for (int c = kFlatBlock - 1 - t; c < 4 * np; c += kFlatBlock) {
-            const int a = c >> 2, k0 = s_off[a] > base ? s_off[a] - base : 0;
-            const int k1 = s_off[a + 1] < base + m ? s_off[a + 1] - base : m;
+        for (int c = kFlatThreads - 1 - t; c < 4 * np; c += kFlatThreads) {
+            const int a = c >> 2, k0 = S.off[a] > base ? S.off[a] - base : 0;
+            const int k1 = S.off[a + 1] < base + m ? S.off[a + 1] - base : m;
             double &x = s_acc[2 * kFlatMax + c];
             x = flat_fold(x, nullptr, s_t[4 + (c & 3)], k0, k1);
         }
         __syncthreads();
     }
     if (t >= np) return;
-    const int64_t i = i0 + t;
+    const int64_t i = Q.i0 + t;
     decltype(auto) I = load_inst<MULTI>(v, i);
-    const double2 xi = v.pos[i], ab = abar[i], pi = prho[i];
+    const double2 pi = prho[i];
     double gx = s_acc[2 * t], gy = s_acc[2 * t + 1];
     const double *o = s_acc + 2 * kFlatMax + 4 * t;
     double gvx = o[0], gvy = o[1], grh = o[2], sumS = o[3];
-    if ((s_serial >> t) & 1u)
-        pass1_sum<double, false>(v, I, i, vel, prho, rho, abar, xi, vel[i], ab, pi, gx, gy, gvx,
-                                 gvy, grh, sumS);
-    const double rhoi = I.p.eos == 1 ? rho[i] : 0.0;
-    pass1_finish<double>(I, i, xi, ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, theta, galpha, gXs,
-                         grho, gV);
+    if ((S.serial >> t) & 1u)
+        pass1_sum<double, false>(v, I, i, vel, prho, rho, abar, v.pos[i], vel[i], abar[i], pi, gx,
+                                 gy, gvx, gvy, grh, sumS);
+    // pass1_finish
+    grh += (-2.0 * I.p.m * pi.x * pi.y) * sumS;
+    if (I.p.eos == 1)
+        grh += I.p.dB * pow_fold<double>(div_rn(rho[i], I.p.rho0), I.p.gam - 1) * I.p.m * pi.y *
+               pi.y * sumS;
+    else
+        grh += I.p.c2 * I.p.m * pi.y * pi.y * sumS;
+    gx += s_side[0][t];
+    gy += s_side[1][t];
+    gXs[i] = make_double2(gx + s_side[2][t], gy + s_side[3][t]);
+    grho[i] = grh;
+    double2 g = gV[i];
+    g.x += gvx;
+    g.y += gvy;
+    gV[i] = g;
 }
 
 // adj_pass2_kernel! + _axpy2!(gX, gXs) + the exact theta write-back
 template <bool MULTI>
-__global__ void __launch_bounds__(kFlatBlock)
+__global__ void __launch_bounds__(kFlatThreads)
     k_pass2_flat(const __grid_constant__ NLView<double> v, const FlatLists B,
                  const double *__restrict__ grho, const double2 *__restrict__ gXs,
                  double2 *__restrict__ gX, const double *__restrict__ galpha,
@@ -487,31 +630,37 @@ __global__ void __launch_bounds__(kFlatBlock)
 {
     pdl_enter();
     __shared__ double s_t[2][kFlatChunk], s_acc[2 * kFlatMax];
-    __shared__ int s_off[kFlatMax + 1];
-    __shared__ uint32_t s_serial;
-    const int t = (int)threadIdx.x;
-    const int64_t i0 = (int64_t)blockIdx.x * B.P, bb = i0 * kFlatRow;
-    const int np = v.N - i0 < B.P ? (int)(v.N - i0) : B.P;
-    flat_offsets(B, np, s_off, &s_serial);
-    const int nt = kFlatBlock - 1 - t; // the last threads load the next state
-    if (nt < np) next.read(i0 + nt);
-    __syncthreads();
-    const int n = s_off[np], a2 = t >> 1, c2 = t & 1;
-    const int b0 = a2 < np ? s_off[a2] : 0, b1 = a2 < np ? s_off[a2 + 1] : 0;
+    __shared__ FlatShared S;
+    const FlatPass<MULTI> Q(v, B, S);
+    const int t = Q.t, np = Q.np;
+    if (t >= kFlatBlock) { // the theta write-back and the next tape state
+        const int64_t own = Q.aside(), i = own >= 0 ? own : Q.i0;
+        if (own >= 0) next.read(i);
+        const int b = MULTI ? inst_of(v, i) : 0;
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        const double2 x = v.pos[i];
+        const double ga = galpha[i];
+        const int em = emax[2 * b + parity];
+        int ci, cj;
+        double fx, fy, ax, ay;
+        interp_cell<double>(x.x, x.y, I.p, ci, cj, fx, fy, ax, ay);
+        theta_add_warp<double>(own >= 0 && ga != 0.0 && em != INT_MIN,
+                               I.toff + cj + ci * I.p.ngy, I.p.ngy, theta_scale(em, I.lgN), ga, fx,
+                               fy, thetaAcc);
+        if (own >= 0) next.write(i);
+    }
+    const int n = S.off[np], a2 = t >> 1, c2 = t & 1;
+    const int b0 = a2 < np ? S.off[a2] : 0, b1 = a2 < np ? S.off[a2 + 1] : 0;
     double acc = 0.0;
-    for (int base = 0; base < n; base += kFlatChunk) {
-        const int m = n - base < kFlatChunk ? n - base : kFlatChunk;
-        for (int p = t; p < m; p += kFlatBlock) {
-            const uint32_t e = B.pair[bb + base + p];
-            const double F = B.F[bb + base + p];
-            const int64_t i = i0 + (e >> kFlatSlotBits);
-            const int j = (int)(e & ((1u << kFlatSlotBits) - 1u));
+    for (int base = 0, at = 0, m; base < n; base += m) {
+        m = Q.chunk(S, base, at);
+        Q.pairs(base, m, [&](int p, int64_t i, int j, double F) {
             decltype(auto) I = load_inst<MULTI>(v, i);
             const double2 xi = v.pos[i], xj = v.pos[j];
             const double w = I.p.m * F * (grho[i] + grho[j]);
             s_t[0][p] = w * (xi.x - xj.x);
             s_t[1][p] = w * (xi.y - xj.y);
-        }
+        });
         __syncthreads();
         if (a2 < np) {
             const int k0 = (b0 > base ? b0 : base) - base;
@@ -521,17 +670,15 @@ __global__ void __launch_bounds__(kFlatBlock)
         __syncthreads();
     }
     if (a2 < np) s_acc[t] = acc;
-    if (nt < np) next.write(i0 + nt);
     __syncthreads();
-    if (t >= 32) return;
-    const bool live = t < np;
-    const int64_t i = i0 + (live ? t : np - 1);
-    const int b = MULTI ? inst_of(v, i) : 0;
-    decltype(auto) I = load_inst<MULTI>(v, i);
-    const double2 xi = v.pos[i];
-    double gx = live ? s_acc[2 * t] : 0.0, gy = live ? s_acc[2 * t + 1] : 0.0;
-    if (live && ((s_serial >> t) & 1u)) pass2_sum<double>(v, I, i, xi, grho, gx, gy);
-    pass2_finish_warp<double>(live, I, b, i, xi, gx, gy, gXs, gX, galpha, emax, parity, thetaAcc);
+    if (t >= np) return;
+    const int64_t i = Q.i0 + t;
+    double gx = s_acc[2 * t], gy = s_acc[2 * t + 1];
+    if ((S.serial >> t) & 1u) {
+        decltype(auto) I = load_inst<MULTI>(v, i);
+        pass2_sum<double>(v, I, i, v.pos[i], grho, gx, gy);
+    }
+    pass2_axpy<double>(i, gx, gy, gXs, gX);
 }
 
 } // namespace sphgb

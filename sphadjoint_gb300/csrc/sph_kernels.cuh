@@ -808,8 +808,8 @@ __device__ __forceinline__ T density_spill_sum(const NLView<T> &v, const IT &I, 
 // Self term and eos_kernel!: rho = sum + m A, pterm = c^2 (rho - rho0) / rho^2
 // (Tait: B ((rho/rho0)^gamma - 1) / rho^2).
 template <typename T, typename IT>
-__device__ __forceinline__ void density_finish(const IT &I, int64_t i, T acc, T *__restrict__ rho,
-                                               T2<T> *__restrict__ prho)
+__device__ __forceinline__ T2<T> density_finish(const IT &I, int64_t i, T acc,
+                                                T *__restrict__ rho, T2<T> *__restrict__ prho)
 {
     const T m = I.p.m, A = I.p.A;
     // explicit roundings: the same result whichever kernel form inlines this
@@ -820,7 +820,9 @@ __device__ __forceinline__ void density_finish(const IT &I, int64_t i, T acc, T 
     T pt;
     if (I.p.eos == 1) pt = I.p.B * pow1m<T>(div_rn(ri - I.p.rho0, I.p.rho0), I.p.gam) * inv * inv;
     else pt = I.p.c2 * (ri - I.p.rho0) * inv * inv;
-    prho[i] = mk2<T>(pt, inv);
+    const T2<T> p = mk2<T>(pt, inv);
+    prho[i] = p;
+    return p;
 }
 
 // density_kernel! + eos_kernel!. It also records, for the rest of this step,
