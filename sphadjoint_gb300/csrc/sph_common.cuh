@@ -325,6 +325,12 @@ template <typename T> __host__ __device__ __forceinline__ int cell_coord(T v, in
 // an integer within reach the floor is already known and the division (some
 // hundred integer instructions, div_rn) is not needed. The estimate is off the
 // FP64 pipe. Non-finite, subnormal and out-of-range values take the division.
+// not inlined: it is rarely taken, and straight-line code that a short kernel
+// runs once is paid for in instruction fetches
+static __device__ __noinline__ int cell_div_exact(double x, double cs, int n)
+{
+    return cell_coord<double>(div_rn(x, cs), n);
+}
 __device__ __forceinline__ int cell_div(float x, float cs, int n)
 {
     return cell_coord<float>(x / cs, n);
@@ -345,7 +351,7 @@ __device__ __forceinline__ int cell_div(double x, double cs, int n)
             return c > n ? n : c;
         }
     }
-    return cell_coord<double>(div_rn(x, cs), n);
+    return cell_div_exact(x, cs, n);
 }
 
 // wall_accel / wall_daccel (src/params.jl:36-46); max(zero(T), -x) keeps +0.

@@ -115,21 +115,32 @@ template <typename T> inline bool step_graph_eligible(int64_t n)
 // device (pdl_enter) for the predecessor's results, which removes the launch
 // gap between the many short kernels of a step.
 template <typename... KArgs, typename... Args>
-inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args)
+inline void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                           unsigned cluster, Args &&...args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = rt_stream();
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
+    cfg.attrs = at;
     if (rt_launch_overlap() && !rt_capturing()) {
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = cluster;
+        at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
     }
     cuda_check(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...), "kernel launch");
+}
+template <typename... KArgs, typename... Args>
+inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args)
+{
+    launch_cluster(kern, grid, block, smem, 0u, std::forward<Args>(args)...);
 }
 
 // Threads per block of each tuned kernel, per precision and per single/batched
@@ -516,10 +527,12 @@ template <typename T> class Sys final : public StateI {
             // graph recording)
             static bool attr = false;
             if (!attr) {
-                SPH_CK(cudaFuncSetAttribute(k_rebuild_small<T>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)(sizeof(int32_t) * (2 * kRebuildSmallMaxCells + 1 +
-                                                                     3 * kRebuildSmallMaxN))));
+                const int most = (int)(sizeof(int32_t) * (2 * kRebuildSmallMaxCells + 1 +
+                                                          kRebuildSmallMaxN));
+                SPH_CK(cudaFuncSetAttribute(k_rebuild_small<T, 1>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+                SPH_CK(cudaFuncSetAttribute(k_rebuild_small<T, kRebuildPer>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, most));
                 attr = true;
             }
         }
@@ -764,9 +777,12 @@ template <typename T> class Sys final : public StateI {
             // faster; in FP64 the cell coordinates' divisions run on the integer
             // pipes, div_rn)
             const int nxt = 1 - cur;
-            const size_t smem = sizeof(int32_t) * (size_t)(2 * ncell + 1 + 3 * N_);
+            const size_t smem = sizeof(int32_t) * (size_t)(2 * ncell + 1 + N_);
             rt_before_launch(K_RANK);
-            launch_k(k_rebuild_small<T>, dim3(1), dim3(kRebuildSmallThreads), smem, (int)N_,
+            const unsigned nblk = N_ <= kRebuildOneMaxN ? 1u : (unsigned)kRebuildSmallBlocks;
+            auto kr = N_ <= kRebuildSmallThreads ? &k_rebuild_small<T, 1>
+                                                 : &k_rebuild_small<T, kRebuildPer>;
+            launch_cluster(kr, dim3(nblk), dim3(kRebuildSmallThreads), smem, nblk > 1 ? nblk : 0u, (int)N_,
                      (int)ncell, hinst[0], check, (const T2<T> *)pos[cur].p,
                      (const T2<T> *)vel[cur].p, pos[nxt].p, vel[nxt].p, xref.p, perm.p,
                      invperm.p, cellStart.p, ex0, ex0N, ex1, ex1N, flags.p);

@@ -266,22 +266,36 @@ __global__ void k_rank_permute(int64_t N, const int32_t *__restrict__ cellTmp,
     if (ex1) ex1N[dst] = ex1[src];
 }
 
-// The whole cell-list rebuild of a small single state in one block: cells
+// The whole cell-list rebuild of a small single state in one launch: cells
 // and the displacement check (k_assign), the exclusive scan (k_scan_*), the
 // bucket and the in-cell rank by particle id (k_bucket, k_rank_permute), with
 // the histogram, scan and buckets in shared memory. Same arithmetic and the
-// same deterministic order as the multi-launch path; it saves four launches
-// per rebuild when the state is too small to keep the GPU busy anyway.
-// Dynamic shared memory: 4 * (ncell + (ncell + 1) + 3 N) bytes.
+// same deterministic order as the multi-launch path.
+//
+// Its time is a chain of latencies and, in one block, the bandwidth of one SM
+// (ten arrays of the state pass through it). So a cluster of eight blocks runs
+// it: each builds the whole cell list for itself (positions and ids only; the
+// histogram's atomic also gives a particle's place in its cell's bucket) and
+// ranks and writes an eighth of the particles. perm and xref are rewritten in
+// place: a cluster barrier separates the last read from the first write. 2072
+// FP64 particles: the earlier one-block form 14.1 us cold, this form in one block
+// 10.8 us and in eight 7.1 us warm; 1500 FP32 6.5 -> 5.3 us; at 240 particles one
+// block is faster (5.1 against 5.5 us), so up to 512 it runs alone.
+// Dynamic shared memory: 4 * (ncell + (ncell + 1) + N) bytes.
 constexpr int kRebuildSmallThreads = 1024;
+constexpr int kRebuildSmallBlocks = 8;
 constexpr int64_t kRebuildSmallMaxN = 4096;
+constexpr int64_t kRebuildOneMaxN = 512;
 constexpr int64_t kRebuildSmallMaxCells = 8192;
+constexpr int kRebuildPer = (int)(kRebuildSmallMaxN / kRebuildSmallThreads); // or 1
+static_assert(kRebuildSmallMaxN / kRebuildSmallBlocks <= kRebuildSmallThreads,
+              "one particle of a block's share per thread");
 
-template <typename T>
+template <typename T, int PER>
 __global__ void __launch_bounds__(kRebuildSmallThreads)
     k_rebuild_small(int N, int ncell, const Inst<T> I, int check, const T2<T> *__restrict__ pos,
                     const T2<T> *__restrict__ vel, T2<T> *__restrict__ posN,
-                    T2<T> *__restrict__ velN, T2<T> *__restrict__ xref, int32_t *__restrict__ perm,
+                    T2<T> *__restrict__ velN, T2<T> *xref, int32_t *perm,
                     int32_t *__restrict__ invperm, int32_t *__restrict__ cellStart,
                     const T2<T> *__restrict__ ex0, T2<T> *__restrict__ ex0N,
                     const T2<T> *__restrict__ ex1, T2<T> *__restrict__ ex1N,
@@ -289,92 +303,110 @@ __global__ void __launch_bounds__(kRebuildSmallThreads)
 {
     pdl_enter();
     extern __shared__ int32_t sm[];
-    int32_t *cursor = sm;                  // ncell: counts, then running cursors
-    int32_t *starts = cursor + ncell;      // ncell + 1
-    int32_t *cellOf = starts + ncell + 1;  // N
-    int32_t *bucketSrc = cellOf + N;       // N
-    int32_t *bucketId = bucketSrc + N;     // N
-    __shared__ int32_t part[kRebuildSmallThreads / 32 + 1];
-    const int t = (int)threadIdx.x, nt = (int)blockDim.x;
-    for (int c = t; c < ncell; c += nt) cursor[c] = 0;
-    __syncthreads();
-    // cells (x / cs as in cell_index) and the displacement check
-    bool moved = false;
-    for (int i = t; i < N; i += nt) {
-        const T2<T> x = pos[i];
-        if (check) {
-            const T2<T> xr = xref[i];
-            const T d2 = r2_exact<T>(sub_rn(x.x, xr.x), sub_rn(x.y, xr.y));
-            moved = moved || d2 > I.dmax2;
+    int32_t *count = sm;                  // ncell
+    int32_t *starts = count + ncell;      // ncell + 1
+    int32_t *bucket = starts + ncell + 1; // N: ids, in arrival order inside a cell
+    __shared__ int32_t part[kRebuildSmallThreads / 32];
+    const int t = (int)threadIdx.x, blk = (int)blockIdx.x, nblk = (int)gridDim.x; // one cluster
+    constexpr int nt = kRebuildSmallThreads;
+    const auto cell_of = [&](const T2<T> &x) {
+        return I.coff + (cell_div(x.x, I.cs, I.nx) - 1) + (cell_div(x.y, I.cs, I.ny) - 1) * I.nx;
+    };
+    // every particle, for the histogram and the buckets
+    T2<T> x[PER];
+    int32_t id[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+        if (t + u * nt < N) {
+            x[u] = pos[t + u * nt];
+            id[u] = perm[t + u * nt];
         }
-        const int cx = cell_div(x.x, I.cs, I.nx);
-        const int cy = cell_div(x.y, I.cs, I.ny);
-        const int c = I.coff + (cx - 1) + (cy - 1) * I.nx;
-        cellOf[i] = c;
-        atomicAdd(&cursor[c], 1);
+    // the particle this thread writes
+    const int own = N * blk / nblk + t;
+    const bool mine = own < N * (blk + 1) / nblk;
+    T2<T> xo, vo, a, b;
+    int32_t ido = 0;
+    bool moved = false;
+    if (mine) {
+        xo = pos[own];
+        vo = vel[own];
+        ido = perm[own];
+        if (ex0) a = ex0[own];
+        if (ex1) b = ex1[own];
+        if (check) {
+            const T2<T> xr = xref[own];
+            moved = r2_exact<T>(sub_rn(xo.x, xr.x), sub_rn(xo.y, xr.y)) > I.dmax2;
+        }
     }
+    for (int c = t; c < ncell; c += nt) count[c] = 0;
     if (__syncthreads_or(moved) && t == 0) atomicOr(flags, FLAG_DISPLACEMENT);
+    int cell[PER], place[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+        if (t + u * nt < N) {
+            cell[u] = cell_of(x[u]);
+            place[u] = atomicAdd(&count[cell[u]], 1);
+        }
+    __syncthreads();
+    // this block's reads of perm and xref are done
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     // exclusive scan of the counts: each thread sums a contiguous chunk
     const int chunk = (ncell + nt - 1) / nt;
     const int c0 = t * chunk, c1 = c0 + chunk < ncell ? c0 + chunk : ncell;
     int32_t sum = 0;
-    for (int c = c0; c < c1; ++c) sum += cursor[c];
-    int32_t x = sum;
+    for (int c = c0; c < c1; ++c) sum += count[c];
+    int32_t y = sum;
     const int lane = t & 31, warp = t >> 5;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
+        const int32_t z = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) y += z;
     }
-    if (lane == 31) part[warp] = x;
+    if (lane == 31) part[warp] = y;
     __syncthreads();
     if (warp == 0) {
-        const int nw = nt >> 5;
-        int32_t w = lane < nw ? part[lane] : 0, v = w;
+        const int32_t w = part[lane];
+        int32_t v = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int32_t y = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += y;
+            const int32_t z = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += z;
         }
-        if (lane < nw) part[lane] = v - w;
+        part[lane] = v - w;
     }
     __syncthreads();
-    int32_t run = x - sum + part[warp];
+    int32_t run = y - sum + part[warp];
     for (int c = c0; c < c1; ++c) {
-        const int32_t n = cursor[c];
         starts[c] = run;
-        cellStart[c] = run;
-        cursor[c] = run;
-        run += n;
+        if (blk == 0) cellStart[c] = run;
+        run += count[c];
     }
     if (t == 0) {
         starts[ncell] = N;
-        cellStart[ncell] = N;
+        if (blk == 0) cellStart[ncell] = N;
     }
     __syncthreads();
-    // buckets: every particle into its cell's range (arbitrary order inside)
-    for (int i = t; i < N; i += nt) {
-        const int p = atomicAdd(&cursor[cellOf[i]], 1);
-        bucketSrc[p] = i;
-        bucketId[p] = perm[i];
-    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+        if (t + u * nt < N) bucket[starts[cell[u]] + place[u]] = id[u];
     __syncthreads();
     // in-cell rank by particle id, and the data into the new order
-    for (int s = t; s < N; s += nt) {
-        const int src = bucketSrc[s], id = bucketId[s], c = cellOf[src];
-        const int b = starts[c], e = starts[c + 1];
+    int dst = 0;
+    if (mine) {
+        const int c = cell_of(xo), s0 = starts[c], s1 = starts[c + 1];
         int rank = 0;
-        for (int k = b; k < e; ++k) rank += bucketId[k] < id ? 1 : 0;
-        const int dst = b + rank;
-        perm[dst] = id;
-        const T2<T> xs = pos[src];
-        posN[dst] = xs;
-        xref[dst] = xs;
-        velN[dst] = vel[src];
-        invperm[id] = dst;
-        if (ex0) ex0N[dst] = ex0[src];
-        if (ex1) ex1N[dst] = ex1[src];
+        for (int k = s0; k < s1; ++k) rank += bucket[k] < ido ? 1 : 0;
+        dst = s0 + rank;
     }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (!mine) return;
+    perm[dst] = ido;
+    posN[dst] = xo;
+    xref[dst] = xo;
+    velN[dst] = vo;
+    invperm[ido] = dst;
+    if (ex0) ex0N[dst] = a;
+    if (ex1) ex1N[dst] = b;
 }
 
 // _nl_build! (src/neighbors.jl:192-245): the scan centre uses x * invcs as
