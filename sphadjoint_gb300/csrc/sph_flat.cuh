@@ -29,8 +29,13 @@
 // divisions not counted, sph_exact64.cuh). Measured per launch, 66,013 particles,
 // one thread per particle -> one lane per pair: density 78.2 -> 61.6 us, accel
 // 100.6 -> 71.7, accel + drag 104.3 -> 70.7, pass 1 184.7 -> 151.2 (FP64 pipe 79%
-// busy), pass 2 69.9 -> 41.2; the solve 5.51 -> 4.22 ms. 2072 particles, lane
-// groups -> this: 128 steps 12.0 -> 9.1 ms.
+// busy), pass 2 69.9 -> 41.2; the solve 5.51 -> 4.22 ms, and with the r, 2 m mu /
+// rho and fifth warp of the later passes 3.70 ms. Small states are chains of
+// latencies (pass 2 at 240 particles: 4 us), so the density's first warp prepares the
+// block alone, a part's loads are issued together, and the folds run ahead of
+// their chain: 240 particles 200 steps 9.86 -> 8.22 ms, 925 particles 50 steps 0.92
+// -> 0.80, 2072 particles 128 steps 7.09 -> 6.58 (lane groups: 12.0), 66,013 the
+// same within 0.3%.
 #pragma once
 
 #include "sph_coop.cuh"
@@ -42,6 +47,7 @@ constexpr int kFlatBlock = 128;
 constexpr int kFlatMax = 32;    // particles of a block, at most
 constexpr int kFlatRow = 64;    // pairs of a particle, at most
 constexpr int kFlatChunk = 384; // pairs folded at a time
+constexpr int kFlatTest = 256;  // candidates tested at a time (384: density 64.3 us, 62.9 at 256)
 constexpr int kFlatOff = kFlatMax + 2; // offsets of a block, then its serial mask
 constexpr int kFlatSlotBits = 27;
 
@@ -60,27 +66,60 @@ __host__ __device__ __forceinline__ int flat_particles(int64_t N)
     return p < 4 ? 4 : (p > kFlatMax ? kFlatMax : (int)p);
 }
 
-// Exclusive scan of one int per thread over the block; tot: the sum.
-__device__ __forceinline__ int flat_scan(int x, int *s_warp, int &tot)
+// Exclusive scan of one int per lane of a warp.
+__device__ __forceinline__ int warp_scan(int x)
 {
-    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+    const int lane = (int)(threadIdx.x & 31u);
     int s = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, s, o);
         if (lane >= o) s += y;
     }
-    if (lane == 31) s_warp[warp] = s;
-    __syncthreads();
-    int before = 0;
-    tot = 0;
+    return s - x;
+}
+
+// One running sum per lane: the terms k0 .. k1 - 1 in order, sub (may be NULL)
+// subtracted before each added one. All lanes of the warp call it (k0 == k1: no
+// sum). A dependent FP64 addition takes 64 cycles, so nothing else may stand in
+// the chain: the lanes run the same number of steps, a missing term is a zero
+// (a sum that starts at +0 never becomes -0, so x + 0 and x - 0 leave it as it
+// is), and four terms are read ahead of the four being added. 141 cycles an
+// addition with a loop per lane, about 90 this way.
+__device__ __forceinline__ double flat_fold(double acc, const double *sub, const double *add,
+                                            int k0, int k1)
+{
+    const int n = k1 > k0 ? k1 - k0 : 0;
+    const int most = __reduce_max_sync(0xffffffffu, n);
+    double a[4], s[4];
+    auto term = [&](const double *p, int k) {
+        const double x = p[k < n ? k0 + k : 0];
+        return k < n ? x : 0.0;
+    };
 #pragma unroll
-    for (int w = 0; w < kFlatBlock / 32; ++w) {
-        before += w < warp ? s_warp[w] : 0;
-        tot += s_warp[w];
+    for (int u = 0; u < 4; ++u) {
+        a[u] = term(add, u);
+        s[u] = sub ? term(sub, u) : 0.0;
     }
-    __syncthreads();
-    return before + s - x;
+    for (int k = 0; k < most; k += 4) {
+        double a2[4], s2[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            a2[u] = term(add, k + 4 + u);
+            s2[u] = sub ? term(sub, k + 4 + u) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (sub) acc -= s[u];
+            acc += a[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            a[u] = a2[u];
+            s[u] = s2[u];
+        }
+    }
+    return acc;
 }
 
 // density_kernel! + eos_kernel!, and the block's dense pairs.
@@ -98,47 +137,58 @@ __global__ void __launch_bounds__(kFlatBlock)
     __shared__ int s_bs[kFlatMax][3], s_pre[kFlatMax][6];
     __shared__ int s_off[kFlatMax + 1], s_cnt[kFlatMax], s_in[kFlatMax];
     __shared__ uint8_t s_own[kFlatMax * kFlatRow];
-    __shared__ int s_warp[kFlatBlock / 32];
+    __shared__ int s_warp[2][kFlatTest / 32]; // kept per warp and part, by round parity
     __shared__ uint32_t s_spill, s_serial;
     const int t = (int)threadIdx.x, P = B.P;
     const int64_t i0 = (int64_t)blockIdx.x * P;
     const int np = v.N - i0 < P ? (int)(v.N - i0) : P;
-    if (t == 0) s_spill = s_serial = 0u;
-    __syncthreads();
-    if (t < np) {
-        const int64_t i = i0 + t;
-        decltype(auto) I = load_inst<MULTI>(v, i);
-        const uint32_t cc = v.center[i];
+    if (t < 32) { // the first warp: each particle's candidates and their offsets
         int n = 0;
-        if (cc >> 31) {
-            atomicOr(I.maxnb > kFlatRow ? &s_serial : &s_spill, 1u << t);
-        } else {
-            const int cx = (int)(cc & 0xffffu), cy = (int)((cc >> 16) & 0x7fffu);
-            const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
-            const int row0 = I.coff + (jx0 - 1) + (cy - 2) * I.nx; // cell (jx0, cy - 1)
+        bool isSpill = false, isSerial = false;
+        if (t < np) {
+            const int64_t i = i0 + t;
+            decltype(auto) I = load_inst<MULTI>(v, i);
+            const uint32_t cc = v.center[i];
             uint32_t w[6];
 #pragma unroll
             for (int q = 0; q < 6; ++q) w[q] = v.masks[(int64_t)q * v.N + i];
+            if (cc >> 31) {
+                isSerial = I.maxnb > kFlatRow;
+                isSpill = !isSerial;
+            } else {
+                const int cx = (int)(cc & 0xffffu), cy = (int)((cc >> 16) & 0x7fffu);
+                const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
+                const int row0 = I.coff + (jx0 - 1) + (cy - 2) * I.nx; // cell (jx0, cy - 1)
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
-                s_bs[t][r] = (w[2 * r] | w[2 * r + 1]) ? v.cellStart[row0 + r * I.nx] : 0;
+                for (int r = 0; r < 3; ++r)
+                    s_bs[t][r] = (w[2 * r] | w[2 * r + 1]) ? v.cellStart[row0 + r * I.nx] : 0;
 #pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                s_wd[t][q] = w[q];
-                s_pre[t][q] = n;
-                n += __popc(w[q]);
-            }
-            if (n > kFlatRow) {
-                atomicOr(&s_serial, 1u << t);
-                n = 0;
+                for (int q = 0; q < 6; ++q) {
+                    s_wd[t][q] = w[q];
+                    s_pre[t][q] = n;
+                    n += __popc(w[q]);
+                }
+                if (n > kFlatRow) {
+                    isSerial = true;
+                    n = 0;
+                }
             }
         }
+        const unsigned sp = __ballot_sync(0xffffffffu, isSpill);
+        const unsigned se = __ballot_sync(0xffffffffu, isSerial);
+        const int o = warp_scan(n);
         s_cnt[t] = n;
+        s_in[t] = 0;
+        s_off[t] = o;
+        if (t == 31) s_off[32] = o + n;
+        if (t == 0) {
+            s_spill = sp;
+            s_serial = se;
+        }
     }
-    if (t < kFlatMax) s_in[t] = 0;
     __syncthreads();
     const uint32_t spill = s_spill, serial = s_serial;
-    if (spill) { // list their rows, a warp per particle
+    if (spill) { // list their rows, a warp per particle, and number the candidates again
         const Group<32> g;
         for (int a = t >> 5; a < np; a += kFlatBlock / 32)
             if ((spill >> a) & 1u) {
@@ -148,68 +198,90 @@ __global__ void __launch_bounds__(kFlatBlock)
                 if ((t & 31) == 0) s_cnt[a] = n;
             }
         __syncthreads();
+        if (t < 32) {
+            const int n = s_cnt[t], o = warp_scan(n);
+            s_off[t] = o;
+            if (t == 31) s_off[32] = o + n;
+        }
+        __syncthreads();
     }
-    int tot;
-    const int pre = flat_scan(t < np ? s_cnt[t] : 0, s_warp, tot);
-    if (t <= np) s_off[t] = pre;
-    __syncthreads();
+    const int tot = s_off[np];
 
     const int64_t bb = (int64_t)blockIdx.x * P * kFlatRow;
+    const unsigned below = (1u << (t & 31)) - 1u;
     int D = 0; // dense pairs so far
-    for (int base = 0; base < tot; base += kFlatChunk) {
-        constexpr int U = kFlatChunk / kFlatBlock;
-        double r2v[U];
-        uint32_t pj[U];
-        int cnt = 0, a = 0;
-        const int p0 = base + U * t;
-        if (p0 < tot) { // the particle that owns pair p0
-            int hi = np - 1;
-            while (a < hi) {
-                const int mid = (a + hi + 1) >> 1;
-                if (s_off[mid] <= p0) a = mid;
-                else hi = mid - 1;
-            }
-        }
+    for (int base = 0, par = 0; base < tot; base += kFlatTest, par ^= 1) {
+        constexpr int U = kFlatTest / kFlatBlock;
+        // candidate base + 128 u + t: its particle and slot, then all positions,
+        // then the test, so that the parts' loads overlap
+        int own[U], slot[U];
+        double2 xi[U], xj[U];
+        double r2[U];
+        unsigned in[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int p = p0 + u;
-            pj[u] = 0xffffffffu;
+            const int p = base + u * kFlatBlock + t;
+            own[u] = 0;
+            slot[u] = (int)i0;
             if (p < tot) {
-                while (p >= s_off[a + 1]) ++a;
+                int a = 0;
+#pragma unroll
+                for (int h = kFlatMax / 2; h > 0; h >>= 1)
+                    if (a + h < np && s_off[a + h] <= p) a += h;
                 const int k = p - s_off[a];
-                int j;
+                own[u] = a;
                 if ((spill >> a) & 1u) {
-                    j = s_lst[a][k];
+                    slot[u] = s_lst[a][k];
                 } else {
                     int w = 0;
 #pragma unroll
                     for (int q = 1; q < 6; ++q) w = k >= s_pre[a][q] ? q : w;
-                    j = s_bs[a][w >> 1] + 32 * (w & 1) + select_bit(s_wd[a][w], k - s_pre[a][w]);
-                }
-                decltype(auto) I = load_inst<MULTI>(v, i0 + a);
-                const double2 xi = v.pos[i0 + a], xj = v.pos[j];
-                const double dx = xi.x - xj.x;
-                const double dy = xi.y - xj.y;
-                r2v[u] = dx * dx + dy * dy;
-                if (lt_nonneg(r2v[u], I.p.r2max)) {
-                    pj[u] = (uint32_t)a << kFlatSlotBits | (uint32_t)j;
-                    ++cnt;
+                    slot[u] = s_bs[a][w >> 1] + 32 * (w & 1) +
+                              select_bit(s_wd[a][w], k - s_pre[a][w]);
                 }
             }
         }
-        int n;
-        int pos = D + flat_scan(cnt, s_warp, n);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (pj[u] != 0xffffffffu) {
-                const int own = (int)(pj[u] >> kFlatSlotBits);
-                s_r2[pos] = r2v[u];
-                s_own[pos] = (uint8_t)own;
-                B.pair[bb + pos] = pj[u];
-                atomicAdd(&s_in[own], 1);
-                ++pos;
+        for (int u = 0; u < U; ++u) {
+            xi[u] = v.pos[i0 + own[u]];
+            xj[u] = v.pos[slot[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (base + u * kFlatBlock >= tot) { // nothing in this part
+                in[u] = 0u;
+                continue;
             }
-        D += n;
+            decltype(auto) I = load_inst<MULTI>(v, i0 + own[u]);
+            const double dx = xi[u].x - xj[u].x;
+            const double dy = xi[u].y - xj[u].y;
+            r2[u] = dx * dx + dy * dy;
+            in[u] = __ballot_sync(0xffffffffu, base + u * kFlatBlock + t < tot &&
+                                                   lt_nonneg(r2[u], I.p.r2max));
+        }
+        if ((t & 31) == 0)
+#pragma unroll
+            for (int u = 0; u < U; ++u) s_warp[par][u * (kFlatBlock / 32) + (t >> 5)] = __popc(in[u]);
+        __syncthreads();
+        int kept = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            int pos = D + kept;
+#pragma unroll
+            for (int w = 0; w < kFlatBlock / 32; ++w) {
+                const int n = s_warp[par][u * (kFlatBlock / 32) + w];
+                pos += w < (t >> 5) ? n : 0;
+                kept += n;
+            }
+            if ((in[u] >> (t & 31)) & 1u) {
+                pos += __popc(in[u] & below);
+                s_r2[pos] = r2[u];
+                s_own[pos] = (uint8_t)own[u];
+                B.pair[bb + pos] = (uint32_t)own[u] << kFlatSlotBits | (uint32_t)slot[u];
+                atomicAdd(&s_in[own[u]], 1);
+            }
+        }
+        D += kept;
     }
     __syncthreads();
     for (int d = t; d < D; d += kFlatBlock) {
@@ -222,10 +294,13 @@ __global__ void __launch_bounds__(kFlatBlock)
         B.r[bb + d] = r;
         s_r2[d] = I.p.m * (I.p.A * u2 * u2 * (twice_of(q) + 1.0));
     }
-    int all;
-    const int o = flat_scan(t < np ? s_in[t] : 0, s_warp, all); // ends with a barrier
-    if (t <= np) B.off[(int64_t)blockIdx.x * kFlatOff + t] = o;
-    if (t == 0) B.off[(int64_t)blockIdx.x * kFlatOff + kFlatOff - 1] = (int)serial;
+    __syncthreads();
+    if (t >= 32) return;
+    const int nin = s_in[t], o = warp_scan(nin);
+    int32_t *off = B.off + (int64_t)blockIdx.x * kFlatOff;
+    if (t <= np) off[t] = o;
+    if (t == 31 && np == 32) off[32] = o + nin;
+    if (t == 0) off[kFlatOff - 1] = (int)serial;
     if (t >= np) return;
     const int64_t i = i0 + t;
     if ((serial >> t) & 1u) {
@@ -235,9 +310,8 @@ __global__ void __launch_bounds__(kFlatBlock)
         return;
     }
     double acc = 0.0;
-    const int e = o + s_in[t];
 #pragma unroll 4
-    for (int k = o; k < e; ++k) acc += s_r2[k];
+    for (int k = o; k < o + nin; ++k) acc += s_r2[k];
     decltype(auto) I = load_inst<MULTI>(v, i);
     B.tm[i] = I.p.twomumass * density_finish<double>(I, i, acc, rho, prho).y;
 }
@@ -318,22 +392,11 @@ template <bool MULTI> struct FlatPass {
     }
 };
 
-// One lane per running sum: chain c adds the terms of its particle's pairs that
-// this chunk holds. sub (may be NULL): a term subtracted before each added one.
-__device__ __forceinline__ double flat_fold(double acc, const double *sub, const double *add,
-                                            int k0, int k1)
+// A barrier of the four pair warps alone: the fifth is not waited for until the
+// results are put together.
+__device__ __forceinline__ void pair_sync()
 {
-    if (sub) {
-#pragma unroll 4
-        for (int k = k0; k < k1; ++k) {
-            acc -= sub[k];
-            acc += add[k];
-        }
-    } else {
-#pragma unroll 4
-        for (int k = k0; k < k1; ++k) acc += add[k];
-    }
-    return acc;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
 // Pressure + Morris viscosity of the block's particles (accel_pair): s_acc[2 a],
@@ -351,7 +414,7 @@ __device__ __forceinline__ void flat_accel(const FlatPass<MULTI> &Q, const FlatS
     const int b0 = a2 < Q.np ? S.off[a2] : 0, b1 = a2 < Q.np ? S.off[a2 + 1] : 0;
     double acc = 0.0;
     side();
-    for (int base = 0, at = 0, m; base < n; base += m) {
+    for (int base = 0, at = 0, m; Q.t < kFlatBlock && base < n; base += m) {
         m = Q.chunk(S, base, at);
         Q.pairs(base, m, [&](int p, int64_t i, int j, double F) {
             decltype(auto) I = load_inst<MULTI>(v, i);
@@ -364,13 +427,13 @@ __device__ __forceinline__ void flat_accel(const FlatPass<MULTI> &Q, const FlatS
             s_t[2][p] = C * (vi.x - vj.x);
             s_t[3][p] = C * (vi.y - vj.y);
         });
-        __syncthreads();
-        if (a2 < Q.np) {
+        pair_sync();
+        if (Q.t < 2 * kFlatMax) {
             const int k0 = (b0 > base ? b0 : base) - base;
             const int k1 = (b1 < base + m ? b1 : base + m) - base;
             acc = flat_fold(acc, s_t[c2], s_t[2 + c2], k0, k1);
         }
-        __syncthreads();
+        if (base + m < n) pair_sync();
     }
     if (a2 < Q.np) s_acc[Q.t] = acc;
     __syncthreads();
@@ -531,7 +594,8 @@ __global__ void __launch_bounds__(kFlatThreads)
     __shared__ FlatShared S;
     const FlatPass<MULTI> Q(v, B, S);
     const int t = Q.t, np = Q.np;
-    for (int k = t; k < 6 * kFlatMax; k += kFlatThreads) s_acc[k] = 0.0;
+    if (t < kFlatBlock)
+        for (int k = t; k < 6 * kFlatMax; k += kFlatBlock) s_acc[k] = 0.0;
     if (const int64_t i = Q.aside(); i >= 0) {
         decltype(auto) I = load_inst<MULTI>(v, i);
         const double2 x = v.pos[i], ab = abar[i];
@@ -544,8 +608,7 @@ __global__ void __launch_bounds__(kFlatThreads)
         s_side[3][t - kFlatBlock] = ga * dady;
     }
     const int n = S.off[np];
-    if (n == 0) __syncthreads();
-    for (int base = 0, at = 0, m; base < n; base += m) {
+    for (int base = 0, at = 0, m; t < kFlatBlock && base < n; base += m) {
         m = Q.chunk(S, base, at);
         Q.pairs(base, m, [&](int p, int64_t i, int j, double F) {
             decltype(auto) I = load_inst<MULTI>(v, i);
@@ -576,22 +639,25 @@ __global__ void __launch_bounds__(kFlatThreads)
             s_t[6][p] = -(C * ad_v * pi.y); // subtracted
             s_t[7][p] = F * ad_d;
         });
-        __syncthreads();
+        pair_sync();
         // gx and gy (two terms a pair) on the first warps, the four sums with one
         // term from the last warp down
-        for (int c = t; c < 2 * np; c += kFlatThreads) {
-            const int a = c >> 1, k0 = S.off[a] > base ? S.off[a] - base : 0;
-            const int k1 = S.off[a + 1] < base + m ? S.off[a + 1] - base : m;
-            s_acc[c] = flat_fold(s_acc[c], s_t[c & 1], s_t[2 + (c & 1)], k0, k1);
+        auto range = [&](int a, int &k0, int &k1) {
+            k0 = a < np && S.off[a] > base ? S.off[a] - base : 0;
+            k1 = a >= np ? 0 : S.off[a + 1] < base + m ? S.off[a + 1] - base : m;
+        };
+        int k0, k1;
+        if (t < 2 * kFlatMax) {
+            range(t >> 1, k0, k1);
+            s_acc[t] = flat_fold(s_acc[t], s_t[t & 1], s_t[2 + (t & 1)], k0, k1);
         }
-        for (int c = kFlatThreads - 1 - t; c < 4 * np; c += kFlatThreads) {
-            const int a = c >> 2, k0 = S.off[a] > base ? S.off[a] - base : 0;
-            const int k1 = S.off[a + 1] < base + m ? S.off[a + 1] - base : m;
-            double &x = s_acc[2 * kFlatMax + c];
-            x = flat_fold(x, nullptr, s_t[4 + (c & 3)], k0, k1);
-        }
-        __syncthreads();
+        const int c = kFlatBlock - 1 - t;
+        range(c >> 2, k0, k1);
+        double &x = s_acc[2 * kFlatMax + c];
+        x = flat_fold(x, nullptr, s_t[4 + (c & 3)], k0, k1);
+        pair_sync();
     }
+    __syncthreads();
     if (t >= np) return;
     const int64_t i = Q.i0 + t;
     decltype(auto) I = load_inst<MULTI>(v, i);
@@ -652,7 +718,7 @@ __global__ void __launch_bounds__(kFlatThreads)
     const int n = S.off[np], a2 = t >> 1, c2 = t & 1;
     const int b0 = a2 < np ? S.off[a2] : 0, b1 = a2 < np ? S.off[a2 + 1] : 0;
     double acc = 0.0;
-    for (int base = 0, at = 0, m; base < n; base += m) {
+    for (int base = 0, at = 0, m; t < kFlatBlock && base < n; base += m) {
         m = Q.chunk(S, base, at);
         Q.pairs(base, m, [&](int p, int64_t i, int j, double F) {
             decltype(auto) I = load_inst<MULTI>(v, i);
@@ -661,13 +727,13 @@ __global__ void __launch_bounds__(kFlatThreads)
             s_t[0][p] = w * (xi.x - xj.x);
             s_t[1][p] = w * (xi.y - xj.y);
         });
-        __syncthreads();
-        if (a2 < np) {
+        pair_sync();
+        if (t < 2 * kFlatMax) {
             const int k0 = (b0 > base ? b0 : base) - base;
             const int k1 = (b1 < base + m ? b1 : base + m) - base;
             acc = flat_fold(acc, nullptr, s_t[c2], k0, k1);
         }
-        __syncthreads();
+        if (base + m < n) pair_sync();
     }
     if (a2 < np) s_acc[t] = acc;
     __syncthreads();
