@@ -609,6 +609,8 @@ static void tape_sizes(const Params *p, int64_t N, int32_t dtype, double skin, i
     const int64_t ncell = nx * ny;
     *snap = 5 * align256(2 * s * n1) + 3 * align256(4 * n1) + align256(24 * n1) +
             align256(4 * (ncell + 1));
+    // (of the 8 bytes a cell 4 are spare since the bucket cursors are gone: plans
+    // made earlier stay what they were)
     *recomp = *snap + (16 + 24 + 6 * s) * n1 + 8 * ncell + 4 * (ncell / 2048 + 2) + 4;
 }
 

@@ -272,23 +272,6 @@ inline void check_params(const Params &p)
 // the model reads per-particle densities (Tait derivative, viscosity average)
 inline bool needs_rho(const Params &p) { return p.eos == 1 || p.visc == 1; }
 
-// exclusive scan of n int32 -> out[0..n] (+ optional copy); tmp >= blocks
-inline void scan_excl(const int32_t *in, int64_t n, int32_t *out, int32_t *out2, int32_t *tmp)
-{
-    const int64_t nb = (n + kScanTile - 1) / kScanTile;
-    if (nb <= 1) {
-        rt_before_launch(K_SCAN);
-        launch_k(k_scan_down, dim3(1), dim3(kBlock), 0, in, n, (const int32_t *)nullptr, out, out2);
-        rt_after_launch(K_SCAN);
-        return;
-    }
-    rt_before_launch(K_SCAN);
-    launch_k(k_scan_reduce, dim3((unsigned)nb), dim3(kBlock), 0, in, n, tmp);
-    launch_k(k_scan_top, dim3(1), dim3(1024), 0, tmp, nb);
-    launch_k(k_scan_down, dim3((unsigned)nb), dim3(kBlock), 0, in, n, (const int32_t *)tmp, out, out2);
-    rt_after_launch(K_SCAN);
-}
-
 // The design field theta of one instance, or the packed fields of a batch
 // (instance b's (ngy, ngx) column-major block at node offset off[b]).
 template <typename T> class Field final : public FieldI {
@@ -358,7 +341,7 @@ template <typename T> class Sys final : public StateI {
     DevBuf<T2<T>> pos[2], vel[2];
     int cur = 0;
     DevBuf<T2<T>> xref;
-    DevBuf<int32_t> perm, invperm, cellStart, nbcount, cellTmp, counts, cursor, bucketSrc,
+    DevBuf<int32_t> perm, invperm, cellStart, nbcount, cellTmp, counts, bucketSrc,
         bucketId, scanTmp;
     DevBuf<uint32_t> center, flags;
     DevBuf<uint32_t> masks;  // 6 words per particle, word-major
@@ -506,10 +489,11 @@ template <typename T> class Sys final : public StateI {
         nbcount.alloc(n1);
         cellTmp.alloc(n1);
         counts.alloc((size_t)ncell);
-        cursor.alloc((size_t)ncell);
+        counts.zero(); // and zero again after every cell list
         bucketSrc.alloc(n1);
         bucketId.alloc(n1);
         scanTmp.alloc((size_t)((ncell + kScanTile - 1) / kScanTile + 1));
+        scanTmp.zero();
         flags.alloc((size_t)B);
         tmask.alloc(6 * n1);
         // staged windows end on multiples of four slots: room for three more
@@ -764,6 +748,23 @@ template <typename T> class Sys final : public StateI {
         }
     }
 
+    // cells, starts and buckets of the current positions; place: N ints of scratch
+    void bucket_cells(int check, int32_t *place, int32_t *starts)
+    {
+        auto ka = B > 1 ? &k_assign<T, true> : &k_assign<T, false>;
+        SPH_LAUNCH(K_ASSIGN, ka, N_, N_, pos[cur].p, xref.p, check, hinst[0], dinst.p, pinst.p,
+                   cellTmp.p, counts.p, scanTmp.p, place, flags.p);
+        const int64_t nb = (ncell + kScanTile - 1) / kScanTile;
+        const int summed = nb > kScanSelf ? 1 : 0;
+        rt_before_launch(K_SCAN);
+        if (summed) launch_k(k_scan_top, dim3(1), dim3(1024), 0, scanTmp.p, nb);
+        launch_k(k_scan_cells, dim3((unsigned)nb), dim3(kBlock), 0, counts.p, ncell,
+                 (const int32_t *)scanTmp.p, summed, starts);
+        rt_after_launch(K_SCAN);
+        SPH_LAUNCH(K_BUCKET, k_bucket, N_, N_, cellTmp.p, place, starts, perm.p, bucketSrc.p,
+                   bucketId.p, scanTmp.p, nb);
+    }
+
     // build_neighbors! (src/neighbors.jl:252-263): cell list, permutation of
     // the particle data (and of up to two extra per-particle arrays) into the
     // new cell order, neighbour masks. ex*N receive the permuted extras.
@@ -790,12 +791,8 @@ template <typename T> class Sys final : public StateI {
             cur = nxt;
             build_masks();
         } else if (N_ > 0) {
-            counts.zero();
-            auto ka = B > 1 ? &k_assign<T, true> : &k_assign<T, false>;
-            SPH_LAUNCH(K_ASSIGN, ka, N_, N_, pos[cur].p, xref.p, check, hinst[0], dinst.p, pinst.p,
-                       cellTmp.p, counts.p, flags.p);
-            scan_excl(counts.p, ncell, cellStart.p, cursor.p, scanTmp.p);
-            SPH_LAUNCH(K_BUCKET, k_bucket, N_, N_, cellTmp.p, perm.p, cursor.p, bucketSrc.p, bucketId.p);
+            // nbcount is rewritten by the mask build: until then it holds the places
+            bucket_cells(check, nbcount.p, cellStart.p);
             const int nxt = 1 - cur;
             SPH_LAUNCH(K_RANK, k_rank_permute<T>, N_, N_, cellTmp.p, cellStart.p, bucketSrc.p,
                        bucketId.p, pos[cur].p, vel[cur].p, pos[nxt].p, vel[nxt].p, xref.p, perm.p,
@@ -844,12 +841,7 @@ template <typename T> class Sys final : public StateI {
             clOrder.alloc((size_t)std::max<int64_t>(N_, 1));
         }
         if (N_ > 0) {
-            counts.zero();
-            auto ka = B > 1 ? &k_assign<T, true> : &k_assign<T, false>;
-            SPH_LAUNCH(K_ASSIGN, ka, N_, N_, pos[cur].p, xref.p, 0, hinst[0], dinst.p, pinst.p,
-                       cellTmp.p, counts.p, flags.p);
-            scan_excl(counts.p, ncell, clStart.p, cursor.p, scanTmp.p);
-            SPH_LAUNCH(K_BUCKET, k_bucket, N_, N_, cellTmp.p, perm.p, cursor.p, bucketSrc.p, bucketId.p);
+            bucket_cells(0, clOrder.p, clStart.p);
             SPH_LAUNCH(K_RANK, k_rank_permute<T>, N_, N_, cellTmp.p, clStart.p, bucketSrc.p,
                        bucketId.p, pos[cur].p, vel[cur].p, (T2<T> *)nullptr, (T2<T> *)nullptr,
                        (T2<T> *)nullptr, clOrder.p, (int32_t *)nullptr, (const T2<T> *)nullptr,

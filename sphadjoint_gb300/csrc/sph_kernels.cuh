@@ -170,18 +170,79 @@ static __global__ void k_scan_down(const int32_t *__restrict__ in, int64_t n,
 // ---------------------------------------------------------------------------
 // Cell list: _cl_assign! / cumsum! / _cl_fill! / _cl_sort_cells!
 // (src/neighbors.jl:44-114), fused with the permutation of particle data into
-// the new cell order.
+// the new cell order. Four launches: cells and histogram (k_assign), starts
+// (k_scan_cells), buckets (k_bucket), in-cell rank and permutation
+// (k_rank_permute). The counters are zero before the first and after the last of
+// them: the scan clears the counts it has read, the bucket pass the tile sums.
+// Bound by the launches' latencies up to some 200k particles, by its memory
+// traffic beyond. With a memset, a sum and a top pass of the scan as launches of
+// their own (seven in all) and cursors counted by atomics in the bucket pass,
+// kernel times without the gaps: 20,000 particles 19.2 us, 249,001 23.5, 1,048,576
+// 42.5; so: 13.0, 17.2, 35.6. 16 steps of 20,000 particles 303 -> 274 us, a
+// 249,001-particle solve 2.05 -> 1.98 ms.
 // ---------------------------------------------------------------------------
 
-// Cell of every particle (division form x / cs as in cell_index), warp-
-// aggregated histogram, and the displacement check of _nl_build!
-// (src/neighbors.jl:207-213) against the previous rebuild positions. Cells are
-// numbered in the packed table (instance offset + local cell).
+// Cell of a particle (division form x / cs as in cell_index) in the packed
+// table (instance offset + local cell), and the displacement check of _nl_build!
+// (src/neighbors.jl:207-213) against its position of the previous rebuild.
+template <typename T, typename IT>
+__device__ __forceinline__ int32_t assign_cell(const IT &I, const T2<T> &x, bool check,
+                                               const T2<T> *__restrict__ xref,
+                                               uint32_t *__restrict__ flags)
+{
+    if (check) {
+        const T2<T> xr = *xref;
+        const T d2 = r2_exact<T>(sub_rn(x.x, xr.x), sub_rn(x.y, xr.y));
+        if (d2 > I.dmax2) atomicOr(flags, FLAG_DISPLACEMENT);
+    }
+    const T cs = I.cs;
+    const int cx = cell_div(x.x, cs, I.nx);
+    const int cy = cell_div(x.y, cs, I.ny);
+    return I.coff + (cx - 1) + (cy - 1) * I.nx;
+}
+
+// Warp-aggregated histogram: the particle's place in its cell's bucket (order of
+// arrival) and the sums of the scan's tiles. A block's particles lie in one or two
+// tiles: those in its first one's tile are added at once (k_assign of 249,001
+// particles, on a dozen tiles: 4.9 us; with an atomic per warp 7.7). All threads
+// call it.
+__device__ __forceinline__ void count_cell(bool live, int32_t c, int64_t i,
+                                           int32_t *__restrict__ counts,
+                                           int32_t *__restrict__ tiles,
+                                           int32_t *__restrict__ place)
+{
+    __shared__ int32_t s_tile;
+    const int lane = (int)lane_id();
+    const int32_t tile = live ? c / kScanTile : -1;
+    if (threadIdx.x == 0) s_tile = tile; // live: a block has a particle
+    const unsigned act = __ballot_sync(0xffffffffu, live);
+    unsigned peers = 0;
+    int32_t base = 0;
+    if (live) { // the atomic's result is read at the end
+        peers = __match_any_sync(act, c);
+        if (lane == __ffs(peers) - 1) base = atomicAdd(counts + c, __popc(peers));
+    }
+    __syncthreads();
+    const int32_t first = s_tile;
+    const int n = __syncthreads_count(live && tile == first);
+    if (threadIdx.x == 0) atomicAdd(tiles + first, n);
+    const unsigned rest = __ballot_sync(0xffffffffu, live && tile != first);
+    if (live && tile != first) {
+        const unsigned same = __match_any_sync(rest, tile);
+        if (lane == __ffs(same) - 1) atomicAdd(tiles + tile, __popc(same));
+    }
+    if (live) {
+        base = __shfl_sync(peers, base, __ffs(peers) - 1);
+        place[i] = base + __popc(peers & ((1u << lane) - 1u));
+    }
+}
+
 template <typename T, bool MULTI>
 __global__ void k_assign(int64_t N, const T2<T> *__restrict__ pos, const T2<T> *__restrict__ xref,
                          int check, const Inst<T> one, const Inst<T> *__restrict__ inst,
                          const uint16_t *__restrict__ pinst, int32_t *__restrict__ cellTmp,
-                         int32_t *__restrict__ counts, uint32_t *__restrict__ flags)
+                         int32_t *__restrict__ counts, int32_t *__restrict__ tiles,
+                         int32_t *__restrict__ place, uint32_t *__restrict__ flags)
 {
     pdl_enter();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -190,45 +251,110 @@ __global__ void k_assign(int64_t N, const T2<T> *__restrict__ pos, const T2<T> *
     if (live) {
         const int b = MULTI ? (int)pinst[i] : 0;
         decltype(auto) I = pick_inst<MULTI>(one, inst, b);
-        const T2<T> x = pos[i];
-        if (check) {
-            const T2<T> xr = xref[i];
-            const T d2 = r2_exact<T>(sub_rn(x.x, xr.x), sub_rn(x.y, xr.y));
-            if (d2 > I.dmax2) atomicOr(flags + b, FLAG_DISPLACEMENT);
-        }
-        const T cs = I.cs;
-        const int cx = cell_div(x.x, cs, I.nx);
-        const int cy = cell_div(x.y, cs, I.ny);
-        c = I.coff + (cx - 1) + (cy - 1) * I.nx;
+        c = assign_cell<T>(I, pos[i], check, xref + i, flags + b);
         cellTmp[i] = c;
     }
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    if (live) {
-        const unsigned peers = __match_any_sync(act, c);
-        if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(counts + c, __popc(peers));
+    count_cell(live, c, i, counts, tiles, place);
+}
+
+// Starts of tile b's cells: its own exclusive scan behind the sums of the tiles
+// before it, which the block adds up itself (at most kScanSelf of them; beyond,
+// k_scan_top has made tiles[b] that sum). Clears the counts.
+constexpr int64_t kScanSelf = 4096;
+__device__ __forceinline__ void scan_cells(int32_t *__restrict__ counts, int64_t n,
+                                           const int32_t *__restrict__ tiles, bool summed,
+                                           int64_t b, int32_t *__restrict__ out)
+{
+    __shared__ int32_t sw[33], s_before[kBlock / 32];
+    constexpr int IPT = kScanTile / kBlock;
+    static_assert(IPT == 8, "two 16-byte words per thread");
+    const int64_t base = b * kScanTile + (int64_t)threadIdx.x * IPT;
+    const bool full = base + IPT <= n;
+    int32_t v[IPT];
+    if (full) {
+        int4 *p = reinterpret_cast<int4 *>(counts + base);
+        const int4 x = p[0], y = p[1];
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+        v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+        p[0] = p[1] = make_int4(0, 0, 0, 0);
+    } else {
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) {
+            v[k] = base + k < n ? counts[base + k] : 0;
+            if (base + k < n) counts[base + k] = 0;
+        }
     }
+    int32_t before = 0;
+    if (!summed) {
+        for (int64_t k = threadIdx.x; k < b; k += kBlock) before += tiles[k];
+    } else if (threadIdx.x == 0) {
+        before = tiles[b];
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane_id() == 0) s_before[threadIdx.x >> 5] = before;
+    int32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) s += v[k];
+    int32_t tot;
+    int32_t run = block_excl_scan(s, sw, tot);
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w) run += s_before[w];
+    int32_t o[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        o[k] = run;
+        run += v[k];
+    }
+    if (full) {
+        int4 *p = reinterpret_cast<int4 *>(out + base);
+        p[0] = make_int4(o[0], o[1], o[2], o[3]);
+        p[1] = make_int4(o[4], o[5], o[6], o[7]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < IPT; ++k)
+            if (base + k < n) out[base + k] = o[k];
+    }
+    if (base < n && base + IPT >= n) out[n] = run; // cells past n count nothing
+}
+
+static __global__ void __launch_bounds__(kBlock)
+    k_scan_cells(int32_t *__restrict__ counts, int64_t n, const int32_t *__restrict__ tiles,
+                 int summed, int32_t *__restrict__ out)
+{
+    pdl_enter();
+    scan_cells(counts, n, tiles, summed != 0, blockIdx.x, out);
 }
 
 // Scatter every particle into its cell's bucket (arbitrary order inside the
-// bucket; the rank step below makes it deterministic).
-static __global__ void k_bucket(int64_t N, const int32_t *__restrict__ cellTmp,
-                                const int32_t *__restrict__ perm, int32_t *__restrict__ cursor,
-                                int32_t *__restrict__ bucketSrc, int32_t *__restrict__ bucketId)
+// bucket; the rank step below makes it deterministic), thread i of `threads`.
+// Clears the nb tile sums.
+__device__ __forceinline__ void bucket_cell(int64_t i, int64_t N, int64_t threads,
+                                            const int32_t *__restrict__ cellTmp,
+                                            const int32_t *__restrict__ place,
+                                            const int32_t *__restrict__ cellStart,
+                                            const int32_t *__restrict__ perm,
+                                            int32_t *__restrict__ bucketSrc,
+                                            int32_t *__restrict__ bucketId,
+                                            int32_t *__restrict__ tiles, int64_t nb)
 {
-    pdl_enter();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < N;
-    const int32_t c = live ? cellTmp[i] : -1;
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    if (!live) return;
-    const unsigned peers = __match_any_sync(act, c);
-    const int leader = __ffs(peers) - 1;
-    int32_t base = 0;
-    if ((int)lane_id() == leader) base = atomicAdd(cursor + c, __popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    const int32_t pos = base + __popc(peers & ((1u << lane_id()) - 1u));
+    for (int64_t k = i; k < nb; k += threads) tiles[k] = 0;
+    if (i >= N) return;
+    const int32_t pos = cellStart[cellTmp[i]] + place[i];
     bucketSrc[pos] = (int32_t)i;
     bucketId[pos] = perm[i];
+}
+
+static __global__ void k_bucket(int64_t N, const int32_t *__restrict__ cellTmp,
+                                const int32_t *__restrict__ place,
+                                const int32_t *__restrict__ cellStart,
+                                const int32_t *__restrict__ perm, int32_t *__restrict__ bucketSrc,
+                                int32_t *__restrict__ bucketId, int32_t *__restrict__ tiles,
+                                int64_t nb)
+{
+    pdl_enter();
+    bucket_cell((int64_t)blockIdx.x * blockDim.x + threadIdx.x, N,
+                (int64_t)gridDim.x * blockDim.x, cellTmp, place, cellStart, perm, bucketSrc,
+                bucketId, tiles, nb);
 }
 
 // _cl_sort_cells! as a rank: each particle counts the smaller ids in its cell

@@ -52,7 +52,7 @@ template <typename T> struct GSys {
     T2<T> *posN, *velN;     // rebuild outputs (the buffers v.pos / vel)
     T2<T> *posOut, *velOut; // forward step outputs
     T2<T> *xref;
-    int32_t *perm, *invperm, *cellStart, *cellTmp, *counts, *cursor, *bucketSrc, *bucketId,
+    int32_t *perm, *invperm, *cellStart, *cellTmp, *counts, *bucketSrc, *bucketId,
         *scanTmp, *nbcount;
     uint32_t *center, *masks, *tmask, *flags;
     T *rho;     // densities (NULL where the model does not read them in the reverse step)
@@ -84,9 +84,9 @@ template <typename T> struct GSys {
 #error "define SPH_PACK_T (this translation unit's precision) before including sph_pack.cuh"
 #endif
 constexpr int kMaxPackSys = 64; // requests one tick can hold
-constexpr int kPackLists = 10;
+constexpr int kPackLists = 9;
 enum PackList : int {
-    PL_GATHER = 0, PL_CELLS, PL_SCANTOP, PL_SCANTILE, PL_PART, PL_ALL, PL_REV, PL_THETA, PL_FWD, PL_LISTS
+    PL_GATHER = 0, PL_SCANTOP, PL_SCANTILE, PL_PART, PL_ALL, PL_REV, PL_THETA, PL_FWD, PL_LISTS
 };
 struct PackLists {
     int32_t cnt[kPackLists];
@@ -133,15 +133,6 @@ __global__ void __launch_bounds__(kPackBlock) g_gather(int l)
     d.velPre[t] = d.sv[s];
 }
 
-template <typename T> __global__ void __launch_bounds__(kBlock) g_zero_counts(int l)
-{
-    pdl_enter();
-    const int2 f = glist_find(l);
-    const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t c = (int64_t)f.y * blockDim.x + threadIdx.x;
-    if (c < d.ncell) d.counts[c] = 0;
-}
-
 // k_assign of one request (single instance, cells from 0)
 template <typename T>
 __global__ void __launch_bounds__(kPackBlock) g_assign(int l)
@@ -153,44 +144,17 @@ __global__ void __launch_bounds__(kPackBlock) g_assign(int l)
     const bool live = i < d.n;
     int32_t c = -1;
     if (live) {
-        const Inst<T> &I = d.v.one;
-        const T2<T> x = d.posPre[i];
-        if (d.check) {
-            const T2<T> xr = d.xref[i];
-            const T d2 = r2_exact<T>(sub_rn(x.x, xr.x), sub_rn(x.y, xr.y));
-            if (d2 > I.dmax2) atomicOr(d.flags, FLAG_DISPLACEMENT);
-        }
-        const T cs = I.cs;
-        const int cx = cell_div(x.x, cs, I.nx);
-        const int cy = cell_div(x.y, cs, I.ny);
-        c = (cx - 1) + (cy - 1) * I.nx;
+        c = assign_cell<T>(d.v.one, d.posPre[i], d.check, d.xref + i, d.flags);
         d.cellTmp[i] = c;
     }
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    if (live) {
-        const unsigned peers = __match_any_sync(act, c);
-        if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(d.counts + c, __popc(peers));
-    }
+    count_cell(live, c, i, d.counts, d.scanTmp, d.nbcount);
 }
 
-// exclusive scan of each request's counts: tile sums, per-request scan of the
-// tile sums (one block each), then the tiles with their offsets
-template <typename T> __global__ void __launch_bounds__(kBlock) g_scan_reduce(int l)
+// exclusive scan of each request's counts; the sums of the tiles before a tile by
+// its own block, or for a very large table by one block per request
+__device__ __forceinline__ int64_t scan_tiles(int64_t ncell)
 {
-    pdl_enter();
-    __shared__ int32_t sw[33];
-    const int2 f = glist_find(l);
-    const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t base = (int64_t)f.y * kScanTile;
-    int32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanTile / kBlock; ++k) {
-        const int64_t i = base + (int64_t)k * kBlock + threadIdx.x;
-        if (i < d.ncell) s += d.counts[i];
-    }
-    int32_t tot;
-    block_excl_scan(s, sw, tot);
-    if (threadIdx.x == 0) d.scanTmp[f.y] = tot;
+    return (ncell + kScanTile - 1) / kScanTile;
 }
 
 template <typename T> __global__ void __launch_bounds__(kBlock) g_scan_top(int l)
@@ -199,7 +163,7 @@ template <typename T> __global__ void __launch_bounds__(kBlock) g_scan_top(int l
     __shared__ int32_t sw[33];
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t nb = (d.ncell + kScanTile - 1) / kScanTile;
+    const int64_t nb = scan_tiles(d.ncell);
     int32_t carry = 0;
     for (int64_t base = 0; base < nb; base += blockDim.x) {
         const int64_t i = base + threadIdx.x;
@@ -211,35 +175,12 @@ template <typename T> __global__ void __launch_bounds__(kBlock) g_scan_top(int l
     }
 }
 
-template <typename T> __global__ void __launch_bounds__(kBlock) g_scan_down(int l)
+template <typename T> __global__ void __launch_bounds__(kBlock) g_scan_cells(int l)
 {
     pdl_enter();
-    __shared__ int32_t sw[33];
-    constexpr int IPT = kScanTile / kBlock;
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t n = d.ncell;
-    const int64_t base = (int64_t)f.y * kScanTile + (int64_t)threadIdx.x * IPT;
-    int32_t v[IPT];
-    int32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int64_t i = base + k;
-        v[k] = i < n ? d.counts[i] : 0;
-        s += v[k];
-    }
-    int32_t tot;
-    int32_t run = block_excl_scan(s, sw, tot) + d.scanTmp[f.y];
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int64_t i = base + k;
-        if (i < n) {
-            d.cellStart[i] = run;
-            d.cursor[i] = run;
-        }
-        run += v[k];
-        if (i == n - 1) d.cellStart[n] = run;
-    }
+    scan_cells(d.counts, d.ncell, d.scanTmp, scan_tiles(d.ncell) > kScanSelf, f.y, d.cellStart);
 }
 
 template <typename T>
@@ -248,19 +189,9 @@ __global__ void __launch_bounds__(kPackBlock) g_bucket(int l)
     pdl_enter();
     const int2 f = glist_find(l);
     const GSys<T> &d = pack_sys<T>(f.x);
-    const int64_t i = (int64_t)f.y * blockDim.x + threadIdx.x;
-    const bool live = i < d.n;
-    const int32_t c = live ? d.cellTmp[i] : -1;
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    if (!live) return;
-    const unsigned peers = __match_any_sync(act, c);
-    const int leader = __ffs(peers) - 1;
-    int32_t base = 0;
-    if ((int)lane_id() == leader) base = atomicAdd(d.cursor + c, __popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    const int32_t p = base + __popc(peers & ((1u << lane_id()) - 1u));
-    d.bucketSrc[p] = (int32_t)i;
-    d.bucketId[p] = d.perm[i];
+    bucket_cell((int64_t)f.y * kPackBlock + threadIdx.x, d.n,
+                (d.n + kPackBlock - 1) / kPackBlock * kPackBlock, d.cellTmp, d.nbcount,
+                d.cellStart, d.perm, d.bucketSrc, d.bucketId, d.scanTmp, scan_tiles(d.ncell));
 }
 
 template <typename T>
@@ -746,7 +677,7 @@ template <typename T> class Packer final : public PackI {
             }
             int32_t blocks() const { return start.back(); }
         };
-        List lGather, lCells, lScanTop, lScanTile, lPart, lAll, lRev, lTheta, lFwd, lLists;
+        List lGather, lScanTop, lScanTile, lPart, lAll, lRev, lTheta, lFwd, lLists;
         bool anyAV = false;
         auto nb = [](int64_t n, int b) { return (n + b - 1) / b; };
         for (int k = 0; k < P; ++k) {
@@ -773,7 +704,6 @@ template <typename T> class Packer final : public PackI {
             d.cellStart = Y.cellStart.p;
             d.cellTmp = Y.cellTmp.p;
             d.counts = Y.counts.p;
-            d.cursor = Y.cursor.p;
             d.bucketSrc = Y.bucketSrc.p;
             d.bucketId = Y.bucketId.p;
             d.scanTmp = Y.scanTmp.p;
@@ -840,8 +770,7 @@ template <typename T> class Packer final : public PackI {
                 q.rstep += 1;
             }
             if (rebuild && N > 0) {
-                lCells.add(k, nb(d.ncell, kBlock));
-                lScanTop.add(k, 1);
+                if (nb(d.ncell, kScanTile) > kScanSelf) lScanTop.add(k, 1);
                 lScanTile.add(k, nb(d.ncell, kScanTile));
                 lPart.add(k, nb(N, kPackBlock));
             }
@@ -863,7 +792,7 @@ template <typename T> class Packer final : public PackI {
         Ring &R = ring_[ringPos_];
         ringPos_ = (ringPos_ + 1) % kRing;
         if (R.used) SPH_CK(cudaEventSynchronize(R.ev));
-        const List *lists[kPackLists] = {&lGather, &lCells, &lScanTop, &lScanTile, &lPart,
+        const List *lists[kPackLists] = {&lGather, &lScanTop, &lScanTile, &lPart,
                                          &lAll, &lRev, &lTheta, &lFwd, &lLists};
         const size_t bytes = sizeof(PackLists) + sizeof(GSys<T>) * (size_t)P;
         if (!R.host) {
@@ -889,11 +818,9 @@ template <typename T> class Packer final : public PackI {
             ++launches_;
         };
         launch(K_GATHER, PL_GATHER, kPackBlock, g_gather<T>);
-        launch(K_ASSIGN, PL_CELLS, kBlock, g_zero_counts<T>);
         launch(K_ASSIGN, PL_PART, kPackBlock, g_assign<T>);
-        launch(K_SCAN, PL_SCANTILE, kBlock, g_scan_reduce<T>);
         launch(K_SCAN, PL_SCANTOP, kBlock, g_scan_top<T>);
-        launch(K_SCAN, PL_SCANTILE, kBlock, g_scan_down<T>);
+        launch(K_SCAN, PL_SCANTILE, kBlock, g_scan_cells<T>);
         launch(K_BUCKET, PL_PART, kPackBlock, g_bucket<T>);
         launch(K_RANK, PL_PART, kPackBlock, g_rank<T>);
         launch(K_NLBUILD, PL_PART, kPackBlock, g_nl_build<T>);
