@@ -50,12 +50,14 @@ constexpr int kRunMax = 8;     // cell-row runs of a tile
 constexpr int kRangeMax = 3 * kRunMax;
 constexpr int kQuads = 12;     // list capacity: 48 entries
 constexpr int kNoList = 255;   // count of a particle without a list
-constexpr int kListStride = 8 * kQuads + 4; // bytes per thread while a list is
-                                            // collected: an odd number of words,
-                                            // so a warp's lanes use all banks
-
-constexpr int kNlStride = 8 * kQuads + 20; // the same with room for eight entries past
-                                          // the capacity (nl_window)
+// While lists are collected, entry k of thread t lies at row k, column t: a store
+// has a two-way bank conflict at most, wherever each lane's list ends (a run of
+// entries per thread, its stride an odd number of words: 3.4 wavefronts on
+// average, mask and list build of 1M particles 69.1 us against 66.5)
+constexpr int kRow = 2 * kTile;            // bytes of a row
+constexpr int kListStride = 8 * kQuads + 4; // bytes per thread: the list and two rows more
+constexpr int kNlStride = 8 * kQuads + 20;  // the same with room for eight entries past
+                                            // the capacity (nl_window)
 
 struct TileWin {
     int32_t nr;               // ranges (0: no window, every particle is marked)
@@ -149,15 +151,16 @@ __device__ __forceinline__ uint32_t entry_of(const uint2 &e, int k)
 // its quads, the last one padded with the last entry.
 __device__ __forceinline__ void write_list(unsigned char *place, int n, uint2 *__restrict__ out)
 {
-    uint16_t *p = reinterpret_cast<uint16_t *>(place);
-    if (n & 3) {
-        const uint16_t last = p[n - 1];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (k < (-n & 3)) p[n + k] = last;
+    const uint16_t *p = reinterpret_cast<const uint16_t *>(place);
+    int q = 0;
+    for (; 4 * q + 4 <= n; ++q, p += 4 * kTile)
+        out[q * kTile] = make_uint2(p[0] | (uint32_t)p[kTile] << 16,
+                                    p[2 * kTile] | (uint32_t)p[3 * kTile] << 16);
+    if (const int left = n & 3) { // padded with the last entry
+        const uint32_t a = p[0], b = p[left > 1 ? kTile : 0];
+        const uint32_t c = left > 2 ? p[2 * kTile] : b;
+        out[q * kTile] = make_uint2(a | b << 16, c | c << 16);
     }
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(place);
-    for (int q = 0; 4 * q < n; ++q) out[q * kTile] = make_uint2(w[2 * q], w[2 * q + 1]);
 }
 
 // The window of a tile whose particles lie in cells (cx, cy) of instance b:
@@ -249,9 +252,9 @@ __device__ __forceinline__ bool tile_window(TileShared &T, const Inst<float> &on
 // _nl_build! (nl_build_one), the tile's window and the candidate lists of a fresh
 // cell list: the rows are scanned in the staged window, and every passing slot
 // goes both to its row mask and to the list. One pass instead of a mask build
-// (52 us at 1M particles) and a walk of the masks (43 us): 73 us, bound by
-// shared-memory wavefronts (81% of their rate) and issue slots (78%); 8.4M dense
-// particles 775 -> 664 us.
+// (52 us at 1M particles) and a walk of the masks (43 us): 66.5 us, bound by issue
+// slots and shared-memory wavefronts (some 80% of either's rate); 8.4M dense
+// particles 775 -> 647 us.
 template <bool MULTI>
 __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
                                           const Inst<float> *inst,
@@ -297,8 +300,8 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
     const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
     const int jx1 = cx + 1 < nx ? cx + 1 : nx;
     const float rc2 = I.rc2, r2min = I.r2min;
-    unsigned char *const place = s_list + t * kNlStride;
-    unsigned char *const full = place + 8 * kQuads;
+    unsigned char *const place = s_list + 2 * t;
+    unsigned char *const full = place + 4 * kQuads * kRow;
     unsigned char *to = place; // the list's end; held at `full` once it is reached
     uint32_t spill = 0;
     uint32_t word[6];
@@ -311,7 +314,7 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
         const float r2 = add_rn(q.x, q.y);
         const bool in = lt_nonneg(r2min, r2) && lt_nonneg(r2, rc2);
         *reinterpret_cast<uint16_t *>(to) = (uint16_t)o;
-        if (in) to += 2;
+        if (in) to += kRow;
         return in;
     };
     // passing slots among the len (at most 32) from offset o, eight at a time
@@ -418,7 +421,7 @@ __device__ __forceinline__ void window_lists(const NLView<float> &v, const WinLi
     decltype(auto) I = pick_inst<MULTI>(v.one, v.inst, b);
     const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
     const int row0 = I.coff + (jx0 - 1) + (cy - 2) * I.nx;
-    unsigned char *const place = s_list + t * kListStride;
+    unsigned char *const place = s_list + 2 * t;
     uint64_t m[3];
     int off[3];
     int n = 0;
@@ -447,7 +450,8 @@ __device__ __forceinline__ void window_lists(const NLView<float> &v, const WinLi
         }
         const int k = __ffs((int)w) - 1;
         w &= w - 1u;
-        *to++ = (uint16_t)(base + 8 * k);
+        *to = (uint16_t)(base + 8 * k);
+        to += kTile;
     }
     write_list(place, n, L.cand + (int64_t)tile * (kQuads * kTile) + t);
     L.candCnt[i] = (uint8_t)n;
@@ -489,7 +493,7 @@ __device__ __forceinline__ void density_window(const NLView<float> &v, const Win
     const float2 one2 = make_float2(1.0f, 1.0f), two2 = make_float2(2.0f, 2.0f);
     const int64_t lbase = (int64_t)tile * (kQuads * kTile) + t;
     const uint2 *cand = L.cand + lbase;
-    unsigned char *const place = s_list + t * kListStride;
+    unsigned char *const place = s_list + 2 * t;
     int ns = 0;
     float acc = 0.0f;
     // one quad of candidates, `left` of them in the list
@@ -521,7 +525,7 @@ __device__ __forceinline__ void density_window(const NLView<float> &v, const Win
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             *reinterpret_cast<uint16_t *>(place + ns) = (uint16_t)entry_of(cur, k);
-            if (in[k]) ns += 2;
+            if (in[k]) ns += kRow;
         }
     };
     uint2 e = n ? cand[0] : make_uint2(0u, 0u);
@@ -532,7 +536,7 @@ __device__ __forceinline__ void density_window(const NLView<float> &v, const Win
         quad(cur, 4);
     }
     if (n & 3) quad(e, n & 3);
-    ns >>= 1;
+    ns /= kRow;
     write_list(place, ns, L.supp + lbase);
     L.suppCnt[i] = (uint8_t)ns;
     acc = mul_rn(mul_rn(m, A), acc);
