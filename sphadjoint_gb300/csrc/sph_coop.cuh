@@ -54,6 +54,44 @@ template <int G> struct Group {
     }
 };
 
+// One running sum over a round's G term slots, n of them dealt out, those with
+// their bit in `inm` in the support: "minus one slot, plus one slot" per pair (sub
+// may be NULL). FP32 adds all of them eight at a time: a slot without a pair is a
+// zero, and a sum that starts at +0 never becomes -0, so x - 0 and x + 0 leave it as
+// it is (pass 1 of 1500 particles, skipping them by their bits: 6.1 us, so 5.5). In
+// FP64 an addition takes 64 cycles, and skipping is the shorter way.
+template <typename T, int G>
+__device__ __forceinline__ T coop_fold(T acc, const T *sub, const T *add, int n, unsigned inm)
+{
+    if constexpr (sizeof(T) == 4) {
+        auto read8 = [](const T *p, float (&x)[8]) {
+            const float4 a = *reinterpret_cast<const float4 *>(p);
+            const float4 c = *reinterpret_cast<const float4 *>(p + 4);
+            x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+            x[4] = c.x, x[5] = c.y, x[6] = c.z, x[7] = c.w;
+        };
+#pragma unroll
+        for (int t = 0; t < G; t += 8) {
+            if (t >= n) break;
+            float a[8], s[8];
+            read8(add + t, a);
+            if (sub) read8(sub + t, s);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (sub) acc -= s[u];
+                acc += a[u];
+            }
+        }
+    } else {
+        for (int t = 0; t < n; ++t)
+            if ((inm >> t) & 1u) {
+                if (sub) acc -= sub[t];
+                acc += add[t];
+            }
+    }
+    return acc;
+}
+
 // The candidates of a particle, numbered 0..total-1 in slot order: the set
 // bits of its six words (row r = words 2r, 2r+1), or for a spilled particle
 // the list spill_list built.
@@ -231,7 +269,7 @@ __global__ void __launch_bounds__(kCoopBlock)
     pdl_enter();
     if (theta_flush<T>(flush)) return;
     constexpr int NG = kCoopBlock / G;
-    __shared__ T buf[NG][G];
+    __shared__ __align__(16) T buf[NG][G];
     __shared__ uint32_t tws[NG][6];
     __shared__ int32_t lst[NG][kSpillList];
     const Group<G> g;
@@ -271,11 +309,8 @@ __global__ void __launch_bounds__(kCoopBlock)
         buf[g.gi][g.gl] = c;
         const unsigned inm = g.ballot(in);
         g.sync();
-        if (g.gl == 0) {
-            const int n = K - base < G ? K - base : G;
-            for (int t = 0; t < n; ++t)
-                if ((inm >> t) & 1u) acc += buf[g.gi][t];
-        }
+        if (g.gl == 0)
+            acc = coop_fold<T, G>(acc, nullptr, buf[g.gi], K - base < G ? K - base : G, inm);
         g.sync();
     }
     if (tmaskOut && g.gl < 6) tmaskOut[(int64_t)g.gl * v.N + i] = tws[g.gi][g.gl];
@@ -336,16 +371,9 @@ __device__ __forceinline__ void accel_sum_coop(const Group<G> &g, T (*buf)[4][G]
         buf[g.gi][3][g.gl] = t.cy;
         const unsigned inm = g.ballot(in);
         g.sync();
-        if (g.gl < 2) {
-            const int n = K - base < G ? K - base : G;
-            const T *ps = buf[g.gi][g.gl];
-            const T *cs = buf[g.gi][2 + g.gl];
-            for (int t2 = 0; t2 < n; ++t2)
-                if ((inm >> t2) & 1u) {
-                    acc -= ps[t2];
-                    acc += cs[t2];
-                }
-        }
+        if (g.gl < 2)
+            acc = coop_fold<T, G>(acc, buf[g.gi][g.gl], buf[g.gi][2 + g.gl],
+                                  K - base < G ? K - base : G, inm);
         g.sync();
     }
     ax = acc;
@@ -365,7 +393,7 @@ __global__ void __launch_bounds__(kCoopBlock)
 {
     pdl_enter();
     constexpr int NG = kCoopBlock / G;
-    __shared__ T buf[NG][4][G];
+    __shared__ __align__(16) T buf[NG][4][G];
     __shared__ int32_t lst[NG][kSpillList];
     const Group<G> g;
     const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
@@ -400,7 +428,7 @@ __global__ void __launch_bounds__(kCoopBlock)
 {
     pdl_enter();
     constexpr int NG = kCoopBlock / G;
-    __shared__ T buf[NG][4][G];
+    __shared__ __align__(16) T buf[NG][4][G];
     __shared__ int32_t lst[NG][kSpillList];
     const Group<G> g;
     const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
@@ -434,7 +462,7 @@ __global__ void __launch_bounds__(kCoopBlock)
 {
     pdl_enter();
     constexpr int NG = kCoopBlock / G;
-    __shared__ T buf[NG][9][G]; // eight term slots and a row of zeros
+    __shared__ __align__(16) T buf[NG][9][G]; // eight term slots and a row of zeros
     __shared__ int32_t lst[NG][kSpillList];
     const Group<G> g;
     const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
@@ -497,14 +525,8 @@ __global__ void __launch_bounds__(kCoopBlock)
             b[7][g.gl] = t.sS;
             const unsigned inm = g.ballot(in);
             g.sync();
-            if (g.gl < 6) {
-                const int n = K - base < G ? K - base : G;
-                for (int t2 = 0; t2 < n; ++t2)
-                    if ((inm >> t2) & 1u) {
-                        acc -= fsub[t2];
-                        acc += fadd[t2];
-                    }
-            }
+            if (g.gl < 6)
+                acc = coop_fold<T, G>(acc, fsub, fadd, K - base < G ? K - base : G, inm);
             g.sync();
         }
         gx = acc;
@@ -520,9 +542,14 @@ __global__ void __launch_bounds__(kCoopBlock)
                     gV);
 }
 
-// adj_pass2_kernel! + _axpy2!(gX, gXs) + the exact theta write-back.
+// adj_pass2_kernel! + _axpy2!(gX, gXs) + the exact theta write-back. A fifth warp
+// writes theta back, a lane per particle and corner (a corner waits for the old
+// value of its accumulator, so one lane took four waits after the pair sums), and
+// loads the next tape state: 1500 FP32 particles 6.4 -> 4.3 us, its floor of a
+// launch being 2.
+constexpr int kCoopPass2 = kCoopBlock + 32;
 template <typename T, int G>
-__global__ void __launch_bounds__(kCoopBlock)
+__global__ void __launch_bounds__(kCoopPass2)
     k_pass2_axpy_coop(const __grid_constant__ NLView<T> v, const T *__restrict__ grho,
                       const T2<T> *__restrict__ gXs, T2<T> *__restrict__ gX,
                       const T *__restrict__ galpha, const int *__restrict__ emax, int parity,
@@ -530,21 +557,28 @@ __global__ void __launch_bounds__(kCoopBlock)
 {
     pdl_enter();
     constexpr int NG = kCoopBlock / G;
-    __shared__ T buf[NG][2][G];
+    __shared__ __align__(16) T buf[NG][2][G];
     __shared__ int32_t lst[NG][kSpillList];
     const Group<G> g;
+    const Inst<T> &I = v.one;
+    if (threadIdx.x >= kCoopBlock) {
+        const int t = (int)threadIdx.x - kCoopBlock;
+        const int64_t i0 = (int64_t)blockIdx.x * NG, it = i0 + (t >> 2);
+        const bool load = t < NG && i0 + t < v.N;
+        if (load) next.read(i0 + t);
+        if (t < 4 * NG && it < v.N)
+            theta_add_corner<T>(I, 0, it, v.pos[it], t & 3, galpha, emax, parity, thetaAcc);
+        if (load) next.write(i0 + t);
+        return;
+    }
     const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
     if (i >= v.N) return;
-    const bool loader = g.gl == G - 1; // a lane with nothing to fold
-    if (loader) next.read(i);
-    const Inst<T> &I = v.one;
     const T r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, Fc = I.p.Fc;
     const T2<T> xi = v.pos[i];
     const T gri = grho[i];
     const uint32_t cc = v.center[i];
     T gx = (T)0, gy = (T)0;
     if ((cc >> 31) && I.maxnb > kSpillList) {
-        if (loader) next.write(i);
         if (g.gl != 0) return;
         for_each_neighbor<T>(v, I, i, [&](int j) {
             const T2<T> xj = v.pos[j];
@@ -583,20 +617,16 @@ __global__ void __launch_bounds__(kCoopBlock)
             buf[g.gi][1][g.gl] = ty;
             const unsigned inm = g.ballot(in);
             g.sync();
-            if (g.gl < 2) {
-                const int n = K - base < G ? K - base : G;
-                const T *src = buf[g.gi][g.gl];
-                for (int t2 = 0; t2 < n; ++t2)
-                    if ((inm >> t2) & 1u) acc += src[t2];
-            }
+            if (g.gl < 2)
+                acc = coop_fold<T, G>(acc, nullptr, buf[g.gi][g.gl], K - base < G ? K - base : G,
+                                      inm);
             g.sync();
         }
         gx = acc;
         gy = g.from(acc, 1);
-        if (loader) next.write(i);
         if (g.gl != 0) return;
     }
-    pass2_finish<T>(I, 0, i, xi, gx, gy, gXs, gX, galpha, emax, parity, thetaAcc);
+    pass2_axpy<T>(i, gx, gy, gXs, gX);
 }
 
 } // namespace sphgb

@@ -198,14 +198,15 @@ template <typename T> int &tuned_block(int kid, bool multi)
 
 // Group-per-particle launch: kCoopBlock threads, kCoopBlock / G particles per
 // block. The _X forms launch extra blocks behind the particles' ones.
-#define SPH_LAUNCH_COOP(kid, G, kern, n, ...) SPH_LAUNCH_COOP_X(kid, G, 0, kern, n, __VA_ARGS__)
-#define SPH_LAUNCH_COOP_X(kid, G, extra, kern, n, ...)                                        \
+#define SPH_LAUNCH_COOP(kid, G, kern, n, ...)                                                 \
+    SPH_LAUNCH_COOP_X(kid, G, 0, ::sphgb::kCoopBlock, kern, n, __VA_ARGS__)
+#define SPH_LAUNCH_COOP_X(kid, G, extra, threads, kern, n, ...)                               \
     do {                                                                                      \
         if ((n) > 0) {                                                                        \
             const int per_ = ::sphgb::kCoopBlock / (G);                                       \
             ::sphgb::rt_before_launch(kid);                                                   \
             ::sphgb::launch_k(kern, dim3((unsigned)(((n) + per_ - 1) / per_) + (extra)),       \
-                              dim3(::sphgb::kCoopBlock), 0, __VA_ARGS__);                       \
+                              dim3(threads), 0, __VA_ARGS__);                                   \
             ::sphgb::rt_after_launch(kid);                                                    \
         }                                                                                     \
     } while (0)
@@ -1496,14 +1497,15 @@ template <typename T> class Work final : public WorkI {
             auto k2 = g32 ? &k_pass2_axpy_coop<T, 32> : &k_pass2_axpy_coop<T, 16>;
             const int per = kCoopBlock / G;
             const ThetaFlush<T> fl = take_flush(S, (N_ + per - 1) / per, extra);
-            SPH_LAUNCH_COOP_X(K_DENSITY, G, extra, kd, N_, v, rhoOut, S.prho.p, S.tmask.p, fl);
+            SPH_LAUNCH_COOP_X(K_DENSITY, G, extra, kCoopBlock, kd, N_, v, rhoOut, S.prho.p,
+                              S.tmask.p, fl);
             v.tmask = S.tmask.p;
             SPH_LAUNCH_COOP(K_ACCEL_DRAG, G, ka, N_, v, vel, S.prho.p, S.rho.p, theta, gX[gcur].p,
                             gV[gcur].p, abar.p, galpha.p, emax.p, parity);
             SPH_LAUNCH_COOP(K_PASS1, G, k1, N_, v, vel, S.prho.p, S.rho.p, theta, abar.p,
                             galpha.p, gXs.p, grho.p, gV[gcur].p);
-            SPH_LAUNCH_COOP(K_PASS2, G, k2, N_, v, grho.p, gXs.p, gX[gcur].p, galpha.p, emax.p,
-                            parity, thetaAcc.p, next);
+            SPH_LAUNCH_COOP_X(K_PASS2, G, 0, kCoopPass2, k2, N_, v, grho.p, gXs.p, gX[gcur].p,
+                              galpha.p, emax.p, parity, thetaAcc.p, next);
             pendingTheta = parity;
             return;
         }

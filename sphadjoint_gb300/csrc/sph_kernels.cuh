@@ -1900,31 +1900,24 @@ __device__ __forceinline__ void pass2_finish_warp(bool live, const IT &I, int b,
     theta_add_warp<T>(live && ga != (T)0 && em != INT_MIN, node, ngy, S, ga, fx, fy, thetaAcc);
 }
 
-// The same of one particle by itself.
+// Corner c of particle i's theta write-back (c & 1: the next column, c >> 1: the
+// next row), as theta_add_warp forms it.
 template <typename T, typename IT>
-__device__ __forceinline__ void pass2_finish(const IT &I, int b, int64_t i, const T2<T> &xi,
-                                             T gx, T gy, const T2<T> *__restrict__ gXs,
-                                             T2<T> *__restrict__ gX,
-                                             const T *__restrict__ galpha,
-                                             const int *__restrict__ emax, int parity,
-                                             unsigned long long *__restrict__ thetaAcc)
+__device__ __forceinline__ void theta_add_corner(const IT &I, int b, int64_t i, const T2<T> &xi,
+                                                 int c, const T *__restrict__ galpha,
+                                                 const int *__restrict__ emax, int parity,
+                                                 unsigned long long *__restrict__ thetaAcc)
 {
-    pass2_axpy<T>(i, gx, gy, gXs, gX);
     const T ga = galpha[i];
     const int em = emax[2 * b + parity];
-    if (ga != (T)0 && em != INT_MIN) {
-        const Phys<T> &p = I.p;
-        int i0, j0;
-        T fx, fy, ax, ay;
-        interp_cell<T>(xi.x, xi.y, p, i0, j0, fx, fy, ax, ay);
-        const int S = theta_scale(em, I.lgN);
-        unsigned long long *acc = thetaAcc + 2 * (int64_t)I.toff;
-        const int64_t l00 = (int64_t)j0 + (int64_t)i0 * p.ngy;
-        fixed_add(acc + 2 * l00, ga * ((T)1 - fx) * ((T)1 - fy), S);
-        fixed_add(acc + 2 * (l00 + p.ngy), ga * fx * ((T)1 - fy), S);
-        fixed_add(acc + 2 * (l00 + 1), ga * ((T)1 - fx) * fy, S);
-        fixed_add(acc + 2 * (l00 + p.ngy + 1), ga * fx * fy, S);
-    }
+    if (ga == (T)0 || em == INT_MIN) return;
+    const Phys<T> &p = I.p;
+    int i0, j0;
+    T fx, fy, ax, ay;
+    interp_cell<T>(xi.x, xi.y, p, i0, j0, fx, fy, ax, ay);
+    const T wx = (c & 1) ? fx : (T)1 - fx, wy = (c >> 1) ? fy : (T)1 - fy;
+    const int64_t node = (int64_t)I.toff + j0 + (int64_t)(i0 + (c & 1)) * p.ngy + (c >> 1);
+    fixed_add(thetaAcc + 2 * node, ga * wx * wy, theta_scale(em, I.lgN));
 }
 
 // Per design node: gtheta += one step's exact sum; clear the accumulator.
