@@ -380,9 +380,15 @@ __device__ __forceinline__ void accel_sum_coop(const Group<G> &g, T (*buf)[4][G]
     ay = g.from(acc, 1);
 }
 
+// The passes below have a fifth warp. While the four with the groups go through
+// their pairs, its lane t does what the block's t-th particle needs besides the pair
+// sums: the design field and the walls (two dependent loads and a division), the
+// tape. One lane per group did that behind the sums: 1500 FP32 particles PERF_SIDE
+constexpr int kCoopThreads = kCoopBlock + 32;
+
 // accel_kernel! + integrate_kernel!
 template <typename T, int G>
-__global__ void __launch_bounds__(kCoopBlock)
+__global__ void __launch_bounds__(kCoopThreads)
     k_accel_integrate_coop(const __grid_constant__ NLView<T> v, const T2<T> *__restrict__ vel,
                            const T2<T> *__restrict__ prho, const T *__restrict__ rho,
                            const T *__restrict__ theta,
@@ -395,30 +401,59 @@ __global__ void __launch_bounds__(kCoopBlock)
     constexpr int NG = kCoopBlock / G;
     __shared__ __align__(16) T buf[NG][4][G];
     __shared__ int32_t lst[NG][kSpillList];
+    __shared__ SideForce<T> side[NG];
     const Group<G> g;
-    const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
-    if (i >= v.N) return;
+    const bool fifth = threadIdx.x >= kCoopBlock;
+    const int q = fifth ? (int)threadIdx.x - kCoopBlock : g.gi;
+    const int64_t i = (int64_t)blockIdx.x * NG + q;
+    const bool live = q < NG && i < v.N; // of a group: all its lanes or none
     const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[i];
-    const T2<T> vi = vel[i];
-    const uint32_t cc = v.center[i];
-    T ax, ay;
-    if ((cc >> 31) && I.maxnb > kSpillList) {
-        if (g.gl != 0) return;
-        accel_sum<T, true>(v, I, vel, prho, rho, i, xi, vi, ax, ay);
-    } else {
-        const Cands<T> cd = pass_cands<T, G>(g, v, I, i, cc, lst[g.gi]);
-        accel_sum_coop<T, G, NG>(g, buf, v, I, i, cd, vel, prho, rho, xi, vi, ax, ay);
-        if (g.gl != 0) return;
+    T2<T> xi = mk2<T>((T)0, (T)0), vi = xi;
+    T ax = (T)0, ay = (T)0;
+    if (live) {
+        xi = v.pos[i];
+        vi = vel[i];
+        if (fifth) {
+            if (tx) {
+                // _tape_store! (src/driver.jl:73-77) of the pre-step state, in
+                // particle-id order
+                const int32_t id = perm[i];
+                tx[id] = xi;
+                tv[id] = vi;
+            }
+            side[q] = side_force<T>(I, xi, theta);
+        } else {
+            const uint32_t cc = v.center[i];
+            if ((cc >> 31) && I.maxnb > kSpillList) {
+                if (g.gl == 0) accel_sum<T, true>(v, I, vel, prho, rho, i, xi, vi, ax, ay);
+            } else {
+                const Cands<T> cd = pass_cands<T, G>(g, v, I, i, cc, lst[g.gi]);
+                accel_sum_coop<T, G, NG>(g, buf, v, I, i, cd, vel, prho, rho, xi, vi, ax, ay);
+            }
+        }
     }
-    accel_integrate_finish<T>(I, 0, i, xi, vi, ax, ay, theta, posOut, velOut, aOut, alphaOut, flags,
-                              perm, tx, tv);
+    __syncthreads();
+    if (!live || fifth || g.gl != 0) return;
+    const SideForce<T> f = side[q];
+    ax += f.gx;
+    ay += f.gy;
+    if (aOut) aOut[i] = mk2<T>(ax, ay);
+    if (alphaOut) alphaOut[i] = f.al;
+    const T dt = I.p.dt;
+    const T v1 = (vi.x + dt * ax) * f.D;
+    const T v2 = (vi.y + dt * ay) * f.D;
+    const T x1 = xi.x + dt * v1;
+    const T x2 = xi.y + dt * v2;
+    velOut[i] = mk2<T>(v1, v2);
+    posOut[i] = mk2<T>(x1, x2);
+    if (!(isfinite(x1) && isfinite(x2) && isfinite(v1) && isfinite(v2)))
+        atomicOr(flags, FLAG_NONFINITE);
 }
 
 // Accel recompute + _adj_integrate! + _adj_drag!; one exponent update per
 // particle (these launches cover few particles).
 template <typename T, int G>
-__global__ void __launch_bounds__(kCoopBlock)
+__global__ void __launch_bounds__(kCoopThreads)
     k_accel_drag_adj_coop(const __grid_constant__ NLView<T> v, const T2<T> *__restrict__ vel,
                           const T2<T> *__restrict__ prho, const T *__restrict__ rho,
                           const T *__restrict__ theta,
@@ -430,30 +465,57 @@ __global__ void __launch_bounds__(kCoopBlock)
     constexpr int NG = kCoopBlock / G;
     __shared__ __align__(16) T buf[NG][4][G];
     __shared__ int32_t lst[NG][kSpillList];
+    __shared__ SideForce<T> side[NG];
+    __shared__ T2<T> s_gv[NG];
     const Group<G> g;
-    const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
-    if (i >= v.N) return;
+    const bool fifth = threadIdx.x >= kCoopBlock;
+    const int q = fifth ? (int)threadIdx.x - kCoopBlock : g.gi;
+    const int64_t i = (int64_t)blockIdx.x * NG + q;
+    const bool live = q < NG && i < v.N;
     const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[i];
-    const T2<T> vi = vel[i];
-    const uint32_t cc = v.center[i];
-    T ax, ay;
-    if ((cc >> 31) && I.maxnb > kSpillList) {
-        if (g.gl != 0) return;
-        accel_sum<T, true>(v, I, vel, prho, rho, i, xi, vi, ax, ay);
-    } else {
-        const Cands<T> cd = pass_cands<T, G>(g, v, I, i, cc, lst[g.gi]);
-        accel_sum_coop<T, G, NG>(g, buf, v, I, i, cd, vel, prho, rho, xi, vi, ax, ay);
-        if (g.gl != 0) return;
+    const T dt = I.p.dt;
+    T2<T> vi = mk2<T>((T)0, (T)0);
+    T ax = (T)0, ay = (T)0;
+    if (live) {
+        const T2<T> xi = v.pos[i];
+        vi = vel[i];
+        if (fifth) {
+            const T2<T> gx = gX[i];
+            T2<T> gv = gV[i];
+            const SideForce<T> f = side_force<T>(I, xi, theta);
+            gv.x += dt * gx.x;
+            gv.y += dt * gx.y;
+            abar[i] = mk2<T>(dt * f.D * gv.x, dt * f.D * gv.y);
+            gV[i] = mk2<T>(f.D * gv.x, f.D * gv.y);
+            side[q] = f;
+            s_gv[q] = gv;
+        } else {
+            const uint32_t cc = v.center[i];
+            if ((cc >> 31) && I.maxnb > kSpillList) {
+                if (g.gl == 0) accel_sum<T, true>(v, I, vel, prho, rho, i, xi, vi, ax, ay);
+            } else {
+                const Cands<T> cd = pass_cands<T, G>(g, v, I, i, cc, lst[g.gi]);
+                accel_sum_coop<T, G, NG>(g, buf, v, I, i, cd, vel, prho, rho, xi, vi, ax, ay);
+            }
+        }
     }
-    const int e = drag_adj_finish<T>(I, i, xi, vi, ax, ay, theta, gX, gV, abar, galpha);
-    if (e != INT_MIN) atomicMax(emax + parity, e);
+    __syncthreads();
+    if (!live || fifth || g.gl != 0) return;
+    const SideForce<T> f = side[q];
+    const T2<T> gv = s_gv[q];
+    ax += f.gx;
+    ay += f.gy;
+    const T vx = (vi.x + dt * ax) * f.D;
+    const T vy = (vi.y + dt * ay) * f.D;
+    const T ga = -dt * f.D * (vx * gv.x + vy * gv.y);
+    galpha[i] = ga;
+    if (ga != (T)0 && isfinite(ga)) atomicMax(emax + parity, ilogb((double)ga) + 1); // |ga| < 2^e
 }
 
 // adj_pass1_kernel! + the gXs half of adj_design_kernel! + _axpy2!(gV, gVs).
 // Lanes 0..5 keep gx, gy, gvx, gvy, grho, S.
 template <typename T, int G>
-__global__ void __launch_bounds__(kCoopBlock)
+__global__ void __launch_bounds__(kCoopThreads)
     k_pass1_design_coop(const __grid_constant__ NLView<T> v, const T2<T> *__restrict__ vel,
                         const T2<T> *__restrict__ prho, const T *__restrict__ rho,
                         const T *__restrict__ theta,
@@ -464,20 +526,27 @@ __global__ void __launch_bounds__(kCoopBlock)
     constexpr int NG = kCoopBlock / G;
     __shared__ __align__(16) T buf[NG][9][G]; // eight term slots and a row of zeros
     __shared__ int32_t lst[NG][kSpillList];
+    __shared__ Pass1Side<T> side[NG];
     const Group<G> g;
-    const int64_t i = (int64_t)blockIdx.x * NG + g.gi;
-    if (i >= v.N) return;
+    const bool fifth = threadIdx.x >= kCoopBlock;
+    const int q = fifth ? (int)threadIdx.x - kCoopBlock : g.gi;
+    const int64_t i = (int64_t)blockIdx.x * NG + q;
+    const bool live = q < NG && i < v.N;
     const Inst<T> &I = v.one;
-    const T2<T> xi = v.pos[i];
-    const T2<T> vi = vel[i];
-    const T2<T> ab = abar[i];
-    const T2<T> pi = prho[i];
-    const uint32_t cc = v.center[i];
-    T gx, gy, gvx, gvy, grh, sumS;
-    if ((cc >> 31) && I.maxnb > kSpillList) {
-        if (g.gl != 0) return;
-        pass1_sum<T, true>(v, I, i, vel, prho, rho, abar, xi, vi, ab, pi, gx, gy, gvx, gvy, grh,
-                           sumS);
+    const T2<T> zero = mk2<T>((T)0, (T)0);
+    const T2<T> xi = live ? v.pos[i] : zero;
+    const T2<T> vi = live ? vel[i] : zero;
+    const T2<T> ab = live ? abar[i] : zero;
+    const T2<T> pi = live ? prho[i] : zero;
+    const uint32_t cc = live ? v.center[i] : 0u;
+    T gx = (T)0, gy = (T)0, gvx = (T)0, gvy = (T)0, grh = (T)0, sumS = (T)0;
+    if (fifth) {
+        if (live) side[q] = pass1_side<T>(I, i, xi, theta, galpha, gV);
+    } else if (!live) {
+    } else if ((cc >> 31) && I.maxnb > kSpillList) {
+        if (g.gl == 0)
+            pass1_sum<T, true>(v, I, i, vel, prho, rho, abar, xi, vi, ab, pi, gx, gy, gvx, gvy,
+                               grh, sumS);
     } else {
         const T r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, Fc = I.p.Fc, Gc = I.p.Gc;
         const Visc<T> vc = visc_of<T>(I);
@@ -535,11 +604,11 @@ __global__ void __launch_bounds__(kCoopBlock)
         gvy = g.from(acc, 3);
         grh = g.from(acc, 4);
         sumS = g.from(acc, 5);
-        if (g.gl != 0) return;
     }
+    __syncthreads();
+    if (!live || fifth || g.gl != 0) return;
     const T rhoi = needs_rho_dev(I) ? rho[i] : (T)0;
-    pass1_finish<T>(I, i, xi, ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, theta, galpha, gXs, grho,
-                    gV);
+    pass1_put<T>(I, i, side[q], ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, gXs, grho, gV);
 }
 
 // adj_pass2_kernel! + _axpy2!(gX, gXs) + the exact theta write-back. A fifth warp
@@ -547,9 +616,8 @@ __global__ void __launch_bounds__(kCoopBlock)
 // value of its accumulator, so one lane took four waits after the pair sums), and
 // loads the next tape state: 1500 FP32 particles 6.4 -> 4.3 us, its floor of a
 // launch being 2.
-constexpr int kCoopPass2 = kCoopBlock + 32;
 template <typename T, int G>
-__global__ void __launch_bounds__(kCoopPass2)
+__global__ void __launch_bounds__(kCoopThreads)
     k_pass2_axpy_coop(const __grid_constant__ NLView<T> v, const T *__restrict__ grho,
                       const T2<T> *__restrict__ gXs, T2<T> *__restrict__ gX,
                       const T *__restrict__ galpha, const int *__restrict__ emax, int parity,

@@ -900,8 +900,8 @@ template <typename T> class Sys final : public StateI {
             SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush());
             v.tmask = tmask.p;
             auto ki = G == 32 ? &k_accel_integrate_coop<T, 32> : &k_accel_integrate_coop<T, 16>;
-            SPH_LAUNCH_COOP(K_ACCEL_INTEGRATE, G, ki, N_, v, vel[cur].p, prho.p, rho.p, theta,
-                            pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
+            SPH_LAUNCH_COOP_X(K_ACCEL_INTEGRATE, G, 0, kCoopThreads, ki, N_, v, vel[cur].p, prho.p,
+                              rho.p, theta, pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
         } else if (tiles()) {
             if constexpr (sizeof(T) == 4) {
                 density_tiles(v, rho.p, prho.p);
@@ -1500,11 +1500,11 @@ template <typename T> class Work final : public WorkI {
             SPH_LAUNCH_COOP_X(K_DENSITY, G, extra, kCoopBlock, kd, N_, v, rhoOut, S.prho.p,
                               S.tmask.p, fl);
             v.tmask = S.tmask.p;
-            SPH_LAUNCH_COOP(K_ACCEL_DRAG, G, ka, N_, v, vel, S.prho.p, S.rho.p, theta, gX[gcur].p,
-                            gV[gcur].p, abar.p, galpha.p, emax.p, parity);
-            SPH_LAUNCH_COOP(K_PASS1, G, k1, N_, v, vel, S.prho.p, S.rho.p, theta, abar.p,
-                            galpha.p, gXs.p, grho.p, gV[gcur].p);
-            SPH_LAUNCH_COOP_X(K_PASS2, G, 0, kCoopPass2, k2, N_, v, grho.p, gXs.p, gX[gcur].p,
+            SPH_LAUNCH_COOP_X(K_ACCEL_DRAG, G, 0, kCoopThreads, ka, N_, v, vel, S.prho.p, S.rho.p,
+                              theta, gX[gcur].p, gV[gcur].p, abar.p, galpha.p, emax.p, parity);
+            SPH_LAUNCH_COOP_X(K_PASS1, G, 0, kCoopThreads, k1, N_, v, vel, S.prho.p, S.rho.p, theta,
+                              abar.p, galpha.p, gXs.p, grho.p, gV[gcur].p);
+            SPH_LAUNCH_COOP_X(K_PASS2, G, 0, kCoopThreads, k2, N_, v, grho.p, gXs.p, gX[gcur].p,
                               galpha.p, emax.p, parity, thetaAcc.p, next);
             pendingTheta = parity;
             return;

@@ -456,23 +456,6 @@ __device__ __forceinline__ void flat_force(const NLView<double> &v, uint32_t ser
     }
 }
 
-// What accel_integrate_finish and drag_adj_finish form without the pair sum:
-// gravity plus wall, the Brinkman alpha and D = 1 / (1 + dt alpha).
-struct FlatForce {
-    double gx, gy, al, D;
-};
-template <typename IT>
-__device__ __forceinline__ FlatForce flat_force_of(const IT &I, const double2 &x,
-                                                   const double *__restrict__ theta)
-{
-    FlatForce f;
-    f.al = interp_alpha_value<double>(theta + I.toff, x.x, x.y, I.p);
-    f.gx = I.p.gx + wall_accel<double>(x.x, I.p.Lx, I.p.kw);
-    f.gy = I.p.gy + wall_accel<double>(x.y, I.p.Ly, I.p.kw);
-    f.D = div_rn(1.0, 1.0 + I.p.dt * f.al);
-    return f;
-}
-
 // accel_kernel! + integrate_kernel! (accel_integrate_finish)
 template <bool MULTI>
 __global__ void __launch_bounds__(kFlatThreads)
@@ -486,7 +469,7 @@ __global__ void __launch_bounds__(kFlatThreads)
 {
     pdl_enter();
     __shared__ double s_t[4][kFlatChunk], s_acc[2 * kFlatMax];
-    __shared__ FlatForce s_f[kFlatMax];
+    __shared__ SideForce<double> s_f[kFlatMax];
     __shared__ FlatShared S;
     const FlatPass<MULTI> Q(v, B, S);
     flat_accel<MULTI>(Q, S, s_t, s_acc, vel, prho, [&] {
@@ -499,7 +482,7 @@ __global__ void __launch_bounds__(kFlatThreads)
             tx[id] = xi;
             tv[id] = vel[i];
         }
-        const FlatForce f = flat_force_of(I, xi, theta);
+        const SideForce<double> f = side_force<double>(I, xi, theta);
         if (alphaOut) alphaOut[i] = f.al;
         s_f[Q.t - kFlatBlock] = f;
     });
@@ -508,7 +491,7 @@ __global__ void __launch_bounds__(kFlatThreads)
     const int b = MULTI ? inst_of(v, i) : 0;
     decltype(auto) I = load_inst<MULTI>(v, i);
     const double2 xi = v.pos[i], vi = vel[i];
-    const FlatForce f = s_f[Q.t];
+    const SideForce<double> f = s_f[Q.t];
     double ax, ay;
     flat_force<MULTI>(v, S.serial, i, s_acc, vel, prho, xi, vi, ax, ay);
     ax += f.gx;
@@ -536,7 +519,7 @@ __global__ void __launch_bounds__(kFlatThreads)
 {
     pdl_enter();
     __shared__ double s_t[4][kFlatChunk], s_acc[2 * kFlatMax];
-    __shared__ FlatForce s_f[kFlatMax];
+    __shared__ SideForce<double> s_f[kFlatMax];
     __shared__ double2 s_gv[kFlatMax];
     __shared__ FlatShared S;
     const FlatPass<MULTI> Q(v, B, S);
@@ -544,7 +527,7 @@ __global__ void __launch_bounds__(kFlatThreads)
         const int64_t i = Q.aside();
         if (i < 0) return;
         decltype(auto) I = load_inst<MULTI>(v, i);
-        const FlatForce f = flat_force_of(I, v.pos[i], theta);
+        const SideForce<double> f = side_force<double>(I, v.pos[i], theta);
         const double dt = I.p.dt;
         const double2 gx = gX[i];
         double2 gv = gV[i];
@@ -562,7 +545,7 @@ __global__ void __launch_bounds__(kFlatThreads)
         b = MULTI ? inst_of(v, i) : 0;
         decltype(auto) I = load_inst<MULTI>(v, i);
         const double2 xi = v.pos[i], vi = vel[i];
-        const FlatForce f = s_f[Q.t];
+        const SideForce<double> f = s_f[Q.t];
         const double2 gv = s_gv[Q.t];
         double ax, ay;
         flat_force<MULTI>(v, S.serial, i, s_acc, vel, prho, xi, vi, ax, ay);

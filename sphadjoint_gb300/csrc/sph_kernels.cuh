@@ -1296,6 +1296,23 @@ __device__ __forceinline__ void accel_integrate_finish(
     T2<T> *__restrict__ aOut, T *__restrict__ alphaOut, uint32_t *__restrict__ flags,
     const int32_t *__restrict__ perm, T2<T> *__restrict__ tx, T2<T> *__restrict__ tv);
 
+// What accel_integrate_finish and drag_adj_finish form without the pair sum:
+// gravity plus wall, the Brinkman alpha and D = 1 / (1 + dt alpha).
+template <typename T> struct SideForce {
+    T gx, gy, al, D;
+};
+template <typename T, typename IT>
+__device__ __forceinline__ SideForce<T> side_force(const IT &I, const T2<T> &x,
+                                                   const T *__restrict__ theta)
+{
+    SideForce<T> f;
+    f.al = interp_alpha_value<T>(theta + I.toff, x.x, x.y, I.p);
+    f.gx = I.p.gx + wall_accel<T>(x.x, I.p.Lx, I.p.kw);
+    f.gy = I.p.gy + wall_accel<T>(x.y, I.p.Ly, I.p.kw);
+    f.D = div_rn((T)1, (T)1 + I.p.dt * f.al);
+    return f;
+}
+
 // accel_kernel! (pressure + viscosity + gravity + wall, and alpha) fused with
 // integrate_kernel! (semi-implicit Euler, implicit Brinkman drag).
 template <typename T, bool MULTI, bool AV = false>
@@ -1599,6 +1616,45 @@ __device__ __forceinline__ void pass1_sum(const NLView<T> &v, const IT &I, int64
 
 // Per-particle tail of adj_pass1_kernel! (src/adjoint.jl:112-121), the gXs
 // half of adj_design_kernel! and _axpy2!(gV, gVs).
+// What pass 1 adds to a particle's pair sums: the walls' derivatives, galpha times
+// the gradient of alpha, and the velocity adjoint so far.
+template <typename T> struct Pass1Side {
+    T wx, wy, ga, dadx, dady;
+    T2<T> gv;
+};
+template <typename T, typename IT>
+__device__ __forceinline__ Pass1Side<T> pass1_side(const IT &I, int64_t i, const T2<T> &xi,
+                                                   const T *__restrict__ theta,
+                                                   const T *__restrict__ galpha,
+                                                   const T2<T> *__restrict__ gV)
+{
+    const Phys<T> &p = I.p;
+    Pass1Side<T> f;
+    f.wx = wall_daccel<T>(xi.x, p.Lx, p.kw);
+    f.wy = wall_daccel<T>(xi.y, p.Ly, p.kw);
+    T al;
+    interp_alpha<T>(theta + I.toff, xi.x, xi.y, p, al, f.dadx, f.dady);
+    f.ga = galpha[i];
+    f.gv = gV[i];
+    return f;
+}
+template <typename T, typename IT>
+__device__ __forceinline__ void pass1_put(const IT &I, int64_t i, const Pass1Side<T> &f,
+                                          const T2<T> &ab, const T2<T> &pi, T rhoi, T gx, T gy,
+                                          T gvx, T gvy, T grh, T sumS, T2<T> *__restrict__ gXs,
+                                          T *__restrict__ grho, T2<T> *__restrict__ gV)
+{
+    const T pti = pi.x, iri = pi.y;
+    const Phys<T> &p = I.p;
+    grh += ((T)(-2) * p.m * pti * iri) * sumS;
+    if (p.eos == 1) grh += p.dB * pow_fold<T>(div_rn(rhoi, p.rho0), p.gam - 1) * p.m * iri * iri * sumS;
+    else grh += p.c2 * p.m * iri * iri * sumS;
+    gx += ab.x * f.wx;
+    gy += ab.y * f.wy;
+    gXs[i] = mk2<T>(gx + f.ga * f.dadx, gy + f.ga * f.dady);
+    grho[i] = grh;
+    gV[i] = mk2<T>(f.gv.x + gvx, f.gv.y + gvy);
+}
 template <typename T, typename IT>
 __device__ __forceinline__ void pass1_finish(const IT &I, int64_t i, const T2<T> &xi,
                                              const T2<T> &ab, const T2<T> &pi, T rhoi, T gx,
@@ -1607,22 +1663,8 @@ __device__ __forceinline__ void pass1_finish(const IT &I, int64_t i, const T2<T>
                                              const T *__restrict__ galpha, T2<T> *__restrict__ gXs,
                                              T *__restrict__ grho, T2<T> *__restrict__ gV)
 {
-    const T pti = pi.x, iri = pi.y;
-    const Phys<T> &p = I.p;
-    grh += ((T)(-2) * p.m * pti * iri) * sumS;
-    if (p.eos == 1) grh += p.dB * pow_fold<T>(div_rn(rhoi, p.rho0), p.gam - 1) * p.m * iri * iri * sumS;
-    else grh += p.c2 * p.m * iri * iri * sumS;
-    gx += ab.x * wall_daccel<T>(xi.x, p.Lx, p.kw);
-    gy += ab.y * wall_daccel<T>(xi.y, p.Ly, p.kw);
-    T al, dadx, dady;
-    interp_alpha<T>(theta + I.toff, xi.x, xi.y, p, al, dadx, dady);
-    const T ga = galpha[i];
-    gXs[i] = mk2<T>(gx + ga * dadx, gy + ga * dady);
-    grho[i] = grh;
-    T2<T> g = gV[i];
-    g.x += gvx;
-    g.y += gvy;
-    gV[i] = g;
+    pass1_put<T>(I, i, pass1_side<T>(I, i, xi, theta, galpha, gV), ab, pi, rhoi, gx, gy, gvx, gvy,
+                 grh, sumS, gXs, grho, gV);
 }
 
 // 128-bit two's-complement fixed-point accumulation: integer addition is
