@@ -88,23 +88,28 @@ cudaError_t rt_malloc(void **p, size_t bytes, cudaStream_t s)
     return cudaMallocAsync(p, bytes, s);
 }
 
-size_t rt_free_memory()
+bool rt_has_free(size_t bytes)
 {
-    size_t fr = 0, tot = 0;
     int dev = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
-    }
     cudaMemPool_t pool;
     uint64_t held = 0, used = 0;
+    size_t spare = 0, fr = 0, tot = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
     if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
         held > used)
-        fr += (size_t)(held - used);
+        spare = (size_t)(held - used);
     (void)cudaGetLastError();
-    return fr;
+    if (spare >= bytes) return true; // without asking the driver
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return fr + spare >= bytes;
 }
 
 void rt_free(void *p, cudaStream_t s)

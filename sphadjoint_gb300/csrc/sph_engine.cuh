@@ -356,6 +356,7 @@ template <typename T> class Sys final : public StateI {
     DevBuf<int32_t> clStart, clOrder; // build! without a neighbour rebuild
     bool cellsOnlyLatest = false;
     bool keepAccel = false;
+    DevBuf<uint8_t> scratch; // holds the two groups of optional buffers below
     DevBuf<TileWin> wwin; // windows and neighbour lists of the FP32 tile passes
     DevBuf<uint2> wcand, wsupp;
     DevBuf<uint8_t> wcnt; // candidate counts, then in-support counts
@@ -489,12 +490,13 @@ template <typename T> class Sys final : public StateI {
         }
         nbcount.alloc(n1);
         cellTmp.alloc(n1);
-        counts.alloc((size_t)ncell);
-        counts.zero(); // and zero again after every cell list
+        // zero now and again after every cell list; the scan's tile sums behind it
+        const size_t ntile = (size_t)((ncell + kScanTile - 1) / kScanTile);
+        counts.alloc((size_t)ncell + ntile);
+        scanTmp.view(counts.p + ncell, ntile);
+        counts.zero();
         bucketSrc.alloc(n1);
         bucketId.alloc(n1);
-        scanTmp.alloc((size_t)((ncell + kScanTile - 1) / kScanTile + 1));
-        scanTmp.zero();
         flags.alloc((size_t)B);
         tmask.alloc(6 * n1);
         // staged windows end on multiples of four slots: room for three more
@@ -572,40 +574,46 @@ template <typename T> class Sys final : public StateI {
         if (want_flat() && !listsTried && !rt_capturing()) {
             listsTried = true;
             const size_t P = (size_t)flat_particles(N_), nb = ((size_t)N_ + P - 1) / P;
-            if (rt_free_memory() / 8 < nb * P * (kFlatRow * 20 + 8) + nb * 4 * kFlatOff) return;
-            try {
-                fF.alloc(nb * P * kFlatRow);
-                fr.alloc(nb * P * kFlatRow);
-                ftm.alloc(nb * P);
-                fpair.alloc(nb * P * kFlatRow);
-                foff.alloc(nb * kFlatOff);
-            } catch (const Error &) {
-                fF.release();
-                fr.release();
-                ftm.release();
-                fpair.release();
-                foff.release();
-            }
+            carve_scratch([&](auto &&part) {
+                part(fF, nb * P * kFlatRow);
+                part(fr, nb * P * kFlatRow);
+                part(ftm, nb * P);
+                part(fpair, nb * P * kFlatRow);
+                part(foff, nb * kFlatOff);
+            });
         }
+    }
+    // Optional buffers in one allocation, if that is at most an eighth of the free
+    // memory: parts(part) names them twice, for their size and for their place.
+    // (An allocation each, and asking the driver for its free memory each time,
+    // showed in streams of small requests.)
+    template <typename F> void carve_scratch(F &&parts)
+    {
+        size_t off = 0;
+        parts([&](auto &b, size_t n) { off += (n * sizeof(*b.p) + 255) & ~(size_t)255; });
+        if (!rt_has_free(8 * off)) return;
+        try {
+            scratch.alloc(off);
+        } catch (const Error &) {
+            return;
+        }
+        uint8_t *at = scratch.p;
+        parts([&](auto &b, size_t n) {
+            b.view(reinterpret_cast<decltype(b.p)>(at), n);
+            at += (n * sizeof(*b.p) + 255) & ~(size_t)255;
+        });
     }
     void alloc_lists()
     {
         if (listsTried || rt_capturing() || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN) return;
         listsTried = true;
         const size_t nt = (size_t)((N_ + kTile - 1) / kTile), e = nt * kQuads * kTile;
-        const size_t bytes = nt * sizeof(TileWin) + 2 * e * sizeof(uint2) + 2 * nt * kTile;
-        if (rt_free_memory() / 8 < bytes) return;
-        try {
-            wcand.alloc(e);
-            wsupp.alloc(e);
-            wcnt.alloc(2 * nt * kTile);
-            wwin.alloc(nt);
-        } catch (const Error &) {
-            wcand.release();
-            wsupp.release();
-            wcnt.release();
-            wwin.release();
-        }
+        carve_scratch([&](auto &&part) {
+            part(wcand, e);
+            part(wsupp, e);
+            part(wcnt, 2 * nt * kTile);
+            part(wwin, nt);
+        });
     }
     WinLists lists() const
     {

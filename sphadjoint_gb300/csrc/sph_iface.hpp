@@ -77,7 +77,7 @@ cudaStream_t rt_stream();
 void rt_set_stream(cudaStream_t s);
 // Stream-ordered device allocation (the device's default memory pool, kept
 // cached between requests).
-size_t rt_free_memory(); // device bytes free now, the pool's unused ones included
+bool rt_has_free(size_t bytes); // are that many device bytes free, the pool's unused ones included?
 cudaError_t rt_malloc(void **p, size_t bytes, cudaStream_t s);
 void rt_free(void *p, cudaStream_t s);
 void rt_before_launch(int kid);
