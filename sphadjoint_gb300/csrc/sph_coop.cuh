@@ -126,6 +126,18 @@ template <typename T> struct Cands {
 #pragma unroll
         for (int w = 0; w < 6; ++w) pre[w + 1] = pre[w] + __popc(wd[w]);
     }
+    // from the words in registers, rows starting at slots b
+    __device__ __forceinline__ void init_words(const uint32_t (&words)[6], const int (&b)[3])
+    {
+        lst = nullptr;
+        pre[0] = 0;
+#pragma unroll
+        for (int w = 0; w < 6; ++w) {
+            wd[w] = words[w];
+            bs[w] = b[w >> 1] + 32 * (w & 1);
+            pre[w + 1] = pre[w] + __popc(wd[w]);
+        }
+    }
     __device__ __forceinline__ int total() const { return lst ? nl : pre[6]; }
     // slot of candidate k < total(); w, bit: its word and bit (w = -1 for a
     // listed candidate: a spilled particle has no in-support words)
@@ -197,18 +209,21 @@ __device__ __forceinline__ int spill_list(const Group<G> &g, const NLView<T> &v,
 
 // _nl_build! (src/neighbors.jl:192-245) with the row scan spread over the
 // group: each round tests G consecutive slots, a ballot gives the passing
-// ones, and the first (maxnb - kept) of them are kept, in slot order.
+// ones, and the first (maxnb - kept) of them are kept, in slot order. The three
+// rows' bounds, then their first rounds' positions, are loaded together. Writes
+// the particle's masks, count and cell and leaves them in wd, n and the return
+// value, with the rows' first slots in bs.
+template <typename T> struct NlOut {
+    uint32_t *center, *masks, *flags;
+    int32_t *nbcount;
+};
 template <typename T, int G>
-__global__ void __launch_bounds__(kCoopBlock)
-    k_nl_build_coop(int64_t N, const Inst<T> I, const T2<T> *__restrict__ pos,
-                    const int32_t *__restrict__ cellStart, uint32_t *__restrict__ center,
-                    uint32_t *__restrict__ masks, int32_t *__restrict__ nbcount,
-                    uint32_t *__restrict__ flags)
+__device__ __forceinline__ uint32_t nl_group(const Group<G> &g, int64_t N, const Inst<T> &I,
+                                             int64_t i, const T2<T> *__restrict__ pos,
+                                             const int32_t *__restrict__ cellStart,
+                                             const NlOut<T> &out, uint32_t (&wd)[6], int (&bs)[3],
+                                             int &n)
 {
-    pdl_enter();
-    const Group<G> g;
-    const int64_t i = (int64_t)blockIdx.x * (kCoopBlock / G) + g.gi;
-    if (i >= N) return; // the whole group
     const int nx = I.nx, ny = I.ny, maxnb = I.maxnb;
     const T2<T> xi = pos[i];
     const NlTest<T> test(I, xi);
@@ -216,55 +231,81 @@ __global__ void __launch_bounds__(kCoopBlock)
     const int cy = cell_coord<T>(xi.y * I.invcs, ny);
     const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
     const int jx1 = cx + 1 < nx ? cx + 1 : nx;
+    int e[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int jy = cy + r - 1;
+        const int row = I.coff + (jy - 1) * nx;
+        const bool is = jy >= 1 && jy <= ny;
+        bs[r] = is ? cellStart[row + jx0 - 1] : 0;
+        e[r] = is ? cellStart[row + jx1] : 0;
+    }
+    T2<T> x0[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) x0[r] = pos[bs[r] + g.gl < e[r] ? bs[r] + g.gl : i];
     uint32_t spill = 0;
     int m = 0;
     bool over = false;
-#pragma unroll 1
+#pragma unroll
     for (int r = 0; r < 3; ++r) {
         uint32_t lo = 0, hi = 0;
-        const int jy = cy + r - 1;
-        if (jy >= 1 && jy <= ny) {
-            const int row = I.coff + (jy - 1) * nx;
-            const int b = cellStart[row + jx0 - 1];
-            const int e = cellStart[row + jx1];
-            if (e - b > 64) spill = 1;
-            for (int base = b; base < e; base += G) {
-                const int j = base + g.gl;
-                bool pass = false;
-                if (j < e && j != (int)i) pass = test(pos[j]);
-                uint32_t kept = g.ballot(pass);
-                const int np = __popc(kept), room = maxnb - m;
-                if (np > room) {
-                    over = true;
-                    kept = room > 0 ? kept & ((1u << select_bit(kept, room)) - 1u) : 0u;
-                }
-                m += __popc(kept);
-                const int off = base - b;
-                if (off < 64) {
-                    const uint64_t w64 = (uint64_t)kept << off;
-                    lo |= (uint32_t)w64;
-                    hi |= (uint32_t)(w64 >> 32);
-                }
+        const int b = bs[r], len = e[r] - b;
+        if (len > 64) spill = 1;
+        for (int off = 0; off < len; off += G) {
+            const int j = b + off + g.gl;
+            bool pass = false;
+            if (off + g.gl < len && j != (int)i) pass = test(off == 0 ? x0[r] : pos[j]);
+            uint32_t kept = g.ballot(pass);
+            const int np = __popc(kept), room = maxnb - m;
+            if (np > room) {
+                over = true;
+                kept = room > 0 ? kept & ((1u << select_bit(kept, room)) - 1u) : 0u;
+            }
+            m += __popc(kept);
+            if (off < 64) {
+                const uint64_t w64 = (uint64_t)kept << off;
+                lo |= (uint32_t)w64;
+                hi |= (uint32_t)(w64 >> 32);
             }
         }
-        if (g.gl == 0) {
-            masks[(int64_t)(2 * r) * N + i] = lo;
-            masks[(int64_t)(2 * r + 1) * N + i] = hi;
-        }
+        wd[2 * r] = lo;
+        wd[2 * r + 1] = hi;
     }
+    const uint32_t cc = (uint32_t)cx | ((uint32_t)cy << 16) | (spill << 31);
+    n = m;
     if (g.gl == 0) {
-        center[i] = (uint32_t)cx | ((uint32_t)cy << 16) | (spill << 31);
-        nbcount[i] = m;
-        if (over) atomicOr(flags, FLAG_NL_OVERFLOW);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) out.masks[(int64_t)q * N + i] = wd[q];
+        out.center[i] = cc;
+        out.nbcount[i] = m;
+        if (over) atomicOr(out.flags, FLAG_NL_OVERFLOW);
     }
+    return cc;
 }
 
-// density_kernel! + eos_kernel!, and this step's in-support words.
 template <typename T, int G>
+__global__ void __launch_bounds__(kCoopBlock)
+    k_nl_build_coop(int64_t N, const Inst<T> I, const T2<T> *__restrict__ pos,
+                    const int32_t *__restrict__ cellStart, const NlOut<T> out)
+{
+    pdl_enter();
+    const Group<G> g;
+    const int64_t i = (int64_t)blockIdx.x * (kCoopBlock / G) + g.gi;
+    if (i >= N) return; // the whole group
+    uint32_t wd[6];
+    int bs[3], n;
+    nl_group<T, G>(g, N, I, i, pos, cellStart, out, wd, bs, n);
+}
+
+// density_kernel! + eos_kernel!, and this step's in-support words. BUILD: of a fresh
+// cell list; the group builds its particle's masks first and takes them from its
+// registers. One launch and one read of the masks less per rebuild: 48 steps of 1500
+// FP32 particles with gradient 1.45 -> 1.38 ms.
+template <typename T, int G, bool BUILD>
 __global__ void __launch_bounds__(kCoopBlock)
     k_density_eos_coop(const __grid_constant__ NLView<T> v, T *__restrict__ rho,
                        T2<T> *__restrict__ prho, uint32_t *__restrict__ tmaskOut,
-                       const ThetaFlush<T> flush)
+                       const ThetaFlush<T> flush, const NlOut<T> out)
 {
     pdl_enter();
     if (theta_flush<T>(flush)) return;
@@ -278,13 +319,18 @@ __global__ void __launch_bounds__(kCoopBlock)
     const Inst<T> &I = v.one;
     const T r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, A = I.p.A;
     const T2<T> xi = v.pos[i];
-    const uint32_t cc = v.center[i];
+    uint32_t wd[6], cc;
+    int bs[3], nb;
+    if (BUILD) cc = nl_group<T, G>(g, v.N, I, i, v.pos, v.cellStart, out, wd, bs, nb);
+    else cc = v.center[i];
     if ((cc >> 31) && I.maxnb > kSpillList) {
+        g.sync(); // the masks just written are read here
         if (g.gl == 0) density_finish<T>(I, i, density_spill_sum<T>(v, I, i, xi, tmaskOut), rho, prho);
         return;
     }
     Cands<T> cd;
     if (cc >> 31) cd.init_list(lst[g.gi], spill_list<T, G>(g, v, I, i, cc, lst[g.gi]));
+    else if (BUILD) cd.init_words(wd, bs);
     else cd.init(v, I, i, cc, v.masks);
     const int K = cd.total();
     if (g.gl < 6) tws[g.gi][g.gl] = 0u;

@@ -365,6 +365,7 @@ template <typename T> class Sys final : public StateI {
     DevBuf<int32_t> foff;
     bool listsTried = false; // the lists were asked for (and may have been refused)
     bool listsFresh = false; // they belong to the masks the state holds
+    bool masksDue = false;   // the next density pass builds the masks (set and taken within a step)
     StepGraphs graphs;   // simulate's steps, replayed in groups
     bool anyRho = false; // some instance's model reads densities in the adjoint
     bool anyAV = false;  // some instance uses the artificial viscosity
@@ -778,7 +779,7 @@ template <typename T> class Sys final : public StateI {
     // the particle data (and of up to two extra per-particle arrays) into the
     // new cell order, neighbour masks. ex*N receive the permuted extras.
     void rebuild(const T2<T> *ex0 = nullptr, T2<T> *ex0N = nullptr, const T2<T> *ex1 = nullptr,
-                 T2<T> *ex1N = nullptr)
+                 T2<T> *ex1N = nullptr, bool defer = false)
     {
         const int check = age != INT64_MAX ? 1 : 0;
         if (N_ > 0 && B == 1 && N_ <= kRebuildSmallMaxN && ncell <= kRebuildSmallMaxCells) {
@@ -798,7 +799,7 @@ template <typename T> class Sys final : public StateI {
                      invperm.p, cellStart.p, ex0, ex0N, ex1, ex1N, flags.p);
             rt_after_launch(K_RANK);
             cur = nxt;
-            build_masks();
+            build_masks(defer);
         } else if (N_ > 0) {
             // nbcount is rewritten by the mask build: until then it holds the places
             bucket_cells(check, nbcount.p, cellStart.p);
@@ -807,10 +808,33 @@ template <typename T> class Sys final : public StateI {
                        bucketId.p, pos[cur].p, vel[cur].p, pos[nxt].p, vel[nxt].p, xref.p, perm.p,
                        invperm.p, ex0, ex0N, ex1, ex1N);
             cur = nxt;
-            build_masks();
+            build_masks(defer);
         }
         age = 0;
         cellsOnlyLatest = false;
+    }
+
+    NlOut<T> nl_out() { return NlOut<T>{center.p, masks.p, flags.p, nbcount.p}; }
+
+    // The masks of the cell list just built, now, or with `defer` and a small single
+    // state by the density pass that its caller launches next (masksDue).
+    void build_masks(bool defer)
+    {
+        masksDue = defer && B == 1 && N_ > 0 && !tiles() &&
+                   (flat() ? flat_particles(N_) <= kFlatBuild : group_lanes() != 0);
+        if (masksDue) listsFresh = false;
+        else build_masks();
+    }
+    static auto density_coop(int G, bool build)
+    {
+        return G == 32 ? (build ? &k_density_eos_coop<T, 32, true> : &k_density_eos_coop<T, 32, false>)
+                       : (build ? &k_density_eos_coop<T, 16, true> : &k_density_eos_coop<T, 16, false>);
+    }
+    bool take_masks_due()
+    {
+        const bool due = masksDue;
+        masksDue = false;
+        return due;
     }
 
     // _nl_build! on the freshly sorted particles
@@ -826,8 +850,7 @@ template <typename T> class Sys final : public StateI {
             }
         } else if (const int G = group_lanes()) {
             auto kn = G == 32 ? &k_nl_build_coop<T, 32> : &k_nl_build_coop<T, 16>;
-            SPH_LAUNCH_COOP(K_NLBUILD, G, kn, N_, N_, hinst[0], pos[cur].p, cellStart.p,
-                            center.p, masks.p, nbcount.p, flags.p);
+            SPH_LAUNCH_COOP(K_NLBUILD, G, kn, N_, N_, hinst[0], pos[cur].p, cellStart.p, nl_out());
         } else {
             auto kn = B > 1 ? &k_nl_build<T, true> : &k_nl_build<T, false>;
             SPH_LAUNCH_TUNED(K_NLBUILD, B > 1, kn, N_, N_, hinst[0], dinst.p, pinst.p,
@@ -868,7 +891,7 @@ template <typename T> class Sys final : public StateI {
         // maybe_rebuild! (src/neighbors.jl:273-279): test, then count
         bool r = false;
         if (age >= opts.interval) {
-            rebuild(ex0, ex0N, ex1, ex1N);
+            rebuild(ex0, ex0N, ex1, ex1N, true);
             r = true;
         }
         age += 1;
@@ -887,6 +910,7 @@ template <typename T> class Sys final : public StateI {
     {
         maybe_rebuild();
         if (N_ == 0) return;
+        const bool due = take_masks_due();
         // the tape slot (tx, tv) is written by the accel pass from the same
         // pre-step state it reads
         NLView<T> v = view();
@@ -896,16 +920,17 @@ template <typename T> class Sys final : public StateI {
         if (flat()) {
             if constexpr (sizeof(T) == 8) {
                 const FlatLists W = flat_lists();
-                auto kd = B > 1 ? &k_density_flat<true> : &k_density_flat<false>;
+                auto kd = B > 1 ? &k_density_flat<true, false>
+                                : due ? &k_density_flat<false, true> : &k_density_flat<false, false>;
                 auto ki = B > 1 ? &k_accel_flat<true> : &k_accel_flat<false>;
                 SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, 0, kFlatBlock, kd, N_, v, W, rho.p, prho.p,
-                                  no_flush());
+                                  no_flush(), nl_out());
                 SPH_LAUNCH_FLAT(K_ACCEL_INTEGRATE, W.P, ki, N_, v, W, vel[cur].p, prho.p, theta,
                                 pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
             }
         } else if (const int G = group_lanes()) {
-            auto kd = G == 32 ? &k_density_eos_coop<T, 32> : &k_density_eos_coop<T, 16>;
-            SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush());
+            auto kd = density_coop(G, due);
+            SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush(), nl_out());
             v.tmask = tmask.p;
             auto ki = G == 32 ? &k_accel_integrate_coop<T, 32> : &k_accel_integrate_coop<T, 16>;
             SPH_LAUNCH_COOP_X(K_ACCEL_INTEGRATE, G, 0, kCoopThreads, ki, N_, v, vel[cur].p, prho.p,
@@ -1462,6 +1487,7 @@ template <typename T> class Work final : public WorkI {
         const int g2 = 1 - gcur;
         S.maybe_rebuild(gX[gcur].p, gX[g2].p, gV[gcur].p, gV[g2].p, &did);
         if (did) gcur = g2;
+        const bool due = S.take_masks_due();
         NLView<T> v = S.view();
         const T2<T> *vel = S.vel[S.cur].p;
         T *rhoOut = S.anyRho ? S.rho.p : (T *)nullptr; // densities only where the model reads them
@@ -1480,13 +1506,14 @@ template <typename T> class Work final : public WorkI {
             if constexpr (sizeof(T) == 8) {
                 const FlatLists W = S.flat_lists();
                 const bool multi = S.B > 1;
-                auto kd = multi ? &k_density_flat<true> : &k_density_flat<false>;
+                auto kd = multi ? &k_density_flat<true, false>
+                                : due ? &k_density_flat<false, true> : &k_density_flat<false, false>;
                 auto ka = multi ? &k_drag_flat<true> : &k_drag_flat<false>;
                 auto k1 = multi ? &k_pass1_flat<true> : &k_pass1_flat<false>;
                 auto k2 = multi ? &k_pass2_flat<true> : &k_pass2_flat<false>;
                 const ThetaFlush<T> fl = take_flush(S, (N_ + W.P - 1) / W.P, extra);
                 SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, extra, kFlatBlock, kd, N_, v, W, rhoOut, S.prho.p,
-                                  fl);
+                                  fl, S.nl_out());
                 SPH_LAUNCH_FLAT(K_ACCEL_DRAG, W.P, ka, N_, v, W, vel, S.prho.p, theta, gX[gcur].p,
                                 gV[gcur].p, abar.p, galpha.p, emax.p, parity);
                 SPH_LAUNCH_FLAT(K_PASS1, W.P, k1, N_, v, W, vel, S.prho.p, S.rho.p, theta, abar.p,
@@ -1499,14 +1526,14 @@ template <typename T> class Work final : public WorkI {
         }
         if (const int G = S.group_lanes()) {
             const bool g32 = G == 32;
-            auto kd = g32 ? &k_density_eos_coop<T, 32> : &k_density_eos_coop<T, 16>;
+            auto kd = S.density_coop(G, due);
             auto ka = g32 ? &k_accel_drag_adj_coop<T, 32> : &k_accel_drag_adj_coop<T, 16>;
             auto k1 = g32 ? &k_pass1_design_coop<T, 32> : &k_pass1_design_coop<T, 16>;
             auto k2 = g32 ? &k_pass2_axpy_coop<T, 32> : &k_pass2_axpy_coop<T, 16>;
             const int per = kCoopBlock / G;
             const ThetaFlush<T> fl = take_flush(S, (N_ + per - 1) / per, extra);
             SPH_LAUNCH_COOP_X(K_DENSITY, G, extra, kCoopBlock, kd, N_, v, rhoOut, S.prho.p,
-                              S.tmask.p, fl);
+                              S.tmask.p, fl, S.nl_out());
             v.tmask = S.tmask.p;
             SPH_LAUNCH_COOP_X(K_ACCEL_DRAG, G, 0, kCoopThreads, ka, N_, v, vel, S.prho.p, S.rho.p,
                               theta, gX[gcur].p, gV[gcur].p, abar.p, galpha.p, emax.p, parity);

@@ -123,11 +123,18 @@ __device__ __forceinline__ double flat_fold(double acc, const double *sub, const
 }
 
 // density_kernel! + eos_kernel!, and the block's dense pairs.
-template <bool MULTI>
+// BUILD: of a fresh cell list of a small single state; the block builds its
+// particles' masks first, a warp per particle. 200 steps of 240 particles with
+// gradient 8.26 -> 7.90 ms, 50 steps of 925 0.80 -> 0.76, 128 of 2072 6.57 -> 6.46. With
+// more particles a block, the warps go through too many in turn: 32 steps at 10 a
+// block 2.00 ms either way, at 16 2.35 (a launch of its own) against 2.37, at 32
+// 3.55 against 3.64.
+constexpr int kFlatBuild = 8; // particles of a block up to which it builds them
+template <bool MULTI, bool BUILD>
 __global__ void __launch_bounds__(kFlatBlock)
     k_density_flat(const __grid_constant__ NLView<double> v, const FlatLists B,
                    double *__restrict__ rho, double2 *__restrict__ prho,
-                   const ThetaFlush<double> flush)
+                   const ThetaFlush<double> flush, const NlOut<double> out)
 {
     pdl_enter();
     if (theta_flush<double>(flush)) return;
@@ -142,10 +149,36 @@ __global__ void __launch_bounds__(kFlatBlock)
     const int t = (int)threadIdx.x, P = B.P;
     const int64_t i0 = (int64_t)blockIdx.x * P;
     const int np = v.N - i0 < P ? (int)(v.N - i0) : P;
+    if constexpr (BUILD) {
+        const Group<32> g;
+        for (int a = t >> 5; a < np; a += kFlatBlock / 32) {
+            uint32_t wd[6];
+            int bs[3], n;
+            const uint32_t cc = nl_group<double, 32>(g, v.N, v.one, i0 + a, v.pos, v.cellStart,
+                                                     out, wd, bs, n);
+            if (g.gl < 3) s_bs[a][g.gl] = g.gl == 0 ? bs[0] : g.gl == 1 ? bs[1] : bs[2];
+            if (g.gl == 0) {
+                int k = 0;
+#pragma unroll
+                for (int q = 0; q < 6; ++q) {
+                    s_wd[a][q] = wd[q];
+                    s_pre[a][q] = k;
+                    k += __popc(wd[q]);
+                }
+                s_cnt[a] = cc >> 31 ? -1 : k;
+            }
+        }
+        __syncthreads();
+    }
     if (t < 32) { // the first warp: each particle's candidates and their offsets
         int n = 0;
         bool isSpill = false, isSerial = false;
-        if (t < np) {
+        if (BUILD) {
+            n = t < np ? s_cnt[t] : 0;
+            isSerial = n > kFlatRow || (n < 0 && v.one.maxnb > kFlatRow);
+            isSpill = n < 0 && !isSerial;
+            if (isSerial || isSpill) n = 0;
+        } else if (t < np) {
             const int64_t i = i0 + t;
             decltype(auto) I = load_inst<MULTI>(v, i);
             const uint32_t cc = v.center[i];
