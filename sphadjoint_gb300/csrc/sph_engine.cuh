@@ -1182,15 +1182,36 @@ template <typename T> void Sys<T>::neighbors(int32_t *indices, int32_t *nbc)
 // On-device objectives: J (deterministic block-ordered reduction in double)
 // and the terminal seeds dJ/dX_T, dJ/dV_T in particle-id order.
 // ---------------------------------------------------------------------------
+// The instances of one launch: a batch's objectives go out in groups of kObjGroup,
+// one launch for the block sums and one for the totals (with a pair of launches per
+// instance, 12 steps of a batch of 24 with gradient took 2.40 ms instead of 2.30).
+constexpr int kObjGroup = 32;
+template <typename T> struct ObjItem {
+    int64_t off, n;     // its particles
+    int64_t partial;    // its first block sum
+    int32_t block, out; // its first block in the launch, its J slot
+    T m, Lx, a0, a1, a2;
+};
+template <typename T> struct ObjItems {
+    int count, kind;
+    int64_t jslots; // the J slots' place behind the block sums
+    ObjItem<T> it[kObjGroup];
+};
+
 template <typename T>
-__global__ void k_objective(int64_t n, int64_t off, int kind, const int32_t *__restrict__ perm,
-                            const T2<T> *__restrict__ pos, const T2<T> *__restrict__ vel, T m,
-                            T Lx, T a0, T a1, T a2, T2<T> *__restrict__ seedX,
-                            T2<T> *__restrict__ seedV, double *__restrict__ partial)
+__global__ void k_objective(const __grid_constant__ ObjItems<T> L, const int32_t *__restrict__ perm,
+                            const T2<T> *__restrict__ pos, const T2<T> *__restrict__ vel,
+                            T2<T> *__restrict__ seedX, T2<T> *__restrict__ seedV,
+                            double *__restrict__ partial)
 {
     pdl_enter();
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t t = off + k;
+    int q = 0;
+    while (q + 1 < L.count && (int)blockIdx.x >= L.it[q + 1].block) ++q;
+    const ObjItem<T> &O = L.it[q];
+    const int kind = L.kind, blk = (int)blockIdx.x - O.block;
+    const T m = O.m, Lx = O.Lx, a0 = O.a0, a1 = O.a1, a2 = O.a2;
+    const int64_t n = O.n, k = (int64_t)blk * blockDim.x + threadIdx.x;
+    const int64_t t = O.off + k;
     double j = 0.0;
     if (k < n) {
         const int32_t id = perm[t];
@@ -1219,24 +1240,26 @@ __global__ void k_objective(int64_t n, int64_t off, int kind, const int32_t *__r
         if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = sm[0];
+    if (threadIdx.x == 0) partial[O.partial + blk] = sm[0];
 }
 
-// single block: fixed-order sum of the block partials
-static __global__ void k_sum_partials(int64_t nb, const double *__restrict__ partial,
-                                      double *__restrict__ out)
+// a block per instance: fixed-order sum of its block sums
+template <typename T>
+__global__ void k_sum_partials(const __grid_constant__ ObjItems<T> L, double *__restrict__ partial)
 {
     pdl_enter();
     __shared__ double sm[kBlock];
+    const ObjItem<T> &O = L.it[blockIdx.x];
+    const int64_t nb = (O.n + kBlock - 1) / kBlock;
     double a = 0.0;
-    for (int64_t i = threadIdx.x; i < nb; i += blockDim.x) a += partial[i];
+    for (int64_t i = threadIdx.x; i < nb; i += blockDim.x) a += partial[O.partial + i];
     sm[threadIdx.x] = a;
     __syncthreads();
     for (int o = kBlock / 2; o > 0; o >>= 1) {
         if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = sm[0];
+    if (threadIdx.x == 0) partial[L.jslots + O.out] = sm[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -1617,22 +1640,42 @@ template <typename T> class Work final : public WorkI {
             partial.alloc((size_t)nbTot + (size_t)B + 1);
         }
         std::vector<double> Jb((size_t)B, 0.0);
+        ObjItems<T> L;
+        L.kind = kind;
+        L.jslots = nbTot;
         int64_t pofs = 0;
-        for (int b = 0; b < B; ++b) {
-            const Inst<T> &I = st->hinst[b];
-            if (!I.n) continue;
-            const Params &q = st->prms[b];
-            const T a0 = args ? (T)args[3 * b] : (T)0, a1 = args ? (T)args[3 * b + 1] : (T)0,
-                    a2 = args ? (T)args[3 * b + 2] : (T)1;
-            SPH_LAUNCH(K_MISC, k_objective<T>, (int64_t)I.n, (int64_t)I.n, (int64_t)I.off, kind,
-                       st->perm.p, st->pos[st->cur].p, st->vel[st->cur].p, (T)q.m, (T)q.Lx, a0, a1,
-                       a2, devSeedX.p, devSeedV.p, partial.p + pofs);
-            const int64_t nb = grid_for(I.n);
+        for (int b = 0; b < B;) {
+            L.count = 0;
+            int64_t blocks = 0;
+            for (; b < B && L.count < kObjGroup; ++b) {
+                const Inst<T> &I = st->hinst[b];
+                if (!I.n) continue;
+                const int64_t nb = grid_for(I.n);
+                if (L.count && blocks + nb > INT32_MAX) break; // the next launch's
+                const Params &q = st->prms[b];
+                ObjItem<T> &O = L.it[L.count++];
+                O.off = I.off;
+                O.n = I.n;
+                O.partial = pofs;
+                O.block = (int32_t)blocks;
+                O.out = b;
+                O.m = (T)q.m;
+                O.Lx = (T)q.Lx;
+                O.a0 = args ? (T)args[3 * b] : (T)0;
+                O.a1 = args ? (T)args[3 * b + 1] : (T)0;
+                O.a2 = args ? (T)args[3 * b + 2] : (T)1;
+                blocks += nb;
+                pofs += nb;
+            }
+            if (!L.count) continue;
             rt_before_launch(K_MISC);
-            launch_k(k_sum_partials, dim3(1), dim3(kBlock), 0, nb, (const double *)(partial.p + pofs),
-                     partial.p + nbTot + b);
+            launch_k(k_objective<T>, dim3((unsigned)blocks), dim3(kBlock), 0, L,
+                     (const int32_t *)st->perm.p, (const T2<T> *)st->pos[st->cur].p,
+                     (const T2<T> *)st->vel[st->cur].p, devSeedX.p, devSeedV.p, partial.p);
             rt_after_launch(K_MISC);
-            pofs += nb;
+            rt_before_launch(K_MISC);
+            launch_k(k_sum_partials<T>, dim3((unsigned)L.count), dim3(kBlock), 0, L, partial.p);
+            rt_after_launch(K_MISC);
         }
         jOff = nbTot;
         haveDevSeeds = true;
