@@ -39,30 +39,31 @@ sys.path.insert(0, ROOT)
 # steps of the short solves that choose the block sizes inside the solve
 TUNE_STEPS = 32
 
-# ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at 1,048,576
-# particles, FP32 (the --set full captures summarised in profiles/*_1M_fp32.md)
+# ncu dram__bytes.sum.per_second times the duration of one launch at 1,048,576
+# particles, FP32 (the captures summarised in profiles/k_*_win_1M_fp32.md)
 TRAFFIC_1M_F32 = {
-    "density": 38.243584e6 + 0.870144e6,
-    "accel_integrate": 55.135488e6 + 2.096640e6,
-    "accel_drag": 71.912192e6 + 3.559680e6,
-    "pass1": 76.111104e6 + 3.872512e6,
-    "pass2": 63.416832e6 + 0.484096e6,
+    "density": 2.220966e12 * 42.528e-6,
+    "accel_integrate": 1.610723e12 * 45.408e-6,
+    "accel_drag": 2.029740e12 * 45.536e-6,
+    "pass1": 1.692239e12 * 58.272e-6,
+    "pass2": 2.444277e12 * 32.864e-6,
 }
 
 # smsp__issue_active.avg.pct_of_peak_sustained_active of the same captures:
-# the fraction of cycles in which a warp scheduler issued, the bound these
-# gather kernels actually meet (HBM throughput stays in single digits)
+# the fraction of cycles in which a warp scheduler issued; with the shared-memory
+# wavefronts (60 to 77% of their rate) the bound these kernels meet (HBM throughput
+# stays at 20 to 31%)
 ISSUE_ACTIVE_1M_F32 = {
-    "density": 0.7623, "accel_integrate": 0.6856, "accel_drag": 0.6692,
-    "pass1": 0.7149, "pass2": 0.7357,
+    "density": 0.6652, "accel_integrate": 0.5616, "accel_drag": 0.5639,
+    "pass1": 0.7156, "pass2": 0.6899,
 }
 
 # lts__throughput.avg.pct_of_peak_sustained_elapsed and
-# l1tex__throughput.avg.pct_of_peak_sustained_active of the same captures:
-# neither cache level is near its peak either
+# l1tex__throughput.avg.pct_of_peak_sustained_active of the same captures (the
+# latter holds the shared memory)
 L2_L1_FRAC_1M_F32 = {
-    "density": (0.0803, 0.3387), "accel_integrate": (0.0900, 0.6129),
-    "accel_drag": (0.0929, 0.5730), "pass1": (0.0983, 0.6216), "pass2": (0.1094, 0.4152),
+    "density": (0.1780, 0.7866), "accel_integrate": (0.1603, 0.8508),
+    "accel_drag": (0.1869, 0.8424), "pass1": (0.1682, 0.8358), "pass2": (0.2057, 0.7245),
 }
 
 # algorithmic HBM bytes per particle per launch (compulsory traffic of the
