@@ -796,10 +796,10 @@ def run_ours(args):
     # (density 4s + accel/integrate 10s), reverse step 48s (tape read 4s,
     # density 4s, accel/drag 15s, pass 1 16s, pass 2 9s), the full tape's
     # write 4s per step, a neighbour rebuild 4s + 12; snapshot copies are not
-    # counted. Rebuilds per solve are the build launches of the breakdown solve
+    # counted. Rebuilds per solve are the rank launches of the breakdown solve
     # when it ran, else one per `interval` executed steps.
     fwd_steps = args.nsteps + rec
-    rebuilds = (kernels["nl_build"]["launches"] if "nl_build" in kernels
+    rebuilds = (kernels["rank"]["launches"] if "rank" in kernels
                 else (fwd_steps + args.nsteps) // max(interval, 1))
     solve_bytes = N * (14 * esz * fwd_steps + 48 * esz * args.nsteps
                        + (4 * esz * args.nsteps if args.snapshots == 0 else 0)

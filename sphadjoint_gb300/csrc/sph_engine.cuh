@@ -817,11 +817,12 @@ template <typename T> class Sys final : public StateI {
     NlOut<T> nl_out() { return NlOut<T>{center.p, masks.p, flags.p, nbcount.p}; }
 
     // The masks of the cell list just built, now, or with `defer` and a small single
-    // state by the density pass that its caller launches next (masksDue).
+    // state, or tiles, by the density pass that its caller launches next (masksDue).
     void build_masks(bool defer)
     {
-        masksDue = defer && B == 1 && N_ > 0 && !tiles() &&
-                   (flat() ? flat_particles(N_) <= kFlatBuild : group_lanes() != 0);
+        masksDue = defer && N_ > 0 &&
+                   (tiles() || (B == 1 && (flat() ? flat_particles(N_) <= kFlatBuild
+                                                  : group_lanes() != 0)));
         if (masksDue) listsFresh = false;
         else build_masks();
     }
@@ -937,7 +938,7 @@ template <typename T> class Sys final : public StateI {
                               rho.p, theta, pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
         } else if (tiles()) {
             if constexpr (sizeof(T) == 4) {
-                density_tiles(v, rho.p, prho.p);
+                density_tiles(v, rho.p, prho.p, due);
                 auto ki = B > 1 ? (anyAV ? &k_accel_win<true, true> : &k_accel_win<true, false>)
                                 : (anyAV ? &k_accel_win<false, true> : &k_accel_win<false, false>);
                 SPH_LAUNCH_TILES(K_ACCEL_INTEGRATE, ki, N_, v, lists(), vel[cur].p, prho.p, rho.p,
@@ -955,9 +956,16 @@ template <typename T> class Sys final : public StateI {
     }
 
     // density_kernel! + eos_kernel! on tiles, and this step's in-support lists
-    void density_tiles(const NLView<T> &v, T *rhoOut, T2<T> *prhoOut)
+    void density_tiles(const NLView<T> &v, T *rhoOut, T2<T> *prhoOut, bool build)
     {
         if constexpr (sizeof(T) == 4) {
+            if (build) {
+                auto kb = B > 1 ? &k_nl_density_win<true> : &k_nl_density_win<false>;
+                SPH_LAUNCH_TILES(K_DENSITY, kb, N_, v, center.p, masks.p, nbcount.p, flags.p,
+                                 lists(), rhoOut, prhoOut);
+                listsFresh = true;
+                return;
+            }
             fresh_lists(v);
             auto kd = B > 1 ? &k_density_win<true> : &k_density_win<false>;
             SPH_LAUNCH_TILES(K_DENSITY, kd, N_, v, lists(), rhoOut, prhoOut);
@@ -1571,7 +1579,7 @@ template <typename T> class Work final : public WorkI {
         const bool av = S.anyAV;
         if (S.tiles()) {
             if constexpr (sizeof(T) == 4) {
-                S.density_tiles(v, rhoOut, S.prho.p);
+                S.density_tiles(v, rhoOut, S.prho.p, due);
                 auto ka = multi ? (av ? &k_drag_win<true, true> : &k_drag_win<true, false>)
                                 : (av ? &k_drag_win<false, true> : &k_drag_win<false, false>);
                 auto k1 = multi ? (av ? &k_pass1_win<true, true> : &k_pass1_win<true, false>)

@@ -249,13 +249,81 @@ __device__ __forceinline__ bool tile_window(TileShared &T, const Inst<float> &on
     return ok;
 }
 
+// density_kernel! + eos_kernel! of one particle and its in-support list, from its n
+// candidates: cand(q) gives the q-th four offsets into the window sw (past the
+// last one, any of them). The list is collected at `place`, which may hold the
+// candidates: an entry is written behind those already read. The arithmetic of
+// density_pairs_f32, two candidates at a time.
+template <bool MULTI, typename Cand>
+__device__ __forceinline__ void density_list(const NLView<float> &v, const WinLists &L, int tile,
+                                             int64_t i, const unsigned char *sw,
+                                             unsigned char *place, int n, Cand &&cand,
+                                             float *__restrict__ rho, float2 *__restrict__ prho)
+{
+    decltype(auto) I = load_inst<MULTI>(v, i);
+    const float r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, A = I.p.A;
+    const float2 xi = v.pos[i];
+    const float2 ih2 = make_float2(invh, invh), mh = make_float2(-0.5f, -0.5f);
+    const float2 one2 = make_float2(1.0f, 1.0f), two2 = make_float2(2.0f, 2.0f);
+    const int64_t lbase = (int64_t)tile * (kQuads * kTile) + (int)threadIdx.x;
+    int ns = 0;
+    float acc = 0.0f;
+    // one quad of candidates, `left` of them in the list
+    auto quad = [&](const uint2 &cur, int left) {
+        float2 xj[4];
+        bool in[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) xj[k] = lds2(sw, entry_of(cur, k));
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            const float2 da = fsub2(xi, xj[h]);
+            const float2 db = fsub2(xi, xj[h + 1]);
+            const float r2a = da.x * da.x + da.y * da.y;
+            const float r2b = db.x * db.x + db.y * db.y;
+            in[h] = h < left && r2a < r2max;
+            in[h + 1] = h + 1 < left && r2b < r2max;
+            const float2 qq = fmul2(make_float2(pair_sqrt(r2a), pair_sqrt(r2b)), ih2);
+            float2 u = ffma2(qq, mh, one2); // 1 - q/2
+            u.x = in[h] ? u.x : 0.0f;
+            u.y = in[h + 1] ? u.y : 0.0f;
+            const float2 u2 = fmul2(u, u);
+            const float2 u4 = fmul2(u2, u2);
+            const float2 w = ffma2(qq, two2, one2); // 2q + 1
+            acc = fmaf(u4.x, w.x, acc);
+            acc = fmaf(u4.y, w.y, acc);
+        }
+        // every entry is written, and kept by moving on (ns <= 48: the write
+        // after the last kept entry stays inside this thread's place)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            *reinterpret_cast<uint16_t *>(place + ns) = (uint16_t)entry_of(cur, k);
+            if (in[k]) ns += kRow;
+        }
+    };
+    uint2 e = n ? cand(0) : make_uint2(0u, 0u);
+    int q = 0;
+    for (; q < (n >> 2); ++q) {
+        const uint2 cur = e;
+        if (4 * q + 4 < n) e = cand(q + 1);
+        quad(cur, 4);
+    }
+    if (n & 3) quad(e, n & 3);
+    ns /= kRow;
+    write_list(place, ns, L.supp + lbase);
+    L.suppCnt[i] = (uint8_t)ns;
+    acc = mul_rn(mul_rn(m, A), acc);
+    density_finish<float>(I, i, acc, rho, prho);
+}
+
 // _nl_build! (nl_build_one), the tile's window and the candidate lists of a fresh
 // cell list: the rows are scanned in the staged window, and every passing slot
 // goes both to its row mask and to the list. One pass instead of a mask build
 // (52 us at 1M particles) and a walk of the masks (43 us): 66.5 us, bound by issue
 // slots and shared-memory wavefronts (some 80% of either's rate); 8.4M dense
 // particles 775 -> 647 us.
-template <bool MULTI>
+// DENS: the density pass of the same particles follows in the staged window, from
+// the lists in shared memory (k_nl_density_win).
+template <bool MULTI, bool DENS = false>
 __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
                                           const Inst<float> *inst,
                                           const uint16_t *__restrict__ pinst,
@@ -264,11 +332,19 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
                                           uint32_t *__restrict__ center,
                                           uint32_t *__restrict__ masks,
                                           int32_t *__restrict__ nbcount,
-                                          uint32_t *__restrict__ flags, const WinLists &L, int tile)
+                                          uint32_t *__restrict__ flags, const WinLists &L, int tile,
+                                          const NLView<float> *v = nullptr, float *rho = nullptr,
+                                          float2 *prho = nullptr)
 {
     __shared__ TileShared T;
     __shared__ __align__(16) unsigned char s_win[kWin8];
     __shared__ __align__(8) unsigned char s_list[kTile * kNlStride];
+    auto walk = [&](int64_t i) { // the density of a particle without a list
+        if constexpr (DENS) {
+            L.suppCnt[i] = kNoList;
+            density_walk<float, MULTI, true>(*v, i, rho, prho, nullptr);
+        }
+    };
     const int t = (int)threadIdx.x;
     const int64_t i = (int64_t)tile * kTile + t;
     const bool live = i < N;
@@ -285,6 +361,7 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
         if (live) {
             nl_build_one<float>(N, I, b, i, pos, cellStart, center, masks, nbcount, flags);
             L.candCnt[i] = kNoList;
+            walk(i);
         }
         return;
     }
@@ -376,10 +453,19 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
     nbcount[i] = n;
     if (spill || n > 4 * kQuads) {
         L.candCnt[i] = kNoList;
+        walk(i);
         return;
     }
     write_list(place, n, L.cand + (int64_t)tile * (kQuads * kTile) + t);
     L.candCnt[i] = (uint8_t)n;
+    if constexpr (DENS) {
+        const uint16_t *p = reinterpret_cast<const uint16_t *>(place);
+        auto four = [&](int q) {
+            auto at = [&](int k) { return (uint32_t)p[(4 * q + k < n ? 4 * q + k : n - 1) * kTile]; };
+            return make_uint2(at(0) | at(1) << 16, at(2) | at(3) << 16);
+        };
+        density_list<MULTI>(*v, L, tile, i, s_win, place, n, four, rho, prho);
+    }
 }
 
 template <bool MULTI>
@@ -393,6 +479,22 @@ __global__ void __launch_bounds__(kTile)
     pdl_enter();
     nl_window<MULTI>(N, one, inst, pinst, pos, cellStart, center, masks, nbcount, flags, L,
                      (int)blockIdx.x);
+}
+
+// The same and the density pass of the step in one launch, which saves the launch, the
+// second staging of the window and the read of the lists: 20,000 particles' 16 steps
+// 271 -> 262 us, 249,001 particles 41.3 -> 34.0 us a rebuild, 1M 116 -> 108, 8.4M 1030
+// -> 995.
+template <bool MULTI>
+__global__ void __launch_bounds__(kTile)
+    k_nl_density_win(const __grid_constant__ NLView<float> v, uint32_t *__restrict__ center,
+                     uint32_t *__restrict__ masks, int32_t *__restrict__ nbcount,
+                     uint32_t *__restrict__ flags, const WinLists L, float *__restrict__ rho,
+                     float2 *__restrict__ prho)
+{
+    pdl_enter();
+    nl_window<MULTI, true>(v.N, v.one, v.inst, v.pinst, v.pos, v.cellStart, center, masks, nbcount,
+                           flags, L, (int)blockIdx.x, &v, rho, prho);
 }
 
 // Windows and candidate lists from the row masks, after a snapshot was restored (a
@@ -465,8 +567,7 @@ __global__ void __launch_bounds__(kTile)
     window_lists<MULTI>(v, L, (int)blockIdx.x);
 }
 
-// density_kernel! + eos_kernel! and this step's in-support lists: the arithmetic of
-// density_pairs_f32, two candidates at a time.
+// density_kernel! + eos_kernel! and this step's in-support lists.
 template <bool MULTI>
 __device__ __forceinline__ void density_window(const NLView<float> &v, const WinLists &L, int tile,
                                                float *__restrict__ rho,
@@ -486,61 +587,9 @@ __device__ __forceinline__ void density_window(const NLView<float> &v, const Win
         density_walk<float, MULTI, true>(v, i, rho, prho, nullptr);
         return;
     }
-    decltype(auto) I = load_inst<MULTI>(v, i);
-    const float r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, A = I.p.A;
-    const float2 xi = v.pos[i];
-    const float2 ih2 = make_float2(invh, invh), mh = make_float2(-0.5f, -0.5f);
-    const float2 one2 = make_float2(1.0f, 1.0f), two2 = make_float2(2.0f, 2.0f);
-    const int64_t lbase = (int64_t)tile * (kQuads * kTile) + t;
-    const uint2 *cand = L.cand + lbase;
-    unsigned char *const place = s_list + 2 * t;
-    int ns = 0;
-    float acc = 0.0f;
-    // one quad of candidates, `left` of them in the list
-    auto quad = [&](const uint2 &cur, int left) {
-        float2 xj[4];
-        bool in[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) xj[k] = lds2(sw, entry_of(cur, k));
-#pragma unroll
-        for (int h = 0; h < 4; h += 2) {
-            const float2 da = fsub2(xi, xj[h]);
-            const float2 db = fsub2(xi, xj[h + 1]);
-            const float r2a = da.x * da.x + da.y * da.y;
-            const float r2b = db.x * db.x + db.y * db.y;
-            in[h] = h < left && r2a < r2max;
-            in[h + 1] = h + 1 < left && r2b < r2max;
-            const float2 qq = fmul2(make_float2(pair_sqrt(r2a), pair_sqrt(r2b)), ih2);
-            float2 u = ffma2(qq, mh, one2); // 1 - q/2
-            u.x = in[h] ? u.x : 0.0f;
-            u.y = in[h + 1] ? u.y : 0.0f;
-            const float2 u2 = fmul2(u, u);
-            const float2 u4 = fmul2(u2, u2);
-            const float2 w = ffma2(qq, two2, one2); // 2q + 1
-            acc = fmaf(u4.x, w.x, acc);
-            acc = fmaf(u4.y, w.y, acc);
-        }
-        // every entry is written, and kept by moving on (ns <= 48: the write
-        // after the last kept entry stays inside this thread's place)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            *reinterpret_cast<uint16_t *>(place + ns) = (uint16_t)entry_of(cur, k);
-            if (in[k]) ns += kRow;
-        }
-    };
-    uint2 e = n ? cand[0] : make_uint2(0u, 0u);
-    int q = 0;
-    for (; q < (n >> 2); ++q) {
-        const uint2 cur = e;
-        if (4 * q + 4 < n) e = cand[(q + 1) * kTile];
-        quad(cur, 4);
-    }
-    if (n & 3) quad(e, n & 3);
-    ns /= kRow;
-    write_list(place, ns, L.supp + lbase);
-    L.suppCnt[i] = (uint8_t)ns;
-    acc = mul_rn(mul_rn(m, A), acc);
-    density_finish<float>(I, i, acc, rho, prho);
+    const uint2 *c = L.cand + (int64_t)tile * (kQuads * kTile) + t;
+    density_list<MULTI>(v, L, tile, i, sw, s_list + 2 * t, n, [&](int q) { return c[q * kTile]; },
+                        rho, prho);
 }
 
 template <bool MULTI>
