@@ -547,11 +547,11 @@ template <typename T> class Sys final : public StateI {
     }
 
     // FP32 states with one thread per particle run their pair passes on tiles
-    // (sph_window.cuh) when their lists are in memory. The lists (about 260
+    // (sph_window.cuh) when their lists are in memory. The lists (about 200
     // bytes a particle) are scratch that the mask walks do without, so they
     // are taken only from memory that is plainly free (an eighth of it at most)
     // and not while a graph is recorded; a state without them gives the same
-    // results. Beyond 2^25 particles they would hold 8.6 GB a state.
+    // results. Beyond 2^25 particles they would hold 6.6 GB a state.
     static constexpr int64_t kListMaxN = int64_t(1) << 25;
     bool want_tiles() const
     {

@@ -31,10 +31,9 @@
 // Bound: shared-memory wavefronts and issue slots together (accel at 1M: 71% of
 // the wavefront rate, 57% of the issue slots, 913 warp instructions a warp where
 // the mask walk ran 1449). Measured per launch at 1,048,576 particles, mask walk
-// -> lists: density 58.1 -> 45.0 us, accel 59.2 -> 46.5, accel + drag 70.8 -> 48.9,
-// pass 1 82.7 -> 60.6, pass 2 64.1 -> 48.2; the lists cost 43 us a rebuild.
-// Solves: 249k particles 2.70 -> 2.17 ms, 8.4M dense (a rebuild a step) 23.5 ->
-// 20.2 ms, 131k with the Tait/artificial-viscosity model 1.83 -> 1.37 ms.
+// -> lists: density 58.1 -> 45.2 us, accel 59.2 -> 46.6, accel + drag 70.8 -> 49.0,
+// pass 1 82.7 -> 60.5, pass 2 64.1 -> 46.8; a rebuild's masks and lists 52 -> 71 us
+// (k_nl_window), 108 with the step's density (k_nl_density_win).
 // Reading the lists two quads ahead (accel 46 -> 49 us), copying a tile's lists
 // to shared memory first (density 45 -> 51) and 16-byte interleaved windows
 // (below) were slower.
