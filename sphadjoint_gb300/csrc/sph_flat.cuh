@@ -426,10 +426,11 @@ template <bool MULTI> struct FlatPass {
 };
 
 // A barrier of the four pair warps alone: the fifth is not waited for until the
-// results are put together.
+// results are put together. Not the aligned form (bar.sync): the lanes of a warp come
+// from pair terms that only some of them had.
 __device__ __forceinline__ void pair_sync()
 {
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    asm volatile("barrier.sync 1, 128;" ::: "memory");
 }
 
 // Pressure + Morris viscosity of the block's particles (accel_pair): s_acc[2 a],

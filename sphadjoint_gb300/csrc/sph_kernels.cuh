@@ -474,8 +474,9 @@ __global__ void __launch_bounds__(kRebuildSmallThreads)
             place[u] = atomicAdd(&count[cell[u]], 1);
         }
     __syncthreads();
-    // this block's reads of perm and xref are done
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    // this block's reads of perm and xref are done (the forms without .aligned: a warp's
+    // lanes come to the wait from loops of different lengths)
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     // exclusive scan of the counts: each thread sums a contiguous chunk
     const int chunk = (ncell + nt - 1) / nt;
     const int c0 = t * chunk, c1 = c0 + chunk < ncell ? c0 + chunk : ncell;
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(kRebuildSmallThreads)
         for (int k = s0; k < s1; ++k) rank += bucket[k] < ido ? 1 : 0;
         dst = s0 + rank;
     }
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     if (!mine) return;
     perm[dst] = ido;
     posN[dst] = xo;
