@@ -213,10 +213,6 @@ __device__ __forceinline__ int spill_list(const Group<G> &g, const NLView<T> &v,
 // rows' bounds, then their first rounds' positions, are loaded together. Writes
 // the particle's masks, count and cell and leaves them in wd, n and the return
 // value, with the rows' first slots in bs.
-template <typename T> struct NlOut {
-    uint32_t *center, *masks, *flags;
-    int32_t *nbcount;
-};
 template <typename T, int G>
 __device__ __forceinline__ uint32_t nl_group(const Group<G> &g, int64_t N, const Inst<T> &I,
                                              int64_t i, const T2<T> *__restrict__ pos,

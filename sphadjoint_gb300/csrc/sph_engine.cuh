@@ -846,7 +846,7 @@ template <typename T> class Sys final : public StateI {
             if constexpr (sizeof(T) == 4) {
                 auto kn = B > 1 ? &k_nl_window<true> : &k_nl_window<false>;
                 SPH_LAUNCH_TILES(K_NLBUILD, kn, N_, N_, hinst[0], dinst.p, pinst.p, pos[cur].p,
-                                 cellStart.p, center.p, masks.p, nbcount.p, flags.p, lists());
+                                 cellStart.p, nl_out(), lists());
                 listsFresh = true;
             }
         } else if (const int G = group_lanes()) {
@@ -961,8 +961,7 @@ template <typename T> class Sys final : public StateI {
         if constexpr (sizeof(T) == 4) {
             if (build) {
                 auto kb = B > 1 ? &k_nl_density_win<true> : &k_nl_density_win<false>;
-                SPH_LAUNCH_TILES(K_DENSITY, kb, N_, v, center.p, masks.p, nbcount.p, flags.p,
-                                 lists(), rhoOut, prhoOut);
+                SPH_LAUNCH_TILES(K_DENSITY, kb, N_, v, nl_out(), lists(), rhoOut, prhoOut);
                 listsFresh = true;
                 return;
             }

@@ -638,6 +638,14 @@ template <> struct NlTest<double> {
     }
 };
 
+// What a neighbour build writes. Plain pointers: where the density pass of the same
+// launch follows, a particle without a list reads the masks and centre just written back
+// through its view (NLView), which a restrict pointer would let the compiler move up.
+template <typename T> struct NlOut {
+    uint32_t *center, *masks, *flags;
+    int32_t *nbcount;
+};
+
 // One particle's neighbour rows (the body of k_nl_build); bi selects its
 // instance's flag word.
 template <typename T, typename IT>

@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(kPackBlock) g_nl_build(int l)
     const GSys<T> &d = pack_sys<T>(f.x);
     if constexpr (sizeof(T) == 4) {
         if (d.W.win) {
-            nl_window<false>(d.n, d.v.one, nullptr, nullptr, d.v.pos, d.cellStart, d.center,
-                             d.masks, d.nbcount, d.flags, d.W, f.y);
+            nl_window<false>(d.n, d.v.one, nullptr, nullptr, d.v.pos, d.cellStart,
+                             NlOut<float>{d.center, d.masks, d.flags, d.nbcount}, d.W, f.y);
             return;
         }
     }

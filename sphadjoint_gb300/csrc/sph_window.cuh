@@ -328,10 +328,7 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
                                           const uint16_t *__restrict__ pinst,
                                           const float2 *__restrict__ pos,
                                           const int32_t *__restrict__ cellStart,
-                                          uint32_t *__restrict__ center,
-                                          uint32_t *__restrict__ masks,
-                                          int32_t *__restrict__ nbcount,
-                                          uint32_t *__restrict__ flags, const WinLists &L, int tile,
+                                          const NlOut<float> &out, const WinLists &L, int tile,
                                           const NLView<float> *v = nullptr, float *rho = nullptr,
                                           float2 *prho = nullptr)
 {
@@ -358,7 +355,8 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
                                        nrun);
     if (!ok) {
         if (live) {
-            nl_build_one<float>(N, I, b, i, pos, cellStart, center, masks, nbcount, flags);
+            nl_build_one<float>(N, I, b, i, pos, cellStart, out.center, out.masks, out.nbcount,
+                                out.flags);
             L.candCnt[i] = kNoList;
             walk(i);
         }
@@ -443,13 +441,13 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
             }
             room -= cnt[r];
         }
-        atomicOr(flags + b, FLAG_NL_OVERFLOW);
+        atomicOr(out.flags + b, FLAG_NL_OVERFLOW);
     }
 #pragma unroll
-    for (int q = 0; q < 6; ++q) masks[(int64_t)q * N + i] = word[q];
+    for (int q = 0; q < 6; ++q) out.masks[(int64_t)q * N + i] = word[q];
     const int n = all < maxnb ? all : maxnb;
-    center[i] = (uint32_t)cx | ((uint32_t)cy << 16) | (spill << 31);
-    nbcount[i] = n;
+    out.center[i] = (uint32_t)cx | ((uint32_t)cy << 16) | (spill << 31);
+    out.nbcount[i] = n;
     if (spill || n > 4 * kQuads) {
         L.candCnt[i] = kNoList;
         walk(i);
@@ -471,13 +469,10 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kTile)
     k_nl_window(int64_t N, const Inst<float> one, const Inst<float> *__restrict__ inst,
                 const uint16_t *__restrict__ pinst, const float2 *__restrict__ pos,
-                const int32_t *__restrict__ cellStart, uint32_t *__restrict__ center,
-                uint32_t *__restrict__ masks, int32_t *__restrict__ nbcount,
-                uint32_t *__restrict__ flags, const WinLists L)
+                const int32_t *__restrict__ cellStart, const NlOut<float> out, const WinLists L)
 {
     pdl_enter();
-    nl_window<MULTI>(N, one, inst, pinst, pos, cellStart, center, masks, nbcount, flags, L,
-                     (int)blockIdx.x);
+    nl_window<MULTI>(N, one, inst, pinst, pos, cellStart, out, L, (int)blockIdx.x);
 }
 
 // The same and the density pass of the step in one launch, which saves the launch, the
@@ -486,14 +481,12 @@ __global__ void __launch_bounds__(kTile)
 // -> 995.
 template <bool MULTI>
 __global__ void __launch_bounds__(kTile)
-    k_nl_density_win(const __grid_constant__ NLView<float> v, uint32_t *__restrict__ center,
-                     uint32_t *__restrict__ masks, int32_t *__restrict__ nbcount,
-                     uint32_t *__restrict__ flags, const WinLists L, float *__restrict__ rho,
-                     float2 *__restrict__ prho)
+    k_nl_density_win(const __grid_constant__ NLView<float> v, const NlOut<float> out,
+                     const WinLists L, float *__restrict__ rho, float2 *__restrict__ prho)
 {
     pdl_enter();
-    nl_window<MULTI, true>(v.N, v.one, v.inst, v.pinst, v.pos, v.cellStart, center, masks, nbcount,
-                           flags, L, (int)blockIdx.x, &v, rho, prho);
+    nl_window<MULTI, true>(v.N, v.one, v.inst, v.pinst, v.pos, v.cellStart, out, L,
+                           (int)blockIdx.x, &v, rho, prho);
 }
 
 // Windows and candidate lists from the row masks, after a snapshot was restored (a
