@@ -365,7 +365,6 @@ template <typename T> class Sys final : public StateI {
     DevBuf<int32_t> foff;
     bool listsTried = false; // the lists were asked for (and may have been refused)
     bool listsFresh = false; // they belong to the masks the state holds
-    bool masksDue = false;   // the next density pass builds the masks (set and taken within a step)
     StepGraphs graphs;   // simulate's steps, replayed in groups
     bool anyRho = false; // some instance's model reads densities in the adjoint
     bool anyAV = false;  // some instance uses the artificial viscosity
@@ -536,11 +535,10 @@ template <typename T> class Sys final : public StateI {
     int64_t N() const override { return N_; }
     int batch() const override { return B; }
 
-    // lanes per particle of this state's pair-sum kernels (0: one thread)
-    int group_lanes() const
+    // lanes per particle of this state's pair-sum kernels (0: one thread) at lane setting f
+    int group_lanes(int f) const
     {
         if (B != 1) return 0;
-        const int f = rt_group_lanes();
         if (f == 16 || f == 32) return f;
         if (f == 1 || N_ > kCoopMaxN) return 0;
         return N_ <= coop32_max_n<T>() ? 32 : 16;
@@ -555,10 +553,9 @@ template <typename T> class Sys final : public StateI {
     static constexpr int64_t kListMaxN = int64_t(1) << 25;
     bool want_tiles() const
     {
-        return sizeof(T) == 4 && N_ > 0 && N_ <= kListMaxN && group_lanes() == 0 &&
+        return sizeof(T) == 4 && N_ > 0 && N_ <= kListMaxN && group_lanes(rt_group_lanes()) == 0 &&
                rt_density_form() == 2;
     }
-    bool tiles() const { return want_tiles() && wwin.p; }
     // FP64 states without artificial viscosity run them one lane per pair
     // (sph_flat.cuh), unless a lane setting is forced; their pair lists (about
     // 1290 bytes a particle) are scratch under the same rule.
@@ -567,7 +564,26 @@ template <typename T> class Sys final : public StateI {
     {
         return sizeof(T) == 8 && N_ > 0 && N_ <= kFlatMaxN && rt_group_lanes() == 0;
     }
-    bool flat() const { return want_flat() && !anyAV && foff.p; }
+    // The kernels of one step or one build, chosen once at its start. The lane and
+    // density settings are process-wide and another thread may move them at any time;
+    // a step's launches have to agree on who builds the masks and who loads the next
+    // tape state, so nothing below reads the settings again.
+    struct Form {
+        bool pairs;  // one lane per pair (FP64)
+        int lanes;   // else a lane group per particle (0: none)
+        bool tiles;  // else tiles (FP32)
+        int density; // else mask walks, with this density form
+    };
+    Form form() const
+    {
+        const int set = rt_group_lanes(), density = sizeof(T) == 4 ? rt_density_form() : 0;
+        Form f;
+        f.pairs = set == 0 && !anyAV && foff.p;
+        f.lanes = group_lanes(set);
+        f.tiles = f.lanes == 0 && density == 2 && wwin.p;
+        f.density = density;
+        return f;
+    }
     FlatLists flat_lists() const { return FlatLists{fF.p, fr.p, ftm.p, fpair.p, foff.p, flat_particles(N_)}; }
     void reserve_lists()
     {
@@ -778,9 +794,12 @@ template <typename T> class Sys final : public StateI {
     // build_neighbors! (src/neighbors.jl:252-263): cell list, permutation of
     // the particle data (and of up to two extra per-particle arrays) into the
     // new cell order, neighbour masks. ex*N receive the permuted extras.
-    void rebuild(const T2<T> *ex0 = nullptr, T2<T> *ex0N = nullptr, const T2<T> *ex1 = nullptr,
-                 T2<T> *ex1N = nullptr, bool defer = false)
+    // Returns whether the density pass that the caller launches next has to build the
+    // masks (only with `defer`, see build_masks).
+    bool rebuild(const Form &f, const T2<T> *ex0 = nullptr, T2<T> *ex0N = nullptr,
+                 const T2<T> *ex1 = nullptr, T2<T> *ex1N = nullptr, bool defer = false)
     {
+        bool due = false;
         const int check = age != INT64_MAX ? 1 : 0;
         if (N_ > 0 && B == 1 && N_ <= kRebuildSmallMaxN && ncell <= kRebuildSmallMaxCells) {
             // small single state: the cell list in one launch (the
@@ -799,7 +818,7 @@ template <typename T> class Sys final : public StateI {
                      invperm.p, cellStart.p, ex0, ex0N, ex1, ex1N, flags.p);
             rt_after_launch(K_RANK);
             cur = nxt;
-            build_masks(defer);
+            due = build_masks(f, defer);
         } else if (N_ > 0) {
             // nbcount is rewritten by the mask build: until then it holds the places
             bucket_cells(check, nbcount.p, cellStart.p);
@@ -808,48 +827,43 @@ template <typename T> class Sys final : public StateI {
                        bucketId.p, pos[cur].p, vel[cur].p, pos[nxt].p, vel[nxt].p, xref.p, perm.p,
                        invperm.p, ex0, ex0N, ex1, ex1N);
             cur = nxt;
-            build_masks(defer);
+            due = build_masks(f, defer);
         }
         age = 0;
         cellsOnlyLatest = false;
+        return due;
     }
 
     NlOut<T> nl_out() { return NlOut<T>{center.p, masks.p, flags.p, nbcount.p}; }
 
     // The masks of the cell list just built, now, or with `defer` and a small single
-    // state, or tiles, by the density pass that its caller launches next (masksDue).
-    void build_masks(bool defer)
+    // state, or tiles, by the density pass that its caller launches next (returns true).
+    bool build_masks(const Form &f, bool defer)
     {
-        masksDue = defer && N_ > 0 &&
-                   (tiles() || (B == 1 && (flat() ? flat_particles(N_) <= kFlatBuild
-                                                  : group_lanes() != 0)));
-        if (masksDue) listsFresh = false;
-        else build_masks();
+        listsFresh = false;
+        if (defer && (f.pairs   ? B == 1 && flat_particles(N_) <= kFlatBuild
+                      : f.lanes ? true
+                                : f.tiles))
+            return true;
+        build_masks(f);
+        return false;
     }
     static auto density_coop(int G, bool build)
     {
         return G == 32 ? (build ? &k_density_eos_coop<T, 32, true> : &k_density_eos_coop<T, 32, false>)
                        : (build ? &k_density_eos_coop<T, 16, true> : &k_density_eos_coop<T, 16, false>);
     }
-    bool take_masks_due()
-    {
-        const bool due = masksDue;
-        masksDue = false;
-        return due;
-    }
-
     // _nl_build! on the freshly sorted particles
-    void build_masks()
+    void build_masks(const Form &f)
     {
-        listsFresh = false;
-        if (tiles()) {
+        if (f.tiles) {
             if constexpr (sizeof(T) == 4) {
                 auto kn = B > 1 ? &k_nl_window<true> : &k_nl_window<false>;
                 SPH_LAUNCH_TILES(K_NLBUILD, kn, N_, N_, hinst[0], dinst.p, pinst.p, pos[cur].p,
                                  cellStart.p, nl_out(), lists());
                 listsFresh = true;
             }
-        } else if (const int G = group_lanes()) {
+        } else if (const int G = f.lanes) {
             auto kn = G == 32 ? &k_nl_build_coop<T, 32> : &k_nl_build_coop<T, 16>;
             SPH_LAUNCH_COOP(K_NLBUILD, G, kn, N_, N_, hinst[0], pos[cur].p, cellStart.p, nl_out());
         } else {
@@ -861,7 +875,7 @@ template <typename T> class Sys final : public StateI {
 
     void build_neighbors() override
     {
-        rebuild();
+        rebuild(form());
         rt_check_launch("build_neighbors");
     }
 
@@ -886,17 +900,16 @@ template <typename T> class Sys final : public StateI {
         rt_check_launch("build_cells");
     }
 
-    void maybe_rebuild(const T2<T> *ex0 = nullptr, T2<T> *ex0N = nullptr,
+    // maybe_rebuild! (src/neighbors.jl:273-279): test, then count. Returns whether the
+    // step's density pass has to build the masks.
+    bool maybe_rebuild(const Form &f, const T2<T> *ex0 = nullptr, T2<T> *ex0N = nullptr,
                        const T2<T> *ex1 = nullptr, T2<T> *ex1N = nullptr, bool *did = nullptr)
     {
-        // maybe_rebuild! (src/neighbors.jl:273-279): test, then count
-        bool r = false;
-        if (age >= opts.interval) {
-            rebuild(ex0, ex0N, ex1, ex1N, true);
-            r = true;
-        }
+        const bool r = age >= opts.interval;
+        const bool due = r && rebuild(f, ex0, ex0N, ex1, ex1N, true);
         age += 1;
         if (did) *did = r;
+        return due;
     }
 
     static ThetaFlush<T> no_flush()
@@ -909,16 +922,16 @@ template <typename T> class Sys final : public StateI {
     // step! (src/forward.jl:161-173); tx/tv: optional tape slot (id order)
     void step_impl(const T *theta, T2<T> *tx, T2<T> *tv)
     {
-        maybe_rebuild();
+        const Form f = form();
+        const bool due = maybe_rebuild(f);
         if (N_ == 0) return;
-        const bool due = take_masks_due();
         // the tape slot (tx, tv) is written by the accel pass from the same
         // pre-step state it reads
         NLView<T> v = view();
         const int nxt = 1 - cur;
         T2<T> *aO = keepAccel ? accOut.p : (T2<T> *)nullptr;
         T *alO = keepAccel ? alphaOut.p : (T *)nullptr;
-        if (flat()) {
+        if (f.pairs) {
             if constexpr (sizeof(T) == 8) {
                 const FlatLists W = flat_lists();
                 auto kd = B > 1 ? &k_density_flat<true, false>
@@ -929,14 +942,14 @@ template <typename T> class Sys final : public StateI {
                 SPH_LAUNCH_FLAT(K_ACCEL_INTEGRATE, W.P, ki, N_, v, W, vel[cur].p, prho.p, theta,
                                 pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
             }
-        } else if (const int G = group_lanes()) {
+        } else if (const int G = f.lanes) {
             auto kd = density_coop(G, due);
             SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush(), nl_out());
             v.tmask = tmask.p;
             auto ki = G == 32 ? &k_accel_integrate_coop<T, 32> : &k_accel_integrate_coop<T, 16>;
             SPH_LAUNCH_COOP_X(K_ACCEL_INTEGRATE, G, 0, kCoopThreads, ki, N_, v, vel[cur].p, prho.p,
                               rho.p, theta, pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
-        } else if (tiles()) {
+        } else if (f.tiles) {
             if constexpr (sizeof(T) == 4) {
                 density_tiles(v, rho.p, prho.p, due);
                 auto ki = B > 1 ? (anyAV ? &k_accel_win<true, true> : &k_accel_win<true, false>)
@@ -945,7 +958,7 @@ template <typename T> class Sys final : public StateI {
                                  theta, pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
             }
         } else {
-            launch_density(v, rho.p, prho.p);
+            launch_density(v, rho.p, prho.p, f.density);
             v.tmask = tmask.p;
             auto ki = B > 1 ? (anyAV ? &k_accel_integrate<T, true, true> : &k_accel_integrate<T, true>)
                             : (anyAV ? &k_accel_integrate<T, false, true> : &k_accel_integrate<T, false>);
@@ -973,9 +986,8 @@ template <typename T> class Sys final : public StateI {
 
     // density_kernel! + eos_kernel! with one thread per particle: the mask
     // walk, or for FP32 states the forms sph_set_density_form selects
-    void launch_density(const NLView<T> &v, T *rhoOut, T2<T> *prhoOut)
+    void launch_density(const NLView<T> &v, T *rhoOut, T2<T> *prhoOut, int form)
     {
-        const int form = sizeof(T) == 4 ? rt_density_form() : 0;
         if (form == 2) {
             auto kd = B > 1 ? &k_density_eos<T, true, true> : &k_density_eos<T, false, true>;
             SPH_LAUNCH_TUNED(K_DENSITY, B > 1, kd, N_, v, rhoOut, prhoOut, tmask.p);
@@ -1493,8 +1505,9 @@ template <typename T> class Work final : public WorkI {
                       const int32_t *srcInv, int parity, const T2<T> *nsx = nullptr,
                       const T2<T> *nsv = nullptr)
     {
-        // the forms below that launch per particle of a small or an FP64 state
-        const bool carries = N_ > 0 && (S.flat() || S.group_lanes());
+        const typename Sys<T>::Form f = S.form();
+        // the forms that load the next tape state and write theta back on the way
+        const bool carries = N_ > 0 && (f.pairs || f.lanes);
         if (nextLoaded) {
             S.cur = 1 - S.cur;
             if (!carries) flush_theta(S);
@@ -1515,9 +1528,8 @@ template <typename T> class Work final : public WorkI {
         }
         bool did = false;
         const int g2 = 1 - gcur;
-        S.maybe_rebuild(gX[gcur].p, gX[g2].p, gV[gcur].p, gV[g2].p, &did);
+        const bool due = S.maybe_rebuild(f, gX[gcur].p, gX[g2].p, gV[gcur].p, gV[g2].p, &did);
         if (did) gcur = g2;
-        const bool due = S.take_masks_due();
         NLView<T> v = S.view();
         const T2<T> *vel = S.vel[S.cur].p;
         T *rhoOut = S.anyRho ? S.rho.p : (T *)nullptr; // densities only where the model reads them
@@ -1532,7 +1544,7 @@ template <typename T> class Work final : public WorkI {
             next.vel = S.vel[nb].p;
         }
         unsigned extra = 0;
-        if (S.flat()) {
+        if (f.pairs) {
             if constexpr (sizeof(T) == 8) {
                 const FlatLists W = S.flat_lists();
                 const bool multi = S.B > 1;
@@ -1554,7 +1566,7 @@ template <typename T> class Work final : public WorkI {
             pendingTheta = parity;
             return;
         }
-        if (const int G = S.group_lanes()) {
+        if (const int G = f.lanes) {
             const bool g32 = G == 32;
             auto kd = S.density_coop(G, due);
             auto ka = g32 ? &k_accel_drag_adj_coop<T, 32> : &k_accel_drag_adj_coop<T, 16>;
@@ -1576,7 +1588,7 @@ template <typename T> class Work final : public WorkI {
         }
         const bool multi = S.B > 1;
         const bool av = S.anyAV;
-        if (S.tiles()) {
+        if (f.tiles) {
             if constexpr (sizeof(T) == 4) {
                 S.density_tiles(v, rhoOut, S.prho.p, due);
                 auto ka = multi ? (av ? &k_drag_win<true, true> : &k_drag_win<true, false>)
@@ -1600,7 +1612,7 @@ template <typename T> class Work final : public WorkI {
         auto k1 = multi ? (av ? &k_pass1_design<T, true, true> : &k_pass1_design<T, true>)
                         : (av ? &k_pass1_design<T, false, true> : &k_pass1_design<T, false>);
         auto k2 = multi ? &k_pass2_axpy<T, true> : &k_pass2_axpy<T, false>;
-        S.launch_density(v, rhoOut, S.prho.p);
+        S.launch_density(v, rhoOut, S.prho.p, f.density);
         v.tmask = S.tmask.p;
         SPH_LAUNCH_TUNED(K_ACCEL_DRAG, multi, ka, N_, v, vel, S.prho.p, S.rho.p, theta, gX[gcur].p,
                          gV[gcur].p, abar.p, galpha.p, emax.p, parity);
@@ -1738,7 +1750,7 @@ template <typename T> class Tuner {
     static void run(Sys<T> &S, Field<T> &th, int reps, int *chosen)
     {
         if (S.N_ == 0) return;
-        if (S.age == INT64_MAX) S.rebuild();
+        if (S.age == INT64_MAX) S.rebuild(S.form());
         const bool multi = S.B > 1;
         const int cand[3] = {64, 128, 256};
         cudaEvent_t e0, e1;
