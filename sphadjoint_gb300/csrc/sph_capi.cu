@@ -147,6 +147,18 @@ void rt_check_launch(const char *name) { cuda_check(cudaGetLastError(), name); }
 
 bool rt_capturing() { return g_capturing || g_recording; }
 
+uint64_t rt_recording()
+{
+    if (g_recording) return 0;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(rt_stream(), &cs, &id) != cudaSuccess) {
+        (void)cudaGetLastError(); // the legacy default stream beside a recording
+        return UINT64_MAX;
+    }
+    return cs == cudaStreamCaptureStatusNone ? 0 : (uint64_t)id;
+}
+
 bool rt_timers_on()
 {
     for (const KTimer &t : g_timer)

@@ -548,7 +548,8 @@ template <typename T> class Sys final : public StateI {
     // (sph_window.cuh) when their lists are in memory. The lists (about 200
     // bytes a particle) are scratch that the mask walks do without, so they
     // are taken only from memory that is plainly free (an eighth of it at most)
-    // and not while a graph is recorded; a state without them gives the same
+    // and not while the stream is recorded, by anyone (the buffers would belong to
+    // that graph); a state without them gives the same
     // results. Beyond 2^25 particles they would hold 6.6 GB a state.
     static constexpr int64_t kListMaxN = int64_t(1) << 25;
     bool want_tiles() const
@@ -588,7 +589,7 @@ template <typename T> class Sys final : public StateI {
     void reserve_lists()
     {
         if (want_tiles()) alloc_lists();
-        if (want_flat() && !listsTried && !rt_capturing()) {
+        if (want_flat() && !listsTried && !rt_recording()) {
             listsTried = true;
             const size_t P = (size_t)flat_particles(N_), nb = ((size_t)N_ + P - 1) / P;
             carve_scratch([&](auto &&part) {
@@ -622,7 +623,7 @@ template <typename T> class Sys final : public StateI {
     }
     void alloc_lists()
     {
-        if (listsTried || rt_capturing() || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN) return;
+        if (listsTried || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN || rt_recording()) return;
         listsTried = true;
         const size_t nt = (size_t)((N_ + kTile - 1) / kTile), e = nt * kQuads * kTile;
         carve_scratch([&](auto &&part) {

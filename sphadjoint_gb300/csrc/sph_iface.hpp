@@ -106,6 +106,10 @@ void rt_set_step_graph(int steps);
 // are skipped (results stay on the device) and device allocations are
 // refused.
 bool rt_capturing();
+// Which recording the launches on the library stream go into: 0 when they run (a group
+// of steps is replayed as soon as it is recorded), else a number of the caller's capture,
+// whether made with this library's calls or on the stream itself.
+uint64_t rt_recording();
 // True when any kernel timer is on (launches are then not grouped, so that
 // each one is timed on its own).
 bool rt_timers_on();
