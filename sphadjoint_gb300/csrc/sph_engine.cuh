@@ -364,7 +364,8 @@ template <typename T> class Sys final : public StateI {
     DevBuf<uint32_t> fpair;
     DevBuf<int32_t> foff;
     bool listsTried = false; // the lists were asked for (and may have been refused)
-    bool listsFresh = false; // they belong to the masks the state holds
+    bool listsFresh = false; // they belong to the masks the state holds,
+    uint64_t listsIn = 0;    // made by this recording's launches (rt_recording)
     StepGraphs graphs;   // simulate's steps, replayed in groups
     bool anyRho = false; // some instance's model reads densities in the adjoint
     bool anyAV = false;  // some instance uses the artificial viscosity
@@ -638,14 +639,21 @@ template <typename T> class Sys final : public StateI {
         const size_t nt = (size_t)((N_ + kTile - 1) / kTile);
         return WinLists{wwin.p, wcand.p, wsupp.p, wcnt.p, wcnt.p + nt * kTile};
     }
+    // Lists made by a recording's launches are there only when it is replayed, and
+    // when it is, those from outside may belong to masks that have been replaced.
+    void lists_made()
+    {
+        listsFresh = true;
+        listsIn = rt_recording();
+    }
     // the candidate lists of the masks the state holds, if they are not there
     void fresh_lists(const NLView<T> &v)
     {
         if constexpr (sizeof(T) == 4) {
-            if (listsFresh) return;
+            if (listsFresh && listsIn == rt_recording()) return;
             auto kl = B > 1 ? &k_window_lists<true> : &k_window_lists<false>;
             SPH_LAUNCH_TILES(K_NLBUILD, kl, N_, v, lists());
-            listsFresh = true;
+            lists_made();
         }
     }
 
@@ -862,7 +870,7 @@ template <typename T> class Sys final : public StateI {
                 auto kn = B > 1 ? &k_nl_window<true> : &k_nl_window<false>;
                 SPH_LAUNCH_TILES(K_NLBUILD, kn, N_, N_, hinst[0], dinst.p, pinst.p, pos[cur].p,
                                  cellStart.p, nl_out(), lists());
-                listsFresh = true;
+                lists_made();
             }
         } else if (const int G = f.lanes) {
             auto kn = G == 32 ? &k_nl_build_coop<T, 32> : &k_nl_build_coop<T, 16>;
@@ -976,7 +984,7 @@ template <typename T> class Sys final : public StateI {
             if (build) {
                 auto kb = B > 1 ? &k_nl_density_win<true> : &k_nl_density_win<false>;
                 SPH_LAUNCH_TILES(K_DENSITY, kb, N_, v, nl_out(), lists(), rhoOut, prhoOut);
-                listsFresh = true;
+                lists_made();
                 return;
             }
             fresh_lists(v);
@@ -1351,6 +1359,26 @@ template <typename T> class Tape final : public TapeI {
     }
 };
 
+// The groups of steps of a call. Left by an exception, it drops an open group and the
+// claim to lists that a group not replayed would have made.
+template <typename T> struct GroupScope {
+    StepGraphs &g;
+    Sys<T> *a, *b; // states that step in it (b may be NULL)
+    bool done = false;
+    void finish()
+    {
+        g.finish();
+        done = true;
+    }
+    ~GroupScope()
+    {
+        g.abandon();
+        if (done) return;
+        a->listsFresh = false;
+        if (b) b->listsFresh = false;
+    }
+};
+
 // simulate! (src/driver.jl:92-115)
 template <typename T>
 void Sys<T>::simulate(FieldI *theta, const Params *p, int64_t nsteps, TapeI *tape)
@@ -1373,7 +1401,7 @@ void Sys<T>::simulate(FieldI *theta, const Params *p, int64_t nsteps, TapeI *tap
                 reserve(tp->slot((int)k));
     reserve_lists();
     graphs.start(step_graph_eligible<T>(N_));
-    StepGraphsGuard guard{graphs};
+    GroupScope<T> group{graphs, this, nullptr};
     for (int64_t s = 0; s < nsteps; ++s) {
         graphs.before_step();
         T2<T> *tx = nullptr, *tv = nullptr;
@@ -1394,7 +1422,7 @@ void Sys<T>::simulate(FieldI *theta, const Params *p, int64_t nsteps, TapeI *tap
         step_impl(th->th.p, tx, tv);
         graphs.after_step();
     }
-    graphs.finish();
+    group.finish();
     rt_sync();
     rt_check_launch("simulate");
 }
@@ -1937,7 +1965,7 @@ void Work<T>::run_backward(TapeI *tape, FieldI *theta, const Params *pp, const v
     S->reserve_lists();
     if (tp->nsnap_ && L > 0) tp->recomp->reserve_lists();
     graphs.start(step_graph_eligible<T>(N_));
-    StepGraphsGuard guard{graphs};
+    GroupScope<T> group{graphs, S, tp->recomp.get()};
     if (tp->nsnap_ == 0) {
         for (int64_t n = L - 1; n >= 0; --n) {
             graphs.before_step();
@@ -2023,7 +2051,7 @@ void Work<T>::run_backward(TapeI *tape, FieldI *theta, const Params *pp, const v
             freeSlots.push_back(taken[k].second);
         }
     }
-    graphs.finish();
+    group.finish();
     flush_theta(*S);
     SPH_LAUNCH(K_MISC, k_scatter_to_ids<T>, N_, N_, S->perm.p, gX[gcur].p, outX.p);
     SPH_LAUNCH(K_MISC, k_scatter_to_ids<T>, N_, N_, S->perm.p, gV[gcur].p, outV.p);

@@ -158,11 +158,6 @@ class StepGraphs {
     uint64_t clock_ = 0;
 };
 
-// Ends an open group of a StepGraphs when the scope is left by an exception.
-struct StepGraphsGuard {
-    StepGraphs &g;
-    ~StepGraphsGuard() { g.abandon(); }
-};
 // Wait for the library stream unless it is being captured.
 void rt_sync();
 
