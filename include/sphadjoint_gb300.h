@@ -227,7 +227,10 @@ SPH_API int32_t sph_batch_objective(sph_workspace ws, sph_state st, int32_t kind
    requests FIFO as soon as a worker is free and the request's device memory
    (states, tape or checkpoints, workspace; sph_request_bytes) fits within
    hbm_budget_bytes next to the requests already running: requests join while
-   others run and their kernels overlap on the device. Each result equals the
+   others run and their kernels overlap on the device. The neighbour lists of
+   its states (scratch: about 195 bytes a particle and state in FP32, 1290 in
+   FP64) are charged beside that, and left out where the budget has no room
+   for them; results do not depend on them. Each result equals the
    same request solved alone. Host inputs of a request (X0, V0, theta) must
    stay valid, and its outputs (gX, gV, gtheta; any may be NULL) are written,
    before sph_server_wait returns. A request whose gX, gV and gtheta are all
@@ -274,12 +277,12 @@ SPH_API int32_t sph_server_wait(sph_server s, int64_t ticket, double *J, double 
 SPH_API int32_t sph_server_poll(sph_server s, int64_t ticket, int32_t *done);
 /* latency percentiles of completed requests, particle-steps/s over the span
    from the first submit to the last completion, completed count, peak
-   admitted bytes and peak number of requests in flight */
+   admitted bytes (lists included) and peak number of requests in flight */
 SPH_API int32_t sph_server_stats(sph_server s, double *p50_ms, double *p99_ms,
                                  double *particle_steps_per_s, int64_t *completed,
                                  int64_t *peak_bytes, int32_t *peak_inflight);
 SPH_API int32_t sph_server_reset_stats(sph_server s);
-/* admission estimate of one request's device bytes */
+/* admission estimate of one request's device bytes, without its lists */
 SPH_API int64_t sph_request_bytes(const sph_request *req, int32_t dtype);
 
 /* ---- design side of the topology-optimisation caller, on the device ----

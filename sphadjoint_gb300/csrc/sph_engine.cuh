@@ -13,6 +13,7 @@
 #pragma once
 
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -536,14 +537,15 @@ template <typename T> class Sys final : public StateI {
     int64_t N() const override { return N_; }
     int batch() const override { return B; }
 
-    // lanes per particle of this state's pair-sum kernels (0: one thread) at lane setting f
-    int group_lanes(int f) const
+    // lanes per particle of the pair-sum kernels (0: one thread) at lane setting f
+    static int lanes_of(int f, int64_t N, int B)
     {
         if (B != 1) return 0;
         if (f == 16 || f == 32) return f;
-        if (f == 1 || N_ > kCoopMaxN) return 0;
-        return N_ <= coop32_max_n<T>() ? 32 : 16;
+        if (f == 1 || N > kCoopMaxN) return 0;
+        return N <= coop32_max_n<T>() ? 32 : 16;
     }
+    int group_lanes(int f) const { return lanes_of(f, N_, B); }
 
     // FP32 states with one thread per particle run their pair passes on tiles
     // (sph_window.cuh) when their lists are in memory. The lists (about 200
@@ -587,52 +589,79 @@ template <typename T> class Sys final : public StateI {
         return f;
     }
     FlatLists flat_lists() const { return FlatLists{fF.p, fr.p, ftm.p, fpair.p, foff.p, flat_particles(N_)}; }
+    // The buffers of the list forms: elements and their size, in the order of the views.
+    struct Part {
+        size_t n, size;
+    };
+    static std::array<Part, 4> tile_parts(int64_t N)
+    {
+        const size_t nt = (size_t)((N + kTile - 1) / kTile), e = nt * kQuads * kTile;
+        return {{{e, sizeof(uint2)}, {e, sizeof(uint2)}, {2 * nt * kTile, 1}, {nt, sizeof(TileWin)}}};
+    }
+    static std::array<Part, 5> pair_parts(int64_t N)
+    {
+        const size_t P = (size_t)flat_particles(N), nb = ((size_t)N + P - 1) / P;
+        const size_t rows = nb * P * kFlatRow, d = sizeof(double), i = sizeof(int32_t);
+        return {{{rows, d}, {rows, d}, {nb * P, d}, {rows, i}, {nb * kFlatOff, i}}};
+    }
+    template <size_t K> static size_t parts_bytes(const std::array<Part, K> &parts)
+    {
+        size_t b = 0;
+        for (const Part &q : parts) b += (q.n * q.size + 255) & ~(size_t)255;
+        return b;
+    }
+    // What a state of N particles takes for them at the present settings (the packed
+    // engine runs every FP32 request on tiles, and no pairs).
+    static int64_t list_bytes(const Params &p, int64_t N, bool packed)
+    {
+        const int set = rt_group_lanes();
+        if (N <= 0) return 0;
+        if (sizeof(T) == 4)
+            return N <= kListMaxN && (packed || lanes_of(set, N, 1) == 0)
+                       ? (int64_t)parts_bytes(tile_parts(N))
+                       : 0;
+        return !packed && set == 0 && p.visc != 1 && N <= kFlatMaxN
+                   ? (int64_t)parts_bytes(pair_parts(N))
+                   : 0;
+    }
     void reserve_lists()
     {
         if (want_tiles()) alloc_lists();
-        if (want_flat() && !listsTried && !rt_recording()) {
+        if (want_flat() && !listsTried && opts.lists && !rt_recording()) {
             listsTried = true;
-            const size_t P = (size_t)flat_particles(N_), nb = ((size_t)N_ + P - 1) / P;
-            carve_scratch([&](auto &&part) {
-                part(fF, nb * P * kFlatRow);
-                part(fr, nb * P * kFlatRow);
-                part(ftm, nb * P);
-                part(fpair, nb * P * kFlatRow);
-                part(foff, nb * kFlatOff);
-            });
+            carve_scratch(pair_parts(N_), fF, fr, ftm, fpair, foff);
         }
     }
     // Optional buffers in one allocation, if that is at most an eighth of the free
-    // memory: parts(part) names them twice, for their size and for their place.
-    // (An allocation each, and asking the driver for its free memory each time,
+    // memory. (An allocation each, and asking the driver for its free memory each time,
     // showed in streams of small requests.)
-    template <typename F> void carve_scratch(F &&parts)
+    template <size_t K, typename... Bufs>
+    void carve_scratch(const std::array<Part, K> &parts, Bufs &...bufs)
     {
-        size_t off = 0;
-        parts([&](auto &b, size_t n) { off += (n * sizeof(*b.p) + 255) & ~(size_t)255; });
-        if (!rt_has_free(8 * off)) return;
+        static_assert(sizeof...(bufs) == K, "a buffer per part");
+        const size_t bytes = parts_bytes(parts);
+        if (!rt_has_free(8 * bytes)) return;
         try {
-            scratch.alloc(off);
+            scratch.alloc(bytes);
         } catch (const Error &) {
             return;
         }
         uint8_t *at = scratch.p;
-        parts([&](auto &b, size_t n) {
-            b.view(reinterpret_cast<decltype(b.p)>(at), n);
-            at += (n * sizeof(*b.p) + 255) & ~(size_t)255;
-        });
+        size_t k = 0;
+        const auto place = [&](auto &b) {
+            b.view(reinterpret_cast<decltype(b.p)>(at), parts[k].n);
+            at += (parts[k].n * parts[k].size + 255) & ~(size_t)255;
+            ++k;
+        };
+        (place(bufs), ...);
     }
     void alloc_lists()
     {
-        if (listsTried || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN || rt_recording()) return;
+        if (listsTried || !opts.lists || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN ||
+            rt_recording())
+            return;
         listsTried = true;
-        const size_t nt = (size_t)((N_ + kTile - 1) / kTile), e = nt * kQuads * kTile;
-        carve_scratch([&](auto &&part) {
-            part(wcand, e);
-            part(wsupp, e);
-            part(wcnt, 2 * nt * kTile);
-            part(wwin, nt);
-        });
+        carve_scratch(tile_parts(N_), wcand, wsupp, wcnt, wwin);
     }
     WinLists lists() const
     {

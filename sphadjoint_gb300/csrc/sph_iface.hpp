@@ -23,11 +23,13 @@ struct Params {
     double alpha = 0.0;
 };
 
-// NeighborList knobs (src/neighbors.jl:174-175).
+// NeighborList knobs (src/neighbors.jl:174-175), and whether the state may take the
+// scratch of the list forms (results do not depend on it).
 struct NLOpts {
     double skin;
     int32_t interval;
     int32_t maxnb;
+    bool lists = true;
 };
 
 enum Dtype : int32_t { F64 = 0, F32 = 1 };
@@ -281,6 +283,7 @@ class PackI {
     virtual int64_t ticks() const = 0;
 };
 
+// (list_bytes: the scratch that one state takes for its lists, at the present settings)
 #define SPH_DECLARE_FACTORIES(SFX)                                                           \
     FieldI *make_field##SFX(const std::vector<int> &ngx, const std::vector<int> &ngy,        \
                             const void *host);                                               \
@@ -288,7 +291,8 @@ class PackI {
     StateI *make_state##SFX(const std::vector<Params> &p, const std::vector<int64_t> &N,     \
                             const void *X0, const void *V0, NLOpts o);                       \
     WorkI *make_work##SFX(const std::vector<Params> &p, const std::vector<int64_t> &N);       \
-    PackI *make_pack##SFX();
+    PackI *make_pack##SFX();                                                                 \
+    int64_t list_bytes##SFX(const Params &p, int64_t N, bool packed);
 
 SPH_DECLARE_FACTORIES(_f32)
 SPH_DECLARE_FACTORIES(_f64)

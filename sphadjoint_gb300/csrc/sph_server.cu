@@ -41,7 +41,8 @@ using Clock = std::chrono::steady_clock;
 struct Req {
     int64_t ticket = 0;
     sph_request spec{};
-    int64_t bytes = 0;
+    int64_t bytes = 0;     // charged to the budget: the estimate, plus its lists once granted
+    int64_t lists = 0;     // scratch of its states' lists
     Clock::time_point submitted, started, finished;
     int status = 0; // 0 queued, 1 running, 2 done, 3 failed
     double J = 0.0;
@@ -118,6 +119,17 @@ class Server {
 
     // device bytes a request holds while it runs
     virtual int64_t bytes_of(const sph_request &r) const { return request_bytes(r, dtype_); }
+    // and those of its lists: the solve state, the reverse scratch state, the recompute state
+    virtual int64_t lists_of(const sph_request &r) const
+    {
+        const bool adjoint = r.gX || r.gV || r.gtheta;
+        return state_lists(r, false) * (1 + (adjoint ? 1 : 0) + (adjoint && r.snapshots > 0 ? 1 : 0));
+    }
+    int64_t state_lists(const sph_request &r, bool packed) const
+    {
+        const Params p = params_of(r.p);
+        return dtype_ == SPH_F64 ? list_bytes_f64(p, r.N, packed) : list_bytes_f32(p, r.N, packed);
+    }
 
     int64_t submit(const sph_request &r0)
     {
@@ -220,14 +232,7 @@ class Server {
                 // fits next to the requests already running
                 cv_work_.wait(g, [&] { return stop_ || admissible(); });
                 if (stop_) break;
-                q = queue_.front();
-                queue_.pop_front();
-                inflight_ += q->bytes;
-                ++running_;
-                peakBytes_ = std::max(peakBytes_, inflight_);
-                peakInflight_ = std::max(peakInflight_, running_);
-                q->status = 1;
-                q->started = Clock::now();
+                q = admit();
             }
             const bool ok = solve(*q);
             {
@@ -262,6 +267,27 @@ class Server {
                inflight_ + queue_.front()->bytes <= budget_;
     }
 
+    // Takes the head of the queue. Its lists are optional scratch: they are granted from
+    // what the budget has left, unless that would keep the next request out that could
+    // start now; a request without them runs the list-free forms (the same bits).
+    std::shared_ptr<Req> admit()
+    {
+        auto q = queue_.front();
+        queue_.pop_front();
+        inflight_ += q->bytes;
+        ++running_;
+        q->lists = lists_of(q->spec);
+        const int64_t next = admissible() ? queue_.front()->bytes : 0;
+        if (inflight_ + q->lists + next > budget_) q->lists = 0;
+        q->bytes += q->lists;
+        inflight_ += q->lists;
+        peakBytes_ = std::max(peakBytes_, inflight_);
+        peakInflight_ = std::max(peakInflight_, running_);
+        q->status = 1;
+        q->started = Clock::now();
+        return q;
+    }
+
     // Runs one request on this worker's stream; results go to the caller's
     // host buffers. Returns false (with q.err / q.msg set) on failure.
     bool solve(Req &q)
@@ -273,7 +299,7 @@ class Server {
             p.gx = r.p.gx; p.gy = r.p.gy; p.dt = r.p.dt; p.Lx = r.p.Lx; p.Ly = r.p.Ly;
             p.kw = r.p.kw; p.ngx = r.p.ngx; p.ngy = r.p.ngy;
             p.eos = r.p.eos; p.gamma = r.p.gamma; p.visc = r.p.visc; p.alpha = r.p.alpha;
-            const NLOpts o{r.skin, r.interval, r.maxnb};
+            const NLOpts o{r.skin, r.interval, r.maxnb, q.lists > 0};
             const std::vector<Params> ps{p};
             const std::vector<int64_t> ns{r.N};
             const std::vector<int> gx{p.ngx}, gy{p.ngy};
@@ -337,6 +363,7 @@ class StreamServer final : public Server {
     StreamServer(int workers, int64_t budget, int dtype) : Server(budget, dtype)
     {
         if (workers < 1) throw Error(ERR_ARG, "need at least one worker");
+        maxInflight_ = workers;
         for (int w = 0; w < workers; ++w) threads_.emplace_back([this] { run_streams(); });
     }
     ~StreamServer() override { stop(); }
@@ -373,6 +400,11 @@ class PackedServer final : public Server {
     }
     ~PackedServer() override { stop(); }
     int64_t bytes_of(const sph_request &r) const override { return packed_request_bytes(r, dtype_); }
+    // the solve state (also the recompute state) and the reverse scratch state
+    int64_t lists_of(const sph_request &r) const override
+    {
+        return state_lists(r, true) * (r.gX || r.gV || r.gtheta ? 2 : 1);
+    }
 
   private:
     void fail(Req &q, int code, const std::string &msg)
@@ -401,25 +433,15 @@ class PackedServer final : public Server {
         }
         for (;;) {
             // admission (FIFO, by bytes and slots)
-            std::vector<std::shared_ptr<Req>> admit;
+            std::vector<std::shared_ptr<Req>> started;
             {
                 std::unique_lock<std::mutex> g(mu_);
                 if (byId.empty())
                     cv_work_.wait(g, [&] { return stop_ || admissible(); });
                 if (stop_ && byId.empty()) break;
-                while (admissible()) {
-                    auto q = queue_.front();
-                    queue_.pop_front();
-                    inflight_ += q->bytes;
-                    ++running_;
-                    peakBytes_ = std::max(peakBytes_, inflight_);
-                    peakInflight_ = std::max(peakInflight_, running_);
-                    q->status = 1;
-                    q->started = Clock::now();
-                    admit.push_back(q);
-                }
+                while (admissible()) started.push_back(admit());
             }
-            for (auto &q : admit) {
+            for (auto &q : started) {
                 const sph_request &r = q->spec;
                 try {
                     if (!pack) throw Error(ERR_CUDA, "packed engine unavailable");
@@ -433,7 +455,7 @@ class PackedServer final : public Server {
                     pr.snapshots = r.snapshots;
                     pr.objective = r.objective;
                     for (int k = 0; k < 3; ++k) pr.obj_args[k] = r.obj_args[k];
-                    pr.opts = NLOpts{r.skin, r.interval, r.maxnb};
+                    pr.opts = NLOpts{r.skin, r.interval, r.maxnb, q->lists > 0};
                     pr.adjoint = r.gX || r.gV || r.gtheta;
                     byId[pack->add(pr)] = q;
                 } catch (const Error &e) {
