@@ -566,7 +566,7 @@ template <typename T> class Sys final : public StateI {
     static constexpr int64_t kFlatMaxN = int64_t(1) << 22;
     bool want_flat() const
     {
-        return sizeof(T) == 8 && N_ > 0 && N_ <= kFlatMaxN && rt_group_lanes() == 0;
+        return sizeof(T) == 8 && N_ > 0 && N_ <= kFlatMaxN && !anyAV && rt_group_lanes() == 0;
     }
     // The kernels of one step or one build, chosen once at its start. The lane and
     // density settings are process-wide and another thread may move them at any time;
