@@ -364,7 +364,7 @@ template <typename T> class Sys final : public StateI {
     DevBuf<double> fF, fr, ftm; // dense pairs of the FP64 flat passes
     DevBuf<uint32_t> fpair;
     DevBuf<int32_t> foff;
-    bool listsTried = false; // the lists were asked for (and may have been refused)
+    int listsWait = 0, listsNext = 1; // calls until the lists are asked for again, after a refusal
     bool listsFresh = false; // they belong to the masks the state holds,
     uint64_t listsIn = 0;    // made by this recording's launches (rt_recording)
     StepGraphs graphs;   // simulate's steps, replayed in groups
@@ -627,10 +627,20 @@ template <typename T> class Sys final : public StateI {
     void reserve_lists()
     {
         if (want_tiles()) alloc_lists();
-        if (want_flat() && !listsTried && opts.lists && !rt_recording()) {
-            listsTried = true;
-            carve_scratch(pair_parts(N_), fF, fr, ftm, fpair, foff);
+        if (want_flat() && may_ask()) carve_scratch(pair_parts(N_), fF, fr, ftm, fpair, foff);
+    }
+    // Memory may be free again later, so a state that was refused its lists asks again,
+    // after 1, 2, 4 ... 256 calls (asking the driver costs as much as a short step).
+    bool may_ask()
+    {
+        if (scratch.p || !opts.lists || rt_recording()) return false;
+        if (listsWait > 0) {
+            --listsWait;
+            return false;
         }
+        listsWait = listsNext;
+        listsNext = std::min(2 * listsNext, 256);
+        return true;
     }
     // Optional buffers in one allocation, if that is at most an eighth of the free
     // memory. (An allocation each, and asking the driver for its free memory each time,
@@ -657,10 +667,7 @@ template <typename T> class Sys final : public StateI {
     }
     void alloc_lists()
     {
-        if (listsTried || !opts.lists || sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN ||
-            rt_recording())
-            return;
-        listsTried = true;
+        if (sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN || !may_ask()) return;
         carve_scratch(tile_parts(N_), wcand, wsupp, wcnt, wwin);
     }
     WinLists lists() const

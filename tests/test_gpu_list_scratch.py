@@ -51,3 +51,32 @@ def test_only_models_with_pair_passes_take_pair_lists(model, takes):
         sp.visc = "morris" if isinstance(sp.visc, str) else 0
         S.step(st, th, sp)
         assert used() - before >= PAIRS * st.N
+
+
+@pytest.mark.parametrize("dtype,nx,ny", [("f64", 700, 700), ("f32", 2000, 1600)])
+def test_refused_lists_are_asked_for_again(dtype, nx, ny):
+    """Lists are taken from an eighth of the free memory at most. A state that starts while
+    less is free steps without them, and takes them once there is room; its results are
+    those of a state that had them from the start."""
+    torch = pytest.importorskip("torch")
+    ref, th, _ = state(nx, ny, dtype)
+    st, _, _ = state(nx, ny, dtype)
+    least = (PAIRS if dtype == "f64" else 195) * st.N
+    before = used()
+    S.step(ref, th)
+    assert used() - before >= least
+    L, p = pool()
+    assert L.cuMemPoolTrimTo(p, C.c_size_t(0)) == 0
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - 5 * least, dtype=torch.uint8, device="cuda")
+    before = used()
+    S.step(st, th)
+    assert used() == before  # refused
+    del hog
+    torch.cuda.empty_cache()
+    for _ in range(2):
+        S.step(st, th)
+    assert used() - before >= least
+    for _ in range(2):
+        S.step(ref, th)
+    for a, b in zip(st.get(), ref.get()):
+        assert np.array_equal(a, b)
