@@ -30,7 +30,7 @@ SOURCES = {
     "sph_design.cu": ["--fmad=false"],
 }
 DEPS = ["sph_common.cuh", "sph_exact64.cuh", "sph_fixed.cuh", "sph_kernels.cuh", "sph_coop.cuh", "sph_window.cuh", "sph_flat.cuh", "sph_engine.cuh", "sph_pack.cuh",
-        "sph_iface.hpp"]
+        "sph_iface.hpp", "sph_once.hpp"]
 
 
 def nvcc() -> str:

@@ -27,6 +27,7 @@
 #include "sph_flat.cuh"
 #include "sph_iface.hpp"
 #include "sph_kernels.cuh"
+#include "sph_once.hpp"
 #include "sph_window.cuh"
 
 namespace sphgb {
@@ -514,16 +515,17 @@ template <typename T> class Sys final : public StateI {
         {
             // the one-launch cell list of small states (set here, outside any
             // graph recording)
-            static bool attr = false;
-            if (!attr) {
+            static OncePerDevice attributes;
+            int device = 0;
+            SPH_CK(cudaGetDevice(&device));
+            attributes(device, [] {
                 const int most = (int)(sizeof(int32_t) * (2 * kRebuildSmallMaxCells + 1 +
                                                           kRebuildSmallMaxN));
                 SPH_CK(cudaFuncSetAttribute(k_rebuild_small<T, 1>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, most));
                 SPH_CK(cudaFuncSetAttribute(k_rebuild_small<T, kRebuildPer>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-                attr = true;
-            }
+            });
         }
         init_identity();
         if (X0 || V0) set(X0, V0);
