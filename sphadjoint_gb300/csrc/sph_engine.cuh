@@ -1809,9 +1809,11 @@ template <typename T> class Work final : public WorkI {
 
 // Block-size autotuner: times each hot kernel of this state's kind (single or
 // batched) at 64, 128 and 256 threads per block on the state's current
-// positions and keeps the fastest. Forward kernels run on the state itself
-// (they only write derived arrays); the adjoint kernels run on a temporary
-// workspace with placeholder gradients, whose values do not change the work.
+// positions and keeps the fastest. The kernels tuned are those of the mask walks with one
+// thread per particle; lane groups, FP32 tiles and FP64 pairs have fixed sizes. Forward
+// kernels run on the state itself (they only write arrays that the next step forms again);
+// the adjoint kernels run on a temporary workspace with placeholder gradients, whose values
+// do not change the work.
 template <typename T> class Tuner {
   public:
     static void run(Sys<T> &S, Field<T> &th, int reps, int *chosen)
@@ -1849,6 +1851,10 @@ template <typename T> class Tuner {
         cudaStream_t st = rt_stream();
         NLView<T> v = S.view();
         const int nxt = 1 - S.cur;
+        // the timed builds write arrays of their own: between rebuilds the particles are
+        // off the cell list, and the state's lists belong to the masks it has
+        DevBuf<uint32_t> center((size_t)N), masks(6 * (size_t)N), flags((size_t)S.B);
+        DevBuf<int32_t> nbcount((size_t)N);
         auto kn = multi ? &k_nl_build<T, true> : &k_nl_build<T, false>;
         auto kd = multi ? &k_density_eos<T, true> : &k_density_eos<T, false>;
         auto ki = multi ? &k_accel_integrate<T, true> : &k_accel_integrate<T, false>;
@@ -1858,8 +1864,7 @@ template <typename T> class Tuner {
         int b;
         b = timeit([&](int c) {
             kn<<<grid(c), c, 0, st>>>(N, S.hinst[0], S.dinst.p, S.pinst.p, S.pos[S.cur].p,
-                                      S.cellStart.p, S.center.p, S.masks.p, S.nbcount.p,
-                                      S.flags.p);
+                                      S.cellStart.p, center.p, masks.p, nbcount.p, flags.p);
         });
         tuned_block<T>(K_NLBUILD, multi) = b;
         b = timeit([&](int c) {
