@@ -452,11 +452,13 @@ SPH_API int64_t sph_launch_count(void);
 SPH_API int32_t sph_profile_enable(int32_t kernel_id, int32_t on);
 SPH_API int32_t sph_profile_read(int32_t kernel_id, double *total_ms, int64_t *launches);
 SPH_API int32_t sph_profile_reset(void);
-/* kernel ids for sph_profile_* */
+/* kernel ids for sph_profile_* (BUILD_DENSITY: the density pass of a rebuild step that also
+   builds the neighbour masks, in forms that do so in one launch; otherwise such a step has
+   an NLBUILD and a DENSITY launch) */
 enum {
     SPH_K_ASSIGN = 0, SPH_K_SCAN, SPH_K_BUCKET, SPH_K_RANK, SPH_K_NLBUILD, SPH_K_DENSITY,
     SPH_K_ACCEL_INTEGRATE, SPH_K_TAPE, SPH_K_GATHER, SPH_K_ACCEL_DRAG, SPH_K_PASS1,
-    SPH_K_PASS2, SPH_K_THETA_NODE, SPH_K_MISC
+    SPH_K_PASS2, SPH_K_THETA_NODE, SPH_K_MISC, SPH_K_BUILD_DENSITY
 };
 
 /* binomial checkpoint schedule (host only): forward steps to reverse l steps

@@ -17,7 +17,8 @@ SPH_F64, SPH_F32 = 0, 1
 FLAG_NL_OVERFLOW, FLAG_DISPLACEMENT, FLAG_NONFINITE = 1, 2, 4
 
 KERNELS = ["assign", "scan", "bucket", "rank", "nl_build", "density", "accel_integrate",
-           "tape", "gather", "accel_drag", "pass1", "pass2", "theta_node", "misc"]
+           "tape", "gather", "accel_drag", "pass1", "pass2", "theta_node", "misc",
+           "build_density"]
 KERNEL_ID = {k: i for i, k in enumerate(KERNELS)}
 
 

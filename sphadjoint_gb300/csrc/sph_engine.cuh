@@ -895,6 +895,8 @@ template <typename T> class Sys final : public StateI {
         build_masks(f);
         return false;
     }
+    // what the density launch of a step is timed as
+    static int density_id(bool due) { return due ? K_BUILD_DENSITY : K_DENSITY; }
     static auto density_coop(int G, bool build)
     {
         return G == 32 ? (build ? &k_density_eos_coop<T, 32, true> : &k_density_eos_coop<T, 32, false>)
@@ -984,14 +986,15 @@ template <typename T> class Sys final : public StateI {
                 auto kd = B > 1 ? &k_density_flat<true, false>
                                 : due ? &k_density_flat<false, true> : &k_density_flat<false, false>;
                 auto ki = B > 1 ? &k_accel_flat<true> : &k_accel_flat<false>;
-                SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, 0, kFlatBlock, kd, N_, v, W, rho.p, prho.p,
+                SPH_LAUNCH_FLAT_X(density_id(due), W.P, 0, kFlatBlock, kd, N_, v, W, rho.p, prho.p,
                                   no_flush(), nl_out());
                 SPH_LAUNCH_FLAT(K_ACCEL_INTEGRATE, W.P, ki, N_, v, W, vel[cur].p, prho.p, theta,
                                 pos[nxt].p, vel[nxt].p, aO, alO, flags.p, perm.p, tx, tv);
             }
         } else if (const int G = f.lanes) {
             auto kd = density_coop(G, due);
-            SPH_LAUNCH_COOP(K_DENSITY, G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush(), nl_out());
+            SPH_LAUNCH_COOP(density_id(due), G, kd, N_, v, rho.p, prho.p, tmask.p, no_flush(),
+                            nl_out());
             v.tmask = tmask.p;
             auto ki = G == 32 ? &k_accel_integrate_coop<T, 32> : &k_accel_integrate_coop<T, 16>;
             SPH_LAUNCH_COOP_X(K_ACCEL_INTEGRATE, G, 0, kCoopThreads, ki, N_, v, vel[cur].p, prho.p,
@@ -1021,7 +1024,7 @@ template <typename T> class Sys final : public StateI {
         if constexpr (sizeof(T) == 4) {
             if (build) {
                 auto kb = B > 1 ? &k_nl_density_win<true> : &k_nl_density_win<false>;
-                SPH_LAUNCH_TILES(K_DENSITY, kb, N_, v, nl_out(), lists(), rhoOut, prhoOut);
+                SPH_LAUNCH_TILES(K_BUILD_DENSITY, kb, N_, v, nl_out(), lists(), rhoOut, prhoOut);
                 lists_made();
                 return;
             }
@@ -1621,8 +1624,8 @@ template <typename T> class Work final : public WorkI {
                 auto k1 = multi ? &k_pass1_flat<true> : &k_pass1_flat<false>;
                 auto k2 = multi ? &k_pass2_flat<true> : &k_pass2_flat<false>;
                 const ThetaFlush<T> fl = take_flush(S, (N_ + W.P - 1) / W.P, extra);
-                SPH_LAUNCH_FLAT_X(K_DENSITY, W.P, extra, kFlatBlock, kd, N_, v, W, rhoOut, S.prho.p,
-                                  fl, S.nl_out());
+                SPH_LAUNCH_FLAT_X(S.density_id(due), W.P, extra, kFlatBlock, kd, N_, v, W, rhoOut,
+                                  S.prho.p, fl, S.nl_out());
                 SPH_LAUNCH_FLAT(K_ACCEL_DRAG, W.P, ka, N_, v, W, vel, S.prho.p, theta, gX[gcur].p,
                                 gV[gcur].p, abar.p, galpha.p, emax.p, parity);
                 SPH_LAUNCH_FLAT(K_PASS1, W.P, k1, N_, v, W, vel, S.prho.p, S.rho.p, theta, abar.p,
@@ -1641,7 +1644,7 @@ template <typename T> class Work final : public WorkI {
             auto k2 = g32 ? &k_pass2_axpy_coop<T, 32> : &k_pass2_axpy_coop<T, 16>;
             const int per = kCoopBlock / G;
             const ThetaFlush<T> fl = take_flush(S, (N_ + per - 1) / per, extra);
-            SPH_LAUNCH_COOP_X(K_DENSITY, G, extra, kCoopBlock, kd, N_, v, rhoOut, S.prho.p,
+            SPH_LAUNCH_COOP_X(S.density_id(due), G, extra, kCoopBlock, kd, N_, v, rhoOut, S.prho.p,
                               S.tmask.p, fl, S.nl_out());
             v.tmask = S.tmask.p;
             SPH_LAUNCH_COOP_X(K_ACCEL_DRAG, G, 0, kCoopThreads, ka, N_, v, vel, S.prho.p, S.rho.p,

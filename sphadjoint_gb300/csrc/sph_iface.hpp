@@ -70,6 +70,7 @@ enum KernelId : int32_t {
     K_PASS2,
     K_THETA_NODE,
     K_MISC,
+    K_BUILD_DENSITY, // neighbour masks and the density pass in one launch
     K_COUNT
 };
 
