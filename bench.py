@@ -80,6 +80,12 @@ ALGO_WORDS = {
 ALGO_INTS = {"build_density": 8}
 
 
+def tuned_kernels_run(args):
+    """Block sizes are tuned for the mask walks with one thread per particle, which FP32
+    states run in the other density forms only, and FP64 states for the neighbour build."""
+    return args.dtype == "f64" or args.density_form != "pairs"
+
+
 def algo_bytes_of(kernel, esz, N):
     return (ALGO_WORDS[kernel] * esz + 4 * ALGO_INTS.get(kernel, 0)) * N
 
@@ -230,7 +236,7 @@ def run_batched(args):
         LB.check(L.sph_batch_objective(ws.h, bt.h, 0, None, Jb))
         LB.check(L.sph_backward_seeded(ws.h, tp.h, th.h, None, None, 0.2, 4, 64, C.byref(flags)))
 
-    if args.autotune:
+    if args.autotune and tuned_kernels_run(args):
         b6 = (C.c_int32 * 6)()
         LB.check(L.sph_autotune(bt.h, th.h, 5, b6))
         tape_t = S.Tape(ntot, TUNE_STEPS, ps[0], snapshots=0)
@@ -687,7 +693,7 @@ def run_ours(args):
                                        C.byref(flags)))
 
     blocks = None
-    if args.autotune:
+    if args.autotune and tuned_kernels_run(args):
         # block sizes: the engine's autotune on this workload's initial state,
         # then each kernel's fastest size inside short solves of the workload
         b6 = (C.c_int32 * 6)()
@@ -1052,7 +1058,8 @@ def main():
     ap.add_argument("--graph", type=int, default=0,
                     help="time replays of the whole solve captured as one CUDA graph")
     ap.add_argument("--autotune", type=int, default=1,
-                    help="measure per-kernel block sizes on the workload before timing")
+                    help="measure per-kernel block sizes on the workload before timing, where "
+                         "kernels that have them run (block_sizes is null otherwise)")
     args = ap.parse_args()
     batched = args.workload == "batched"
     if args.fp64_check < 0:
