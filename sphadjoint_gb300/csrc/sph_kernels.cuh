@@ -802,6 +802,31 @@ __device__ __forceinline__ AccelPair<T> accel_pair(T r2, T dx, T dy, T invh, T m
     return o;
 }
 
+// One pair of the FP32 force sum with the artificial viscosity, added to (ax, ay) with
+// explicit roundings: every walk and list gives the same bits. (Left to the compiler, the
+// product K d of the branch on approaching pairs was rounded before the addition in some
+// loops and contracted in others.)
+__device__ __forceinline__ void accel_add_av(float dx, float dy, float r2, float invh, float m,
+                                             float Fc, const Visc<float> &vc, float pti,
+                                             float rhoi, float rhoj, const float2 &vi, float ptj,
+                                             const float2 &vj, float &ax, float &ay)
+{
+    const float q = __fmul_rn(pair_sqrt(r2), invh);
+    const float u = __fmaf_rn(-0.5f, q, 1.0f);
+    const float F = __fmul_rn(__fmul_rn(__fmul_rn(Fc, u), u), u);
+    const float PF = __fmul_rn(__fmul_rn(m, __fadd_rn(pti, ptj)), F);
+    ax = __fmaf_rn(-PF, dx, ax);
+    ay = __fmaf_rn(-PF, dy, ay);
+    const float s = __fmaf_rn(__fsub_rn(vi.x, vj.x), dx, __fmul_rn(__fsub_rn(vi.y, vj.y), dy));
+    if (s < 0.0f) {
+        const float D = __fadd_rn(r2, vc.eh2);
+        const float rb = __fmul_rn(0.5f, __fadd_rn(rhoi, rhoj));
+        const float K = __fmul_rn(__fmul_rn(vc.avc, s), F) / __fmul_rn(D, rb);
+        ax = __fmaf_rn(K, dx, ax);
+        ay = __fmaf_rn(K, dy, ay);
+    }
+}
+
 // adj_pass1_kernel!: gx -= P F da_x, gx += w d_x (same for y), gv += C da,
 // grho -= C ad_v ir_i, S += F ad_d.
 template <typename T> struct Pass1Pair {
@@ -1251,7 +1276,8 @@ __device__ __forceinline__ void accel_sum(const NLView<T> &v, const Inst<T> &I,
     const Visc<T> vc = visc_of<T>(I);
     const T2<T> pi = prho[i];
     const T pti = pi.x, iri = pi.y;
-    if constexpr (sizeof(T) == 4 && !AV && kPackedPairs) {
+    if constexpr (sizeof(T) == 4 && kPackedPairs)
+    if (!AV || vc.kind != 1) { // in a batch of both models too, with a solo run's bits
         // a_i -= (P_ij F) d, a_i += C (v_i - v_j), both components at once
         const float tmm = vc.twomumass;
         float2 acc = make_float2(0.0f, 0.0f);
@@ -1281,6 +1307,20 @@ __device__ __forceinline__ void accel_sum(const NLView<T> &v, const Inst<T> &I,
     const T rhoi = (AV && vc.kind == 1) ? rho[i] : (T)0;
     ax = (T)0;
     ay = (T)0;
+    if constexpr (sizeof(T) == 4 && AV) {
+        if (vc.kind == 1) {
+            for_each_neighbor<T>(v, I, i, [&](int j) {
+                const float2 xj = v.pos[j];
+                const float dx = xi.x - xj.x;
+                const float dy = xi.y - xj.y;
+                const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+                if (lt_nonneg(r2, r2max))
+                    accel_add_av(dx, dy, r2, invh, m, Fc, vc, pti, rhoi, rho[j], vi, prho[j].x,
+                                 vel[j], ax, ay);
+            });
+            return;
+        }
+    }
     for_each_neighbor<T>(v, I, i, [&](int j) {
         const T2<T> xj = v.pos[j];
         const T dx = xi.x - xj.x;
@@ -1556,7 +1596,8 @@ __device__ __forceinline__ void pass1_sum(const NLView<T> &v, const IT &I, int64
     const T r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, Fc = I.p.Fc, Gc = I.p.Gc;
     const Visc<T> vc = visc_of<T>(I);
     const T pti = pi.x, iri = pi.y;
-    if constexpr (sizeof(T) == 4 && !AV && kPackedPairs) {
+    if constexpr (sizeof(T) == 4 && kPackedPairs)
+    if (!AV || vc.kind != 1) { // in a batch of both models too, with a solo run's bits
         // the Morris-model pair of adj_pass1_kernel! with (x, y) packed:
         // g -= (P F) da, g += w d, gv += C da
         const float tmm = vc.twomumass;

@@ -644,7 +644,6 @@ __device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsign
         ax = acc.x;
         ay = acc.y;
     } else {
-        vc.kind = 1;
         ax = 0.0f;
         ay = 0.0f;
         for_each_entry(list, n, [&](uint32_t o) {
@@ -654,13 +653,8 @@ __device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsign
             const float rhoj = lds1(sw + 3 * kWin8, o >> 1);
             const float dx = xi.x - xj.x;
             const float dy = xi.y - xj.y;
-            const float r2 = dx * dx + dy * dy;
-            const AccelPair<float> t = accel_pair<float, AV>(r2, dx, dy, invh, m, Fc, vc, pti, iri,
-                                                             rhoi, rhoj, vi, pj, vj);
-            ax -= t.px;
-            ay -= t.py;
-            ax += t.cx;
-            ay += t.cy;
+            const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+            accel_add_av(dx, dy, r2, invh, m, Fc, vc, pti, rhoi, rhoj, vi, pj.x, vj, ax, ay);
         });
     }
 }
