@@ -285,12 +285,13 @@ __device__ __forceinline__ void g_accel_sum(const GSys<T> &d, int tile, int64_t 
     const NLView<T> &v = d.v;
     if constexpr (sizeof(T) == 4) {
         __shared__ __align__(16) unsigned char s_win[kAccelSmem<AV>];
+        int nr = 0;
         if (d.W.win)
-            stage_window<3, AV>(d.W.win + tile, s_win, v.pos, d.vel, d.prho, nullptr, d.rhoAll);
+            nr = stage_window<3, AV>(d.W.win + tile, s_win, v.pos, d.vel, d.prho, nullptr, d.rhoAll);
         if (!live) return;
         xi = v.pos[i];
         vi = d.vel[i];
-        accel_any<false, AV>(v, d.W, tile, s_win, i, v.one, d.vel, d.prho, d.rhoAll, xi, vi, ax, ay);
+        accel_any<false, AV>(v, d.W, tile, s_win, nr, i, v.one, d.vel, d.prho, d.rhoAll, xi, vi, ax, ay);
     } else {
         if (!live) return;
         xi = v.pos[i];

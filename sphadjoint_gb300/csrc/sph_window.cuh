@@ -24,9 +24,10 @@
 // sums are those of the mask walks (for_each_neighbor), operation by operation,
 // so results are the same bits; what goes away is the walk itself: finding set
 // bits, moving from word to word (some lane of a warp does that in nearly every
-// iteration), and 64-bit addresses for every array. Particles that have no
-// list (a row beyond the 64-slot masks, more than 48 candidates, or a tile
-// whose window exceeds its capacity) are marked and take the mask walk.
+// iteration), and 64-bit addresses for every array. A tile whose window exceeds
+// its capacity keeps lists of slots, and its passes read memory (TileKind). Particles
+// that have no list (more than 48 candidates, or in a tile of more than 8 runs or with
+// a window wider than 16 bits) are marked and take the mask walk.
 //
 // Bound: shared-memory wavefronts and issue slots together (accel at 1M: 71% of
 // the wavefront rate, 57% of the issue slots, 913 warp instructions a warp where
@@ -49,6 +50,8 @@ constexpr int kRunMax = 8;     // cell-row runs of a tile
 constexpr int kRangeMax = 3 * kRunMax;
 constexpr int kQuads = 12;     // list capacity: 48 entries
 constexpr int kNoList = 255;   // count of a particle without a list
+constexpr int kSpilled = 64;   // flag beside the candidate count of a particle whose rows
+                               // exceed the 64-slot masks
 // While lists are collected, entry k of thread t lies at row k, column t: a store
 // has a two-way bank conflict at most, wherever each lane's list ends (a run of
 // entries per thread, its stride an odd number of words: 3.4 wavefronts on
@@ -59,9 +62,9 @@ constexpr int kNlStride = 8 * kQuads + 20;  // the same with room for eight entr
                                             // the capacity (nl_window)
 
 struct TileWin {
-    int32_t nr;               // ranges (0: no window, every particle is marked)
+    int32_t nr;               // ranges (0: no window)
     int32_t pad[3];
-    int32_t start[kRangeMax]; // first slot, a multiple of 4
+    int32_t start[kRangeMax]; // first slot, a multiple of 4 (no window: of all ranges)
     int32_t base[kRangeMax + 1]; // first window slot; base[nr] = window slots
     int32_t pad2[3];
 };
@@ -100,17 +103,38 @@ __device__ __forceinline__ void copy_wait()
 constexpr int kWin8 = 8 * kWinMax;
 constexpr int kWin4 = 4 * kWinMax;
 
+// Where a pass reads its neighbours: float2 array k and, behind N8 of those, a float
+// array, at a list's entry e.
+struct InWindow { // staged, e a byte offset
+    const unsigned char *sw;
+    __device__ __forceinline__ float2 a(int k, uint32_t e) const { return lds2(sw + k * kWin8, e); }
+    template <int N8> __device__ __forceinline__ float f(uint32_t e) const
+    {
+        return lds1(sw + N8 * kWin8, e >> 1);
+    }
+};
+struct InMemory { // of a tile without a window, e a slot from its first one on
+    const float2 *p0, *p1, *p2, *p3;
+    const float *pf;
+    __device__ __forceinline__ float2 a(int k, uint32_t e) const
+    {
+        return (k == 0 ? p0 : k == 1 ? p1 : k == 2 ? p2 : p3)[e];
+    }
+    template <int N8> __device__ __forceinline__ float f(uint32_t e) const { return pf[e]; }
+};
+
 // Copy the tile's window of the given arrays into shared memory at sw, sw +
 // kWin8, ... (N8 float2 arrays), then a float array. Range ends are multiples of
 // four slots, so a copy may read up to three elements past the last particle:
-// every staged array has room for them. All threads of the block call it.
+// every staged array has room for them. All threads of the block call it. Returns the
+// ranges: 0 is a tile without a window, whose lists hold slots from w->start[0] on.
 //
 // Neighbours are then read eight bytes at a time: 4.2 wavefronts a warp read
 // (2.1 per 16 lanes; bank padding, swizzles, 4-byte arrays were no better), and
 // 16-byte reads of interleaved arrays measured slower (8.8 wavefronts where two
 // 8-byte reads take 8.4: accel 46 -> 55 us, pass 1 60 -> 74 us at 1M).
 template <int N8, bool F4>
-__device__ __forceinline__ void stage_window(const TileWin *__restrict__ w,
+__device__ __forceinline__ int stage_window(const TileWin *__restrict__ w,
                                              const unsigned char *sw, const float2 *a0,
                                              const float2 *a1, const float2 *a2, const float2 *a3,
                                              const float *f)
@@ -138,6 +162,7 @@ __device__ __forceinline__ void stage_window(const TileWin *__restrict__ w,
     }
     copy_wait();
     __syncthreads();
+    return nr;
 }
 
 __device__ __forceinline__ uint32_t entry_of(const uint2 &e, int k)
@@ -164,16 +189,22 @@ __device__ __forceinline__ void write_list(unsigned char *place, int n, uint2 *_
 
 // The window of a tile whose particles lie in cells (cx, cy) of instance b:
 // TileWin, and for this thread's run the window slot of a slot j of row r as
-// T.base[3 run + r] + j - T.start[3 run + r]. Returns whether the window fits
-// (otherwise the tile's particles take the mask walk). All threads call it; it
-// ends with a barrier.
+// T.base[3 run + r] + j - T.start[3 run + r]. Returns kWindow if the window fits. If it
+// does not, but its slots span 16 bits, kFar: the lists hold slots from T.first on and the
+// passes read memory. (Where a column has pressed through a wall, a border cell holds
+// what would be many cells, and such a tile's walk over rows of some hundred slots was
+// the end of every pass: a batch of eight, 51,500 particles, 1000 steps on, 32 steps with
+// gradient 8.8 ms, so 2.7; 90,000 particles 6.4 ms, so 2.5.) Otherwise kNone: the mask walk. All threads call it; it ends with a
+// barrier.
+enum TileKind : int { kNone = 0, kFar, kWindow };
 struct TileShared {
     int key[kTile], cnt[kTile / 32];
     int lo[kRunMax], hi[kRunMax], inst[kRunMax], cy[kRunMax];
     int start[32], len[32], base[33];
+    int first, span;
 };
 template <bool MULTI>
-__device__ __forceinline__ bool tile_window(TileShared &T, const Inst<float> &one,
+__device__ __forceinline__ int tile_window(TileShared &T, const Inst<float> &one,
                                             const Inst<float> *inst,
                                             const int32_t *__restrict__ cellStart, bool live, int b,
                                             int cx, int cy, TileWin *W, int &run, int &nrun)
@@ -238,26 +269,80 @@ __device__ __forceinline__ bool tile_window(TileShared &T, const Inst<float> &on
             if (lane >= o) x += y;
         }
         T.base[t] = x - n;
-        if (t == 31) T.base[32] = x;
+        const int lo = __reduce_min_sync(0xffffffffu, n ? T.start[t] : INT_MAX);
+        const int hi = __reduce_max_sync(0xffffffffu, n ? T.start[t] + n : 0);
+        if (t == 31) {
+            T.base[32] = x;
+            T.first = x ? lo : 0;
+            T.span = x ? hi - lo : 0;
+        }
     }
     __syncthreads();
+    const bool far = ok && T.base[32] > kWinMax && T.span <= 65536;
     ok = ok && T.base[32] <= kWinMax;
     if (t == 0) W->nr = ok ? 3 * nrun : 0;
-    if (t < kRangeMax) W->start[t] = t < 3 * nrun ? T.start[t] : 0;
+    if (t < kRangeMax) W->start[t] = ok && t < 3 * nrun ? T.start[t] : t == 0 ? T.first : 0;
     if (t <= kRangeMax) W->base[t] = ok ? T.base[t] : 0;
-    return ok;
+    return ok ? kWindow : far ? kFar : kNone;
+}
+
+// Which of the kAhead slots from j on (below e) are neighbours of a particle at xr, by the
+// positions x of the rebuild. Their loads overlap: such a row has hundreds of slots.
+constexpr int kAhead = 8;
+__device__ __forceinline__ uint32_t test_slots(const Inst<float> &I, const float2 &xr,
+                                               const float2 *x, int j, int e)
+{
+    float2 xj[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) xj[k] = x[j + k < e ? j + k : j];
+    uint32_t in = 0;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+        const float r2 = r2_exact<float>(sub_rn(xr.x, xj[k].x), sub_rn(xr.y, xj[k].y));
+        in |= (uint32_t)(j + k < e && lt_nonneg(I.r2min, r2) && lt_nonneg(r2, I.rc2)) << k;
+    }
+    return in;
+}
+
+// The candidate list of a particle in cell (cx, cy) by the test of its rows' rebuild
+// positions x (its own is xr), as for_each_neighbor takes it: entries off(slot), at most
+// maxnb of them; its length, or kNoList if it does not fit.
+template <typename Off>
+__device__ __forceinline__ int scan_list(const Inst<float> &I, int cx, int cy, const float2 &xr,
+                                         const float2 *x, const int32_t *cellStart, uint16_t *to,
+                                         Off &&off)
+{
+    const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
+    const int jx1 = cx + 1 < I.nx ? cx + 1 : I.nx;
+    int n = 0;
+#pragma unroll 1
+    for (int r = 0; r < 3; ++r) {
+        const int jy = cy + r - 1;
+        if (jy < 1 || jy > I.ny) continue;
+        const int row = I.coff + (jy - 1) * I.nx;
+        const int e = cellStart[row + jx1];
+        for (int j = cellStart[row + jx0 - 1]; j < e; j += kAhead) {
+            uint32_t in = test_slots(I, xr, x, j, e);
+            for (; in; in &= in - 1u) {
+                if (n >= I.maxnb) return n;
+                if (n == 4 * kQuads) return kNoList;
+                to[kTile * n++] = (uint16_t)off(r, j + __ffs((int)in) - 1);
+            }
+        }
+    }
+    return n;
 }
 
 // density_kernel! + eos_kernel! of one particle and its in-support list, from its n
-// candidates: cand(q) gives the q-th four offsets into the window sw (past the
-// last one, any of them). The list is collected at `place`, which may hold the
+// candidates: cand(q) gives the q-th four entries (past the last one, any of them). The list is collected at `place`, which may hold the
 // candidates: an entry is written behind those already read. The arithmetic of
-// density_pairs_f32, two candidates at a time.
-template <bool MULTI, typename Cand>
+// density_pairs_f32, two candidates at a time, or for a particle with spilled rows that
+// of density_spill_sum, which scales each pair's term.
+template <bool MULTI, typename Read, typename Cand>
 __device__ __forceinline__ void density_list(const NLView<float> &v, const WinLists &L, int tile,
-                                             int64_t i, const unsigned char *sw,
-                                             unsigned char *place, int n, Cand &&cand,
-                                             float *__restrict__ rho, float2 *__restrict__ prho)
+                                             int64_t i, const Read &rd, unsigned char *place, int n, bool spilled,
+                                             Cand &&cand, float *__restrict__ rho,
+                                             float2 *__restrict__ prho)
 {
     decltype(auto) I = load_inst<MULTI>(v, i);
     const float r2max = I.p.r2max, invh = I.p.invh, m = I.p.m, A = I.p.A;
@@ -272,7 +357,7 @@ __device__ __forceinline__ void density_list(const NLView<float> &v, const WinLi
         float2 xj[4];
         bool in[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) xj[k] = lds2(sw, entry_of(cur, k));
+        for (int k = 0; k < 4; ++k) xj[k] = rd.a(0, entry_of(cur, k));
 #pragma unroll
         for (int h = 0; h < 4; h += 2) {
             const float2 da = fsub2(xi, xj[h]);
@@ -299,18 +384,38 @@ __device__ __forceinline__ void density_list(const NLView<float> &v, const WinLi
             if (in[k]) ns += kRow;
         }
     };
-    uint2 e = n ? cand(0) : make_uint2(0u, 0u);
-    int q = 0;
-    for (; q < (n >> 2); ++q) {
-        const uint2 cur = e;
-        if (4 * q + 4 < n) e = cand(q + 1);
-        quad(cur, 4);
+    if (!spilled) {
+        uint2 e = n ? cand(0) : make_uint2(0u, 0u);
+        int q = 0;
+        for (; q < (n >> 2); ++q) {
+            const uint2 cur = e;
+            if (4 * q + 4 < n) e = cand(q + 1);
+            quad(cur, 4);
+        }
+        if (n & 3) quad(e, n & 3);
+        acc = mul_rn(mul_rn(m, A), acc);
+    } else {
+#pragma unroll 1
+        for (int q = 0; 4 * q < n; ++q) {
+            const uint2 cur = cand(q);
+#pragma unroll 1
+            for (int k = 0; k < 4 && 4 * q + k < n; ++k) {
+                const uint32_t o = entry_of(cur, k);
+                const float2 xj = rd.a(0, o);
+                const float dx = xi.x - xj.x;
+                const float dy = xi.y - xj.y;
+                const float r2 = dx * dx + dy * dy;
+                if (r2 < r2max) {
+                    acc += density_pair<float>(r2, invh, m, A);
+                    *reinterpret_cast<uint16_t *>(place + ns) = (uint16_t)o;
+                    ns += kRow;
+                }
+            }
+        }
     }
-    if (n & 3) quad(e, n & 3);
     ns /= kRow;
     write_list(place, ns, L.supp + lbase);
     L.suppCnt[i] = (uint8_t)ns;
-    acc = mul_rn(mul_rn(m, A), acc);
     density_finish<float>(I, i, acc, rho, prho);
 }
 
@@ -351,15 +456,40 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
     const int cx = cell_coord<float>(xi.x * I.invcs, nx);
     const int cy = cell_coord<float>(xi.y * I.invcs, ny);
     int run, nrun;
-    const bool ok = tile_window<MULTI>(T, one, inst, cellStart, live, b, cx, cy, L.win + tile, run,
-                                       nrun);
-    if (!ok) {
-        if (live) {
-            nl_build_one<float>(N, I, b, i, pos, cellStart, out.center, out.masks, out.nbcount,
-                                out.flags);
+    const int kind = tile_window<MULTI>(T, one, inst, cellStart, live, b, cx, cy, L.win + tile,
+                                        run, nrun);
+    unsigned char *const place = s_list + 2 * t;
+    uint2 *const list = L.cand + (int64_t)tile * (kQuads * kTile) + t;
+    // the density from the list just collected
+    auto density = [&](const auto &rd, int n, bool spilled) {
+        if constexpr (DENS) {
+            const uint16_t *p = reinterpret_cast<const uint16_t *>(place);
+            auto four = [&](int q) {
+                auto at = [&](int k) {
+                    return (uint32_t)p[(4 * q + k < n ? 4 * q + k : n - 1) * kTile];
+                };
+                return make_uint2(at(0) | at(1) << 16, at(2) | at(3) << 16);
+            };
+            density_list<MULTI>(*v, L, tile, i, rd, place, n, spilled, four, rho, prho);
+        }
+    };
+    if (kind != kWindow) {
+        if (!live) return;
+        nl_build_one<float>(N, I, b, i, pos, cellStart, out.center, out.masks, out.nbcount,
+                            out.flags);
+        int n = kNoList;
+        if (kind == kFar)
+            n = scan_list(I, cx, cy, xi, pos, cellStart, reinterpret_cast<uint16_t *>(place),
+                          [&](int, int j) { return j - T.first; });
+        if (n == kNoList) {
             L.candCnt[i] = kNoList;
             walk(i);
+            return;
         }
+        const bool spilled = out.center[i] >> 31;
+        write_list(place, n, list);
+        L.candCnt[i] = (uint8_t)(spilled ? n | kSpilled : n);
+        density(InMemory{pos + T.first, nullptr, nullptr, nullptr, nullptr}, n, spilled);
         return;
     }
     const int total = T.base[32];
@@ -374,7 +504,6 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
     const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
     const int jx1 = cx + 1 < nx ? cx + 1 : nx;
     const float rc2 = I.rc2, r2min = I.r2min;
-    unsigned char *const place = s_list + 2 * t;
     unsigned char *const full = place + 4 * kQuads * kRow;
     unsigned char *to = place; // the list's end; held at `full` once it is reached
     uint32_t spill = 0;
@@ -448,21 +577,14 @@ __device__ __forceinline__ void nl_window(int64_t N, const Inst<float> &one,
     const int n = all < maxnb ? all : maxnb;
     out.center[i] = (uint32_t)cx | ((uint32_t)cy << 16) | (spill << 31);
     out.nbcount[i] = n;
-    if (spill || n > 4 * kQuads) {
+    if (n > 4 * kQuads) {
         L.candCnt[i] = kNoList;
         walk(i);
         return;
     }
-    write_list(place, n, L.cand + (int64_t)tile * (kQuads * kTile) + t);
-    L.candCnt[i] = (uint8_t)n;
-    if constexpr (DENS) {
-        const uint16_t *p = reinterpret_cast<const uint16_t *>(place);
-        auto four = [&](int q) {
-            auto at = [&](int k) { return (uint32_t)p[(4 * q + k < n ? 4 * q + k : n - 1) * kTile]; };
-            return make_uint2(at(0) | at(1) << 16, at(2) | at(3) << 16);
-        };
-        density_list<MULTI>(*v, L, tile, i, s_win, place, n, four, rho, prho);
-    }
+    write_list(place, n, list);
+    L.candCnt[i] = (uint8_t)(spill ? n | kSpilled : n);
+    density(InWindow{s_win}, n, spill != 0);
 }
 
 template <bool MULTI>
@@ -504,10 +626,10 @@ __device__ __forceinline__ void window_lists(const NLView<float> &v, const WinLi
     const int cy = (int)((cc >> 16) & 0x7fffu);
     const int b = MULTI && live ? (int)v.pinst[i] : 0;
     int run, nrun;
-    const bool ok = tile_window<MULTI>(T, v.one, v.inst, v.cellStart, live, b, cx, cy,
-                                       L.win + tile, run, nrun);
+    const int kind = tile_window<MULTI>(T, v.one, v.inst, v.cellStart, live, b, cx, cy,
+                                        L.win + tile, run, nrun);
     if (!live) return;
-    if (!ok || (cc >> 31)) {
+    if (kind == kNone) {
         L.candCnt[i] = kNoList;
         return;
     }
@@ -516,6 +638,18 @@ __device__ __forceinline__ void window_lists(const NLView<float> &v, const WinLi
     const int jx0 = cx - 1 > 1 ? cx - 1 : 1;
     const int row0 = I.coff + (jx0 - 1) + (cy - 2) * I.nx;
     unsigned char *const place = s_list + 2 * t;
+    uint2 *const list = L.cand + (int64_t)tile * (kQuads * kTile) + t;
+    if (kind == kFar || (cc >> 31)) { // no window, or rows beyond the masks
+        const int n = scan_list(I, cx, cy, v.xref[i], v.xref, v.cellStart,
+                                reinterpret_cast<uint16_t *>(place), [&](int r, int j) {
+                                    return kind == kFar ? j - T.first
+                                                        : 8 * (T.base[3 * run + r] + j -
+                                                               T.start[3 * run + r]);
+                                });
+        if (n != kNoList) write_list(place, n, list);
+        L.candCnt[i] = (uint8_t)(n != kNoList && (cc >> 31) ? n | kSpilled : n);
+        return;
+    }
     uint64_t m[3];
     int off[3];
     int n = 0;
@@ -547,7 +681,7 @@ __device__ __forceinline__ void window_lists(const NLView<float> &v, const WinLi
         *to = (uint16_t)(base + 8 * k);
         to += kTile;
     }
-    write_list(place, n, L.cand + (int64_t)tile * (kQuads * kTile) + t);
+    write_list(place, n, list);
     L.candCnt[i] = (uint8_t)n;
 }
 
@@ -571,17 +705,27 @@ __device__ __forceinline__ void density_window(const NLView<float> &v, const Win
     const int64_t i = (int64_t)tile * kTile + t;
     const bool live = i < v.N;
     const unsigned char *sw = s_win;
-    const int n = live ? (int)L.candCnt[i] : 0;
-    stage_window<1, false>(L.win + tile, sw, v.pos, nullptr, nullptr, nullptr, nullptr);
+    const int c = live ? (int)L.candCnt[i] : 0;
+    const int nr =
+        stage_window<1, false>(L.win + tile, sw, v.pos, nullptr, nullptr, nullptr, nullptr);
     if (!live) return;
-    if (n == kNoList) {
+    if (c == kNoList) {
         L.suppCnt[i] = kNoList;
         density_walk<float, MULTI, true>(v, i, rho, prho, nullptr);
         return;
     }
-    const uint2 *c = L.cand + (int64_t)tile * (kQuads * kTile) + t;
-    density_list<MULTI>(v, L, tile, i, sw, s_list + 2 * t, n, [&](int q) { return c[q * kTile]; },
-                        rho, prho);
+    const uint2 *list = L.cand + (int64_t)tile * (kQuads * kTile) + t;
+    const auto cand = [&](int q) { return list[q * kTile]; };
+    const int n = c & (kSpilled - 1);
+    const bool spilled = (c & kSpilled) != 0;
+    unsigned char *const place = s_list + 2 * t;
+    if (nr)
+        density_list<MULTI>(v, L, tile, i, InWindow{sw}, place, n, spilled, cand, rho, prho);
+    else
+        density_list<MULTI>(v, L, tile, i,
+                            InMemory{v.pos + L.win[tile].start[0], nullptr, nullptr, nullptr,
+                                     nullptr},
+                            place, n, spilled, cand, rho, prho);
 }
 
 template <bool MULTI>
@@ -611,10 +755,10 @@ __device__ __forceinline__ void for_each_entry(const uint2 *__restrict__ list, i
         if (k < (n & 3)) f(entry_of(e, k));
 }
 
-// Pressure + viscosity sum of accel_sum over the staged window: positions,
-// velocities, {p/rho^2, 1/rho} (and densities for the artificial viscosity).
-template <bool AV>
-__device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsigned char *sw,
+// Pressure + viscosity sum of accel_sum over a list: positions, velocities,
+// {p/rho^2, 1/rho} (and densities for the artificial viscosity).
+template <bool AV, typename Read>
+__device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const Read &rd,
                                               const uint2 *__restrict__ list, int n,
                                               const float2 &xi, const float2 &vi,
                                               const float2 &pi, float rhoi, float &ax, float &ay)
@@ -628,9 +772,9 @@ __device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsign
         const float tmm = vc.twomumass;
         float2 acc = make_float2(0.0f, 0.0f);
         for_each_entry(list, n, [&](uint32_t o) {
-            const float2 xj = lds2(sw, o);
-            const float2 vj = lds2(sw + kWin8, o);
-            const float2 pj = lds2(sw + 2 * kWin8, o);
+            const float2 xj = rd.a(0, o);
+            const float2 vj = rd.a(1, o);
+            const float2 pj = rd.a(2, o);
             const float2 d = fsub2(xi, xj);
             const float r2 = d.x * d.x + d.y * d.y;
             const float q = pair_sqrt(r2) * invh;
@@ -647,10 +791,10 @@ __device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsign
         ax = 0.0f;
         ay = 0.0f;
         for_each_entry(list, n, [&](uint32_t o) {
-            const float2 xj = lds2(sw, o);
-            const float2 vj = lds2(sw + kWin8, o);
-            const float2 pj = lds2(sw + 2 * kWin8, o);
-            const float rhoj = lds1(sw + 3 * kWin8, o >> 1);
+            const float2 xj = rd.a(0, o);
+            const float2 vj = rd.a(1, o);
+            const float2 pj = rd.a(2, o);
+            const float rhoj = rd.template f<3>(o);
             const float dx = xi.x - xj.x;
             const float dy = xi.y - xj.y;
             const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
@@ -659,10 +803,11 @@ __device__ __forceinline__ void accel_sum_win(const Inst<float> &I, const unsign
     }
 }
 
-// The sum of particle i of a tile: its list, or the mask walk of a marked one.
+// The sum of particle i of a tile: its list (nr: ranges of the tile's window), or the mask
+// walk of a marked one.
 template <bool MULTI, bool AV>
 __device__ __forceinline__ void accel_any(const NLView<float> &v, const WinLists &L, int tile,
-                                          const unsigned char *sw, int64_t i, const Inst<float> &I,
+                                          const unsigned char *sw, int nr, int64_t i, const Inst<float> &I,
                                           const float2 *__restrict__ vel,
                                           const float2 *__restrict__ prho,
                                           const float *__restrict__ rho, const float2 &xi,
@@ -674,8 +819,14 @@ __device__ __forceinline__ void accel_any(const NLView<float> &v, const WinLists
         return;
     }
     const float rhoi = AV && I.p.visc == 1 ? rho[i] : 0.0f;
-    accel_sum_win<AV>(I, sw, L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n, xi, vi,
-                      prho[i], rhoi, ax, ay);
+    const uint2 *list = L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x;
+    if (nr) {
+        accel_sum_win<AV>(I, InWindow{sw}, list, n, xi, vi, prho[i], rhoi, ax, ay);
+    } else {
+        const int f = L.win[tile].start[0];
+        accel_sum_win<AV>(I, InMemory{v.pos + f, vel + f, prho + f, nullptr, AV ? rho + f : nullptr},
+                          list, n, xi, vi, prho[i], rhoi, ax, ay);
+    }
 }
 
 template <bool AV> constexpr int kAccelSmem = 3 * kWin8 + (AV ? kWin4 : 0);
@@ -694,7 +845,7 @@ __global__ void __launch_bounds__(kTile, AV ? 1 : 12)
     pdl_enter();
     __shared__ __align__(16) unsigned char s_win[kAccelSmem<AV>];
     const unsigned char *sw = s_win;
-    stage_window<3, AV>(L.win + blockIdx.x, sw, v.pos, vel, prho, nullptr, rho);
+    const int nr = stage_window<3, AV>(L.win + blockIdx.x, sw, v.pos, vel, prho, nullptr, rho);
     const int64_t i = (int64_t)blockIdx.x * kTile + threadIdx.x;
     if (i >= v.N) return;
     const int b = MULTI ? inst_of(v, i) : 0;
@@ -702,7 +853,7 @@ __global__ void __launch_bounds__(kTile, AV ? 1 : 12)
     const float2 xi = v.pos[i];
     const float2 vi = vel[i];
     float ax, ay;
-    accel_any<MULTI, AV>(v, L, (int)blockIdx.x, sw, i, I, vel, prho, rho, xi, vi, ax, ay);
+    accel_any<MULTI, AV>(v, L, (int)blockIdx.x, sw, nr, i, I, vel, prho, rho, xi, vi, ax, ay);
     accel_integrate_finish<float>(I, b, i, xi, vi, ax, ay, theta, posOut, velOut, aOut, alphaOut,
                                   flags, perm, tx, tv);
 }
@@ -731,7 +882,7 @@ __global__ void __launch_bounds__(kTile, AV ? 1 : 12)
     pdl_enter();
     __shared__ __align__(16) unsigned char s_win[kAccelSmem<AV>];
     const unsigned char *sw = s_win;
-    stage_window<3, AV>(L.win + blockIdx.x, sw, v.pos, vel, prho, nullptr, rho);
+    const int nr = stage_window<3, AV>(L.win + blockIdx.x, sw, v.pos, vel, prho, nullptr, rho);
     const int64_t i = (int64_t)blockIdx.x * kTile + threadIdx.x;
     const bool live = i < v.N;
     int e = INT_MIN, b = 0;
@@ -741,16 +892,16 @@ __global__ void __launch_bounds__(kTile, AV ? 1 : 12)
         const float2 xi = v.pos[i];
         const float2 vi = vel[i];
         float ax, ay;
-        accel_any<MULTI, AV>(v, L, (int)blockIdx.x, sw, i, I, vel, prho, rho, xi, vi, ax, ay);
+        accel_any<MULTI, AV>(v, L, (int)blockIdx.x, sw, nr, i, I, vel, prho, rho, xi, vi, ax, ay);
         e = drag_adj_finish<float>(I, i, xi, vi, ax, ay, theta, gX, gV, abar, galpha);
     }
     warp_emax(live, b, e, emax, parity, MULTI);
 }
 
-// The pair sums of pass1_sum over the staged window: positions, velocities,
-// {p/rho^2, 1/rho}, abar (and densities).
-template <bool AV>
-__device__ __forceinline__ void pass1_sum_win(const Inst<float> &I, const unsigned char *sw,
+// The pair sums of pass1_sum over a list: positions, velocities, {p/rho^2, 1/rho}, abar
+// (and densities).
+template <bool AV, typename Read>
+__device__ __forceinline__ void pass1_sum_win(const Inst<float> &I, const Read &rd,
                                               const uint2 *__restrict__ list, int n,
                                               const float2 &xi, const float2 &vi,
                                               const float2 &ab, const float2 &pi, float rhoi,
@@ -765,10 +916,10 @@ __device__ __forceinline__ void pass1_sum_win(const Inst<float> &I, const unsign
         float2 g = make_float2(0.0f, 0.0f), gv = make_float2(0.0f, 0.0f);
         float gr = 0.0f, sS = 0.0f;
         for_each_entry(list, n, [&](uint32_t o) {
-            const float2 xj = lds2(sw, o);
-            const float2 vj = lds2(sw + kWin8, o);
-            const float2 pj = lds2(sw + 2 * kWin8, o);
-            const float2 abj = lds2(sw + 3 * kWin8, o);
+            const float2 xj = rd.a(0, o);
+            const float2 vj = rd.a(1, o);
+            const float2 pj = rd.a(2, o);
+            const float2 abj = rd.a(3, o);
             const float2 d = fsub2(xi, xj);
             const float r2 = d.x * d.x + d.y * d.y;
             const float rinv = r2 > 0.0f ? rsqrtf(r2) : 0.0f;
@@ -802,11 +953,11 @@ __device__ __forceinline__ void pass1_sum_win(const Inst<float> &I, const unsign
         vc.kind = 1;
         gx = 0, gy = 0, gvx = 0, gvy = 0, grh = 0, sumS = 0;
         for_each_entry(list, n, [&](uint32_t o) {
-            const float2 xj = lds2(sw, o);
-            const float2 vj = lds2(sw + kWin8, o);
-            const float2 pj = lds2(sw + 2 * kWin8, o);
-            const float2 abj = lds2(sw + 3 * kWin8, o);
-            const float rhoj = lds1(sw + 4 * kWin8, o >> 1);
+            const float2 xj = rd.a(0, o);
+            const float2 vj = rd.a(1, o);
+            const float2 pj = rd.a(2, o);
+            const float2 abj = rd.a(3, o);
+            const float rhoj = rd.template f<4>(o);
             const float dx = xi.x - xj.x;
             const float dy = xi.y - xj.y;
             const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
@@ -837,7 +988,8 @@ __device__ __forceinline__ void pass1_window(const NLView<float> &v, const WinLi
                                              float2 *__restrict__ gXs, float *__restrict__ grho,
                                              float2 *__restrict__ gV)
 {
-    if (L.win) stage_window<4, AV>(L.win + tile, sw, v.pos, vel, prho, abar, rho);
+    int nr = 0;
+    if (L.win) nr = stage_window<4, AV>(L.win + tile, sw, v.pos, vel, prho, abar, rho);
     const int64_t i = (int64_t)tile * kTile + threadIdx.x;
     if (i >= v.N) return;
     decltype(auto) I = load_inst<MULTI>(v, i);
@@ -850,9 +1002,19 @@ __device__ __forceinline__ void pass1_window(const NLView<float> &v, const WinLi
     if (n == kNoList)
         pass1_sum<float, AV>(v, I, i, vel, prho, rho, abar, xi, vi, ab, pi, gx, gy, gvx, gvy, grh,
                              sumS);
-    else
-        pass1_sum_win<AV>(I, sw, L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n, xi, vi,
-                          ab, pi, AV && I.p.visc == 1 ? rho[i] : 0.0f, gx, gy, gvx, gvy, grh, sumS);
+    else {
+        const uint2 *list = L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x;
+        const float r = AV && I.p.visc == 1 ? rho[i] : 0.0f;
+        if (nr) {
+            pass1_sum_win<AV>(I, InWindow{sw}, list, n, xi, vi, ab, pi, r, gx, gy, gvx, gvy, grh,
+                              sumS);
+        } else {
+            const int f = L.win[tile].start[0];
+            pass1_sum_win<AV>(I, InMemory{v.pos + f, vel + f, prho + f, abar + f,
+                                          AV ? rho + f : nullptr},
+                              list, n, xi, vi, ab, pi, r, gx, gy, gvx, gvy, grh, sumS);
+        }
+    }
     const float rhoi = I.p.eos == 1 || (AV && I.p.visc == 1) ? rho[i] : 0.0f;
     pass1_finish<float>(I, i, xi, ab, pi, rhoi, gx, gy, gvx, gvy, grh, sumS, theta, galpha, gXs,
                         grho, gV);
@@ -883,7 +1045,8 @@ __device__ __forceinline__ void pass2_window(const NLView<float> &v, const WinLi
                                              const int *__restrict__ emax, int parity,
                                              unsigned long long *__restrict__ thetaAcc)
 {
-    if (L.win) stage_window<1, true>(L.win + tile, sw, v.pos, nullptr, nullptr, nullptr, grho);
+    int nr = 0;
+    if (L.win) nr = stage_window<1, true>(L.win + tile, sw, v.pos, nullptr, nullptr, nullptr, grho);
     const int64_t i = (int64_t)tile * kTile + threadIdx.x;
     const bool live = i < v.N;
     const int64_t s = live ? i : v.N - 1;
@@ -899,15 +1062,23 @@ __device__ __forceinline__ void pass2_window(const NLView<float> &v, const WinLi
             const float invh = I.p.invh, m = I.p.m, Fc = I.p.Fc;
             const float gri = grho[i];
             float2 acc = make_float2(0.0f, 0.0f);
-            for_each_entry(L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n,
-                           [&](uint32_t o) {
-                               const float2 xj = lds2(sw, o);
-                               const float grj = lds1(sw + kWin8, o >> 1);
-                               const float2 d = fsub2(xi, xj);
-                               const float r2 = d.x * d.x + d.y * d.y;
-                               const float w = pass2_weight<float>(r2, invh, m, Fc, gri, grj);
-                               acc = ffma2(make_float2(w, w), d, acc);
-                           });
+            const auto sum = [&](const auto &rd) {
+                for_each_entry(L.supp + (int64_t)tile * (kQuads * kTile) + threadIdx.x, n,
+                               [&](uint32_t o) {
+                                   const float2 xj = rd.a(0, o);
+                                   const float grj = rd.template f<1>(o);
+                                   const float2 d = fsub2(xi, xj);
+                                   const float r2 = d.x * d.x + d.y * d.y;
+                                   const float w = pass2_weight<float>(r2, invh, m, Fc, gri, grj);
+                                   acc = ffma2(make_float2(w, w), d, acc);
+                               });
+            };
+            if (nr) {
+                sum(InWindow{sw});
+            } else {
+                const int f = L.win[tile].start[0];
+                sum(InMemory{v.pos + f, nullptr, nullptr, nullptr, grho + f});
+            }
             gx = acc.x;
             gy = acc.y;
         }

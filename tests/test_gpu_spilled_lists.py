@@ -1,6 +1,7 @@
 """FP32 tiles: particles whose cell rows exceed the 64-slot masks but whose neighbours fit a
 list (what a column that presses through a wall leaves in the border cells: everything beyond
-a wall is clamped into them) take lists like the others, with the bits of the mask walks:
+a wall is clamped into them) take lists like the others, with the bits of the mask walks, also
+in tiles whose window is too large to be staged (lists of slots, up to a span of 16 bits):
 from a fresh cell list, from restored snapshots, with rows cut at maxnb, in batches, with the
 model variants and in the packed server."""
 import numpy as np
@@ -16,11 +17,11 @@ S = pytest.importorskip("sphadjoint_gb300")
 SKIN = 0.2
 
 
-def beyond(nx, ny, inside, model=None):
+def beyond(nx, ny, inside, model=None, hfac=1.3):
     """A block of which `inside` columns are in the tank and the rest beyond its right wall."""
     dx = 0.01
     p = K.dambreak_params(dx=dx, col_h=ny * dx, Lx=(inside + 0.5) * dx, Ly=1.25 * ny * dx)
-    p.update(kw=0.5, **(model or {}))
+    p.update(kw=0.5, h=hfac * dx, **(model or {}))
     rng = np.random.default_rng(nx * 31 + ny)
     X0 = K.lattice_block(nx, ny, dx, dx, dx, 0.05 * dx, rng)
     return dict(p=p, X0=X0, V0=0.05 * rng.standard_normal(X0.shape),
@@ -50,6 +51,9 @@ CASES = {
     "restored": (lambda: beyond(60, 30, 25), 15, 4, 64, 3),
     "cut-at-maxnb": (lambda: beyond(60, 30, 25), 6, 2, 20, 0),
     "restored-cut-at-maxnb": (lambda: beyond(60, 30, 25), 15, 4, 20, 3),
+    "wide": (lambda: beyond(200, 18, 4), 5, 2, 64, 0),           # no tile has a window
+    "wide-restored": (lambda: beyond(120, 24, 4), 15, 4, 64, 3),
+    "too-long-for-a-list": (lambda: beyond(60, 30, 25, hfac=1.75), 5, 2, 64, 0),
     "tait-av": (lambda: beyond(60, 30, 25, TAIT_AV), 6, 3, 64, 0),
     "tait-av-restored": (lambda: beyond(61, 30, 25, TAIT_AV), 15, 4, 64, 3),
 }
@@ -68,7 +72,7 @@ def test_lists_of_spilled_rows_equal_the_mask_walks(forms, name):
     make, n, interval, maxnb, snapshots = CASES[name]
     case = make()
     rows, most = spilled(case)
-    assert rows > 300 and most <= 48
+    assert rows > 300 and (most <= 48) == (name != "too-long-for-a-list")
     out = {}
     for f in ("mask", "pairs"):
         forms(f)
@@ -76,6 +80,17 @@ def test_lists_of_spilled_rows_equal_the_mask_walks(forms, name):
                          maxnb=maxnb, snapshots=snapshots)
     assert out["mask"]["flags"] == out["pairs"]["flags"]
     assert np.all(np.isfinite(out["pairs"]["gX"]))
+    for k in ("X", "V", "gX", "gV", "gtheta"):
+        assert np.array_equal(out["pairs"][k], out["mask"][k]), k
+
+
+def test_rows_that_span_more_than_16_bits(forms):
+    """Three rows of 22,200 slots: neither a window nor 16-bit slots."""
+    case = beyond(7400, 9, 3)
+    out = {}
+    for f in ("mask", "pairs"):
+        forms(f)
+        out[f] = run_gpu(case, 2, dtype="f32", seeds=linear_seeds(case), interval=2)
     for k in ("X", "V", "gX", "gV", "gtheta"):
         assert np.array_equal(out["pairs"][k], out["mask"][k]), k
 
