@@ -369,6 +369,7 @@ template <typename T> class Sys final : public StateI {
     bool listsFresh = false; // they belong to the masks the state holds,
     uint64_t listsIn = 0;    // made by this recording's launches (rt_recording)
     StepGraphs graphs;   // simulate's steps, replayed in groups
+    bool listsFit = true; // FP32 lists hold the neighbours of most particles
     bool anyRho = false; // some instance's model reads densities in the adjoint
     bool anyAV = false;  // some instance uses the artificial viscosity
 
@@ -438,6 +439,9 @@ template <typename T> class Sys final : public StateI {
         N_ = off;
         ncell = coff;
         nnode = toff;
+        int64_t over = 0;
+        for (int b = 0; b < B; ++b) over += list_fits(ps[b], o) ? 0 : ns[b];
+        listsFit = 2 * over <= N_;
         for (const Params &q : ps) {
             anyRho = anyRho || needs_rho(q);
             anyAV = anyAV || q.visc == 1;
@@ -556,11 +560,21 @@ template <typename T> class Sys final : public StateI {
     // and not while the stream is recorded, by anyone (the buffers would belong to
     // that graph); a state without them gives the same
     // results. Beyond 2^25 particles they would hold 6.6 GB a state.
+    // A list holds 48 candidates (sph_window.cuh), and a particle with more walks its masks
+    // inside the tile, which is slower than the mask-walk kernels: 90,000 particles, 16
+    // steps with gradient, mask walks -> tiles: h = 1.6 spacings (44 candidates) 2.18 ->
+    // 1.41 ms, 1.66 2.20 -> 2.06, 1.68 2.23 -> 2.35, 1.75 2.34 -> 2.89. So tiles are for
+    // states whose instances at rest expect at most 49 (1.66), for half of their particles.
     static constexpr int64_t kListMaxN = int64_t(1) << 25;
+    static bool list_fits(const Params &p, const NLOpts &o)
+    {
+        const double rc = 2.0 * p.h * (1.0 + o.skin);
+        return 3.141592653589793 * rc * rc * p.rho0 <= (49.0 + 1.0) * p.m; // itself among them
+    }
     bool want_tiles() const
     {
-        return sizeof(T) == 4 && N_ > 0 && N_ <= kListMaxN && group_lanes(rt_group_lanes()) == 0 &&
-               rt_density_form() == 2;
+        return sizeof(T) == 4 && N_ > 0 && N_ <= kListMaxN && listsFit &&
+               group_lanes(rt_group_lanes()) == 0 && rt_density_form() == 2;
     }
     // FP64 states without artificial viscosity run them one lane per pair
     // (sph_flat.cuh), unless a lane setting is forced; their pair lists (about
@@ -614,12 +628,12 @@ template <typename T> class Sys final : public StateI {
     }
     // What a state of N particles takes for them at the present settings (the packed
     // engine runs every FP32 request on tiles, and no pairs).
-    static int64_t list_bytes(const Params &p, int64_t N, bool packed)
+    static int64_t list_bytes(const Params &p, int64_t N, const NLOpts &o, bool packed)
     {
         const int set = rt_group_lanes();
         if (N <= 0) return 0;
         if (sizeof(T) == 4)
-            return N <= kListMaxN && (packed || lanes_of(set, N, 1) == 0)
+            return N <= kListMaxN && list_fits(p, o) && (packed || lanes_of(set, N, 1) == 0)
                        ? (int64_t)parts_bytes(tile_parts(N))
                        : 0;
         return !packed && set == 0 && p.visc != 1 && N <= kFlatMaxN
@@ -669,7 +683,7 @@ template <typename T> class Sys final : public StateI {
     }
     void alloc_lists()
     {
-        if (sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN || !may_ask()) return;
+        if (sizeof(T) != 4 || N_ == 0 || N_ > kListMaxN || !listsFit || !may_ask()) return;
         carve_scratch(tile_parts(N_), wcand, wsupp, wcnt, wwin);
     }
     WinLists lists() const

@@ -21,9 +21,9 @@ WorkI *make_work_f32(const std::vector<Params> &p, const std::vector<int64_t> &N
     return new Work<float>(p, N);
 }
 PackI *make_pack_f32() { return new Packer<float>(); }
-int64_t list_bytes_f32(const Params &p, int64_t N, bool packed)
+int64_t list_bytes_f32(const Params &p, int64_t N, const NLOpts &o, bool packed)
 {
-    return Sys<float>::list_bytes(p, N, packed);
+    return Sys<float>::list_bytes(p, N, o, packed);
 }
 
 } // namespace sphgb

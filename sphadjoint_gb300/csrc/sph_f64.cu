@@ -23,9 +23,9 @@ WorkI *make_work_f64(const std::vector<Params> &p, const std::vector<int64_t> &N
     return new Work<double>(p, N);
 }
 PackI *make_pack_f64() { return new Packer<double>(); }
-int64_t list_bytes_f64(const Params &p, int64_t N, bool packed)
+int64_t list_bytes_f64(const Params &p, int64_t N, const NLOpts &o, bool packed)
 {
-    return Sys<double>::list_bytes(p, N, packed);
+    return Sys<double>::list_bytes(p, N, o, packed);
 }
 
 } // namespace sphgb

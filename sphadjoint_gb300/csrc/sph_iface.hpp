@@ -293,7 +293,7 @@ class PackI {
                             const void *X0, const void *V0, NLOpts o);                       \
     WorkI *make_work##SFX(const std::vector<Params> &p, const std::vector<int64_t> &N);       \
     PackI *make_pack##SFX();                                                                 \
-    int64_t list_bytes##SFX(const Params &p, int64_t N, bool packed);
+    int64_t list_bytes##SFX(const Params &p, int64_t N, const NLOpts &o, bool packed);
 
 SPH_DECLARE_FACTORIES(_f32)
 SPH_DECLARE_FACTORIES(_f64)

@@ -128,7 +128,9 @@ class Server {
     int64_t state_lists(const sph_request &r, bool packed) const
     {
         const Params p = params_of(r.p);
-        return dtype_ == SPH_F64 ? list_bytes_f64(p, r.N, packed) : list_bytes_f32(p, r.N, packed);
+        const NLOpts o{r.skin, r.interval, r.maxnb};
+        return dtype_ == SPH_F64 ? list_bytes_f64(p, r.N, o, packed)
+                                 : list_bytes_f32(p, r.N, o, packed);
     }
 
     int64_t submit(const sph_request &r0)

@@ -17,13 +17,15 @@ S = pytest.importorskip("sphadjoint_gb300")
 SKIN = 0.2
 
 
-def beyond(nx, ny, inside, model=None, hfac=1.3):
-    """A block of which `inside` columns are in the tank and the rest beyond its right wall."""
+def beyond(nx, ny, inside, model=None, crowd=0):
+    """A block of which `inside` columns are in the tank and the rest beyond its right wall;
+    the first `crowd` particles are within half a spacing's distance of each other."""
     dx = 0.01
     p = K.dambreak_params(dx=dx, col_h=ny * dx, Lx=(inside + 0.5) * dx, Ly=1.25 * ny * dx)
-    p.update(kw=0.5, h=hfac * dx, **(model or {}))
+    p.update(kw=0.5, **(model or {}))
     rng = np.random.default_rng(nx * 31 + ny)
     X0 = K.lattice_block(nx, ny, dx, dx, dx, 0.05 * dx, rng)
+    X0[:, :crowd] = X0[:, :1] + 0.5 * dx * rng.random((2, crowd))
     return dict(p=p, X0=X0, V0=0.05 * rng.standard_normal(X0.shape),
                 theta=20.0 * rng.random((p["ngy"], p["ngx"])),
                 cX=rng.standard_normal(X0.shape), cV=rng.standard_normal(X0.shape))
@@ -53,7 +55,7 @@ CASES = {
     "restored-cut-at-maxnb": (lambda: beyond(60, 30, 25), 15, 4, 20, 3),
     "wide": (lambda: beyond(200, 18, 4), 5, 2, 64, 0),           # no tile has a window
     "wide-restored": (lambda: beyond(120, 24, 4), 15, 4, 64, 3),
-    "too-long-for-a-list": (lambda: beyond(60, 30, 25, hfac=1.75), 5, 2, 64, 0),
+    "too-long-for-a-list": (lambda: beyond(60, 30, 25, crowd=60), 4, 2, 90, 0),
     "tait-av": (lambda: beyond(60, 30, 25, TAIT_AV), 6, 3, 64, 0),
     "tait-av-restored": (lambda: beyond(61, 30, 25, TAIT_AV), 15, 4, 64, 3),
 }

@@ -28,5 +28,5 @@ def test_no_process_wide_flag_beside_kernel_attributes():
         with open(os.path.join(CSRC, name)) as f:
             text = f.read()
         if "cudaFuncSetAttribute" in text:
-            assert not re.search(r"\bstatic bool\b", text), name
+            assert not re.search(r"\bstatic bool \w+ *[=;]", text), name
             assert "OncePerDevice" in text, name
