@@ -42,28 +42,30 @@ TUNE_STEPS = 32
 # ncu dram__bytes.sum.per_second times the duration of one launch at 1,048,576
 # particles, FP32 (the captures summarised in profiles/k_*_win_1M_fp32.md)
 TRAFFIC_1M_F32 = {
-    "density": 2.220966e12 * 42.528e-6,
-    "accel_integrate": 1.610723e12 * 45.408e-6,
-    "accel_drag": 2.029740e12 * 45.536e-6,
-    "pass1": 1.692239e12 * 58.272e-6,
-    "pass2": 2.444277e12 * 32.864e-6,
+    "density": 2.257210e12 * 41.888e-6,
+    "build_density": 0.944795e12 * 108.864e-6,
+    "accel_integrate": 1.602263e12 * 45.824e-6,
+    "accel_drag": 2.019603e12 * 46.048e-6,
+    "pass1": 1.628691e12 * 60.416e-6,
+    "pass2": 2.377234e12 * 33.824e-6,
 }
 
 # smsp__issue_active.avg.pct_of_peak_sustained_active of the same captures:
 # the fraction of cycles in which a warp scheduler issued; with the shared-memory
-# wavefronts (60 to 77% of their rate) the bound these kernels meet (HBM throughput
-# stays at 20 to 31%)
+# wavefronts (63 to 75% of their rate) the bound these kernels meet (HBM throughput
+# stays at 12 to 30%)
 ISSUE_ACTIVE_1M_F32 = {
-    "density": 0.6652, "accel_integrate": 0.5616, "accel_drag": 0.5639,
-    "pass1": 0.7156, "pass2": 0.6899,
+    "density": 0.6675, "build_density": 0.7662, "accel_integrate": 0.5648, "accel_drag": 0.5710,
+    "pass1": 0.6840, "pass2": 0.6887,
 }
 
 # lts__throughput.avg.pct_of_peak_sustained_elapsed and
 # l1tex__throughput.avg.pct_of_peak_sustained_active of the same captures (the
 # latter holds the shared memory)
 L2_L1_FRAC_1M_F32 = {
-    "density": (0.1780, 0.7866), "accel_integrate": (0.1603, 0.8508),
-    "accel_drag": (0.1869, 0.8424), "pass1": (0.1682, 0.8358), "pass2": (0.2057, 0.7245),
+    "density": (0.1815, 0.7967), "build_density": (0.1380, 0.7899),
+    "accel_integrate": (0.1596, 0.8451), "accel_drag": (0.1860, 0.8502),
+    "pass1": (0.1594, 0.8018), "pass2": (0.2105, 0.7387),
 }
 
 # algorithmic HBM bytes per particle per launch (compulsory traffic of the

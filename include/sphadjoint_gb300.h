@@ -355,8 +355,11 @@ SPH_API int32_t sph_build_cells_noalloc(const void *X_dev, int64_t N, int32_t dt
    per block on this state's current positions (reps launches each) and uses
    the fastest from then on for every object of the same precision and kind
    (single or batched). blocks[6] (may be NULL) receives the choices in that
-   order. Runs on the state's own arrays and a temporary workspace; the state's
-   positions and velocities are not changed. */
+   order. These are the kernels of the mask walks with one thread per particle;
+   lane groups, the tiles of FP32 states and the pairs of FP64 states have
+   fixed sizes (FP64 pairs beyond 2432 particles use the tuned list build).
+   Runs on the state's own arrays and a temporary workspace; the state's
+   positions, velocities and neighbour rows are not changed. */
 SPH_API int32_t sph_autotune(sph_state st, sph_field theta, int32_t reps, int32_t *blocks);
 /* Set or read the six block sizes directly (same order; each 64, 128 or 256,
    else SPH_ERR_ARG), for this state's precision and kind. A caller can time
@@ -368,26 +371,32 @@ SPH_API int32_t sph_set_block_sizes(sph_state st, const int32_t *blocks);
 SPH_API int32_t sph_get_block_sizes(sph_state st, int32_t *blocks);
 
 /* Lanes per particle of the neighbour-list and pair-sum kernels (no
-   counterpart in the reference), process-wide. 0 (default): by state size --
-   single states of up to 16384 particles give each particle a group of 32
-   lanes (up to 512 particles in FP64, 2048 in FP32) or 16 lanes, larger
-   states one thread. 1: always one thread. 16 or 32: groups for every
-   single-instance state. Every setting adds each particle's pair terms in the
-   same order, so FP64 results are bit-identical across settings; FP32 results
-   may differ in the last bits (multiply-add contraction differs between the
-   forms). Batches always use one thread per particle, so an FP32 batch member
-   equals a solo run made with lanes = 1. Other values: SPH_ERR_ARG. */
+   counterpart in the reference), process-wide; a step reads it once. 0
+   (default): by state. FP64 states and batches with the Morris viscosity, up
+   to 2^22 particles, run one lane per pair where the scratch for the pair
+   lists is free (about 1290 bytes a particle). Otherwise single states of up
+   to 16384 particles give each particle a group of 32 lanes (up to 512
+   particles in FP64, 2048 in FP32) or 16 lanes, larger states and batches one
+   thread (FP32: see sph_set_density_form). 1: always one thread. 16 or 32:
+   groups for every single-instance state. Every setting adds each particle's
+   pair terms in the same order, so FP64 results are bit-identical across
+   settings; FP32 results may differ in the last bits between groups and one
+   thread (multiply-add contraction differs), so an FP32 batch member equals a
+   solo run made with lanes = 1. Other values: SPH_ERR_ARG. */
 SPH_API int32_t sph_set_group_lanes(int32_t lanes);
-/* Density kernel form of FP32 states that run one thread per particle (no
-   counterpart in the reference), process-wide: 0 walks each particle's
-   neighbour row masks one candidate at a time; 1 (single states) uses the
-   cell-tile form, where a warp stages the neighbouring cell rows of its 32
-   consecutive particles in shared memory once and every lane scans all staged
-   candidates; 2 (default) walks the masks taking two candidates per
-   iteration, their kernel arithmetic in packed f32x2 instructions (7% faster
-   than 0 on 1M particles; 1 is 3.4x slower). Every form adds the same
-   terms in the same order; they may differ in the last bits of FP32 through
-   multiply-add contraction. Other values: SPH_ERR_ARG. */
+/* Kernel form of FP32 states that run one thread per particle (no counterpart
+   in the reference), process-wide; a step reads it once. 2 (default): tiles of
+   128 particles, whose pair passes read neighbour lists (scratch, about 195
+   bytes a particle) and windows staged in shared memory; states that expect
+   more than 49 neighbours a particle, or whose lists are not free, walk the
+   masks with two candidates per iteration of the density sum in packed f32x2
+   instructions. 0: every pass walks each particle's neighbour row masks, the
+   density one candidate at a time (the bits of 2). 1 (single states): mask
+   walks with the cell-tile density, where a warp stages the neighbouring cell
+   rows of its 32 consecutive particles in shared memory once and every lane
+   scans all staged candidates (its density pass takes 3.4 times that of 0);
+   its sums may differ in the last bits through multiply-add contraction. Other
+   values: SPH_ERR_ARG. */
 SPH_API int32_t sph_set_density_form(int32_t form);
 /* Programmatic dependent launch (no counterpart in the reference),
    process-wide: 1 (default) launches the engine's kernels so that each may be
@@ -399,8 +408,8 @@ SPH_API int32_t sph_set_density_form(int32_t form);
    sequences use plain launches. */
 SPH_API int32_t sph_set_launch_overlap(int32_t on);
 /* Steps per recorded group (no counterpart in the reference), process-wide:
-   simulate and backward record the launches of `steps` consecutive steps
-   (forward, recomputed and reverse steps alike, with the snapshot copies
+   simulate and backward record the launches of up to `steps` consecutive steps,
+   a call's first groups shorter (forward, recomputed and reverse steps alike, with the snapshot copies
    between them) and replay each group as one CUDA graph, which shortens the
    gaps between the short kernels of small states. It applies to FP64 states
    and to FP32 states of up to 2^18 particles (larger FP32 states run faster
@@ -430,7 +439,8 @@ SPH_API int32_t sph_get_group_lanes(int32_t *lanes);
    (host seeds) fail while capturing: run the sequence once, then capture it.
    A graph replays only the device work; the handles' host bookkeeping
    (neighbour-list age, tape length, snapshot slots) stays as the capture left
-   it, so capture a sequence that starts from a reset -- for instance one whole
+   it (the scratch lists of FP32 states are made again where a recording, or a
+   step after it, needs them), so capture a sequence that starts from a reset -- for instance one whole
    solve: sph_state_assign from a pristine state, sph_tape_reset, sph_simulate,
    sph_objective, sph_backward_seeded -- and replay it as a unit. */
 typedef struct sph_graph_s *sph_graph;

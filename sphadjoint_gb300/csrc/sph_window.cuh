@@ -32,9 +32,9 @@
 // Bound: shared-memory wavefronts and issue slots together (accel at 1M: 71% of
 // the wavefront rate, 57% of the issue slots, 913 warp instructions a warp where
 // the mask walk ran 1449). Measured per launch at 1,048,576 particles, mask walk
-// -> lists: density 58.1 -> 45.2 us, accel 59.2 -> 46.6, accel + drag 70.8 -> 49.0,
-// pass 1 82.7 -> 60.5, pass 2 64.1 -> 46.8; a rebuild's masks and lists 52 -> 71 us
-// (k_nl_window), 108 with the step's density (k_nl_density_win).
+// -> lists: density 58.1 -> 45.5 us, accel 59.2 -> 47.8, accel + drag 70.8 -> 49.8,
+// pass 1 82.7 -> 61.5, pass 2 64.1 -> 48.3; a rebuild's masks and lists 52 -> 72 us
+// (k_nl_window), 111 with the step's density (k_nl_density_win).
 // Reading the lists two quads ahead (accel 46 -> 49 us), copying a tile's lists
 // to shared memory first (density 45 -> 51) and 16-byte interleaved windows
 // (below) were slower.
@@ -422,7 +422,7 @@ __device__ __forceinline__ void density_list(const NLView<float> &v, const WinLi
 // _nl_build! (nl_build_one), the tile's window and the candidate lists of a fresh
 // cell list: the rows are scanned in the staged window, and every passing slot
 // goes both to its row mask and to the list. One pass instead of a mask build
-// (52 us at 1M particles) and a walk of the masks (43 us): 66.5 us, bound by issue
+// (52 us at 1M particles) and a walk of the masks (43 us): 72 us, bound by issue
 // slots and shared-memory wavefronts (some 80% of either's rate); 8.4M dense
 // particles 775 -> 647 us.
 // DENS: the density pass of the same particles follows in the staged window, from
@@ -599,8 +599,8 @@ __global__ void __launch_bounds__(kTile)
 
 // The same and the density pass of the step in one launch, which saves the launch, the
 // second staging of the window and the read of the lists: 20,000 particles' 16 steps
-// 271 -> 262 us, 249,001 particles 41.3 -> 34.0 us a rebuild, 1M 116 -> 108, 8.4M 1030
-// -> 995.
+// 271 -> 267 us, 249,001 particles 41.3 -> 35.9 us a rebuild, 1M 116 -> 111, 8.4M 1030
+// -> 1014.
 template <bool MULTI>
 __global__ void __launch_bounds__(kTile)
     k_nl_density_win(const __grid_constant__ NLView<float> v, const NlOut<float> out,
