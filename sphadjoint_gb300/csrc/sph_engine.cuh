@@ -672,6 +672,9 @@ template <typename T> class Sys final : public StateI {
         } catch (const Error &) {
             return;
         }
+        // freed as the state's other buffers are, on the stream that it was created on: the
+        // one of this call may be gone by then
+        scratch.s = core.s;
         uint8_t *at = scratch.p;
         size_t k = 0;
         const auto place = [&](auto &b) {
